@@ -244,7 +244,7 @@ int launch_mma(const void* x, PlaneView xv, long x_rows_stored, const void* w, i
 }  // namespace
 
 bool conv2d_mma_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int W, int R, int S, int dtype) {
-    return dtype != MTA_F32 && S <= 17 && R <= 64 && W % 8 == 0 && xv.width == W && yv.width == W &&
+    return dtype != MTA_F32 && S <= 17 && R <= 64 && xv.width % 8 == 0 && yv.width % 8 == 0 &&
            xv.plane_stride % 8 == 0 && yv.plane_stride % 8 == 0 && aligned16(x) && aligned16(y);
 }
 

@@ -495,7 +495,7 @@ int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, 
 
 bool conv2d_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int W, int R, int S, int dtype,
                            int w_dtype) {
-    return dtype != MTA_F32 && S <= 17 && R <= 16 && conv2d_tc05_smem_bytes(R, w_dtype == MTA_F32) <= 227 * 1024 && W % 8 == 0 && xv.width == W && yv.width == W &&
+    return dtype != MTA_F32 && S <= 17 && R <= 16 && conv2d_tc05_smem_bytes(R, w_dtype == MTA_F32) <= 227 * 1024 && xv.width % 8 == 0 && yv.width % 8 == 0 &&
            xv.plane_stride % 8 == 0 && yv.plane_stride % 8 == 0 && aligned16(x) && aligned16(y);
 }
 

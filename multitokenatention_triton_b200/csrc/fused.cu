@@ -15,20 +15,33 @@ namespace {
 
 struct Plan {
     int ra, rb, r0, r1;      // first score row, first softmax row, first and one-past-last output row
+    int pitch;               // elements between rows of a scratch plane
     size_t buf_bytes;        // one scratch buffer
     size_t total() const { return 2 * buf_bytes; }
 };
 
 size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-Plan make_plan(int B, int H, int S, int cq, int cq2, int r0, int r1, int dtype) {
+// Rows of a 16-bit scratch plane start on 128-byte boundaries whatever S is: TMA and the vector accesses of the tensor-core
+// kernels need 16, and a box of 64 columns then touches one line per row instead of two.  Nothing in the padding is ever read
+// as a score (the tensor maps end at column S).
+int padded_pitch(int S, int dtype) { return dtype == MTA_F32 ? S : (int)round_up((size_t)S, 64); }
+
+Plan make_plan(int B, int H, int S, int cq, int cq2, int r0, int r1, int dtype, int pitch) {
     Plan p;
     p.r0 = r0;
     p.r1 = r1;
     p.rb = r0 - (cq2 - 1) > 0 ? r0 - (cq2 - 1) : 0;
     p.ra = p.rb - (cq - 1) > 0 ? p.rb - (cq - 1) : 0;
-    p.buf_bytes = round_up((size_t)B * H * (size_t)(r1 - p.ra) * S * dtype_size(dtype), 256);
+    p.pitch = pitch;
+    p.buf_bytes = round_up((size_t)B * H * (size_t)(r1 - p.ra) * p.pitch * dtype_size(dtype), 256);
     return p;
+}
+
+// The plan with padded rows, or with rows of S elements when the caller's workspace only holds that.
+Plan fit_plan(int B, int H, int S, int cq, int cq2, int r0, int r1, int dtype, size_t workspace_bytes) {
+    const Plan padded = make_plan(B, H, S, cq, cq2, r0, r1, dtype, padded_pitch(S, dtype));
+    return padded.total() <= workspace_bytes ? padded : make_plan(B, H, S, cq, cq2, r0, r1, dtype, S);
 }
 
 // Stage tracing of mta_fused_fwd: when switched on, the forward records a CUDA event on its stream before every stage
@@ -84,7 +97,7 @@ size_t mta_workspace_bytes(int B, int H, int S, int D, int cq, int ck, int cq2, 
     if (B <= 0 || H <= 0 || S <= 0 || cq < 1 || cq2 < 1 || q_row_begin < 0 || q_row_end > S ||
         q_row_end <= q_row_begin || !dtype_ok(dtype))
         return 0;
-    return make_plan(B, H, S, cq, cq2, q_row_begin, q_row_end, dtype).total();
+    return make_plan(B, H, S, cq, cq2, q_row_begin, q_row_end, dtype, padded_pitch(S, dtype)).total();
 }
 
 int mta_fused_fwd(const void* q, const void* k, const void* v, const void* w1, const void* W1, const void* w2,
@@ -113,7 +126,7 @@ int mta_fused_fwd_dropout(const void* q, const void* k, const void* v, const voi
     if ((long)B * S == 0 || q_row_begin == q_row_end) return MTA_OK;
     MTA_REQUIRE(q && k && v && w1 && W1 && w2 && W2 && o, "fused_fwd: null pointer");
     MTA_REQUIRE((long)B * H <= 65535, "fused_fwd: B*H = %ld exceeds 65535", (long)B * H);
-    const Plan pl = make_plan(B, H, S, cq, cq2, q_row_begin, q_row_end, dtype);
+    const Plan pl = fit_plan(B, H, S, cq, cq2, q_row_begin, q_row_end, dtype, workspace_bytes);
     MTA_REQUIRE(workspace && workspace_bytes >= pl.total(), "fused_fwd: workspace of %zu bytes is smaller than the %zu needed",
                 workspace_bytes, pl.total());
     MTA_REQUIRE(aligned16(workspace), "fused_fwd: workspace must be 16-byte aligned");
@@ -122,7 +135,7 @@ int mta_fused_fwd_dropout(const void* q, const void* k, const void* v, const voi
     char* ws = static_cast<char*>(workspace);
     void* bufA = ws;
     void* bufB = ws + pl.buf_bytes;
-    const PlaneView pv{(long)(pl.r1 - pl.ra) * S, pl.ra, S};
+    const PlaneView pv{(long)(pl.r1 - pl.ra) * pl.pitch, pl.ra, pl.pitch};
     const long planes = (long)B * H;
     const float scale = 1.0f / sqrtf((float)D);
     const int round16 = dtype != MTA_F32;
@@ -171,8 +184,17 @@ static bool conv_attn_one_kernel(int S, int D, int cq, int ck, int causal, int d
 size_t mta_conv_attn_workspace_bytes(int B, int H, int S, int D, int cq, int ck, int causal, int dtype, int w_dtype) {
     if (B <= 0 || H <= 0 || S <= 0 || cq < 1 || !dtype_ok(dtype) || !dtype_ok(w_dtype)) return 0;
     if (conv_attn_one_kernel(S, D, cq, ck, causal, dtype, w_dtype)) return 0;
-    return 2 * make_plan(B, H, S, cq, 1, 0, S, dtype).buf_bytes;      // this path uses the two score planes only
+    return make_plan(B, H, S, cq, 1, 0, S, dtype, padded_pitch(S, dtype)).total();
 }
+
+}  // extern "C"
+
+// What mta_conv_attn_fwd can do with at the least: rows without padding.
+size_t mta::conv_attn_least_workspace(int B, int H, int S, int D, int cq, int ck, int causal, int dtype, int w_dtype) {
+    return mta_conv_attn_workspace_bytes(B, H, S, D, cq, ck, causal, dtype, w_dtype) == 0 ? 0 : make_plan(B, H, S, cq, 1, 0, S, dtype, S).total();
+}
+
+extern "C" {
 
 int mta_conv_attn_fwd(const void* q, const void* k, const void* v, const void* w, void* o, void* workspace,
                       size_t workspace_bytes, int B, int H, int S, int D, int cq, int ck, int causal, float scale,
@@ -192,13 +214,13 @@ int mta_conv_attn_fwd(const void* q, const void* k, const void* v, const void* w
         // raw scores into the conv (score scale 1), the softmax scale after it, as the reference orders them
         return conv_attn_fused_launch(q, k, v, w, w_dtype, o, B, H, S, D, cq, ck, 1.0f, scale, 0, S, dtype, st);
     }
-    const Plan pl = make_plan(B, H, S, cq, 1, 0, S, dtype);
-    MTA_REQUIRE(workspace && workspace_bytes >= 2 * pl.buf_bytes, "conv_attn_fwd: workspace of %zu bytes is smaller than the %zu needed",
-                workspace_bytes, 2 * pl.buf_bytes);
+    const Plan pl = fit_plan(B, H, S, cq, 1, 0, S, dtype, workspace_bytes);
+    MTA_REQUIRE(workspace && workspace_bytes >= pl.total(), "conv_attn_fwd: workspace of %zu bytes is smaller than the %zu needed",
+                workspace_bytes, pl.total());
     MTA_REQUIRE(aligned16(workspace), "conv_attn_fwd: workspace must be 16-byte aligned");
     void* bufA = workspace;
     void* bufB = static_cast<char*>(workspace) + pl.buf_bytes;
-    const PlaneView pv{(long)S * S, 0, S};
+    const PlaneView pv{(long)S * pl.pitch, 0, pl.pitch};
     const long planes = (long)B * H;
     int rc;
     // 16-bit dtypes: the raw scores are computed inside the conv's kernel (scale 1: the conv attention scales after its conv)

@@ -345,7 +345,7 @@ int launch_pv(const void* p, PlaneView pview, const void* v, void* o, int B, int
               int row_end, long p_rows_stored, cudaStream_t st, DropoutSpec drop) {
     CUtensorMap mp, mv;
     int rc;
-    if ((rc = make_tensor_map_3d(&mp, p, (uint64_t)B * H, (uint64_t)p_rows_stored, S, S, (uint64_t)pview.plane_stride, 64, TILE, true))) return rc;
+    if ((rc = make_tensor_map_3d(&mp, p, (uint64_t)B * H, (uint64_t)p_rows_stored, S, (uint64_t)pview.width, (uint64_t)pview.plane_stride, 64, TILE, true))) return rc;
     if ((rc = make_tensor_map_3d(&mv, v, (uint64_t)B * H, S, D, D, (uint64_t)S * D, 64, PV_KEYS, true))) return rc;
     int* flag = nullptr;
     if ((rc = wait_flag_ptr(&flag))) return rc;
@@ -368,7 +368,7 @@ int launch_pv(const void* p, PlaneView pview, const void* v, void* o, int B, int
 }  // namespace
 
 bool tc05_contractions_supported(int S, int D, int dtype, const void* a, const void* b, const void* c, PlaneView view) {
-    return dtype != MTA_F32 && (D == 64 || D == 128) && S % 8 == 0 && view.width == S && view.plane_stride % 8 == 0 &&
+    return dtype != MTA_F32 && (D == 64 || D == 128) && view.width >= S && view.width % 8 == 0 && view.plane_stride % 8 == 0 &&
            aligned16(a) && aligned16(b) && aligned16(c);
 }
 

@@ -664,7 +664,7 @@ head_mix_softmax_kernel(const T* __restrict__ x, PlaneView xv, const void* __res
         if (cur_whole) load_pair(blk + 2 * WARPS, raw);
     }
     if (write_upper) {                                     // probabilities above the diagonal are exactly 0
-        const int v0 = (n_keys + 7) >> 3, nv = Q >> 3;
+        const int v0 = (n_keys + 7) >> 3, nv = (Q + 7) >> 3;
         for (int o = 0; o < C; ++o) {
             uint4* row = reinterpret_cast<uint4*>(y + yv.at(n * C + o, p, 0));
             for (int i = v0 + (int)threadIdx.x; i < nv; i += WARPS * 32) row[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -762,7 +762,7 @@ bool vector_ok(const void* p, PlaneView v) {
 
 namespace {
 bool mix_softmax_mma_ok(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int causal, int dtype) {
-    return causal && dtype != MTA_F32 && C <= 32 && Q % 8 == 0 && x != y && vector_ok(x, xv) && vector_ok(y, yv);
+    return causal && dtype != MTA_F32 && C <= 32 && x != y && vector_ok(x, xv) && vector_ok(y, yv);
 }
 }  // namespace
 
@@ -809,7 +809,7 @@ int head_linear_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype,
     MTA_REQUIRE(N <= 65535 && row_end - row_begin <= 65535, "head_linear: N or the row count exceeds 65535");
     // variant "head_linear": 0 auto, 1 CUDA cores, 2 mma.sync, 3 tcgen05
     const int want = variant("head_linear");
-    const bool mma_able = dtype != MTA_F32 && C <= 32 && Q % 8 == 0 && vector_ok(x, xv) && vector_ok(y, yv);
+    const bool mma_able = dtype != MTA_F32 && C <= 32 && vector_ok(x, xv) && vector_ok(y, yv);
     const bool tc05_able = head_linear_tc05_supported(x, xv, y, yv, C, Q, dtype, w_dtype);
     MTA_REQUIRE(want != 2 || mma_able, "head_linear: the mma.sync variant needs a 16-bit dtype, C <= 32, Q %% 8 == 0 and 16-byte aligned rows");
     MTA_REQUIRE(want != 3 || tc05_able,

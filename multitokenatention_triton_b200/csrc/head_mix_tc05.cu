@@ -533,7 +533,7 @@ int launch_hm(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv
 
 bool hm_tc05_ok(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int dtype, int w_dtype) {
     const bool pow2 = C >= 8 && C <= 128 && (C & (C - 1)) == 0;
-    return dtype != MTA_F32 && w_dtype == dtype && pow2 && Q % 8 == 0 && x != y && aligned16(x) && aligned16(y) &&
+    return dtype != MTA_F32 && w_dtype == dtype && pow2 && x != y && aligned16(x) && aligned16(y) &&
            xv.width % 8 == 0 && xv.plane_stride % 8 == 0 && yv.width % 8 == 0 && yv.plane_stride % 8 == 0;
 }
 

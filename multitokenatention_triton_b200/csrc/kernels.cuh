@@ -110,6 +110,8 @@ bool conv_attn_fused_supported(const void* q, const void* k, const void* v, cons
                                int dtype, int w_dtype);
 int conv_attn_fused_launch(const void* q, const void* k, const void* v, const void* w, int w_dtype, void* o, int B, int H, int S, int D,
                            int R, int KS, float score_scale, float sm_scale, int row_begin, int row_end, int dtype, cudaStream_t st);
+// Scratch that mta_conv_attn_fwd needs at the least (0: none); with mta_conv_attn_workspace_bytes(...) its rows are padded.
+size_t conv_attn_least_workspace(int B, int H, int S, int D, int cq, int ck, int causal, int dtype, int w_dtype);
 // Reads and clears the flag raised by a device-side bounded wait that gave up (synchronises `st`).
 int device_wait_status(cudaStream_t st, int* timed_out);
 // True when such a wait has given up on the current device since the last device_wait_status; reads the flag's mirror in

@@ -64,10 +64,11 @@ int mta_conv_attn_fwd_static(const void* q, const void* k, const void* v, const 
                 "conv_attn_fwd_static: bad shape or dtype (B=%d H=%d S=%d D=%d cq=%d ck=%d dtype=%d)", B, H, S, D, cq, ck, dtype);
     if ((long)B * S == 0) return MTA_OK;
     const size_t need = mta_conv_attn_workspace_bytes(B, H, S, D, cq, ck, causal, dtype, w_dtype);
-    MTA_REQUIRE(need <= kStaticScratchBytes,
+    const size_t least = mta::conv_attn_least_workspace(B, H, S, D, cq, ck, causal, dtype, w_dtype);
+    MTA_REQUIRE(least <= kStaticScratchBytes,
                 "conv_attn_fwd_static: B=%d H=%d S=%d needs %zu bytes of scratch, the built-in array holds %zu; "
                 "use mta_conv_attn_fwd with a caller workspace for larger problems",
-                B, H, S, need, kStaticScratchBytes);
+                B, H, S, least, kStaticScratchBytes);
     // the array belongs to the current device: a stream of another device would run the kernels there with this address
     int dev = 0, stream_dev = 0;
     MTA_CUDA_OK(cudaGetDevice(&dev));
@@ -75,7 +76,7 @@ int mta_conv_attn_fwd_static(const void* q, const void* k, const void* v, const 
     MTA_REQUIRE(stream_dev == dev, "conv_attn_fwd_static: the stream belongs to device %d but device %d is current", stream_dev, dev);
     unsigned char* scratch = nullptr;
     if (int rc = static_scratch_ptr(&scratch)) return rc;
-    return mta_conv_attn_fwd(q, k, v, w, o, scratch, need, B, H, S, D, cq, ck, causal, scale, dtype, w_dtype, stream);
+    return mta_conv_attn_fwd(q, k, v, w, o, scratch, need < kStaticScratchBytes ? need : kStaticScratchBytes, B, H, S, D, cq, ck, causal, scale, dtype, w_dtype, stream);
 }
 
 }  // extern "C"

@@ -356,8 +356,8 @@ int launch_qc(const void* q, const void* k, const void* w, int w_dtype, void* y,
 
 bool qk_conv_supported(const void* q, const void* k, const void* y, PlaneView yv, int S, int D, int R, int KS, int causal, int dtype,
                        int w_dtype) {
-    return causal && dtype != MTA_F32 && (D == 64 || D == 128) && S % 8 == 0 && KS % 2 == 1 && KS <= 17 && R >= 1 && R <= 16 &&
-           qk_conv_smem_bytes(D, R, w_dtype == MTA_F32) <= 225 * 1024 && yv.width == S && yv.plane_stride % 8 == 0 && aligned16(q) &&
+    return causal && dtype != MTA_F32 && (D == 64 || D == 128) && KS % 2 == 1 && KS <= 17 && R >= 1 && R <= 16 &&
+           qk_conv_smem_bytes(D, R, w_dtype == MTA_F32) <= 225 * 1024 && yv.width >= S && yv.width % 8 == 0 && yv.plane_stride % 8 == 0 && aligned16(q) &&
            aligned16(k) && aligned16(y);
 }
 

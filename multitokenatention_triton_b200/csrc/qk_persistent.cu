@@ -253,7 +253,7 @@ int launch(const void* a, const void* b, void* c, PlaneView cv, int BH, QkGeom g
     int rc;
     if ((rc = make_tensor_map_3d(&ma, a, (uint64_t)BH, g.S, D, D, (uint64_t)g.S * D, 64, TILE, true))) return rc;
     if ((rc = make_tensor_map_3d(&mb, b, (uint64_t)BH * g.NI, g.S, D, D, (uint64_t)g.S * D, 64, TILE, true))) return rc;
-    if ((rc = make_tensor_map_3d(&mc, c, (uint64_t)BH, (uint64_t)(g.row_end - cv.row0), g.S, g.S, (uint64_t)cv.plane_stride, 64, TILE, true)))
+    if ((rc = make_tensor_map_3d(&mc, c, (uint64_t)BH, (uint64_t)(g.row_end - cv.row0), g.S, (uint64_t)cv.width, (uint64_t)cv.plane_stride, 64, TILE, true)))
         return rc;
     int* flag = nullptr;
     if ((rc = wait_flag_ptr(&flag))) return rc;

@@ -184,7 +184,7 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
         }
     }
     if (write_upper)
-        for (int ch = nch + tid; ch < (Q >> 3); ch += VT) yr[ch] = make_uint4(0u, 0u, 0u, 0u);
+        for (int ch = nch + tid; ch < ((Q + 7) >> 3); ch += VT) yr[ch] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <typename T, int NCH>
@@ -200,7 +200,7 @@ int launch_vec(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, 
 template <typename T>
 int launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int Q, int causal, int row_begin,
            int row_end, bool write_upper, float pre_scale, int round_prescaled, cudaStream_t st) {
-    if constexpr (sizeof(T) == 2) if (Q % 8 == 0 && Q <= 16 * 8 * VT && xv.plane_stride % 8 == 0 && yv.plane_stride % 8 == 0 &&
+    if constexpr (sizeof(T) == 2) if (Q <= 16 * 8 * VT && xv.plane_stride % 8 == 0 && yv.plane_stride % 8 == 0 &&
         xv.width % 8 == 0 && yv.width % 8 == 0 && aligned16(x) && aligned16(y)) {
         const int longest = causal ? (row_end < Q ? row_end : Q) : Q;
         const int need = (longest + 8 * VT - 1) / (8 * VT);
