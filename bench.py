@@ -261,7 +261,8 @@ def reference_arm(args, wl: MTAWorkload, rank: int, world: int):
             if i >= args.warmup:
                 vals.append(v)
                 secs.append(t)
-        value, sec, kind = statistics.mean(vals), statistics.mean(secs), "port"
+        sec, kind = statistics.mean(secs), "port"
+        value = statistics.mean(v * t for v, t in zip(vals, secs)) / sec
         scaled = {"batch": "each step is a block of query rows of batch element 0 centred on S/2 (mean cost per token)", "seq": None}
     line = {
         "impl": "reference", "metric": METRIC, "value": value, "unit": "tokens/s", "n_gpus": args.gpus,
