@@ -145,8 +145,8 @@ int mta_conv2d_bwd_input(const void* dy, const void* w, void* dx, int N, int C, 
     MTA_REQUIRE(dy && w && dx, "conv2d_bwd_input: null pointer");
     MTA_REQUIRE(dy != dx, "conv2d_bwd_input: in-place operation is not supported");
     if (int rc = check_device()) return rc;
-    return conv2d_bwd_input_launch(dy, w, w_dtype, dx, (long)N * C, C, H, W, R, S, causal ? 1 : 0, dtype,
-                                   static_cast<cudaStream_t>(stream));
+    return conv2d_bwd_input_launch(dy, full_view(H, W), w, w_dtype, dx, full_view(H, W), (long)N * C, C, H, W, R, S, causal ? 1 : 0, true,
+                                   dtype, static_cast<cudaStream_t>(stream));
 }
 
 size_t mta_conv2d_bwd_weight_workspace_bytes(int N, int C, int H, int W, int R, int S) {
@@ -171,7 +171,7 @@ int mta_conv2d_bwd_weight(const void* x, const void* dy, float* dw, void* worksp
     const size_t need = conv2d_bwd_weight_workspace(N, C, H, W, R, S);
     MTA_REQUIRE(workspace && workspace_bytes >= need, "conv2d_bwd_weight: workspace of %zu bytes is smaller than the %zu needed",
                 workspace_bytes, need);
-    return conv2d_bwd_weight_launch(x, dy, dw, workspace, N, C, H, W, R, S, causal ? 1 : 0, dtype, st);
+    return conv2d_bwd_weight_launch(x, full_view(H, W), dy, full_view(H, W), dw, workspace, N, C, H, W, R, S, causal ? 1 : 0, dtype, st);
 }
 
 int mta_head_linear_bwd_input(const void* dy, const void* Wm, void* dx, int N, int C, int P, int Q, int causal, int dtype,
@@ -209,7 +209,7 @@ int mta_head_linear_bwd_weight(const void* x, const void* dy, float* dW, void* w
     const size_t need = head_linear_bwd_weight_workspace(C);
     MTA_REQUIRE(workspace && workspace_bytes >= need, "head_linear_bwd_weight: workspace of %zu bytes is smaller than the %zu needed",
                 workspace_bytes, need);
-    return head_linear_bwd_weight_launch(x, dy, dW, workspace, N, C, P, Q, causal ? 1 : 0, dtype, st);
+    return head_linear_bwd_weight_launch(x, full_view(P, Q), dy, full_view(P, Q), dW, workspace, N, C, P, Q, causal ? 1 : 0, dtype, st);
 }
 
 int mta_qk_scores_fwd(const void* q, const void* k, void* s, int B, int H, int S, int D, float scale, int round_scale,

@@ -29,8 +29,8 @@ constexpr int WT_THREADS = WT_M * (WT_N / WT_CPT) / 2;     // 256: a thread owns
 // indexes it statically), 0 = any size (the window is re-read from shared memory per tap).
 template <typename T, int SC>
 __global__ void __launch_bounds__(WT_THREADS)
-conv2d_bwd_weight_kernel(const T* __restrict__ x, const T* __restrict__ dy, float* __restrict__ partial, int H, int W,
-                         int R, int S, int causal, int tiles_n) {
+conv2d_bwd_weight_kernel(const T* __restrict__ x, PlaneView xv, const T* __restrict__ dy, PlaneView dyv, float* __restrict__ partial,
+                         int H, int W, int R, int S, int causal, int tiles_n) {
     extern __shared__ __align__(16) float smem[];
     const int pad_h = R - 1, pad_w = (S - 1) / 2;
     const int tw = (WT_N + S - 1 + 3) & ~3, th = WT_M + R - 1;      // row pitch a multiple of 4 floats: 16-byte window loads
@@ -46,13 +46,13 @@ conv2d_bwd_weight_kernel(const T* __restrict__ x, const T* __restrict__ dy, floa
         for (int i = tid; i < taps; i += WT_THREADS) out[i] = 0.0f;
         return;
     }
-    const T* xp = x + plane * (long)H * W;
-    const T* dp = dy + plane * (long)H * W;
+    const T* xp = x + plane * xv.plane_stride;
+    const T* dp = dy + plane * dyv.plane_stride;
     for (int idx = tid; idx < th * tw; idx += WT_THREADS) {
         const int rr = idx / tw, cc = idx - rr * tw;
         const int qq = m0 - pad_h + rr, kk = n0 - pad_w + cc;
         float v = 0.0f;
-        if (qq >= 0 && qq < H && kk >= 0 && kk < W && (!causal || kk <= qq)) v = to_f32<T>(xp[(long)qq * W + kk]);
+        if (qq >= 0 && qq < H && kk >= 0 && kk < W && (!causal || kk <= qq)) v = to_f32<T>(xp[(long)qq * xv.width + kk]);
         xs[idx] = v;
     }
     // this thread's output positions: rows (ry, ry + WT_M/2), columns [cx, cx + 8)
@@ -61,8 +61,8 @@ conv2d_bwd_weight_kernel(const T* __restrict__ x, const T* __restrict__ dy, floa
 #pragma unroll
     for (int e = 0; e < WT_CPT; ++e) {
         const int k = n0 + cx + e, q0 = m0 + ry, q1 = m0 + ry + WT_M / 2;
-        g0[e] = (q0 < H && k < W && (!causal || k <= q0)) ? to_f32<T>(dp[(long)q0 * W + k]) : 0.0f;
-        g1[e] = (q1 < H && k < W && (!causal || k <= q1)) ? to_f32<T>(dp[(long)q1 * W + k]) : 0.0f;
+        g0[e] = (q0 < H && k < W && (!causal || k <= q0)) ? to_f32<T>(dp[(long)q0 * dyv.width + k]) : 0.0f;
+        g1[e] = (q1 < H && k < W && (!causal || k <= q1)) ? to_f32<T>(dp[(long)q1 * dyv.width + k]) : 0.0f;
     }
     __syncthreads();
     for (int i = 0; i < R; ++i) {
@@ -130,8 +130,8 @@ constexpr int HW_THREADS = 256;
 // PPT = (o,h) pairs per thread; KT = keys per tile.  Persistent CTAs walk the (n, row, key block) tiles.
 template <typename T, int PPT, int KT>
 __global__ void __launch_bounds__(HW_THREADS)
-head_linear_bwd_weight_kernel(const T* __restrict__ x, const T* __restrict__ dy, float* __restrict__ partial, int N, int C,
-                              int P, int Q, int causal) {
+head_linear_bwd_weight_kernel(const T* __restrict__ x, PlaneView xv, const T* __restrict__ dy, PlaneView dyv,
+                              float* __restrict__ partial, int N, int C, int P, int Q, int causal) {
     extern __shared__ __align__(16) float smem[];
     float* xs = smem;                   // C x KT
     float* gs = smem + (size_t)C * KT;  // C x KT
@@ -152,9 +152,8 @@ head_linear_bwd_weight_kernel(const T* __restrict__ x, const T* __restrict__ dy,
         for (int idx = tid; idx < C * KT; idx += HW_THREADS) {
             const int h = idx / KT, kk = idx - h * KT, k = k0 + kk;
             const bool ok = k < Q && (!causal || k <= p);
-            const long off = ((n * C + h) * P + p) * (long)Q + k;
-            xs[idx] = ok ? to_f32<T>(x[off]) : 0.0f;
-            gs[idx] = ok ? to_f32<T>(dy[off]) : 0.0f;
+            xs[idx] = ok ? to_f32<T>(x[xv.at(n * C + h, p, k)]) : 0.0f;
+            gs[idx] = ok ? to_f32<T>(dy[dyv.at(n * C + h, p, k)]) : 0.0f;
         }
         __syncthreads();
 #pragma unroll
@@ -207,8 +206,8 @@ constexpr int HM_KEYS = 128;       // keys per item
 
 template <typename T, int MT>
 __global__ void __launch_bounds__(HM_WARPS * 32)
-head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, const T* __restrict__ dy, float* __restrict__ partial, int N, int C,
-                                  int P, int Q, int causal) {
+head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, PlaneView xview, const T* __restrict__ dy, PlaneView dyview,
+                                  float* __restrict__ partial, int N, int C, int P, int Q, int causal) {
     constexpr int CP = 16 * MT, NV = 2 * MT;            // padded heads; 16-byte vectors per lane, side and 32-key group
     __shared__ float red[HM_WARPS][CP * CP];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -220,7 +219,6 @@ head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, const T* __restrict__
         for (int b = 0; b < 2 * MT; ++b) acc[a][b][0] = acc[a][b][1] = acc[a][b][2] = acc[a][b][3] = 0.0f;
     const int kblocks = (Q + HM_KEYS - 1) / HM_KEYS;
     const long items = (long)N * P * kblocks;
-    const long plane = (long)P * Q;
     for (long item = (long)blockIdx.x * HM_WARPS + warp; item < items; item += (long)gridDim.x * HM_WARPS) {
         const int kb = (int)(item % kblocks);
         const int p = (int)((item / kblocks) % P);
@@ -228,7 +226,6 @@ head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, const T* __restrict__
         const int k0 = kb * HM_KEYS;
         if (causal && k0 > p) continue;
         const int n_keys = causal ? min(p + 1, Q) : Q;   // keys of this row that carry a gradient
-        const long row_off = n * C * plane + (long)p * Q;
         uint4 gv[4][NV], xv[4][NV];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -237,8 +234,8 @@ head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, const T* __restrict__
             for (int r = 0; r < NV; ++r) {
                 const int head = g + 8 * r;
                 if (head < C && kq < n_keys) {
-                    gv[j][r] = __ldg(reinterpret_cast<const uint4*>(dy + row_off + head * plane + kq));
-                    xv[j][r] = __ldg(reinterpret_cast<const uint4*>(x + row_off + head * plane + kq));
+                    gv[j][r] = __ldg(reinterpret_cast<const uint4*>(dy + dyview.at(n * C + head, p, kq)));
+                    xv[j][r] = __ldg(reinterpret_cast<const uint4*>(x + xview.at(n * C + head, p, kq)));
                 } else {
                     gv[j][r] = make_uint4(0u, 0u, 0u, 0u);
                     xv[j][r] = make_uint4(0u, 0u, 0u, 0u);
@@ -298,22 +295,22 @@ __global__ void head_linear_bwd_weight_reduce_kernel(const float* __restrict__ p
 int hw_grid(int sms) { return sms * 4; }
 
 template <typename T, int PPT, int KT>
-int launch_hw(const void* x, const void* dy, float* partial, int N, int C, int P, int Q, int causal, int grid, cudaStream_t st) {
+int launch_hw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, int N, int C, int P, int Q, int causal, int grid, cudaStream_t st) {
     const size_t smem = 2 * (size_t)C * KT * sizeof(float);
     if (smem > 48 * 1024)
         MTA_CUDA_OK(cudaFuncSetAttribute(head_linear_bwd_weight_kernel<T, PPT, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    head_linear_bwd_weight_kernel<T, PPT, KT><<<grid, HW_THREADS, smem, st>>>(static_cast<const T*>(x), static_cast<const T*>(dy),
+    head_linear_bwd_weight_kernel<T, PPT, KT><<<grid, HW_THREADS, smem, st>>>(static_cast<const T*>(x), xv, static_cast<const T*>(dy), dyv,
                                                                               partial, N, C, P, Q, causal);
     MTA_LAUNCH_OK("head_linear_bwd_weight_kernel");
     return MTA_OK;
 }
 
 template <typename T>
-int dispatch_hw(const void* x, const void* dy, float* partial, int N, int C, int P, int Q, int causal, int grid, cudaStream_t st) {
-    if (C <= 16) return launch_hw<T, 1, 256>(x, dy, partial, N, C, P, Q, causal, grid, st);
-    if (C <= 32) return launch_hw<T, 4, 256>(x, dy, partial, N, C, P, Q, causal, grid, st);
-    if (C <= 64) return launch_hw<T, 16, 128>(x, dy, partial, N, C, P, Q, causal, grid, st);
-    return launch_hw<T, 64, 64>(x, dy, partial, N, C, P, Q, causal, grid, st);
+int dispatch_hw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, int N, int C, int P, int Q, int causal, int grid, cudaStream_t st) {
+    if (C <= 16) return launch_hw<T, 1, 256>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
+    if (C <= 32) return launch_hw<T, 4, 256>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
+    if (C <= 64) return launch_hw<T, 16, 128>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
+    return launch_hw<T, 64, 64>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
 }
 
 }  // namespace
@@ -323,8 +320,8 @@ size_t conv2d_bwd_weight_workspace(int N, int C, int H, int W, int R, int S) {
     return (size_t)N * C * tiles * R * S * sizeof(float);
 }
 
-int conv2d_bwd_weight_launch(const void* x, const void* dy, float* dw, void* workspace, int N, int C, int H, int W, int R,
-                             int S, int causal, int dtype, cudaStream_t st) {
+int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dw, void* workspace, int N, int C, int H,
+                             int W, int R, int S, int causal, int dtype, cudaStream_t st) {
     const int tiles_m = (H + WT_M - 1) / WT_M, tiles_n = (W + WT_N - 1) / WT_N;
     const long planes = (long)N * C;
     MTA_REQUIRE(planes <= 65535, "conv2d_bwd_weight: N*C = %ld exceeds 65535", planes);
@@ -338,7 +335,7 @@ int conv2d_bwd_weight_launch(const void* x, const void* dy, float* dw, void* wor
     do {                                                                                                                 \
         if (smem > 48 * 1024)                                                                                            \
             MTA_CUDA_OK(cudaFuncSetAttribute(conv2d_bwd_weight_kernel<TT, SCV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        conv2d_bwd_weight_kernel<TT, SCV><<<grid, WT_THREADS, smem, st>>>(static_cast<const TT*>(x), static_cast<const TT*>(dy), \
+        conv2d_bwd_weight_kernel<TT, SCV><<<grid, WT_THREADS, smem, st>>>(static_cast<const TT*>(x), xv, static_cast<const TT*>(dy), dyv, \
                                                                           partial, H, W, R, S, causal, tiles_n);          \
     } while (0)
 #define MTA_BW_CASE(TT)                                     \
@@ -369,8 +366,8 @@ size_t head_linear_bwd_weight_workspace(int C) {
     return (size_t)hw_grid(sms) * C * C * sizeof(float);
 }
 
-int head_linear_bwd_weight_launch(const void* x, const void* dy, float* dW, void* workspace, int N, int C, int P, int Q,
-                                  int causal, int dtype, cudaStream_t st) {
+int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dW, void* workspace, int N, int C,
+                                  int P, int Q, int causal, int dtype, cudaStream_t st) {
     int dev = 0, sms = 0;
     MTA_CUDA_OK(cudaGetDevice(&dev));
     MTA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -378,19 +375,20 @@ int head_linear_bwd_weight_launch(const void* x, const void* dy, float* dW, void
     const int grid = hw_grid(sms);
     float* partial = static_cast<float*>(workspace);
     int rc;
-    const bool vec_ok = dtype != MTA_F32 && C <= 32 && Q % 8 == 0 && aligned16(x) && aligned16(dy);
+    const bool vec_ok = dtype != MTA_F32 && C <= 32 && aligned16(x) && aligned16(dy) && xv.width % 8 == 0 && dyv.width % 8 == 0 &&
+                        xv.plane_stride % 8 == 0 && dyv.plane_stride % 8 == 0;
     if (vec_ok && variant("head_linear") != 1) {         // tensor cores (mta_set_variant("head_linear", 1): CUDA cores)
 #define MTA_HM_CASE(TT, MTV)                                                                                              \
-    head_linear_bwd_weight_mma_kernel<TT, MTV><<<grid, HM_WARPS * 32, 0, st>>>(static_cast<const TT*>(x), static_cast<const TT*>(dy), \
+    head_linear_bwd_weight_mma_kernel<TT, MTV><<<grid, HM_WARPS * 32, 0, st>>>(static_cast<const TT*>(x), xv, static_cast<const TT*>(dy), dyv, \
                                                                                partial, N, C, P, Q, causal)
         if (dtype == MTA_BF16) { if (C <= 16) MTA_HM_CASE(__nv_bfloat16, 1); else MTA_HM_CASE(__nv_bfloat16, 2); }
         else { if (C <= 16) MTA_HM_CASE(__half, 1); else MTA_HM_CASE(__half, 2); }
 #undef MTA_HM_CASE
         MTA_LAUNCH_OK("head_linear_bwd_weight_mma_kernel");
         rc = MTA_OK;
-    } else if (dtype == MTA_F32) rc = dispatch_hw<float>(x, dy, partial, N, C, P, Q, causal, grid, st);
-    else if (dtype == MTA_BF16) rc = dispatch_hw<__nv_bfloat16>(x, dy, partial, N, C, P, Q, causal, grid, st);
-    else rc = dispatch_hw<__half>(x, dy, partial, N, C, P, Q, causal, grid, st);
+    } else if (dtype == MTA_F32) rc = dispatch_hw<float>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
+    else if (dtype == MTA_BF16) rc = dispatch_hw<__nv_bfloat16>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
+    else rc = dispatch_hw<__half>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
     if (rc) return rc;
     const int pairs = C * C;
     head_linear_bwd_weight_reduce_kernel<<<(pairs + 255) / 256, 256, 0, st>>>(partial, dW, grid, pairs);

@@ -37,9 +37,6 @@
 
 namespace mta {
 
-int make_tensor_map_chunked(CUtensorMap* out, const void* base, uint64_t planes, uint64_t rows, uint64_t cols,
-                            uint64_t row_pitch_elems, uint64_t plane_pitch_elems, uint32_t box_rows, uint32_t box_chunks);
-
 namespace {
 using namespace tc05;
 

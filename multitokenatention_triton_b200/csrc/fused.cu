@@ -22,10 +22,10 @@ struct Plan {
 
 size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Rows of a 16-bit scratch plane start on 128-byte boundaries whatever S is: TMA and the vector accesses of the tensor-core
+// Rows of a scratch plane start on 128-byte boundaries whatever S is: TMA and the vector accesses of the tensor-core
 // kernels need 16, and a box of 64 columns then touches one line per row instead of two.  Nothing in the padding is ever read
 // as a score (the tensor maps end at column S).
-int padded_pitch(int S, int dtype) { return dtype == MTA_F32 ? S : (int)round_up((size_t)S, 64); }
+int padded_pitch(int S, int dtype) { return (int)round_up((size_t)S, dtype == MTA_F32 ? 32 : 64); }
 
 Plan make_plan(int B, int H, int S, int cq, int cq2, int r0, int r1, int dtype, int pitch) {
     Plan p;

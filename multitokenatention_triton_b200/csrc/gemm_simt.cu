@@ -1,6 +1,7 @@
 // CUDA-core (fp32 FMA) versions of the two contractions of the forward: scores = Q K^T * scale and
-// out = P V, restricted to keys k <= q when causal.  They serve float32 runs (where tensor-core
-// TF32 would miss the 1e-3 absolute tolerance) and shapes the tensor-core kernels do not take.
+// out = P V (or P^T V), restricted to keys k <= q when causal: the general kernels, for 16-bit
+// shapes the tensor-core kernels do not take and for float32 whose rows are not 16-byte aligned (gemm_f32.cu takes the rest;
+// tensor-core TF32 would miss the 1e-3 absolute tolerance of float32) or that applies dropout.
 // Stand in for the torch.matmul calls at mta_attention_triton.py:68-71 and :89.
 #include "kernels.cuh"
 
@@ -62,24 +63,28 @@ qk_scores_simt_kernel(const T* __restrict__ q, const T* __restrict__ k, T* __res
     }
 }
 
-// out tile (BT queries x BT features) of one (b,h): o[q,d] = sum_{k<=q} P[q,k] V[k,d]
-template <typename T>
+// out tile (BT rows x BT features) of one (b,h): o[q,d] = scale * sum_{k<=q} P[q,k] V[k,d]; TRANS: the plane read as its
+// transpose, o[k,d] = scale * sum_{q>=k} P[q,k] V[q,d]
+template <typename T, bool TRANS>
 __global__ void __launch_bounds__(GT)
 pv_simt_kernel(const T* __restrict__ p, PlaneView pv, const T* __restrict__ v, T* __restrict__ o, int S, int D,
-               int causal, int row_begin, int row_end, int tiles_d, DropoutSpec drop) {
+               int causal, int row_begin, int row_end, int tiles_d, float scale, DropoutSpec drop) {
     __shared__ float ps[BK][BT + 1];
     __shared__ float vs[BK][BT + 1];
     const long bh = blockIdx.y;
     const int tq = blockIdx.x / tiles_d, td = blockIdx.x % tiles_d;
     const int q0 = row_begin + tq * BT, d0 = td * BT;
     const int q_end = min(q0 + BT, row_end);
-    const int k_end = causal ? min(q_end, S) : S;
+    const int k_begin = TRANS && causal ? q0 / BK * BK : 0, k_end = !TRANS && causal ? min(q_end, S) : S;
     const T* vp = v + bh * (long)S * D;
     const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
     float acc[4][4] = {};
-    for (int k0 = 0; k0 < k_end; k0 += BK) {
+    for (int k0 = k_begin; k0 < k_end; k0 += BK) {
         for (int idx = tid; idx < BT * BK; idx += GT) {
-            {   // P: BT rows x BK keys, consecutive threads along keys
+            if (TRANS) {   // P: BK query rows x BT keys, consecutive threads along keys
+                const int qq = k0 + idx / BT, kk = q0 + idx % BT;
+                ps[idx / BT][idx % BT] = (qq < k_end && kk < q_end && (!causal || kk <= qq)) ? to_f32<T>(p[pv.at(bh, qq, kk)]) : 0.0f;
+            } else {   // P: BT rows x BK keys, consecutive threads along keys
                 const int r = idx / BK, kk = k0 + idx % BK;
                 const int qq = q0 + r;
                 float val = 0.0f;
@@ -117,7 +122,7 @@ pv_simt_kernel(const T* __restrict__ p, PlaneView pv, const T* __restrict__ v, T
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int d = d0 + tx * 4 + j;
-            if (d < D) op[(long)qq * D + d] = from_f32<T>(acc[i][j]);
+            if (d < D) op[(long)qq * D + d] = from_f32<T>(acc[i][j] * scale);
         }
     }
 }
@@ -141,16 +146,18 @@ int qk_scores_simt_launch(const void* q, const void* k, void* s, PlaneView sv, i
 }
 
 int pv_simt_launch(const void* p, PlaneView pview, const void* v, void* o, int B, int H, int S, int D, int causal,
-                   int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop) {
+                   int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop, bool trans, float scale) {
     const int tiles_q = (row_end - row_begin + BT - 1) / BT, tiles_d = (D + BT - 1) / BT;
     dim3 grid((unsigned)(tiles_q * tiles_d), (unsigned)(B * H));
-#define MTA_PV(TT)                                                                                              \
-    pv_simt_kernel<TT><<<grid, GT, 0, st>>>(static_cast<const TT*>(p), pview, static_cast<const TT*>(v),          \
-                                            static_cast<TT*>(o), S, D, causal, row_begin, row_end, tiles_d, drop)
+#define MTA_PV_RUN(TT, TR)                                                                                        \
+    pv_simt_kernel<TT, TR><<<grid, GT, 0, st>>>(static_cast<const TT*>(p), pview, static_cast<const TT*>(v),       \
+                                                static_cast<TT*>(o), S, D, causal, row_begin, row_end, tiles_d, scale, drop)
+#define MTA_PV(TT) do { if (trans) MTA_PV_RUN(TT, true); else MTA_PV_RUN(TT, false); } while (0)
     if (dtype == MTA_F32) MTA_PV(float);
     else if (dtype == MTA_BF16) MTA_PV(__nv_bfloat16);
     else MTA_PV(__half);
 #undef MTA_PV
+#undef MTA_PV_RUN
     MTA_LAUNCH_OK("pv_simt_kernel");
     return MTA_OK;
 }

@@ -1,5 +1,6 @@
-// The two contractions of the forward on the 5th-generation tensor cores (tcgen05), 16-bit dtypes:
-//   output tile  O[128 q x D]     = sum over key tiles  P[128 q x 128 k] V[128 k x D]   (A K-major, B MN-major)
+// Products of a causal score plane with (rows x D) matrices on the 5th-generation tensor cores (tcgen05), 16-bit dtypes:
+//   O[128 q x D] = scale * sum over keys <= q     P[q x k] V[k x D]     (A K-major, B MN-major): P V, and dS K of a backward
+//   O[128 k x D] = scale * sum over queries >= k  P[q x k] X[q x D]     (A and B MN-major): P^T dO and dS^T Q of a backward
 // Operand tiles arrive by TMA (128-byte swizzle, out-of-range rows and columns read as zero), the
 // accumulator lives in tensor memory, and only tiles that touch keys k <= q are visited when causal.
 // They stand in for the torch.matmul calls at mta_attention_triton.py:68-71 and :89.
@@ -114,42 +115,22 @@ int make_tensor_map_3d_mode(CUtensorMap* out, const void* base, uint64_t planes,
                 "tensor map: box %u x %u with a %d-byte swizzle is not supported", box_cols, box_rows, swizzle_bytes);
     cuuint32_t box[3] = {box_cols, box_rows, box_planes};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                               : (swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                                      : (swizzle_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE)),
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUtensorMapSwizzle swizzle =
+        swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                   : (swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : (swizzle_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE));
+    auto encode = [&] {
+        return fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {
+        // A thread whose first CUDA work is this call (autograd's, for one) has no current context yet: a driver function does
+        // not set one up as the runtime's do.
+        MTA_CUDA_OK(cudaFree(nullptr));
+        r = encode();
+    }
     if (r != CUDA_SUCCESS) {
         set_error("cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-        return MTA_ERR_CUDA;
-    }
-    return MTA_OK;
-}
-
-// 4-D map (8 columns, rows, 8-column chunks, planes) of a [planes][rows][cols] tensor of 16-bit elements: a box
-// {8, box_rows, box_chunks, 1} lands in shared memory as [chunk][row][8 columns], the layout a tcgen05 matrix
-// descriptor without swizzle reads with any row offset.  Out-of-range rows and chunks read as zero.
-int make_tensor_map_chunked(CUtensorMap* out, const void* base, uint64_t planes, uint64_t rows, uint64_t cols,
-                            uint64_t row_pitch_elems, uint64_t plane_pitch_elems, uint32_t box_rows, uint32_t box_chunks) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) {
-        set_error("cuTensorMapEncodeTiled is not available from this driver");
-        return MTA_ERR_CUDA;
-    }
-    MTA_REQUIRE(aligned16(base) && cols % 8 == 0 && (row_pitch_elems * 2) % 16 == 0 && (plane_pitch_elems * 2) % 16 == 0 &&
-                    box_rows <= 256 && box_chunks <= 256,
-                "chunked tensor map: unsupported geometry");
-    cuuint64_t dims[4] = {8, rows, cols / 8, planes};
-    cuuint64_t strides[3] = {row_pitch_elems * 2, 16, plane_pitch_elems * 2};
-    cuuint32_t box[4] = {8, box_rows, box_chunks, 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        set_error("cuTensorMapEncodeTiled (chunked view) failed with CUresult %d", (int)r);
         return MTA_ERR_CUDA;
     }
     return MTA_OK;
@@ -180,41 +161,51 @@ __device__ __forceinline__ uint8_t* align_1024(uint8_t* p) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// O tile = sum over key tiles of P tile x V tile.  Warp 0: TMA producer; warp 1: zeroes the part of a
-// diagonal P tile that lies above the diagonal, then issues the MMAs; warps 2..5: epilogue.
+// Output tile of 128 rows = sum over steps of 64 contraction indices (keys, or queries when TRANS).  Warp 0: TMA producer;
+// warp 1: MMA issuer; warps 2..5: before the accumulator is complete they zero what lies above the diagonal in the few tiles
+// that straddle it (128 threads; one warp doing it was a serial stretch of about a microsecond per tile) and apply the
+// dropout, then they are the epilogue.
 constexpr int PV_STAGES = 3;
 constexpr int PV_THREADS = 192;
-constexpr int PV_KEYS = 64;               // keys per pipeline stage: 32 KB stages, so two CTAs fit on an SM and one CTA's
-                                          // start-up and epilogue overlap the other's steady state
-constexpr int PV_VBOX_BYTES = PV_KEYS * 128;   // one box of the V tile: 64 keys x 64 elements
+constexpr int PV_KEYS = 64;               // contraction indices per pipeline stage: 32 KB stages, so two CTAs fit on an SM and
+                                          // one CTA's start-up and epilogue overlap the other's steady state
+constexpr int PV_VBOX_BYTES = PV_KEYS * 128;   // one box of the V tile: 64 rows x 64 elements
+constexpr int PV_DIAG = 3;                // most steps of a tile that straddle the diagonal (128 rows from any row on)
 
-// DROP: the four epilogue warps, idle until the accumulator is complete, apply the dropout of dropout.cuh to every P tile
-// in shared memory before its MMAs are issued (a thread owns a row of the tile).
-template <typename T, int D, bool DROP>
+// DROP: the dropout of dropout.cuh is applied to every P tile in shared memory before its MMAs (a thread owns a row).
+// TRANS: the P tile is read as its transpose: 64 query rows x 128 keys, two boxes of 64 keys.
+template <typename T, int D, bool DROP, bool TRANS>
 __global__ void __launch_bounds__(PV_THREADS)
 pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ CUtensorMap mv, T* __restrict__ o,
-               int p_row0, int S, int causal, int row_begin, int row_end, int* err_flag, DropoutSpec drop) {
+               int p_row0, int S, int causal, int row_begin, int row_end, float scale, int* err_flag, DropoutSpec drop) {
     constexpr int NBOX_V = D / 64;
-    constexpr int P_BYTES = BOX_BYTES;                     // 128 q x 64 k
-    constexpr int V_BYTES = NBOX_V * PV_VBOX_BYTES;        // 64 k x D
+    constexpr int P_BYTES = BOX_BYTES;                     // 128 q x 64 k, or 64 q x 128 k
+    constexpr int V_BYTES = NBOX_V * PV_VBOX_BYTES;        // 64 rows x D
     constexpr int STAGE_BYTES = P_BYTES + V_BYTES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = align_1024(smem_raw);
-    __shared__ __align__(8) uint64_t full_bar[PV_STAGES], empty_bar[PV_STAGES], mask_bar[PV_STAGES], acc_bar;
+    __shared__ __align__(8) uint64_t full_bar[PV_STAGES], empty_bar[PV_STAGES], drop_bar[PV_STAGES], go_bar[PV_DIAG], diag_bar[PV_DIAG],
+        acc_bar;
     __shared__ uint32_t tmem_slot;
 
     __shared__ int abort_flag;      // an earlier bounded wait on this device gave up: the whole CTA does nothing
     if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
     __syncthreads();
     if (abort_flag != 0) return;
-    // heaviest query tiles first: tile index counts down from the last
+    // heaviest tiles first: the last query tile (all keys), or the first key tile (all queries)
     const int n_qt = (row_end - row_begin + TILE - 1) / TILE;
-    const int tq = n_qt - 1 - (int)blockIdx.x;
-    const int bh = (int)blockIdx.y;
-    const int q0 = row_begin + tq * TILE;
+    const int tq = TRANS ? (int)blockIdx.y : n_qt - 1 - (int)blockIdx.y;
+    const int bh = (int)blockIdx.x;
+    const int q0 = row_begin + tq * TILE;                  // first output row (a query, or a key when TRANS)
     const int q_end = min(q0 + TILE, row_end);
-    // 64-key steps that hold a key <= the tile's last query
-    const int nk = causal ? min((q_end + PV_KEYS - 1) / PV_KEYS, (S + PV_KEYS - 1) / PV_KEYS) : (S + PV_KEYS - 1) / PV_KEYS;
+    // steps [kt0, kt1) of 64 contraction indices: keys up to the tile's last query, or queries from the tile's first key on
+    const int n_steps = (S + PV_KEYS - 1) / PV_KEYS;
+    const int kt0 = TRANS && causal ? q0 / PV_KEYS : 0;
+    const int kt1 = !TRANS && causal ? min((q_end + PV_KEYS - 1) / PV_KEYS, n_steps) : n_steps;
+    // steps [d0, d1) straddle the diagonal
+    const int d0 = !causal ? kt1 : (TRANS ? kt0 : min((q0 + 1) / PV_KEYS, kt1));
+    const int d1 = !causal ? kt1 : (TRANS ? min((q0 + TILE - 2) / PV_KEYS + 1, kt1) : kt1);
+    const int nk = kt1 - kt0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (warp == 0) {
@@ -222,7 +213,11 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
             for (int i = 0; i < PV_STAGES; ++i) {
                 mbar_init(&full_bar[i], 1);
                 mbar_init(&empty_bar[i], 1);
-                mbar_init(&mask_bar[i], 4);
+                mbar_init(&drop_bar[i], 4);
+            }
+            for (int i = 0; i < PV_DIAG; ++i) {
+                mbar_init(&go_bar[i], 1);
+                mbar_init(&diag_bar[i], 4);
             }
             mbar_init(&acc_bar, 1);
             fence_mbar_init();
@@ -239,77 +234,92 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
 
     if (warp == 0) {
         if (lane == 0) {
-            for (int kt = 0; kt < nk; ++kt) {
-                const int st = kt % PV_STAGES, use = kt / PV_STAGES;
+            for (int it = 0; it < nk; ++it) {
+                const int kt = kt0 + it, st = it % PV_STAGES, use = it / PV_STAGES;
                 if (use > 0) mbar_wait(&empty_bar[st], (use - 1) & 1, err_flag);
                 uint8_t* sp = smem + st * STAGE_BYTES;
                 uint8_t* sv = sp + P_BYTES;
                 mbar_expect_tx(&full_bar[st], STAGE_BYTES);
-                tma_load_3d(sp, &mp, &full_bar[st], kt * PV_KEYS, q0 - p_row0, bh);
+                if (TRANS) {
+                    tma_load_3d(sp, &mp, &full_bar[st], q0, kt * PV_KEYS - p_row0, bh);
+                    tma_load_3d(sp + P_BYTES / 2, &mp, &full_bar[st], q0 + 64, kt * PV_KEYS - p_row0, bh);
+                } else {
+                    tma_load_3d(sp, &mp, &full_bar[st], kt * PV_KEYS, q0 - p_row0, bh);
+                }
 #pragma unroll
                 for (int j = 0; j < NBOX_V; ++j) tma_load_3d(sv + j * PV_VBOX_BYTES, &mv, &full_bar[st], j * 64, kt * PV_KEYS, bh);
             }
         }
     } else if (warp == 1) {
-        constexpr uint32_t idesc = instr_desc_f16(AbFormat<T>::value, 0, 1, TILE, D);
-        for (int kt = 0; kt < nk; ++kt) {
-            const int st = kt % PV_STAGES, use = kt / PV_STAGES;
+        constexpr uint32_t idesc = instr_desc_f16(AbFormat<T>::value, TRANS ? 1 : 0, 1, TILE, D);
+        for (int it = 0; it < nk; ++it) {
+            const int kt = kt0 + it, st = it % PV_STAGES, use = it / PV_STAGES;
             uint8_t* sp = smem + st * STAGE_BYTES;
             uint8_t* sv = sp + P_BYTES;
             mbar_wait(&full_bar[st], use & 1, err_flag);
-            if (DROP) mbar_wait(&mask_bar[st], use & 1, err_flag);         // the epilogue warps have applied the dropout
-            const int k0 = kt * PV_KEYS;
-            if (causal && k0 + PV_KEYS - 1 > q0) {
-                // Keys above the diagonal must contribute nothing, whatever the buffer holds there.
-                // Element (row r, key c) of the swizzled tile: byte r*128 + ((c/8) ^ (r%8))*16 + (c%8)*2.
-                for (int idx = lane; idx < TILE * 8; idx += 32) {
-                    const int r = idx >> 3, ch = idx & 7;              // 16-byte chunk ch covers keys 8ch..8ch+7
-                    const int qrow = q0 + r, kfirst = k0 + ch * 8;
-                    if (kfirst + 7 <= qrow) continue;
-                    uint8_t* chunk = sp + r * 128 + ((ch ^ (r & 7)) << 4);
-                    if (kfirst > qrow) {
-                        *reinterpret_cast<uint4*>(chunk) = make_uint4(0u, 0u, 0u, 0u);
-                    } else {
-                        uint16_t* e16 = reinterpret_cast<uint16_t*>(chunk);
-                        for (int e = 0; e < 8; ++e)
-                            if (kfirst + e > qrow) e16[e] = 0;
-                    }
-                }
-                fence_proxy_async();
+            if (DROP) mbar_wait(&drop_bar[st], use & 1, err_flag);                      // the dropout has been applied
+            if (kt >= d0 && kt < d1) {                                                  // the part above the diagonal becomes zero
+                // The warps that zero it visit few of the stages, so they cannot follow full_bar's phases themselves (a wait
+                // tells two phases apart, no more): this warp, which sees every phase, calls them.
+                if (!DROP && lane == 0) mbar_arrive(&go_bar[kt - d0]);
+                mbar_wait_spin(&diag_bar[kt - d0], 0, err_flag);
             }
-            __syncwarp();
             fence_after_sync();
             if (lane == 0) {
 #pragma unroll
                 for (int kk = 0; kk < PV_KEYS / 16; ++kk) {
-                    const uint64_t da = smem_desc_sw128(smem_u32(sp) + kk * 32, 16, 1024);
+                    const uint64_t da = TRANS ? smem_desc_sw128(smem_u32(sp) + kk * 16 * 128, P_BYTES / 2, 1024)
+                                              : smem_desc_sw128(smem_u32(sp) + kk * 32, 16, 1024);
                     const uint64_t db = smem_desc_sw128(smem_u32(sv) + kk * 16 * 128, PV_VBOX_BYTES, 1024);
-                    mma_f16_ss(tmem, da, db, idesc, (kt > 0 || kk > 0) ? 1u : 0u);
+                    mma_f16_ss(tmem, da, db, idesc, (it > 0 || kk > 0) ? 1u : 0u);
                 }
                 mma_commit(&empty_bar[st]);
-                if (kt == nk - 1) mma_commit(&acc_bar);
+                if (it == nk - 1) mma_commit(&acc_bar);
             }
             __syncwarp();
         }
     } else {
-        if (DROP) {
-            const int r = (int)threadIdx.x - 64;             // row of the P tile this thread owns
-            const uint32_t thr = drop.keep_threshold();
-            const float scale = drop.scale();
-            for (int kt = 0; kt < nk; ++kt) {
-                const int st = kt % PV_STAGES, use = kt / PV_STAGES;
-                uint8_t* sp = smem + st * STAGE_BYTES;
-                mbar_wait(&full_bar[st], use & 1, err_flag);
+        const int et = (int)threadIdx.x - 64;                // 0..127
+        for (int it = DROP ? 0 : d0 - kt0; it < (DROP ? nk : d1 - kt0); ++it) {
+            const int kt = kt0 + it, st = it % PV_STAGES, use = it / PV_STAGES;
+            uint8_t* sp = smem + st * STAGE_BYTES;
+            const int k0 = kt * PV_KEYS;
+            if (DROP) mbar_wait(&full_bar[st], use & 1, err_flag);
+            else mbar_wait(&go_bar[kt - d0], 0, err_flag);
+            if (DROP) {
+                const uint32_t thr = drop.keep_threshold();
+                const float keep_scale = drop.scale();
 #pragma unroll 2
                 for (int ch = 0; ch < 8; ++ch) {
-                    const uint32_t keep = dropout_keep8(drop.seed, (uint32_t)bh, (uint32_t)(q0 + r), (uint32_t)(kt * (PV_KEYS / 8) + ch), thr);
-                    T* e8 = reinterpret_cast<T*>(sp + r * 128 + ((ch ^ (r & 7)) << 4));
+                    const uint32_t keep = dropout_keep8(drop.seed, (uint32_t)bh, (uint32_t)(q0 + et), (uint32_t)(kt * (PV_KEYS / 8) + ch), thr);
+                    T* e8 = reinterpret_cast<T*>(sp + et * 128 + ((ch ^ (et & 7)) << 4));
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) e8[e] = (keep >> e) & 1u ? from_f32<T>(to_f32<T>(e8[e]) * scale) : from_f32<T>(0.0f);
+                    for (int e = 0; e < 8; ++e) e8[e] = (keep >> e) & 1u ? from_f32<T>(to_f32<T>(e8[e]) * keep_scale) : from_f32<T>(0.0f);
                 }
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&mask_bar[st]);
+            }
+            if (kt >= d0 && kt < d1) {
+                // Keys above the diagonal must contribute nothing, whatever the buffer holds there: a thread takes one line of
+                // 64 keys (a row of the tile; when TRANS one of the two halves of a row) and zeroes it from the first such key on.
+                const int line = TRANS ? et & 63 : et, key_first = TRANS ? q0 + (et >> 6) * 64 : k0;
+                const int qrow = TRANS ? k0 + line : q0 + line;
+                uint8_t* lp = sp + (TRANS ? (et >> 6) * (P_BYTES / 2) : 0) + line * 128;
+                int first = qrow + 1 - key_first;            // first key of the line to zero
+                if (first < 0) first = 0;
+                for (int ch = first >> 3; ch < 8; ++ch) {
+                    uint4* chunk = reinterpret_cast<uint4*>(lp + ((ch ^ (line & 7)) << 4));
+                    if (ch * 8 >= first) {
+                        *chunk = make_uint4(0u, 0u, 0u, 0u);
+                    } else {
+                        uint16_t* e16 = reinterpret_cast<uint16_t*>(chunk);
+                        for (int e = first & 7; e < 8; ++e) e16[e] = 0;
+                    }
+                }
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                if (DROP) mbar_arrive(&drop_bar[st]);
+                if (kt >= d0 && kt < d1) mbar_arrive(&diag_bar[kt - d0]);
             }
         }
         mbar_wait(&acc_bar, 0, err_flag);
@@ -326,11 +336,14 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
             if (q >= q_end) continue;
 #pragma unroll
             for (int v8 = 0; v8 < 4; ++v8) {
+                float f[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[v8 * 8 + e]) * scale;
                 uint4 w;
-                w.x = pack2<T>(__uint_as_float(r[v8 * 8 + 0]), __uint_as_float(r[v8 * 8 + 1]));
-                w.y = pack2<T>(__uint_as_float(r[v8 * 8 + 2]), __uint_as_float(r[v8 * 8 + 3]));
-                w.z = pack2<T>(__uint_as_float(r[v8 * 8 + 4]), __uint_as_float(r[v8 * 8 + 5]));
-                w.w = pack2<T>(__uint_as_float(r[v8 * 8 + 6]), __uint_as_float(r[v8 * 8 + 7]));
+                w.x = pack2<T>(f[0], f[1]);
+                w.y = pack2<T>(f[2], f[3]);
+                w.z = pack2<T>(f[4], f[5]);
+                w.w = pack2<T>(f[6], f[7]);
                 *reinterpret_cast<uint4*>(orow + c * 32 + v8 * 8) = w;
             }
         }
@@ -340,29 +353,36 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
     if (warp == 0) tmem_dealloc(tmem, D < 32 ? 32 : D);
 }
 
-template <typename T, int D>
+template <typename T, int D, bool DROP, bool TRANS>
 int launch_pv(const void* p, PlaneView pview, const void* v, void* o, int B, int H, int S, int causal, int row_begin,
-              int row_end, long p_rows_stored, cudaStream_t st, DropoutSpec drop) {
+              int row_end, long p_rows_stored, float scale, cudaStream_t st, DropoutSpec drop) {
     CUtensorMap mp, mv;
     int rc;
-    if ((rc = make_tensor_map_3d(&mp, p, (uint64_t)B * H, (uint64_t)p_rows_stored, S, (uint64_t)pview.width, (uint64_t)pview.plane_stride, 64, TILE, true))) return rc;
+    if ((rc = make_tensor_map_3d(&mp, p, (uint64_t)B * H, (uint64_t)p_rows_stored, S, (uint64_t)pview.width, (uint64_t)pview.plane_stride, 64,
+                                 TRANS ? PV_KEYS : TILE, true)))
+        return rc;
     if ((rc = make_tensor_map_3d(&mv, v, (uint64_t)B * H, S, D, D, (uint64_t)S * D, 64, PV_KEYS, true))) return rc;
     int* flag = nullptr;
     if ((rc = wait_flag_ptr(&flag))) return rc;
     const int n_qt = (row_end - row_begin + TILE - 1) / TILE;
     const size_t smem = (size_t)PV_STAGES * (BOX_BYTES + (D / 64) * PV_VBOX_BYTES) + 1024;
-    dim3 grid((unsigned)n_qt, (unsigned)(B * H));
-    if (drop.on()) {
-        MTA_CUDA_OK(cudaFuncSetAttribute(pv_tc05_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        pv_tc05_kernel<T, D, true><<<grid, PV_THREADS, smem, st>>>(mp, mv, static_cast<T*>(o), pview.row0, S, causal, row_begin,
-                                                                   row_end, flag, drop);
-    } else {
-        MTA_CUDA_OK(cudaFuncSetAttribute(pv_tc05_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        pv_tc05_kernel<T, D, false><<<grid, PV_THREADS, smem, st>>>(mp, mv, static_cast<T*>(o), pview.row0, S, causal, row_begin,
-                                                                    row_end, flag, drop);
-    }
+    dim3 grid((unsigned)(B * H), (unsigned)n_qt);      // planes along x: the heaviest tiles of ALL planes come first
+    auto kernel = pv_tc05_kernel<T, D, DROP, TRANS>;
+    MTA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, PV_THREADS, smem, st>>>(mp, mv, static_cast<T*>(o), pview.row0, S, causal, row_begin, row_end, scale, flag, drop);
     MTA_LAUNCH_OK("pv_tc05_kernel");
     return MTA_OK;
+}
+
+template <typename T, int D>
+int launch_pv_kind(const void* p, PlaneView pview, const void* v, void* o, int B, int H, int S, int causal, int row_begin, int row_end,
+                   long p_rows_stored, bool trans, float scale, cudaStream_t st, DropoutSpec drop) {
+#define MTA_PV_KIND(DROP, TRANS) \
+    return launch_pv<T, D, DROP, TRANS>(p, pview, v, o, B, H, S, causal, row_begin, row_end, p_rows_stored, scale, st, drop)
+    if (trans) MTA_PV_KIND(false, true);
+    if (drop.on()) MTA_PV_KIND(true, false);
+    MTA_PV_KIND(false, false);
+#undef MTA_PV_KIND
 }
 
 }  // namespace
@@ -373,8 +393,8 @@ bool tc05_contractions_supported(int S, int D, int dtype, const void* a, const v
 }
 
 int pv_tc05_launch(const void* p, PlaneView pview, long p_rows_stored, const void* v, void* o, int B, int H, int S, int D,
-                   int causal, int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop) {
-#define MTA_PV(TT, DD) return launch_pv<TT, DD>(p, pview, v, o, B, H, S, causal, row_begin, row_end, p_rows_stored, st, drop)
+                   int causal, int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop, bool trans, float scale) {
+#define MTA_PV(TT, DD) return launch_pv_kind<TT, DD>(p, pview, v, o, B, H, S, causal, row_begin, row_end, p_rows_stored, trans, scale, st, drop)
     if (dtype == MTA_BF16) { if (D == 64) MTA_PV(__nv_bfloat16, 64); MTA_PV(__nv_bfloat16, 128); }
     if (D == 64) MTA_PV(__half, 64);
     MTA_PV(__half, 128);

@@ -26,16 +26,16 @@ int head_linear_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype,
                        int C, int P, int Q, int causal, float fill, int row_begin, int row_end, bool write_upper,
                        int dtype, cudaStream_t st, bool w_transposed = false);
 
-// Gradients of the two stand-alone ops (backward.cu, conv2d.cu).  dx of the conv: layout of x, zeros above the diagonal
-// when causal.  The weight gradients are float32, reduced in a fixed order through a caller workspace of the given size.
-int conv2d_bwd_input_launch(const void* dy, const void* w, int w_dtype, void* dx, long planes, int C, int H, int W, int R,
-                            int S, int causal, int dtype, cudaStream_t st);
+// Gradients of the two stand-alone ops (backward.cu, conv2d.cu).  dx of the conv: zeros above the diagonal when causal and
+// `write_upper`.  The weight gradients are float32, reduced in a fixed order through a caller workspace of the given size.
+int conv2d_bwd_input_launch(const void* dy, PlaneView dyv, const void* w, int w_dtype, void* dx, PlaneView dxv, long planes, int C, int H,
+                            int W, int R, int S, int causal, bool write_upper, int dtype, cudaStream_t st);
 size_t conv2d_bwd_weight_workspace(int N, int C, int H, int W, int R, int S);
-int conv2d_bwd_weight_launch(const void* x, const void* dy, float* dw, void* workspace, int N, int C, int H, int W, int R,
-                             int S, int causal, int dtype, cudaStream_t st);
+int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dw, void* workspace, int N, int C, int H,
+                             int W, int R, int S, int causal, int dtype, cudaStream_t st);
 size_t head_linear_bwd_weight_workspace(int C);
-int head_linear_bwd_weight_launch(const void* x, const void* dy, float* dW, void* workspace, int N, int C, int P, int Q,
-                                  int causal, int dtype, cudaStream_t st);
+int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dW, void* workspace, int N, int C,
+                                  int P, int Q, int causal, int dtype, cudaStream_t st);
 
 // Head mix followed by the causal row softmax of the mixed logits, in one pass (16-bit dtypes, C <= 32, causal);
 // entries above the diagonal of y are written as 0 when `write_upper`, else left untouched.
@@ -61,6 +61,10 @@ int head_linear_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y
 int softmax_launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int P, int Q, int causal,
                    int row_begin, int row_end, bool write_upper, float pre_scale, int dtype, cudaStream_t st);
 
+// ds = p (g - sum over the row of g p), keys k <= query when causal; ds may be g.  Nothing above the diagonal is touched.
+int softmax_bwd_launch(const void* p, PlaneView pv, const void* g, PlaneView gv, void* ds, PlaneView dv, long planes, int P, int Q,
+                       int causal, int dtype, cudaStream_t st);
+
 // s = round(round(Q K^T) * scale) for rows [row_begin,row_end), keys k <= q when causal.
 int qk_scores_launch(const void* q, const void* k, void* s, PlaneView sv, int B, int H, int S, int D, float scale,
                      int round_scale, int causal, int row_begin, int row_end, int dtype, cudaStream_t st);
@@ -68,13 +72,24 @@ int qk_scores_launch(const void* q, const void* k, void* s, PlaneView sv, int B,
 // o[rows] = p[rows, k<=q] V.  `p_rows_stored` = number of rows each plane of p holds (from pview.row0 on).
 // `drop`: dropout on the weights as they are read (dropout.cuh); the default leaves them as they are.
 int pv_launch(const void* p, PlaneView pview, long p_rows_stored, const void* v, void* o, int B, int H, int S, int D,
-              int causal, int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop = DropoutSpec());
+              int causal, int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop = DropoutSpec(), float scale = 1.0f);
+// o[key] = scale * sum over queries >= key (all when not causal) of p[query, key] x[query]: the product with the transposed plane.
+int ptx_launch(const void* p, PlaneView pview, const void* x, void* o, int B, int H, int S, int D, int causal, float scale, int dtype,
+               cudaStream_t st);
 
 // CUDA-core versions of the two contractions (gemm_simt.cu).
 int qk_scores_simt_launch(const void* q, const void* k, void* s, PlaneView sv, int B, int H, int S, int D, float scale,
                           int round_scale, int causal, int row_begin, int row_end, int dtype, cudaStream_t st);
 int pv_simt_launch(const void* p, PlaneView pview, const void* v, void* o, int B, int H, int S, int D, int causal,
-                   int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop = DropoutSpec());
+                   int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop = DropoutSpec(), bool trans = false,
+                   float scale = 1.0f);
+
+// float32 with 16-byte aligned rows (gemm_f32.cu).
+bool gemm_f32_supported(const void* a, const void* b, const void* c, PlaneView plane, int S, int D, int dtype);
+int qk_f32_launch(const void* q, const void* k, void* s, PlaneView sv, int B, int H, int S, int D, float scale, int causal, int row_begin,
+                  int row_end, cudaStream_t st);
+int pv_f32_launch(const void* p, PlaneView pview, const void* v, void* o, int B, int H, int S, int D, int causal, int row_begin, int row_end,
+                  bool trans, float scale, cudaStream_t st);
 
 // tcgen05 version of the conv (conv2d_tc05.cu): 16-bit dtypes, S <= 17, W a multiple of 8, R small enough for its
 // shared-memory rings (R <= 13 with 16-bit weights).
@@ -89,7 +104,8 @@ int conv2d_tc05_launch(const void* x, PlaneView xv, long x_rows_stored, const vo
 // tcgen05 tensor-core versions (gemm_tc05.cu): 16-bit dtypes, D in {64,128}, S a multiple of 8.
 bool tc05_contractions_supported(int S, int D, int dtype, const void* a, const void* b, const void* c, PlaneView view);
 int pv_tc05_launch(const void* p, PlaneView pview, long p_rows_stored, const void* v, void* o, int B, int H, int S, int D,
-                   int causal, int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop = DropoutSpec());
+                   int causal, int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop = DropoutSpec(),
+                   bool trans = false, float scale = 1.0f);
 // Persistent, warp-specialised score-tile kernel (qk_persistent.cu); same domain as the kernels above.
 // NI = 1: c = scale * a b^T.  mode 0: all tiles with keys <= query; 1 / 2: the band of a (band_cq x (2 band_pw + 1))
 // conv / the tiles wholly below it.
