@@ -165,6 +165,27 @@ int mta_fused_fwd(const void* q, const void* k, const void* v, const void* w1, c
                   int w_dtype, void* stream);
 
 /*
+ * A training step's share of the MTA module (causal, no mask, no dropout): the forward that keeps what its backward reads,
+ * and that backward.  They replace MTAAttentionTriton.forward under autograd (mta_attention_triton.py:61-92 with
+ * convolution_2d_trit.py:143-295, triton_linear_head.py:142-278 and torch's backward of the softmax and the two products).
+ *   saved      mta_train_saved_bytes(...) bytes: five score planes (scores, conv 1, probabilities, conv 2, head mix 2) with
+ *              padded rows, written by mta_train_fwd, only read by mta_train_bwd; the part above the diagonal is undefined
+ *   workspace  mta_train_workspace_bytes(...) bytes of scratch
+ *   dout       gradient of o, (B,H,S,D) contiguous in `dtype`; dq, dk, dv: the same; dw1 (H,cq,ck), dW1 (H,H),
+ *              dw2 (H,cq2,ck2), dW2 (H,H): float32.  A gradient whose pointer is NULL is not computed.
+ * ck and ck2 must be odd, H at most 128.  Accumulation is fp32 (weight gradients: fp32 per block, double across blocks).
+ */
+size_t mta_train_saved_bytes(int B, int H, int S, int dtype);
+size_t mta_train_workspace_bytes(int B, int H, int S, int cq, int ck, int cq2, int ck2, int dtype);
+int mta_train_fwd(const void* q, const void* k, const void* v, const void* w1, const void* W1, const void* w2,
+                  const void* W2, void* o, void* saved, size_t saved_bytes, int B, int H, int S, int D, int cq, int ck,
+                  int cq2, int ck2, int dtype, int w_dtype, void* stream);
+int mta_train_bwd(const void* q, const void* k, const void* v, const void* w1, const void* W1, const void* w2,
+                  const void* W2, const void* dout, const void* saved, void* dq, void* dk, void* dv, float* dw1,
+                  float* dW1, float* dw2, float* dW2, void* workspace, size_t workspace_bytes, int B, int H, int S, int D,
+                  int cq, int ck, int cq2, int ck2, int dtype, int w_dtype, void* stream);
+
+/*
  * mta_fused_fwd with dropout on the attention weights between the second head mix and the product with V, where
  * MTAAttentionTriton.forward applies F.dropout(scores, p=self.dropout, training=self.training)
  * (mta_attention_triton.py:87).  No mask tensor exists: whether weight (batch, head, query, key) is kept is a function

@@ -16,6 +16,25 @@ def _tril_(t: torch.Tensor) -> torch.Tensor:
     return torch.tril(t)
 
 
+class MTAFunction(torch.autograd.Function):
+    """The whole causal module (q, k, v, conv weight, head mix, post-softmax conv weight, post-softmax head mix) -> (B,H,S,D)
+    as one node: mta_train_fwd and mta_train_bwd."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, w1, W1, w2, W2):
+        out, saved = ops.mta_train_fwd(q, k, v, w1, W1, w2, W2)
+        ctx.save_for_backward(q, k, v, w1, W1, w2, W2, saved)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        *args, saved = ctx.saved_tensors
+        if args[0].numel() == 0:
+            return tuple(torch.zeros_like(t) if n else None for t, n in zip(args, ctx.needs_input_grad))
+        grads = ops.mta_train_bwd(grad_out.to(args[0].dtype), saved, *args, ctx.needs_input_grad)
+        return tuple(None if g is None else g.to(t.dtype) for g, t in zip(grads, args))
+
+
 class QKScoresFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, scale, causal):

@@ -221,7 +221,74 @@ int launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int 
     return MTA_OK;
 }
 
+// Gradient of the causal row softmax: ds = p (g - sum_k g p) over keys k <= query, fp32 arithmetic; nothing is read or written
+// above the diagonal.  ds may be g.  Bound by memory (two planes in, one out): one warp per row, 16-byte chunks; the row is
+// walked twice, and the second walk finds it in L1.
+constexpr int SB_WARPS = 8;
+
+template <typename T, int VEC>
+__global__ void __launch_bounds__(SB_WARPS * 32)
+softmax_bwd_kernel(const T* __restrict__ p, PlaneView pv, const T* g, PlaneView gv, T* ds, PlaneView dv, int P, int Q, int causal) {
+    struct alignas(sizeof(T) * VEC) V { T e[VEC]; };
+    const int row = P - 1 - ((int)blockIdx.x * SB_WARPS + (threadIdx.x >> 5));     // longest rows first
+    if (row < 0) return;
+    const long plane = blockIdx.y;
+    const int lane = threadIdx.x & 31;
+    const int n = causal ? min(row + 1, Q) : Q;
+    const T* pr = p + pv.at(plane, row, 0);
+    const T* gr = g + gv.at(plane, row, 0);
+    T* dr = ds + dv.at(plane, row, 0);
+    const int whole = n / VEC;
+    float dot = 0.0f;
+#pragma unroll 4
+    for (int c = lane; c < whole; c += 32) {
+        const V a = reinterpret_cast<const V*>(pr)[c], b = reinterpret_cast<const V*>(gr)[c];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) dot = fmaf(to_f32<T>(a.e[e]), to_f32<T>(b.e[e]), dot);
+    }
+    const int tail = whole * VEC + lane;
+    float tp = 0.0f, tg = 0.0f;
+    if (tail < n) {
+        tp = to_f32<T>(pr[tail]);
+        tg = to_f32<T>(gr[tail]);
+        dot = fmaf(tp, tg, dot);
+    }
+    dot = warp_sum(dot);
+#pragma unroll 4
+    for (int c = lane; c < whole; c += 32) {
+        const V a = reinterpret_cast<const V*>(pr)[c], b = reinterpret_cast<const V*>(gr)[c];
+        V o;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) o.e[e] = from_f32<T>(to_f32<T>(a.e[e]) * (to_f32<T>(b.e[e]) - dot));
+        reinterpret_cast<V*>(dr)[c] = o;
+    }
+    if (tail < n) dr[tail] = from_f32<T>(tp * (tg - dot));
+}
+
+template <typename T>
+int launch_bwd(const void* p, PlaneView pv, const void* g, PlaneView gv, void* ds, PlaneView dv, long planes, int P, int Q, int causal,
+               cudaStream_t st) {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    auto ok = [](const void* b, const PlaneView& v) { return aligned16(b) && v.width % VEC == 0 && v.plane_stride % VEC == 0; };
+    const dim3 grid((unsigned)((P + SB_WARPS - 1) / SB_WARPS), (unsigned)planes);
+    if (ok(p, pv) && ok(g, gv) && ok(ds, dv))
+        softmax_bwd_kernel<T, VEC><<<grid, SB_WARPS * 32, 0, st>>>(static_cast<const T*>(p), pv, static_cast<const T*>(g), gv, static_cast<T*>(ds), dv, P, Q, causal);
+    else
+        softmax_bwd_kernel<T, 1><<<grid, SB_WARPS * 32, 0, st>>>(static_cast<const T*>(p), pv, static_cast<const T*>(g), gv, static_cast<T*>(ds), dv, P, Q, causal);
+    MTA_LAUNCH_OK("softmax_bwd_kernel");
+    return MTA_OK;
+}
+
 }  // namespace
+
+int softmax_bwd_launch(const void* p, PlaneView pv, const void* g, PlaneView gv, void* ds, PlaneView dv, long planes, int P, int Q,
+                       int causal, int dtype, cudaStream_t st) {
+    if (planes == 0 || P == 0 || Q == 0) return MTA_OK;
+    MTA_REQUIRE(planes <= 65535, "softmax_bwd: N*C = %ld exceeds 65535", planes);
+    if (dtype == MTA_F32) return launch_bwd<float>(p, pv, g, gv, ds, dv, planes, P, Q, causal, st);
+    if (dtype == MTA_BF16) return launch_bwd<__nv_bfloat16>(p, pv, g, gv, ds, dv, planes, P, Q, causal, st);
+    return launch_bwd<__half>(p, pv, g, gv, ds, dv, planes, P, Q, causal, st);
+}
 
 int softmax_launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int P, int Q, int causal,
                    int row_begin, int row_end, bool write_upper, float pre_scale, int dtype, cudaStream_t st) {

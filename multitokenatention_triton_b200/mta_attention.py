@@ -5,7 +5,8 @@ parameter names (mta_conv_triton.weight, wpsm_triton.weight, mta_conv_after_sm_t
 wposm_triton.weight), reset_mta_parameters / copy_mta_parameters, and forward(xq, xk, xv, mask,
 chunk_start_ids) returning the (B,S,H,D) transpose view of a (B,H,S,D) tensor.
 
-`fused=True` (default) runs the whole forward through mta_fused_fwd.  `fused=False` runs the reference's
+`fused=True` (default) runs the whole forward through mta_fused_fwd, or through mta_train_fwd / mta_train_bwd when a
+gradient is needed (without dropout).  `fused=False` runs the reference's
 seven steps one by one through the stand-alone entry points, which keeps every 16-bit rounding point of
 the reference.  `use_mask=True` runs the reference's explicit-mask path (None, boolean, additive, padding or
 (1,1,S,S) masks) stage by stage over full score planes.
@@ -15,7 +16,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from .autograd_ops import CausalSoftmaxFunction, PVFunction, QKScoresFunction
+from .autograd_ops import CausalSoftmaxFunction, MTAFunction, PVFunction, QKScoresFunction
 from .convolution_2d import Conv2dTriton
 from .linear_head import TritonLinearHead
 
@@ -69,6 +70,9 @@ class MTAAttentionTriton(nn.Module):
                                     self.mta_conv_after_sm_triton.effective_weight(), self.wposm_triton.weight, causal=True,
                                     dropout_p=self.dropout if dropping else 0.0, dropout_seed=seed)
             return out.transpose(1, 2)
+        w1, w2 = self.mta_conv_triton.effective_weight(), self.mta_conv_after_sm_triton.effective_weight()
+        if self.fused and not dropping and xk.shape == xq.shape and xv.shape == xq.shape and w1.size(-1) % 2 and w2.size(-1) % 2:
+            return MTAFunction.apply(xq, xk, xv, w1, self.wpsm_triton.weight, w2, self.wposm_triton.weight).transpose(1, 2)
         # stage by stage; every stage is differentiable (the conv and the head mix through their backward kernels, the
         # scores, the softmax and the product with V through autograd_ops), so this is the path a training step uses
         head_dim = xq.size(-1)

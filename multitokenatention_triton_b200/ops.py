@@ -232,6 +232,47 @@ def mta_fused_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w1: torch.T
     return out
 
 
+def _mta_weights(q, w1, W1, w2, W2):
+    """The four weights as the library takes them: on the device, contiguous, of one dtype (the activations' or float32)."""
+    w = [_weight(w1, q, "conv weight"), _weight(W1, q, "head-mix weight"), _weight(w2, q, "post-softmax conv weight"),
+         _weight(W2, q, "post-softmax head-mix weight")]
+    return w if len({t.dtype for t in w}) == 1 else [t.float() for t in w]
+
+
+def mta_train_fwd(q, k, v, w1, W1, w2, W2) -> Tuple[torch.Tensor, torch.Tensor]:
+    """The causal MTA forward of a training step: (output (B,H,S,D), the score planes that mta_train_bwd reads)."""
+    q, k, v = _cuda_contig(q, "xq"), _cuda_contig(k, "xk"), _cuda_contig(v, "xv")
+    B, H, S, D = q.shape
+    assert k.shape == q.shape and v.shape == q.shape
+    w = _mta_weights(q, w1, W1, w2, W2)
+    out = torch.empty_like(q)
+    L = lib()
+    nbytes = L.mta_train_saved_bytes(B, H, S, dtype_code(q))
+    saved = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
+    with torch.cuda.device(q.device):
+        check(L.mta_train_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), *(t.data_ptr() for t in w), out.data_ptr(), saved.data_ptr(),
+                              saved.numel(), B, H, S, D, *w1.shape[1:], *w2.shape[1:], dtype_code(q), dtype_code(w[0]),
+                              stream_ptr(q.device)), "mta_train_fwd")
+    return out, saved
+
+
+def mta_train_bwd(grad_out, saved, q, k, v, w1, W1, w2, W2, needs) -> list:
+    """Gradients of (q, k, v, w1, W1, w2, W2) where `needs` says so (None elsewhere); those of the weights are float32."""
+    q, k, v, g = (_cuda_contig(q, "xq"), _cuda_contig(k, "xk"), _cuda_contig(v, "xv"), _cuda_contig(grad_out, "grad_output"))
+    B, H, S, D = q.shape
+    w = _mta_weights(q, w1, W1, w2, W2)
+    grads = [torch.empty_like(t) if n else None for t, n in zip((q, k, v), needs)]
+    grads += [torch.empty(t.shape, dtype=torch.float32, device=q.device) if n else None for t, n in zip(w, needs[3:])]
+    L = lib()
+    nbytes = L.mta_train_workspace_bytes(B, H, S, *w1.shape[1:], *w2.shape[1:], dtype_code(q))
+    ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
+    with torch.cuda.device(q.device):
+        check(L.mta_train_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), *(t.data_ptr() for t in w), g.data_ptr(), saved.data_ptr(),
+                              *(None if t is None else t.data_ptr() for t in grads), ws.data_ptr(), ws.numel(), B, H, S, D,
+                              *w1.shape[1:], *w2.shape[1:], dtype_code(q), dtype_code(w[0]), stream_ptr(q.device)), "mta_train_bwd")
+    return grads
+
+
 def mta_fused_fwd_host(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w1: torch.Tensor, W1: torch.Tensor,
                        w2: torch.Tensor, W2: torch.Tensor, causal: bool = True, out: Optional[torch.Tensor] = None,
                        chunk_batch: int = 0) -> torch.Tensor:

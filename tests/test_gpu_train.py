@@ -1,0 +1,79 @@
+"""The one-node training path (mta_train_fwd / mta_train_bwd) against autograd through a plain PyTorch evaluation in float64,
+at lengths around the tile edges, and the float32 score-plane products behind it."""
+import types
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from multitokenatention_triton_b200 import MTAAttentionTriton, _lib, ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def torch_mta(q, k, v, w1, W1, w2, W2):
+    S = q.size(-2)
+    dead = torch.ones(S, S, dtype=torch.bool, device=q.device).triu(1)
+
+    def conv(x, w):
+        p = (w.size(-1) - 1) // 2
+        return F.conv2d(F.pad(x.masked_fill(dead, 0.0), (p, p, w.size(-2) - 1, 0)), w.unsqueeze(1), groups=x.size(1))
+
+    s = conv(q @ k.transpose(2, 3) * q.size(-1) ** -0.5, w1)
+    s = torch.einsum("oh,bhqk->boqk", W1, s).masked_fill(dead, float("-inf")).softmax(-1)
+    s = torch.einsum("oh,bhqk->boqk", W2, conv(s, w2).masked_fill(dead, 0.0))
+    return (s @ v).transpose(1, 2)
+
+
+@pytest.mark.parametrize("S,H,D,ker,ker2,dtype", [
+    (1, 8, 64, (3, 5), (3, 3), torch.bfloat16), (127, 16, 128, (6, 11), (3, 3), torch.bfloat16),
+    (129, 8, 64, (2, 3), (6, 11), torch.float16), (200, 12, 64, (11, 15), (7, 9), torch.bfloat16),
+    (321, 16, 128, (6, 11), (6, 11), torch.float16), (67, 8, 32, (3, 5), (3, 3), torch.float32),
+    (130, 16, 64, (11, 15), (11, 15), torch.float32), (96, 64, 128, (5, 5), (3, 3), torch.bfloat16)])
+def test_training_step(S, H, D, ker, ker2, dtype):
+    cfg = types.SimpleNamespace(use_mta=True, query_kernel_size=ker[0], key_kernel_size=ker[1], after_sm_query_kernel_size=ker2[0],
+                                after_sm_key_kernel_size=ker2[1], pre_sm_linear_head=True, post_sm_linear_head=True, pad_key="both",
+                                init_method="identity", dim=H * D)
+    g = torch.Generator(device=DEV).manual_seed(S)
+    m = MTAAttentionTriton(H, cfg, dropout=0.0, causal=True).to(DEV, dtype)
+    with torch.no_grad():
+        for p in m.parameters():
+            if p.dim() == 2:
+                p.copy_(torch.eye(H, device=DEV) + 0.1 * torch.randn(H, H, device=DEV, generator=g))
+            else:
+                p.copy_(torch.randn(p.shape, device=DEV, generator=g) * (p[0].numel()) ** -0.5)
+                p[:, -1, p.shape[2] // 2] += 1.0
+    x = [torch.randn(2, H, S, D, device=DEV, generator=g).to(dtype).requires_grad_() for _ in range(3)]
+    up = torch.randn(2, S, H, D, device=DEV, generator=g).to(dtype)
+    out = m(*x, None, None)
+    out.backward(up)
+    _lib.device_status()
+    w = [m.mta_conv_triton.weight, m.wpsm_triton.weight, m.mta_conv_after_sm_triton.weight, m.wposm_triton.weight]
+    ref_in = [t.detach().double().requires_grad_() for t in x + w]
+    ref = torch_mta(*ref_in)
+    ref.backward(up.double())
+    tol = {torch.float32: 2e-5, torch.float16: 6e-3, torch.bfloat16: 4e-2}[dtype]
+    for name, got, want in zip(("out", "dq", "dk", "dv", "dw1", "dW1", "dw2", "dW2"), [out] + [t.grad for t in x + w],
+                               [ref] + [t.grad for t in ref_in]):
+        err = float((got.detach().double() - want.detach()).norm() / want.detach().norm().clamp_min(1e-30))
+        if S == 1 and name in ("dq", "dk", "dw1", "dW1"):       # a softmax over one key has no gradient
+            assert float(want.abs().max()) < 1e-12 and float(got.abs().max()) < 1e-2, name
+            continue
+        assert err <= tol, f"{name}: relative error {err:.3e}"
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("S,D", [(4, 8), (60, 100), (64, 64), (68, 128), (132, 36), (260, 128)])
+def test_float32_products(S, D, causal):
+    g = torch.Generator(device=DEV).manual_seed(S + D)
+    q, k, v = (torch.randn(2, 3, S, D, device=DEV, generator=g) for _ in range(3))
+    p = torch.rand(2, 3, S, S, device=DEV, generator=g)
+    mask = (lambda t: t.tril()) if causal else (lambda t: t)
+    s = ops.qk_scores_fwd(q, k, 0.25, causal)
+    assert torch.allclose(s.double(), mask(q.double() @ k.double().transpose(2, 3) * 0.25), atol=2e-5, rtol=1e-5)
+    pn = p.clone()
+    if causal:
+        pn.masked_fill_(torch.ones(S, S, dtype=torch.bool, device=DEV).triu(1), float("nan"))
+    o = ops.pv_fwd(pn, v, causal)
+    assert torch.allclose(o.double(), mask(p.double()) @ v.double(), atol=5e-5, rtol=1e-5)
