@@ -126,7 +126,7 @@ struct TileIter {
 // 0..15 onto block b1 for s = b1 + 1.  Per (row tap i, term) the k-steps b0+1, b0+3, ... come first: they touch every
 // owned block exactly once, so in the first batch they carry accumulate = 0.
 template <typename T, int ISSUER>
-__device__ __forceinline__ void issue_tile(uint32_t xa_addr, uint32_t d0, int R, int split_w, int box_bytes, int tb_off) {
+__device__ __forceinline__ void issue_tile(uint32_t xa_addr, uint32_t d0, int R, int split_w, int box_bytes, int tb_off, uint32_t el) {
     constexpr uint32_t idesc32 = instr_desc_f16(AbFmt<T>::value, 0, 0, TM, 32);
     constexpr uint32_t idesc16 = instr_desc_f16(AbFmt<T>::value, 0, 0, TM, 16);
     constexpr int b0 = issuer_block0(ISSUER), b1 = issuer_block0(ISSUER + 1) - 1;
@@ -152,7 +152,7 @@ __device__ __forceinline__ void issue_tile(uint32_t xa_addr, uint32_t d0, int R,
                     const uint64_t bdesc = db + (upper ? 16u : 0u);
                     const uint32_t dcol = upper ? 16u * (uint32_t)s : 16u * (uint32_t)(s - 1);
                     const uint32_t acc = (batch > 0 || pass > 0) ? 1u : 0u;
-                    mma_f16_ss(d0 + dcol, adesc, bdesc, (upper || lower) ? idesc16 : idesc32, acc);
+                    mma_f16_ss(d0 + dcol, adesc, bdesc, (upper || lower) ? idesc16 : idesc32, acc, el);
                 }
         }
 }
@@ -178,7 +178,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
     uint8_t* out_base = smem;                                  // 1024-byte aligned, as the swizzled TMA store needs
     uint8_t* zero_box = smem + 2 * OUT_BYTES;                 // 16 KB of zeros: source of the zero tiles above the diagonal
     uint8_t* stage_base = zero_box + TM * 128;                // then the stage ring
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int pad_w = (S - 1) / 2;
     const int pad8 = (pad_w + 7) & ~7;
     const int a_off = pad8 - pad_w;
@@ -281,23 +281,23 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
     } else if (warp == 1 || (warp == 8 && NISS >= 2)) {
         // ---------------- MMA issuers ----------------
         // Two threads issue, each onto its own output blocks, so no ordering between them is needed and none affects
-        // the result (measured at B8 H16 S4096, 6 x 11: one issuer 1.19 ms, two 0.94 ms, three 1.01 ms; the tensor pipe
-        // takes ~49 cycles per MMA, a single thread issues one per ~76).  The schedule of an issuer is compile-time (issue_tile<ISSUER>): every descriptor is the stage's
+        // the result.  With MMAs issued from uniform code (tc05.cuh) one issuer keeps up in this kernel (B4 H16 S2048 6x11: 186 us
+        // with one or two); in the two kernels that compute the scores themselves two are better (qk_conv B1 H16 S2048 7x7 fp16:
+        // 51 against 56 us; conv attention B8 H16 S4096 6x11: 1.21 against 1.24 ms).  The schedule of an issuer is compile-time (issue_tile<ISSUER>): every descriptor is the stage's
         // base descriptor plus a constant and a multiple of the row tap, all warp-uniform values.
+        const uint32_t el = elect_one();
         for (int n = 0; n < my_tiles; ++n) {
             const int st = n % NSTAGE, ab = n & 1;
             mbar_wait(&ready_bar[st], (n / NSTAGE) & 1, err_flag);
             mbar_wait(&acc_empty[ab], ((n >> 1) & 1) ^ 1, err_flag);
-            fence_after_sync();
-            if (lane == 0) {
-                const uint32_t xa_addr = smem_u32(stage_base + st * stage_bytes);
-                const uint32_t d0 = tmem + (uint32_t)(ab * TN);
-                if (warp == 1) issue_tile<T, 0>(xa_addr, d0, R, g.split_w, box_bytes, tb_off);
-                else issue_tile<T, NISS >= 2 ? 1 : 0>(xa_addr, d0, R, g.split_w, box_bytes, tb_off);
-                mma_commit(&empty_bar[st]);
-                mma_commit(&acc_full[ab]);
-            }
             __syncwarp();
+            fence_after_sync();
+            const uint32_t xa_addr = smem_u32(stage_base + st * stage_bytes);
+            const uint32_t d0 = tmem + (uint32_t)(ab * TN);
+            if (warp == 1) issue_tile<T, 0>(xa_addr, d0, R, g.split_w, box_bytes, tb_off, el);
+            else issue_tile<T, NISS >= 2 ? 1 : 0>(xa_addr, d0, R, g.split_w, box_bytes, tb_off, el);
+            mma_commit(&empty_bar[st], el);
+            mma_commit(&acc_full[ab], el);
         }
     } else if (warp == 8 || warp == 9) {
         // issuer warp that this build does not use

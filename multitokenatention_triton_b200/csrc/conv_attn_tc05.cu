@@ -83,7 +83,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     uint8_t* v_base = k_base + K_BYTES;
     uint8_t* stage_base = v_base + V_BYTES;        // NSTAGE staged tiles of TB_OFF bytes
     uint8_t* tb_base = stage_base + NSTAGE * TB_OFF;     // two sets of Toeplitz slices: units alternate between them
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int a_off = 8 - (KS - 1) / 2;
     const int lead = R - 1;
 
@@ -140,6 +140,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
         // read the buffer have completed, which is this thread's own commit.  The ring of staged tiles downstream
         // keeps the conv MMAs fed while a load is in flight.
         constexpr uint32_t idesc = instr_desc_f16(AbFmtQ<T>::value, 0, 0, TM, SN);
+        const uint32_t el = elect_one();
         int n = 0, un = 0;
         CA_FOR_UNITS
             mbar_wait(&q_free, (un & 1) ^ 1, err_flag);        // the previous unit's score MMAs have read its Q tile
@@ -160,24 +161,22 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 mbar_wait(&s_free, (n & 1) ^ 1, err_flag);       // the drain warps have read the previous score tile
                 __syncwarp();
                 fence_after_sync();
-                if (lane == 0) {
-                    const uint32_t qa = smem_u32(q_base), ka = smem_u32(k_base);
+                const uint32_t qa = smem_u32(q_base), ka = smem_u32(k_base);
 #pragma unroll
-                    for (int kk = 0; kk < D / 16; ++kk) {
-                        const uint32_t qoff = (kk / 4) * BOX_BYTES + (kk % 4) * 32, koff = (kk / 4) * KBOX_BYTES + (kk % 4) * 32;
-                        mma_f16_ss(tmem + S_COL, smem_desc_sw128(qa + qoff, 16, 1024), smem_desc_sw128(ka + koff, 16, 1024), idesc,
-                                   kk > 0 ? 1u : 0u);
-                    }
-                    mma_commit(&k_free);
-                    mma_commit(&s_full);
-                    if (tn == nk - 1) mma_commit(&q_free);
+                for (int kk = 0; kk < D / 16; ++kk) {
+                    const uint32_t qoff = (kk / 4) * BOX_BYTES + (kk % 4) * 32, koff = (kk / 4) * KBOX_BYTES + (kk % 4) * 32;
+                    mma_f16_ss(tmem + S_COL, smem_desc_sw128(qa + qoff, 16, 1024), smem_desc_sw128(ka + koff, 16, 1024), idesc,
+                               kk > 0 ? 1u : 0u, el);
                 }
-                __syncwarp();
+                mma_commit(&k_free, el);
+                mma_commit(&s_full, el);
+                if (tn == nk - 1) mma_commit(&q_free, el);
             }
             ++un;
         }
     } else if (warp == 2 || warp == 3) {
         // ---------------- conv MMAs ----------------
+        const uint32_t el = elect_one();
         int n = 0, un = 0;
         CA_FOR_UNITS
             const uint32_t tb_addr = smem_u32(tb_base + (un & 1) * tb_bytes);
@@ -185,15 +184,13 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 const int st = n % NSTAGE;
                 mbar_wait_spin(&ready_bar[st], (n / NSTAGE) & 1, err_flag);
                 mbar_wait_spin(&acc_empty, (n & 1) ^ 1, err_flag);    // the softmax warps have read the previous conv tile
-                fence_after_sync();
-                if (lane == 0) {
-                    const uint32_t xa_addr = smem_u32(stage_base + st * TB_OFF);
-                    if (warp == 2) issue_conv<T, 0>(xa_addr, tb_addr, tmem + C_COL, R, g.split_w);
-                    else issue_conv<T, 1>(xa_addr, tb_addr, tmem + C_COL, R, g.split_w);
-                    mma_commit(&empty_bar[st]);
-                    mma_commit(&acc_full);
-                }
                 __syncwarp();
+                fence_after_sync();
+                const uint32_t xa_addr = smem_u32(stage_base + st * TB_OFF);
+                if (warp == 2) issue_conv<T, 0>(xa_addr, tb_addr, tmem + C_COL, R, g.split_w, el);
+                else issue_conv<T, 1>(xa_addr, tb_addr, tmem + C_COL, R, g.split_w, el);
+                mma_commit(&empty_bar[st], el);
+                mma_commit(&acc_full, el);
             }
             ++un;
         }
@@ -355,6 +352,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     } else {
         // ---------------- (warp 1) V loads and P.V MMAs: O[128 x D] (+)= P[128 x 128] V[128 x D] ----------------
         constexpr uint32_t idesc = instr_desc_f16(AbFmtQ<T>::value, 0, 1, TM, D);
+        const uint32_t el = elect_one();
         int n = 0;
         CA_FOR_UNITS
             for (int tn = 0; tn < nk; ++tn, ++n) {
@@ -368,16 +366,13 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 mbar_wait(&v_full, n & 1, err_flag);
                 __syncwarp();
                 fence_after_sync();
-                if (lane == 0) {
-                    const uint32_t va = smem_u32(v_base);
+                const uint32_t va = smem_u32(v_base);
 #pragma unroll
-                    for (int kk = 0; kk < TN / 16; ++kk) {
-                        const uint64_t db = smem_desc_sw128(va + kk * 16 * 128, VBOX_BYTES, 1024);
-                        mma_f16_ts(tmem + O_COL, tmem + P_COL + (uint32_t)(kk * 8), db, idesc, (tn > 0 || kk > 0) ? 1u : 0u);
-                    }
-                    mma_commit(&pv_done);
+                for (int kk = 0; kk < TN / 16; ++kk) {
+                    const uint64_t db = smem_desc_sw128(va + kk * 16 * 128, VBOX_BYTES, 1024);
+                    mma_f16_ts(tmem + O_COL, tmem + P_COL + (uint32_t)(kk * 8), db, idesc, (tn > 0 || kk > 0) ? 1u : 0u, el);
                 }
-                __syncwarp();
+                mma_commit(&pv_done, el);
             }
         }
     }

@@ -8,9 +8,9 @@
 // its source bytes, which is how the causal edge and the ends of the tensors become zeros.  For QK the groups are a 2 x 2
 // block of output tiles.  For PV and PT, whose contraction is as long as the sequence while the output is D wide, they share
 // one output tile and take every fourth block: four times the parallelism for the few heavy tiles; the partial tiles are
-// added in group order, so a row's sum depends only on which index lies in which block.  The heaviest tiles of all planes
-// are launched first (planes along grid x).
+// added in group order, so a row's sum depends only on which index lies in which block.
 // The accumulators are packed pairs of columns: the packed FMA needs half the issue slots, which the operand loads then use.
+// Measured at B1 H16 S2048 D64: P V 115 us (the general kernel: 532), Q K^T 131 us (183); the FMAs alone would take 64.
 #include "kernels.cuh"
 
 namespace mta {
@@ -22,6 +22,7 @@ constexpr int GROUPS = 4;
 constexpr int GTHREADS = 64;
 constexpr int THREADS = GROUPS * GTHREADS;
 constexpr int NST = 3;               // ring depth
+constexpr int PLANE_GROUP = 16;
 constexpr int KPITCH = BK + 4;       // row pitch of an operand staged [row][index]: four rows of a warp land in different banks
 constexpr int OPER_K = BT * KPITCH;  // floats of an operand staged [row][index]
 constexpr int OPER_N = BK * BT;      // floats of an operand staged [index][row]
@@ -150,12 +151,15 @@ qk_f32_kernel(const float* __restrict__ q, const float* __restrict__ k, float* _
 
 template <Kind KIND>
 __global__ void __launch_bounds__(THREADS, 2)
-pv_f32_kernel(const float* __restrict__ p, PlaneView pv, const float* __restrict__ v, float* __restrict__ o, int S, int D, int causal,
-              int row_begin, int row_end, int tiles_d, float scale) {
+pv_f32_kernel(const float* __restrict__ p, PlaneView pv, const float* __restrict__ v, float* __restrict__ o, int planes, int S, int D,
+              int causal, int row_begin, int row_end, int tiles_d, float scale) {
     extern __shared__ __align__(16) float smem[];
-    const long bh = blockIdx.x;
+    // heaviest tiles first over groups of planes (as in gemm_tc05.cu: few enough for their V to stay in L2)
     const int n_q = (row_end - row_begin + BT - 1) / BT;
-    const int tq = KIND == PT ? (int)blockIdx.y / tiles_d : n_q - 1 - (int)blockIdx.y / tiles_d, td = blockIdx.y % tiles_d;   // heaviest first
+    const int per_group = n_q * tiles_d * PLANE_GROUP, in_group = (int)(blockIdx.x % per_group), p0 = (int)(blockIdx.x / per_group) * PLANE_GROUP;
+    const int width = min(PLANE_GROUP, planes - p0);
+    const long bh = p0 + in_group % width;
+    const int t = in_group / width / tiles_d, td = in_group / width % tiles_d, tq = KIND == PT ? t : n_q - 1 - t;
     const int q0 = row_begin + tq * BT, d0 = td * BT;
     const int q_end = min(q0 + BT, row_end);
     // contraction indices [c_lo, c_hi), c_lo a multiple of BK
@@ -261,8 +265,8 @@ int launch_pv(const float* p, PlaneView pview, const float* v, float* o, int B, 
               float scale, cudaStream_t st) {
     const int tiles_q = (row_end - row_begin + BT - 1) / BT, tiles_d = (D + BT - 1) / BT;
     MTA_CUDA_OK(cudaFuncSetAttribute(pv_f32_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(KIND)));
-    pv_f32_kernel<KIND><<<dim3((unsigned)(B * H), (unsigned)(tiles_q * tiles_d)), THREADS, smem_bytes(KIND), st>>>(
-        p, pview, v, o, S, D, causal, row_begin, row_end, tiles_d, scale);
+    pv_f32_kernel<KIND><<<(unsigned)(B * H * tiles_q * tiles_d), THREADS, smem_bytes(KIND), st>>>(
+        p, pview, v, o, B * H, S, D, causal, row_begin, row_end, tiles_d, scale);
     MTA_LAUNCH_OK("pv_f32_kernel");
     return MTA_OK;
 }

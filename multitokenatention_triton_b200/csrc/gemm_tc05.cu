@@ -170,6 +170,7 @@ constexpr int PV_THREADS = 192;
 constexpr int PV_KEYS = 64;               // contraction indices per pipeline stage: 32 KB stages, so two CTAs fit on an SM and
                                           // one CTA's start-up and epilogue overlap the other's steady state
 constexpr int PV_VBOX_BYTES = PV_KEYS * 128;   // one box of the V tile: 64 rows x 64 elements
+constexpr int PV_PLANE_GROUP = 16;
 constexpr int PV_DIAG = 3;                // most steps of a tile that straddle the diagonal (128 rows from any row on)
 
 // DROP: the dropout of dropout.cuh is applied to every P tile in shared memory before its MMAs (a thread owns a row).
@@ -177,7 +178,7 @@ constexpr int PV_DIAG = 3;                // most steps of a tile that straddle 
 template <typename T, int D, bool DROP, bool TRANS>
 __global__ void __launch_bounds__(PV_THREADS)
 pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ CUtensorMap mv, T* __restrict__ o,
-               int p_row0, int S, int causal, int row_begin, int row_end, float scale, int* err_flag, DropoutSpec drop) {
+               int planes, int p_row0, int S, int causal, int row_begin, int row_end, float scale, int* err_flag, DropoutSpec drop) {
     constexpr int NBOX_V = D / 64;
     constexpr int P_BYTES = BOX_BYTES;                     // 128 q x 64 k, or 64 q x 128 k
     constexpr int V_BYTES = NBOX_V * PV_VBOX_BYTES;        // 64 rows x D
@@ -192,10 +193,14 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
     if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
     __syncthreads();
     if (abort_flag != 0) return;
-    // heaviest tiles first: the last query tile (all keys), or the first key tile (all queries)
+    // Heaviest tiles first (the last query tile has all keys, or the first key tile all queries), over groups of planes: plane by
+    // plane, the last planes' heavy tiles start when little else is left (B1 H16 S2048: 30 us against 25); all planes at once,
+    // the V tiles of 128 planes do not stay in L2 (B8 H16 S4096: 549 us against 441).
     const int n_qt = (row_end - row_begin + TILE - 1) / TILE;
-    const int tq = TRANS ? (int)blockIdx.y : n_qt - 1 - (int)blockIdx.y;
-    const int bh = (int)blockIdx.x;
+    const int per_group = n_qt * PV_PLANE_GROUP, group = (int)blockIdx.x / per_group, in_group = (int)blockIdx.x % per_group;
+    const int width = min(PV_PLANE_GROUP, planes - group * PV_PLANE_GROUP);
+    const int bh = group * PV_PLANE_GROUP + in_group % width, t = in_group / width;
+    const int tq = TRANS ? t : n_qt - 1 - t;
     const int q0 = row_begin + tq * TILE;                  // first output row (a query, or a key when TRANS)
     const int q_end = min(q0 + TILE, row_end);
     // steps [kt0, kt1) of 64 contraction indices: keys up to the tile's last query, or queries from the tile's first key on
@@ -206,7 +211,7 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
     const int d0 = !causal ? kt1 : (TRANS ? kt0 : min((q0 + 1) / PV_KEYS, kt1));
     const int d1 = !causal ? kt1 : (TRANS ? min((q0 + TILE - 2) / PV_KEYS + 1, kt1) : kt1);
     const int nk = kt1 - kt0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -252,6 +257,7 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
         }
     } else if (warp == 1) {
         constexpr uint32_t idesc = instr_desc_f16(AbFormat<T>::value, TRANS ? 1 : 0, 1, TILE, D);
+        const uint32_t el = elect_one();
         for (int it = 0; it < nk; ++it) {
             const int kt = kt0 + it, st = it % PV_STAGES, use = it / PV_STAGES;
             uint8_t* sp = smem + st * STAGE_BYTES;
@@ -264,19 +270,17 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
                 if (!DROP && lane == 0) mbar_arrive(&go_bar[kt - d0]);
                 mbar_wait_spin(&diag_bar[kt - d0], 0, err_flag);
             }
-            fence_after_sync();
-            if (lane == 0) {
-#pragma unroll
-                for (int kk = 0; kk < PV_KEYS / 16; ++kk) {
-                    const uint64_t da = TRANS ? smem_desc_sw128(smem_u32(sp) + kk * 16 * 128, P_BYTES / 2, 1024)
-                                              : smem_desc_sw128(smem_u32(sp) + kk * 32, 16, 1024);
-                    const uint64_t db = smem_desc_sw128(smem_u32(sv) + kk * 16 * 128, PV_VBOX_BYTES, 1024);
-                    mma_f16_ss(tmem, da, db, idesc, (it > 0 || kk > 0) ? 1u : 0u);
-                }
-                mma_commit(&empty_bar[st]);
-                if (it == nk - 1) mma_commit(&acc_bar);
-            }
             __syncwarp();
+            fence_after_sync();
+#pragma unroll
+            for (int kk = 0; kk < PV_KEYS / 16; ++kk) {
+                const uint64_t da = TRANS ? smem_desc_sw128(smem_u32(sp) + kk * 16 * 128, P_BYTES / 2, 1024)
+                                          : smem_desc_sw128(smem_u32(sp) + kk * 32, 16, 1024);
+                const uint64_t db = smem_desc_sw128(smem_u32(sv) + kk * 16 * 128, PV_VBOX_BYTES, 1024);
+                mma_f16_ss(tmem, da, db, idesc, (it > 0 || kk > 0) ? 1u : 0u, el);
+            }
+            mma_commit(&empty_bar[st], el);
+            if (it == nk - 1) mma_commit(&acc_bar, el);
         }
     } else {
         const int et = (int)threadIdx.x - 64;                // 0..127
@@ -366,10 +370,10 @@ int launch_pv(const void* p, PlaneView pview, const void* v, void* o, int B, int
     if ((rc = wait_flag_ptr(&flag))) return rc;
     const int n_qt = (row_end - row_begin + TILE - 1) / TILE;
     const size_t smem = (size_t)PV_STAGES * (BOX_BYTES + (D / 64) * PV_VBOX_BYTES) + 1024;
-    dim3 grid((unsigned)(B * H), (unsigned)n_qt);      // planes along x: the heaviest tiles of ALL planes come first
+    const unsigned grid = (unsigned)(B * H * n_qt);
     auto kernel = pv_tc05_kernel<T, D, DROP, TRANS>;
     MTA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, PV_THREADS, smem, st>>>(mp, mv, static_cast<T*>(o), pview.row0, S, causal, row_begin, row_end, scale, flag, drop);
+    kernel<<<grid, PV_THREADS, smem, st>>>(mp, mv, static_cast<T*>(o), B * H, pview.row0, S, causal, row_begin, row_end, scale, flag, drop);
     MTA_LAUNCH_OK("pv_tc05_kernel");
     return MTA_OK;
 }

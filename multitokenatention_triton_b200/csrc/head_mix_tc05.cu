@@ -221,7 +221,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
     uint8_t* out_base = stage_base + HM_NSTAGE * HM_STAGE_BYTES;      // HM_NACC staging buffers of HM_OUT_BYTES
     uint8_t* fill_base = out_base + HM_NACC * HM_OUT_BYTES;           // one more, holding `fill` (0 for the softmax) everywhere
     constexpr int PASSES = SOFTMAX ? 2 : 1;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int C = g.C, R = g.R;
 
     if (tid == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
@@ -303,9 +303,10 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
             }
         }
     } else if (warp <= HM_ISSUERS) {
-        // Two issuers take alternate tiles (a thread issues an MMA every ~75 cycles, 8 MMAs a tile would be the kernel's pace).
+        // Two issuers take alternate tiles .
         constexpr uint32_t idesc = instr_desc_f16(AbFmtH<T>::value, 0, 1, 128, HM_KEYS);
         const uint32_t a_addr = smem_u32(a_base);
+        const uint32_t el = elect_one();
         const int issuer = warp - 1;
         int it = 0;
         bool ok = true;
@@ -343,18 +344,18 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                 __syncwarp();
                 if (ok && au > 0) ok = mbar_wait_spin(&acc_empty[ab], (uint32_t)((au - 1) & 1), err_flag);
                 fence_after_sync();
-                if (lane == 0 && ok) {
+                ok = __all_sync(0xffffffffu, ok);
+                if (ok) {
                     const uint32_t b_addr = smem_u32(sb);
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk) {
                         const uint64_t da = smem_desc_sw128(a_addr + (kk >> 2) * HM_BOX_BYTES + (kk & 3) * 32, 16, 1024);
                         const uint64_t db = smem_desc_sw128(b_addr + kk * 16 * 128, HM_BOX_BYTES, 1024);
-                        mma_f16_ss(tmem + (uint32_t)(ab * HM_KEYS), da, db, idesc, kk > 0 ? 1u : 0u);
+                        mma_f16_ss(tmem + (uint32_t)(ab * HM_KEYS), da, db, idesc, kk > 0 ? 1u : 0u, el);
                     }
-                    mma_commit(&empty_bar[st]);
-                    mma_commit(&acc_full[ab]);
+                    mma_commit(&empty_bar[st], el);
+                    mma_commit(&acc_full[ab], el);
                 }
-                __syncwarp();
             }
             if (!ok) break;
         }

@@ -90,7 +90,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
     uint8_t* k_base = q_base + Q_BYTES;                        // one K tile: the ring of staged tiles hides its reload
     uint8_t* stage_base = k_base + K_BYTES;                    // NSTAGE staged tiles of TB_OFF bytes
     uint8_t* tb_base = stage_base + NSTAGE * TB_OFF;           // two sets of Toeplitz slices: successive heads alternate
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int pad_w = (KS - 1) / 2;
     const int a_off = 8 - pad_w;
     const int lead = R - 1;
@@ -159,6 +159,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
     } else if (warp == 1) {
         // ---------------- score MMAs: S[128 x 144] = Q K^T into TMEM columns S_COL.. ----------------
         constexpr uint32_t idesc = instr_desc_f16(AbFmtQ<T>::value, 0, 0, TM, SN);
+        const uint32_t el = elect_one();
         QcIter it;
         it.init(g, t_begin);
         bool new_q = true;
@@ -170,26 +171,25 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
             }
             mbar_wait(&k_full, n & 1, err_flag);
             mbar_wait(&s_free, (n & 1) ^ 1, err_flag);           // the drain warps have read the previous score tile
+            __syncwarp();
             fence_after_sync();
             new_q = it.next(g);
-            if (lane == 0) {
-                const uint32_t qa = smem_u32(q_base), ka = smem_u32(k_base);
+            const uint32_t qa = smem_u32(q_base), ka = smem_u32(k_base);
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t qoff = (kk / 4) * BOX_BYTES + (kk % 4) * 32, koff = (kk / 4) * KBOX_BYTES + (kk % 4) * 32;
-                    mma_f16_ss(tmem + S_COL, smem_desc_sw128(qa + qoff, 16, 1024), smem_desc_sw128(ka + koff, 16, 1024), idesc,
-                               kk > 0 ? 1u : 0u);
-                }
-                mma_commit(&k_free);
-                mma_commit(&s_full);
-                if (new_q || n == my_tiles - 1) mma_commit(&q_free);     // last tile of this row of tiles
+            for (int kk = 0; kk < D / 16; ++kk) {
+                const uint32_t qoff = (kk / 4) * BOX_BYTES + (kk % 4) * 32, koff = (kk / 4) * KBOX_BYTES + (kk % 4) * 32;
+                mma_f16_ss(tmem + S_COL, smem_desc_sw128(qa + qoff, 16, 1024), smem_desc_sw128(ka + koff, 16, 1024), idesc,
+                           kk > 0 ? 1u : 0u, el);
             }
-            __syncwarp();
+            mma_commit(&k_free, el);
+            mma_commit(&s_full, el);
+            if (new_q || n == my_tiles - 1) mma_commit(&q_free, el);     // last tile of this row of tiles
         }
     } else if (warp == 2 || warp == 3) {
         // ---------------- conv MMAs ----------------
         QcIter it;
         it.init(g, t_begin);
+        const uint32_t el = elect_one();
         int cur_head = -1, hn = -1;                          // the running head and how many times it has changed
         for (int n = 0; n < my_tiles; ++n, it.next(g)) {
             const int st = n % NSTAGE, ab = n & 1;
@@ -197,17 +197,15 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
             if (head != cur_head) { cur_head = head; ++hn; }
             mbar_wait(&ready_bar[st], (n / NSTAGE) & 1, err_flag);
             mbar_wait(&acc_empty[ab], ((n >> 1) & 1) ^ 1, err_flag);
-            fence_after_sync();
-            if (lane == 0) {
-                const uint32_t xa_addr = smem_u32(stage_base + st * TB_OFF);
-                const uint32_t tb_addr = smem_u32(tb_base + (hn & 1) * tb_bytes);
-                const uint32_t d0 = tmem + (uint32_t)(ab * TN);
-                if (warp == 2) issue_conv<T, 0>(xa_addr, tb_addr, d0, R, g.split_w);
-                else issue_conv<T, 1>(xa_addr, tb_addr, d0, R, g.split_w);
-                mma_commit(&empty_bar[st]);
-                mma_commit(&acc_full[ab]);
-            }
             __syncwarp();
+            fence_after_sync();
+            const uint32_t xa_addr = smem_u32(stage_base + st * TB_OFF);
+            const uint32_t tb_addr = smem_u32(tb_base + (hn & 1) * tb_bytes);
+            const uint32_t d0 = tmem + (uint32_t)(ab * TN);
+            if (warp == 2) issue_conv<T, 0>(xa_addr, tb_addr, d0, R, g.split_w, el);
+            else issue_conv<T, 1>(xa_addr, tb_addr, d0, R, g.split_w, el);
+            mma_commit(&empty_bar[st], el);
+            mma_commit(&acc_full[ab], el);
         }
     } else if (warp < 8) {
         // ---------------- drain: score tile TMEM -> rounded, scaled, masked -> staged tile; Toeplitz slices ----------------
@@ -235,9 +233,9 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
             mbar_wait(&s_full, n & 1, err_flag);
             __syncwarp();
             fence_after_sync();
-            // The causal comparison runs on every tile, also those wholly below the diagonal (measured: skipping it there
-            // made an earlier two-stage version of this kernel slower, because the drain's shared-memory stores then came
-            // in denser bursts and held up the operand reads of the conv MMAs).
+            // The causal comparison runs on every tile, also those wholly below the diagonal (measured: skipping it there makes
+            // the kernel slower - B8 H16 S4096 1.44 against 1.32 ms, B1 H16 S2048 7x7 57 against 51 us - because the drain's
+            // shared-memory stores then come in denser bursts and hold up the operand reads of the conv MMAs).
             drain_row<T, true>(tmem + ((uint32_t)(quarter * 32) << 16) + S_COL, smem_u32(xa), sr, m0 - lead + sr, n0 - 8, sc, true);
             fence_before_sync();
             fence_proxy_async();          // generic-proxy writes above must be visible to the MMAs (async proxy)

@@ -102,7 +102,7 @@ qk_persistent_kernel(const __grid_constant__ CUtensorMap ma, const __grid_consta
     __shared__ __align__(8) uint64_t full_bar[4], empty_bar[4], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int NST = g.nstage, NI = g.NI;
 
     const long per = (g.total + gridDim.x - 1) / gridDim.x;
@@ -162,6 +162,7 @@ qk_persistent_kernel(const __grid_constant__ CUtensorMap ma, const __grid_consta
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         constexpr uint32_t idesc = instr_desc_f16(AbF<T>::value, 0, 0, TILE, TILE);
+        const uint32_t el = elect_one();
         int f = 0;
         for (int n = 0; n < my_tiles; ++n) {
             const int ab = n & 1;
@@ -169,19 +170,17 @@ qk_persistent_kernel(const __grid_constant__ CUtensorMap ma, const __grid_consta
             for (int i = 0; i < NI; ++i, ++f) {
                 const int st = f % NST;
                 mbar_wait(&full_bar[st], (f / NST) & 1, err_flag);
-                fence_after_sync();
-                if (lane == 0) {
-                    const uint32_t sa = smem_u32(stage_base + st * STAGE_BYTES), sb = sa + OPER_BYTES;
-#pragma unroll
-                    for (int kk = 0; kk < D / 16; ++kk) {
-                        const uint32_t off = (kk / 4) * BOX_BYTES + (kk % 4) * 32;
-                        mma_f16_ss(tmem + (uint32_t)(ab * TILE), smem_desc_sw128(sa + off, 16, 1024),
-                                   smem_desc_sw128(sb + off, 16, 1024), idesc, (i > 0 || kk > 0) ? 1u : 0u);
-                    }
-                    mma_commit(&empty_bar[st]);
-                    if (i == NI - 1) mma_commit(&acc_full[ab]);
-                }
                 __syncwarp();
+                fence_after_sync();
+                const uint32_t sa = smem_u32(stage_base + st * STAGE_BYTES), sb = sa + OPER_BYTES;
+#pragma unroll
+                for (int kk = 0; kk < D / 16; ++kk) {
+                    const uint32_t off = (kk / 4) * BOX_BYTES + (kk % 4) * 32;
+                    mma_f16_ss(tmem + (uint32_t)(ab * TILE), smem_desc_sw128(sa + off, 16, 1024), smem_desc_sw128(sb + off, 16, 1024), idesc,
+                               (i > 0 || kk > 0) ? 1u : 0u, el);
+                }
+                mma_commit(&empty_bar[st], el);
+                if (i == NI - 1) mma_commit(&acc_full[ab], el);
             }
         }
     } else {

@@ -19,14 +19,14 @@ constexpr uint32_t WAIT_LIMIT = 1u << 20;     // polls of mbarrier.try_wait (eac
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ bool elect_one() {
+__device__ __forceinline__ uint32_t elect_one() {
     uint32_t pred = 0;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "elect.sync _|p, 0xffffffff;\n\t"
         "selp.b32 %0, 1, 0, p;\n\t}\n"
         : "=r"(pred));
-    return pred != 0;
+    return pred;
 }
 
 // ---- mbarrier ------------------------------------------------------------------------------------
@@ -189,28 +189,41 @@ __host__ __device__ constexpr uint32_t instr_desc_f16(int ab_format, int a_mn_ma
            ((uint32_t)b_mn_major << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by one thread.  No "memory" clobber: the instruction is ordered against the
-// barriers and fences around it because all of them are volatile asm statements, and a clobber would stop the
-// compiler from overlapping the issuing thread's own loads with the MMAs it issues.
-__device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// Index of the calling warp in its CTA, in a form the compiler knows to be the same for the whole warp.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
+// D[tmem] (+)= A[smem] * B[smem].  Called by a whole warp, executed by the thread whose `el` is 1 (from elect_one(), the same
+// thread for everything that one commit covers).  The instruction takes its descriptors from uniform registers: when it sits
+// in code that only one lane enters (if (lane == 0)), every operand has to be moved there first and one thread issues an MMA
+// per ~75 to 113 cycles, which was the pace of the conv kernels; predicated inside warp-uniform code it issues several times
+// faster (conv2d_dw_tc05_kernel with one issuer, B4 H16 S2048 6x11: 225 -> 148 us).
+// No "memory" clobber: the instruction is ordered against the barriers and fences around it because all of them are volatile
+// asm statements, and a clobber would stop the compiler from overlapping the warp's own loads with the MMAs it issues.
+__device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t el) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate));
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(el));
 }
 // The same with the A operand in tensor memory: row r of A in lane r, the 16 contraction elements of one MMA packed two
 // per 32-bit column in 8 consecutive columns starting at tmem_a (element 2j in the low half of column j).
-__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t el) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate));
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(el));
 }
-// Arrive on `bar` once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+// Arrive on `bar` once every MMA issued so far by the elected thread has completed.
+__device__ __forceinline__ void mma_commit(uint64_t* bar, uint32_t el) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar)), "r"(el)
+        : "memory");
 }
 
 // 32 lanes x 32 consecutive fp32 columns: lane i of the warp receives row (lane base + i).

@@ -55,7 +55,7 @@ __host__ __device__ inline int stage_bytes(int R, int split_w) { return TB_OFF +
 // conv2d_tc05.cu over a staged tile at shared-memory address xa_addr with the Toeplitz slices at tb_addr, accumulating
 // into TMEM columns d0 .. d0 + 127.
 template <typename T, int ISSUER>
-__device__ __forceinline__ void issue_conv(uint32_t xa_addr, uint32_t tb_addr, uint32_t d0, int R, int split_w) {
+__device__ __forceinline__ void issue_conv(uint32_t xa_addr, uint32_t tb_addr, uint32_t d0, int R, int split_w, uint32_t el) {
     constexpr uint32_t idesc32 = instr_desc_f16(AbFmtQ<T>::value, 0, 0, TM, 32);
     constexpr uint32_t idesc16 = instr_desc_f16(AbFmtQ<T>::value, 0, 0, TM, 16);
     constexpr int b0 = ISSUER == 0 ? 0 : 4, b1 = ISSUER == 0 ? 3 : 7;
@@ -80,7 +80,7 @@ __device__ __forceinline__ void issue_conv(uint32_t xa_addr, uint32_t tb_addr, u
                     const uint64_t bdesc = db + (upper ? 16u : 0u);
                     const uint32_t dcol = upper ? 16u * (uint32_t)s : 16u * (uint32_t)(s - 1);
                     const uint32_t acc = (batch > 0 || pass > 0) ? 1u : 0u;
-                    mma_f16_ss(d0 + dcol, adesc, bdesc, (upper || lower) ? idesc16 : idesc32, acc);
+                    mma_f16_ss(d0 + dcol, adesc, bdesc, (upper || lower) ? idesc16 : idesc32, acc, el);
                 }
         }
 }
