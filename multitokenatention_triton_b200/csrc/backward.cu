@@ -10,6 +10,8 @@
 // Both reduce over every position of every plane.  The reference accumulates with floating-point atomics; here each
 // CTA writes its partial sums to a workspace and a second kernel adds them in a fixed order in double precision, so
 // the result does not depend on scheduling.
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace mta {
@@ -317,7 +319,7 @@ int dispatch_hw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, floa
 
 size_t conv2d_bwd_weight_workspace(int N, int C, int H, int W, int R, int S) {
     const long tiles = (long)((H + WT_M - 1) / WT_M) * ((W + WT_N - 1) / WT_N);
-    return (size_t)N * C * tiles * R * S * sizeof(float);
+    return std::max((size_t)N * C * tiles * R * S * sizeof(float), conv2d_dw_tc05_workspace(N, C, H, W, R, S));
 }
 
 int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dw, void* workspace, int N, int C, int H,
@@ -326,10 +328,13 @@ int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneV
     const long planes = (long)N * C;
     MTA_REQUIRE(planes <= 65535, "conv2d_bwd_weight: N*C = %ld exceeds 65535", planes);
     const int taps = R * S;
+    float* partial = static_cast<float*>(workspace);
+    // 16-bit dtypes with aligned rows: tensor cores (mta_set_variant("conv2d", 1): CUDA cores)
+    if (variant("conv2d") != 1 && conv2d_dw_tc05_supported(x, xv, dy, dyv, R, S, dtype))
+        return conv2d_dw_tc05_launch(x, xv, dy, dyv, dw, workspace, N, C, H, W, R, S, causal, dtype, st);
     // rows padded to a multiple of 4 floats, plus slack for the last window's 16-byte over-read
     const size_t smem = ((size_t)(WT_M + R - 1) * ((WT_N + S - 1 + 3) & ~3) + 8 + (size_t)(WT_THREADS / 32) * taps) * sizeof(float);
     MTA_REQUIRE(smem <= 200 * 1024, "conv2d_bwd_weight: kernel %dx%d needs %zu bytes of shared memory (max 204800)", R, S, smem);
-    float* partial = static_cast<float*>(workspace);
     dim3 grid((unsigned)(tiles_m * tiles_n), (unsigned)planes);
 #define MTA_BW_LAUNCH(TT, SCV)                                                                                           \
     do {                                                                                                                 \

@@ -33,6 +33,11 @@ int conv2d_bwd_input_launch(const void* dy, PlaneView dyv, const void* w, int w_
 size_t conv2d_bwd_weight_workspace(int N, int C, int H, int W, int R, int S);
 int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dw, void* workspace, int N, int C, int H,
                              int W, int R, int S, int causal, int dtype, cudaStream_t st);
+// The conv's weight gradient on tcgen05 (conv2d_dw_tc05.cu).
+bool conv2d_dw_tc05_supported(const void* x, PlaneView xv, const void* dy, PlaneView dyv, int R, int S, int dtype);
+size_t conv2d_dw_tc05_workspace(int N, int C, int H, int W, int R, int S);
+int conv2d_dw_tc05_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dw, void* workspace, int N, int C, int H, int W,
+                          int R, int S, int causal, int dtype, cudaStream_t st);
 size_t head_linear_bwd_weight_workspace(int C);
 int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dW, void* workspace, int N, int C,
                                   int P, int Q, int causal, int dtype, cudaStream_t st);

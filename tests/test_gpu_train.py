@@ -77,3 +77,25 @@ def test_float32_products(S, D, causal):
         pn.masked_fill_(torch.ones(S, S, dtype=torch.bool, device=DEV).triu(1), float("nan"))
     o = ops.pv_fwd(pn, v, causal)
     assert torch.allclose(o.double(), mask(p.double()) @ v.double(), atol=5e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("H,W,R,S,dtype", [(8, 8, 1, 1, torch.bfloat16), (127, 120, 6, 11, torch.float16), (128, 96, 2, 16, torch.bfloat16),
+                                           (129, 136, 7, 17, torch.bfloat16), (260, 48, 16, 15, torch.float16), (64, 328, 20, 3, torch.bfloat16),
+                                           (640, 640, 11, 15, torch.bfloat16)])
+def test_conv_weight_gradient_tensor_cores(H, W, R, S, dtype, causal):
+    """Planes around the 128-row, 48-key step, odd and even tap counts, several flushes; NaN above the diagonal."""
+    g = torch.Generator(device=DEV).manual_seed(H + W)
+    x, dy = (torch.randn(2, 3, H, W, device=DEV, generator=g).to(dtype) for _ in range(2))
+    dead = torch.arange(W, device=DEV)[None, :] > torch.arange(H, device=DEV)[:, None]
+    xr, dr = x.double(), dy.double()
+    if causal:
+        xr, dr = xr.masked_fill(dead, 0.0), dr.masked_fill(dead, 0.0)
+        x, dy = x.masked_fill(dead, float("nan")), dy.masked_fill(dead, float("nan"))
+    got = ops.conv2d_bwd_weight(x, dy, (R, S), causal)
+    _lib.device_status()
+    pad = (S - 1) // 2
+    xp = F.pad(xr, (pad, S - 1 - pad, R - 1, 0))
+    want = torch.stack([torch.stack([(xp[:, :, i:i + H, j:j + W] * dr).sum((0, 2, 3)) for j in range(S)], -1) for i in range(R)], -2)
+    bound = (xr.abs().sum((0, 2, 3)).max() * 3).item()
+    assert float((got.double() - want).abs().max()) <= 2e-6 * bound + 1e-5
