@@ -95,7 +95,27 @@ def dtype_code(t: torch.Tensor) -> int:
 
 
 def stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    if device.index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)      # what current_stream() wraps in an object
+
+
+class _Here:
+    """The context of a device that is already the current one: nothing to do."""
+
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_HERE = _Here()
+
+
+def on_device(device: torch.device):
+    """torch.cuda.device(device), which costs microseconds, only where it would change the device."""
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def device_status(device=None) -> None:

@@ -36,8 +36,12 @@ int variant(const char* key) {
 int check_device() {
     int dev = 0;
     MTA_CUDA_OK(cudaGetDevice(&dev));
-    int major = 0;
-    MTA_CUDA_OK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+    static std::atomic<int> known[MAX_DEVICES_KNOWN];         // major compute capability, 0 = not looked up yet
+    int major = dev < MAX_DEVICES_KNOWN ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (major == 0) {
+        MTA_CUDA_OK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+        if (dev < MAX_DEVICES_KNOWN) known[dev].store(major, std::memory_order_relaxed);
+    }
     if (major != 10) {
         set_error("device %d has compute capability %d.x; this library is built for sm_100a only", dev, major);
         return MTA_ERR_ARCH;
@@ -47,6 +51,19 @@ int check_device() {
                   "computing; mta_device_status() reports and clears the condition", dev);
         return MTA_ERR_TIMEOUT;
     }
+    return MTA_OK;
+}
+
+int sm_count(int* out) {
+    static std::atomic<int> known[MAX_DEVICES_KNOWN];
+    int dev = 0;
+    MTA_CUDA_OK(cudaGetDevice(&dev));
+    int n = dev < MAX_DEVICES_KNOWN ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        MTA_CUDA_OK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+        if (dev < MAX_DEVICES_KNOWN) known[dev].store(n, std::memory_order_relaxed);
+    }
+    *out = n;
     return MTA_OK;
 }
 

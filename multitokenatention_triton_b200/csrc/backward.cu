@@ -360,22 +360,20 @@ int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneV
 #undef MTA_BW_CASE
 #undef MTA_BW_LAUNCH
     MTA_LAUNCH_OK("conv2d_bwd_weight_kernel");
-    conv2d_bwd_weight_reduce_kernel<<<(unsigned)(C * taps), 256, 0, st>>>(partial, dw, N, C, tiles_m * tiles_n, taps);
-    MTA_LAUNCH_OK("conv2d_bwd_weight_reduce_kernel");
-    return MTA_OK;
+    return launch_kernel<conv2d_bwd_weight_reduce_kernel>("conv2d_bwd_weight_reduce_kernel", (unsigned)(C * taps), 256, 0, st, partial, dw, N, C,
+                                                          tiles_m * tiles_n, taps);
 }
 
 size_t head_linear_bwd_weight_workspace(int C) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 148;
+    if (sm_count(&sms) != MTA_OK) sms = 148;
     return (size_t)hw_grid(sms) * C * C * sizeof(float);
 }
 
 int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dW, void* workspace, int N, int C,
                                   int P, int Q, int causal, int dtype, cudaStream_t st) {
-    int dev = 0, sms = 0;
-    MTA_CUDA_OK(cudaGetDevice(&dev));
-    MTA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 0;
+    if (int bad = sm_count(&sms)) return bad;
     MTA_REQUIRE(C >= 1 && C <= 128, "head_linear_bwd_weight: C = %d heads is outside the supported range 1..128", C);
     const int grid = hw_grid(sms);
     float* partial = static_cast<float*>(workspace);
@@ -383,22 +381,19 @@ int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, P
     const bool vec_ok = dtype != MTA_F32 && C <= 32 && aligned16(x) && aligned16(dy) && xv.width % 8 == 0 && dyv.width % 8 == 0 &&
                         xv.plane_stride % 8 == 0 && dyv.plane_stride % 8 == 0;
     if (vec_ok && variant("head_linear") != 1) {         // tensor cores (mta_set_variant("head_linear", 1): CUDA cores)
-#define MTA_HM_CASE(TT, MTV)                                                                                              \
-    head_linear_bwd_weight_mma_kernel<TT, MTV><<<grid, HM_WARPS * 32, 0, st>>>(static_cast<const TT*>(x), xv, static_cast<const TT*>(dy), dyv, \
-                                                                               partial, N, C, P, Q, causal)
+#define MTA_HM_CASE(TT, MTV)                                                                                                            \
+    rc = launch_kernel<head_linear_bwd_weight_mma_kernel<TT, MTV>>("head_linear_bwd_weight_mma_kernel", (unsigned)grid, HM_WARPS * 32, 0, st, \
+                                                                   static_cast<const TT*>(x), xv, static_cast<const TT*>(dy), dyv, partial, N, C, P, Q, causal)
         if (dtype == MTA_BF16) { if (C <= 16) MTA_HM_CASE(__nv_bfloat16, 1); else MTA_HM_CASE(__nv_bfloat16, 2); }
         else { if (C <= 16) MTA_HM_CASE(__half, 1); else MTA_HM_CASE(__half, 2); }
 #undef MTA_HM_CASE
-        MTA_LAUNCH_OK("head_linear_bwd_weight_mma_kernel");
-        rc = MTA_OK;
     } else if (dtype == MTA_F32) rc = dispatch_hw<float>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
     else if (dtype == MTA_BF16) rc = dispatch_hw<__nv_bfloat16>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
     else rc = dispatch_hw<__half>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
     if (rc) return rc;
     const int pairs = C * C;
-    head_linear_bwd_weight_reduce_kernel<<<(pairs + 255) / 256, 256, 0, st>>>(partial, dW, grid, pairs);
-    MTA_LAUNCH_OK("head_linear_bwd_weight_reduce_kernel");
-    return MTA_OK;
+    return launch_kernel<head_linear_bwd_weight_reduce_kernel>("head_linear_bwd_weight_reduce_kernel", (unsigned)((pairs + 255) / 256), 256, 0, st, partial,
+                                                               dW, grid, pairs);
 }
 
 }  // namespace mta

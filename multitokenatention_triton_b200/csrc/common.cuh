@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
@@ -47,6 +48,44 @@ int check_device();                            // MTA_OK when the current device
         }                                                                                   \
         ::mta::count_launch();                                                              \
     } while (0)
+
+int sm_count(int* out);                        // SMs of the current device (looked up once per device)
+
+constexpr int MAX_DEVICES_KNOWN = 64;
+
+// Makes `bytes` of dynamic shared memory available to KERNEL on the current device.  The attribute is a maximum, so it is only
+// set when a launch needs more than any before it: setting it costs more than the launch's other host work.
+template <auto KERNEL> int ensure_smem(size_t bytes) {
+    static std::atomic<int> have[MAX_DEVICES_KNOWN];
+    if (bytes <= 32 * 1024) return MTA_OK;      // leaves room for static arrays inside the default 48 KB
+    int dev = 0;
+    MTA_CUDA_OK(cudaGetDevice(&dev));
+    if (dev < MAX_DEVICES_KNOWN && have[dev].load(std::memory_order_relaxed) >= (int)bytes) return MTA_OK;
+    MTA_CUDA_OK(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (dev < MAX_DEVICES_KNOWN) {
+        int old = have[dev].load(std::memory_order_relaxed);
+        while (old < (int)bytes && !have[dev].compare_exchange_weak(old, (int)bytes, std::memory_order_relaxed)) {}
+    }
+    return MTA_OK;
+}
+
+template <auto KERNEL, typename... Args>
+int launch_kernel(const char* name, dim3 grid, unsigned block, size_t smem, cudaStream_t st, Args... args) {
+    if (int rc = ensure_smem<KERNEL>(smem)) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, KERNEL, args...);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_error("launch of %s failed: %s", name, cudaGetErrorString(e));
+        return MTA_ERR_CUDA;
+    }
+    count_launch();
+    return MTA_OK;
+}
 
 inline size_t dtype_size(int dt) { return dt == MTA_F32 ? 4 : 2; }
 inline bool dtype_ok(int dt) { return dt == MTA_F32 || dt == MTA_BF16 || dt == MTA_F16; }

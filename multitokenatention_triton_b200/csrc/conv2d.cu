@@ -113,14 +113,10 @@ int launch_tile(const void* x, PlaneView xv, const void* w, int w_dtype, void* y
     const size_t smem = ((size_t)(TM + R - 1) * (TN + S - 1) + (size_t)R * S) * sizeof(float);
     MTA_REQUIRE(smem <= 200 * 1024, "conv2d: kernel %dx%d needs %zu bytes of shared memory (max 204800)", R, S, smem);
     MTA_REQUIRE(planes <= 65535, "conv2d: N*C = %ld exceeds 65535", planes);
-    if (smem > 48 * 1024)
-        MTA_CUDA_OK(cudaFuncSetAttribute(conv2d_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((unsigned)(tiles_m * tiles_n), (unsigned)planes);
-    conv2d_tile_kernel<T><<<grid, NTHREADS, smem, st>>>(static_cast<const T*>(x), xv, w, w_dtype, static_cast<T*>(y), yv,
-                                                         C, H, W, R, S, causal, row_begin, row_end, write_upper ? 1 : 0,
-                                                         tiles_n, grad_input ? 1 : 0);
-    MTA_LAUNCH_OK("conv2d_tile_kernel");
-    return MTA_OK;
+    const dim3 grid((unsigned)(tiles_m * tiles_n), (unsigned)planes);
+    return launch_kernel<conv2d_tile_kernel<T>>("conv2d_tile_kernel", grid, NTHREADS, smem, st, static_cast<const T*>(x), xv, w, w_dtype,
+                                                static_cast<T*>(y), yv, C, H, W, R, S, causal, row_begin, row_end, write_upper ? 1 : 0, tiles_n,
+                                                grad_input ? 1 : 0);
 }
 
 }  // namespace

@@ -319,20 +319,10 @@ int launch_dw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float*
     const size_t stage = (size_t)((th * 128 + 1023) & ~1023) + DW_DY_BYTES;
     g.nstage = (int)std::min<size_t>(DW_MAX_STAGES, (218 * 1024) / stage);
     const size_t smem = 1024 + g.nstage * stage;
-    MTA_CUDA_OK(cudaFuncSetAttribute(conv2d_dw_tc05_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    conv2d_dw_tc05_kernel<T><<<(unsigned)ctas, DW_THREADS, smem, st>>>(mx, mdy, partial, g, flag);
-    MTA_LAUNCH_OK("conv2d_dw_tc05_kernel");
+    if ((rc = launch_kernel<conv2d_dw_tc05_kernel<T>>("conv2d_dw_tc05_kernel", (unsigned)ctas, DW_THREADS, smem, st, mx, mdy, partial, g, flag))) return rc;
     const int taps = g.R * g.S;
-    conv2d_dw_reduce_kernel<<<(unsigned)((C * taps + 63) / 64), 64, 0, st>>>(partial, dw, N, C, taps, g.slots, g.steps, g.total, ctas);
-    MTA_LAUNCH_OK("conv2d_dw_reduce_kernel");
-    return MTA_OK;
-}
-
-int sm_count(int* sms) {
-    int dev = 0;
-    MTA_CUDA_OK(cudaGetDevice(&dev));
-    MTA_CUDA_OK(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
-    return MTA_OK;
+    return launch_kernel<conv2d_dw_reduce_kernel>("conv2d_dw_reduce_kernel", (unsigned)((C * taps + 63) / 64), 64, 0, st, partial, dw, N, C, taps,
+                                                  g.slots, g.steps, g.total, ctas);
 }
 
 }  // namespace

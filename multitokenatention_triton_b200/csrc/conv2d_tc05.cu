@@ -475,16 +475,12 @@ int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, 
     g.total_tiles = per_plane * planes;
     g.zero_per_plane = (causal && write_upper) ? (long)tiles_m * g.tiles_n - per_plane : 0;
     g.zero_total = g.zero_per_plane * planes;
-    int dev = 0, sms = 0;
-    MTA_CUDA_OK(cudaGetDevice(&dev));
-    MTA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 0;
+    if (int bad = sm_count(&sms)) return bad;
     const size_t smem = conv2d_tc05_smem_bytes(R, g.split_w != 0);
     MTA_REQUIRE(smem <= 227 * 1024, "conv2d (tcgen05): kernel with %d row taps needs %zu bytes of shared memory", R, smem);
-    MTA_CUDA_OK(cudaFuncSetAttribute(conv2d_tc05_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)std::min<long>(g.total_tiles, sms);
-    conv2d_tc05_kernel<T><<<grid, THREADS, smem, st>>>(mx, mx3, my, w, w_dtype, yv.row0, g, flag);
-    MTA_LAUNCH_OK("conv2d_tc05_kernel");
-    return MTA_OK;
+    return launch_kernel<conv2d_tc05_kernel<T>>("conv2d_tc05_kernel", grid, THREADS, smem, st, mx, mx3, my, w, w_dtype, yv.row0, g, flag);
 }
 
 }  // namespace

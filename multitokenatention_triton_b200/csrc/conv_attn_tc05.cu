@@ -405,15 +405,11 @@ int launch_ca(const void* q, const void* k, const void* v, const void* w, int w_
     if ((rc = make_tensor_map_3d(&mv, v, (uint64_t)planes, S, D, D, (uint64_t)S * D, 64, TN, true))) return rc;
     int* flag = nullptr;
     if ((rc = wait_flag_ptr(&flag))) return rc;
-    int dev = 0, sms = 0;
-    MTA_CUDA_OK(cudaGetDevice(&dev));
-    MTA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 0;
+    if (int bad = sm_count(&sms)) return bad;
     const size_t smem = conv_attn_smem_bytes(D, R, g.split_w != 0);
-    MTA_CUDA_OK(cudaFuncSetAttribute(conv_attn_tc05_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)std::min<long>(g.units, sms);
-    conv_attn_tc05_kernel<T, D><<<grid, CA_THREADS, smem, st>>>(mq, mk, mv, static_cast<T*>(o), w, w_dtype, g, flag);
-    MTA_LAUNCH_OK("conv_attn_tc05_kernel");
-    return MTA_OK;
+    return launch_kernel<conv_attn_tc05_kernel<T, D>>("conv_attn_tc05_kernel", grid, CA_THREADS, smem, st, mq, mk, mv, static_cast<T*>(o), w, w_dtype, g, flag);
 }
 
 constexpr size_t CA_STATIC_SMEM = 4608;     // barriers, the exchange arrays and the weight buffer, rounded up

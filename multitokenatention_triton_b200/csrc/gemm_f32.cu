@@ -264,11 +264,8 @@ template <Kind KIND>
 int launch_pv(const float* p, PlaneView pview, const float* v, float* o, int B, int H, int S, int D, int causal, int row_begin, int row_end,
               float scale, cudaStream_t st) {
     const int tiles_q = (row_end - row_begin + BT - 1) / BT, tiles_d = (D + BT - 1) / BT;
-    MTA_CUDA_OK(cudaFuncSetAttribute(pv_f32_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(KIND)));
-    pv_f32_kernel<KIND><<<(unsigned)(B * H * tiles_q * tiles_d), THREADS, smem_bytes(KIND), st>>>(
-        p, pview, v, o, B * H, S, D, causal, row_begin, row_end, tiles_d, scale);
-    MTA_LAUNCH_OK("pv_f32_kernel");
-    return MTA_OK;
+    return launch_kernel<pv_f32_kernel<KIND>>("pv_f32_kernel", (unsigned)(B * H * tiles_q * tiles_d), THREADS, smem_bytes(KIND), st, p, pview, v,
+                                              o, B * H, S, D, causal, row_begin, row_end, tiles_d, scale);
 }
 
 }  // namespace
@@ -283,11 +280,9 @@ bool gemm_f32_supported(const void* a, const void* b, const void* c, PlaneView p
 int qk_f32_launch(const void* q, const void* k, void* s, PlaneView sv, int B, int H, int S, int D, float scale, int causal, int row_begin,
                   int row_end, cudaStream_t st) {
     const int tiles_q = (row_end - row_begin + 2 * BT - 1) / (2 * BT), tiles_k = (S + 2 * BT - 1) / (2 * BT);
-    MTA_CUDA_OK(cudaFuncSetAttribute(qk_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(QK)));
-    qk_f32_kernel<<<dim3((unsigned)(B * H), (unsigned)(tiles_q * tiles_k)), THREADS, smem_bytes(QK), st>>>(
-        static_cast<const float*>(q), static_cast<const float*>(k), static_cast<float*>(s), sv, S, D, scale, causal, row_begin, row_end, tiles_k);
-    MTA_LAUNCH_OK("qk_f32_kernel");
-    return MTA_OK;
+    return launch_kernel<qk_f32_kernel>("qk_f32_kernel", dim3((unsigned)(B * H), (unsigned)(tiles_q * tiles_k)), THREADS, smem_bytes(QK), st,
+                                        static_cast<const float*>(q), static_cast<const float*>(k), static_cast<float*>(s), sv, S, D, scale, causal,
+                                        row_begin, row_end, tiles_k);
 }
 
 int pv_f32_launch(const void* p, PlaneView pview, const void* v, void* o, int B, int H, int S, int D, int causal, int row_begin, int row_end,

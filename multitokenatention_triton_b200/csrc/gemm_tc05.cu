@@ -4,7 +4,9 @@
 // Operand tiles arrive by TMA (128-byte swizzle, out-of-range rows and columns read as zero), the
 // accumulator lives in tensor memory, and only tiles that touch keys k <= q are visited when causal.
 // They stand in for the torch.matmul calls at mta_attention_triton.py:68-71 and :89.
+#include <atomic>
 #include <cstddef>
+#include <cstring>
 #include <mutex>
 
 #include "kernels.cuh"
@@ -23,7 +25,7 @@ struct WaitFlag {
 };
 __device__ WaitFlag g_wait_timeout = {0, 0, nullptr};
 std::mutex g_flag_mutex;
-int* g_flag_dev[64] = {};          // per device: address of g_wait_timeout.flag
+std::atomic<int*> g_flag_dev[64];  // per device: address of g_wait_timeout.flag
 int* g_flag_host[64] = {};         // per device: the host mirror (mapped page-locked memory)
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -48,8 +50,9 @@ int wait_flag_ptr(int** out) {
     int dev = 0;
     MTA_CUDA_OK(cudaGetDevice(&dev));
     MTA_REQUIRE(dev >= 0 && dev < 64, "device index %d out of range", dev);
+    if ((*out = g_flag_dev[dev].load(std::memory_order_acquire))) return MTA_OK;
     std::lock_guard<std::mutex> lock(g_flag_mutex);
-    if (!g_flag_dev[dev]) {
+    if (!g_flag_dev[dev].load(std::memory_order_relaxed)) {
         // first tcgen05 launch on this device: look up the flag and give it a host-visible mirror (4 bytes of mapped
         // page-locked memory, kept until the process ends)
         void* p = nullptr;
@@ -61,9 +64,9 @@ int wait_flag_ptr(int** out) {
         MTA_CUDA_OK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&host_dev), host, 0));
         MTA_CUDA_OK(cudaMemcpy(static_cast<char*>(p) + offsetof(WaitFlag, host_mirror), &host_dev, sizeof(host_dev), cudaMemcpyHostToDevice));
         g_flag_host[dev] = host;
-        g_flag_dev[dev] = static_cast<int*>(p);
+        g_flag_dev[dev].store(static_cast<int*>(p), std::memory_order_release);
     }
-    *out = g_flag_dev[dev];
+    *out = g_flag_dev[dev].load(std::memory_order_relaxed);
     return MTA_OK;
 }
 
@@ -99,6 +102,30 @@ int make_tensor_map_3d(CUtensorMap* out, const void* base, uint64_t planes, uint
 int make_tensor_map_3d_mode(CUtensorMap* out, const void* base, uint64_t planes, uint64_t rows, uint64_t cols,
                             uint64_t row_pitch_elems, uint64_t plane_pitch_elems, uint32_t box_cols, uint32_t box_rows,
                             int swizzle_bytes, uint32_t box_planes) {
+    // A map is a pure function of its description, and a program calls with the same few descriptions again and again: each
+    // thread keeps the last maps it encoded (direct-mapped by a hash of the description, 24 KB).
+    struct Key {
+        const void* base;
+        uint64_t planes, rows, cols, row_pitch, plane_pitch;
+        uint32_t box_cols, box_rows, box_planes;
+        int swizzle;
+    };
+    struct Entry {
+        Key key;
+        CUtensorMap map;
+    };
+    constexpr int ENTRIES = 128;
+    static thread_local Entry cache[ENTRIES] = {};
+    const Key key{base, planes, rows, cols, row_pitch_elems, plane_pitch_elems, box_cols, box_rows, box_planes, swizzle_bytes};
+    static_assert(sizeof(Key) == 64, "compared and hashed as bytes: no padding");
+    uint64_t words[8], hash = 0;
+    memcpy(words, &key, sizeof(key));
+    for (uint64_t w : words) hash = (hash ^ w) * 0x9E3779B97F4A7C15ull ^ (hash >> 29);
+    Entry& entry = cache[(hash >> 40) % ENTRIES];
+    if (base && memcmp(&entry.key, &key, sizeof(key)) == 0) {
+        *out = entry.map;
+        return MTA_OK;
+    }
     const bool swizzle128 = swizzle_bytes == 128;
     EncodeTiledFn fn = encode_fn();
     if (!fn) {
@@ -133,6 +160,8 @@ int make_tensor_map_3d_mode(CUtensorMap* out, const void* base, uint64_t planes,
         set_error("cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
         return MTA_ERR_CUDA;
     }
+    entry.key = key;
+    entry.map = *out;
     return MTA_OK;
 }
 
@@ -371,11 +400,8 @@ int launch_pv(const void* p, PlaneView pview, const void* v, void* o, int B, int
     const int n_qt = (row_end - row_begin + TILE - 1) / TILE;
     const size_t smem = (size_t)PV_STAGES * (BOX_BYTES + (D / 64) * PV_VBOX_BYTES) + 1024;
     const unsigned grid = (unsigned)(B * H * n_qt);
-    auto kernel = pv_tc05_kernel<T, D, DROP, TRANS>;
-    MTA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, PV_THREADS, smem, st>>>(mp, mv, static_cast<T*>(o), B * H, pview.row0, S, causal, row_begin, row_end, scale, flag, drop);
-    MTA_LAUNCH_OK("pv_tc05_kernel");
-    return MTA_OK;
+    return launch_kernel<pv_tc05_kernel<T, D, DROP, TRANS>>("pv_tc05_kernel", grid, PV_THREADS, smem, st, mp, mv, static_cast<T*>(o), B * H,
+                                                            pview.row0, S, causal, row_begin, row_end, scale, flag, drop);
 }
 
 template <typename T, int D>

@@ -699,12 +699,8 @@ int launch_simt(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* 
                 int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st) {
     dim3 grid((unsigned)((Q + 255) / 256), (unsigned)(row_end - row_begin), (unsigned)N);
     const size_t smem = (size_t)C * C * sizeof(float);
-    if (smem > 48 * 1024)
-        MTA_CUDA_OK(cudaFuncSetAttribute(head_linear_simt_kernel<T, CP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    head_linear_simt_kernel<T, CP><<<grid, 256, smem, st>>>(static_cast<const T*>(x), xv, Wm, w_dtype, static_cast<T*>(y),
-                                                            yv, C, Q, causal, fill, row_begin, write_upper ? 1 : 0, wt ? 1 : 0);
-    MTA_LAUNCH_OK("head_linear_simt_kernel");
-    return MTA_OK;
+    return launch_kernel<head_linear_simt_kernel<T, CP>>("head_linear_simt_kernel", grid, 256, smem, st, static_cast<const T*>(x), xv, Wm, w_dtype,
+                                                         static_cast<T*>(y), yv, C, Q, causal, fill, row_begin, write_upper ? 1 : 0, wt ? 1 : 0);
 }
 
 template <typename T>
@@ -727,10 +723,10 @@ int launch_mma(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y
     const int rows_per_cta = rows >= 2048 ? 8 : (rows >= 256 ? 4 : 1);
     dim3 grid((unsigned)((Q + MMA_WARPS * MMA_KEYS_PER_WARP - 1) / (MMA_WARPS * MMA_KEYS_PER_WARP)),
               (unsigned)((rows + rows_per_cta - 1) / rows_per_cta), (unsigned)N);
-#define MTA_HL_LAUNCH(KERNEL, SPLIT)                                                                                     \
-    KERNEL<T, CP, SPLIT><<<grid, MMA_WARPS * 32, 0, st>>>(static_cast<const T*>(x), xv, Wm, w_dtype, static_cast<T*>(y), yv, C, \
-                                                         Q, causal, fill, row_begin, row_end, rows_per_cta,            \
-                                                         write_upper ? 1 : 0, wt ? 1 : 0)
+#define MTA_HL_LAUNCH(KERNEL, SPLIT)                                                                                                   \
+    return launch_kernel<KERNEL<T, CP, SPLIT>>("head_linear_mma_kernel", grid, MMA_WARPS * 32, 0, st, static_cast<const T*>(x), xv, Wm,   \
+                                               w_dtype, static_cast<T*>(y), yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,    \
+                                               write_upper ? 1 : 0, wt ? 1 : 0)
     if constexpr (CP > 16) {
         if (w_dtype == MTA_F32) MTA_HL_LAUNCH(head_linear_mma_wide_kernel, true);
         else MTA_HL_LAUNCH(head_linear_mma_wide_kernel, false);
@@ -739,8 +735,6 @@ int launch_mma(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y
         else MTA_HL_LAUNCH(head_linear_mma_kernel, false);
     }
 #undef MTA_HL_LAUNCH
-    MTA_LAUNCH_OK("head_linear_mma_kernel");
-    return MTA_OK;
 }
 
 template <typename T>

@@ -517,19 +517,14 @@ int launch_hm(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv
         return rc;
     int* flag = nullptr;
     if ((rc = wait_flag_ptr(&flag))) return rc;
-    int dev = 0, sms = 0;
-    MTA_CUDA_OK(cudaGetDevice(&dev));
-    MTA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 0;
+    if (int bad = sm_count(&sms)) return bad;
     const unsigned grid = (unsigned)std::min<long>(g.units, sms);
-    if constexpr (SOFTMAX) {
-        MTA_CUDA_OK(cudaFuncSetAttribute(head_mix_softmax_tc05_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HM_SMEM_BYTES));
-        head_mix_softmax_tc05_kernel<T><<<grid, HM_THREADS, HM_SMEM_BYTES, st>>>(mx, my, static_cast<const T*>(Wm), yv.row0, g, flag);
-    } else {
-        MTA_CUDA_OK(cudaFuncSetAttribute(head_mix_plain_tc05_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HM_SMEM_BYTES));
-        head_mix_plain_tc05_kernel<T><<<grid, HM_THREADS, HM_SMEM_BYTES, st>>>(mx, my, static_cast<const T*>(Wm), yv.row0, g, flag);
-    }
-    MTA_LAUNCH_OK(SOFTMAX ? "head_mix_softmax_tc05_kernel" : "head_mix_plain_tc05_kernel");
-    return MTA_OK;
+    if constexpr (SOFTMAX)
+        return launch_kernel<head_mix_softmax_tc05_kernel<T>>("head_mix_softmax_tc05_kernel", grid, HM_THREADS, HM_SMEM_BYTES, st, mx, my,
+                                                              static_cast<const T*>(Wm), yv.row0, g, flag);
+    return launch_kernel<head_mix_plain_tc05_kernel<T>>("head_mix_plain_tc05_kernel", grid, HM_THREADS, HM_SMEM_BYTES, st, mx, my,
+                                                        static_cast<const T*>(Wm), yv.row0, g, flag);
 }
 
 bool hm_tc05_ok(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int dtype, int w_dtype) {

@@ -339,15 +339,11 @@ int launch_qc(const void* q, const void* k, const void* w, int w_dtype, void* y,
         return rc;
     int* flag = nullptr;
     if ((rc = wait_flag_ptr(&flag))) return rc;
-    int dev = 0, sms = 0;
-    MTA_CUDA_OK(cudaGetDevice(&dev));
-    MTA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 0;
+    if (int bad = sm_count(&sms)) return bad;
     const size_t smem = qk_conv_smem_bytes(D, R, g.split_w != 0);
-    MTA_CUDA_OK(cudaFuncSetAttribute(qk_conv_tc05_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)std::min<long>(g.total_tiles, sms);
-    qk_conv_tc05_kernel<T, D><<<grid, THREADS, smem, st>>>(mq, mk, my, w, w_dtype, g, flag);
-    MTA_LAUNCH_OK("qk_conv_tc05_kernel");
-    return MTA_OK;
+    return launch_kernel<qk_conv_tc05_kernel<T, D>>("qk_conv_tc05_kernel", grid, THREADS, smem, st, mq, mk, my, w, w_dtype, g, flag);
 }
 
 }  // namespace

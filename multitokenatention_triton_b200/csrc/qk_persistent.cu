@@ -271,14 +271,10 @@ int launch(const void* a, const void* b, void* c, PlaneView cv, int BH, QkGeom g
     constexpr int STAGE = 2 * (D / 64) * BOX_BYTES;
     g.nstage = D == 128 ? 3 : 4;
     const size_t smem = 1024 + OUT_BYTES + (size_t)g.nstage * STAGE;
-    int dev = 0, sms = 0;
-    MTA_CUDA_OK(cudaGetDevice(&dev));
-    MTA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MTA_CUDA_OK(cudaFuncSetAttribute(qk_persistent_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int sms = 0;
+    if (int bad = sm_count(&sms)) return bad;
     const unsigned grid = (unsigned)std::min<long>(g.total, sms);
-    qk_persistent_kernel<T, D><<<grid, QK_THREADS, smem, st>>>(ma, mb, mc, g, flag);
-    MTA_LAUNCH_OK("qk_persistent_kernel");
-    return MTA_OK;
+    return launch_kernel<qk_persistent_kernel<T, D>>("qk_persistent_kernel", grid, QK_THREADS, smem, st, ma, mb, mc, g, flag);
 }
 
 }  // namespace

@@ -191,10 +191,8 @@ template <typename T, int NCH>
 int launch_vec(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int Q, int causal, int row_begin,
                int row_end, bool write_upper, float pre_scale, int round_prescaled, cudaStream_t st) {
     dim3 grid((unsigned)(row_end - row_begin), (unsigned)planes);
-    softmax_rows_vec_kernel<T, NCH><<<grid, VT, 0, st>>>(static_cast<const T*>(x), xv, static_cast<T*>(y), yv, Q, causal,
-                                                        row_begin, write_upper ? 1 : 0, pre_scale, round_prescaled);
-    MTA_LAUNCH_OK("softmax_rows_vec_kernel");
-    return MTA_OK;
+    return launch_kernel<softmax_rows_vec_kernel<T, NCH>>("softmax_rows_vec_kernel", grid, VT, 0, st, static_cast<const T*>(x), xv,
+                                                          static_cast<T*>(y), yv, Q, causal, row_begin, write_upper ? 1 : 0, pre_scale, round_prescaled);
 }
 
 template <typename T>
@@ -212,13 +210,9 @@ int launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int 
     }
     const int cache = Q < ROW_CACHE ? Q : ROW_CACHE;
     const size_t smem = (size_t)cache * sizeof(float);
-    if (smem > 48 * 1024)
-        MTA_CUDA_OK(cudaFuncSetAttribute(softmax_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((unsigned)(row_end - row_begin), (unsigned)planes);
-    softmax_rows_kernel<T><<<grid, SM_THREADS, smem, st>>>(static_cast<const T*>(x), xv, static_cast<T*>(y), yv, Q, causal,
-                                                           row_begin, write_upper ? 1 : 0, cache, pre_scale, round_prescaled);
-    MTA_LAUNCH_OK("softmax_rows_kernel");
-    return MTA_OK;
+    const dim3 grid((unsigned)(row_end - row_begin), (unsigned)planes);
+    return launch_kernel<softmax_rows_kernel<T>>("softmax_rows_kernel", grid, SM_THREADS, smem, st, static_cast<const T*>(x), xv, static_cast<T*>(y),
+                                                 yv, Q, causal, row_begin, write_upper ? 1 : 0, cache, pre_scale, round_prescaled);
 }
 
 // Gradient of the causal row softmax: ds = p (g - sum_k g p) over keys k <= query, fp32 arithmetic; nothing is read or written
@@ -271,12 +265,11 @@ int launch_bwd(const void* p, PlaneView pv, const void* g, PlaneView gv, void* d
     constexpr int VEC = 16 / (int)sizeof(T);
     auto ok = [](const void* b, const PlaneView& v) { return aligned16(b) && v.width % VEC == 0 && v.plane_stride % VEC == 0; };
     const dim3 grid((unsigned)((P + SB_WARPS - 1) / SB_WARPS), (unsigned)planes);
+    const T *pt = static_cast<const T*>(p), *gt = static_cast<const T*>(g);
+    T* dt = static_cast<T*>(ds);
     if (ok(p, pv) && ok(g, gv) && ok(ds, dv))
-        softmax_bwd_kernel<T, VEC><<<grid, SB_WARPS * 32, 0, st>>>(static_cast<const T*>(p), pv, static_cast<const T*>(g), gv, static_cast<T*>(ds), dv, P, Q, causal);
-    else
-        softmax_bwd_kernel<T, 1><<<grid, SB_WARPS * 32, 0, st>>>(static_cast<const T*>(p), pv, static_cast<const T*>(g), gv, static_cast<T*>(ds), dv, P, Q, causal);
-    MTA_LAUNCH_OK("softmax_bwd_kernel");
-    return MTA_OK;
+        return launch_kernel<softmax_bwd_kernel<T, VEC>>("softmax_bwd_kernel", grid, SB_WARPS * 32, 0, st, pt, pv, gt, gv, dt, dv, P, Q, causal);
+    return launch_kernel<softmax_bwd_kernel<T, 1>>("softmax_bwd_kernel", grid, SB_WARPS * 32, 0, st, pt, pv, gt, gv, dt, dv, P, Q, causal);
 }
 
 }  // namespace

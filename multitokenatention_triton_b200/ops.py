@@ -5,12 +5,13 @@ enqueues the kernels on PyTorch's current stream.  Nothing here computes on the 
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional, Tuple
 
 import torch
 
 from . import _lib
-from ._lib import MTALibraryError, check, dtype_code, lib, stream_ptr
+from ._lib import MTALibraryError, check, dtype_code, lib, on_device, stream_ptr
 
 
 def _cuda_contig(t: torch.Tensor, name: str) -> torch.Tensor:
@@ -20,10 +21,16 @@ def _cuda_contig(t: torch.Tensor, name: str) -> torch.Tensor:
 
 
 def _weight(w: torch.Tensor, like: torch.Tensor, name: str) -> torch.Tensor:
-    w = _cuda_contig(w.detach(), name)
+    w = _cuda_contig(w, name)
     if w.dtype not in (torch.float32, like.dtype):
-        w = w.to(like.dtype)
+        w = w.detach().to(like.dtype)
     return w
+
+
+@functools.lru_cache(maxsize=256)
+def _size(name: str, *args: int) -> int:
+    """A workspace size of the library: a function of the shape alone."""
+    return getattr(lib(), name)(*args)
 
 
 def conv2d_fwd(x: torch.Tensor, weight: torch.Tensor, causal: bool) -> torch.Tensor:
@@ -36,7 +43,7 @@ def conv2d_fwd(x: torch.Tensor, weight: torch.Tensor, causal: bool) -> torch.Ten
     assert C == Cw, "This implementation assumes depthwise convolution (C_in == C_out)"
     w = _weight(weight, x, "weight")
     y = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         check(lib().mta_conv2d_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, C, H, W, R, S, int(bool(causal)),
                                    dtype_code(x), dtype_code(w), stream_ptr(x.device)), "mta_conv2d_fwd")
     return y
@@ -53,7 +60,7 @@ def head_linear_fwd(x: torch.Tensor, weight: torch.Tensor, causal: bool = True, 
     assert C == L, f"Channel dimension {C} must match weight dimension {L}"
     w = _weight(weight, x, "weight")
     y = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         check(lib().mta_head_linear_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, C, P, Q, int(bool(causal)),
                                         float(output_value), dtype_code(x), dtype_code(w), stream_ptr(x.device)),
               "mta_head_linear_fwd")
@@ -68,7 +75,7 @@ def conv2d_bwd_input(grad_output: torch.Tensor, weight: torch.Tensor, causal: bo
     assert C == Cw, "This implementation assumes depthwise convolution (C_in == C_out)"
     w = _weight(weight, g, "weight")
     dx = torch.empty_like(g)
-    with torch.cuda.device(g.device):
+    with on_device(g.device):
         check(lib().mta_conv2d_bwd_input(g.data_ptr(), w.data_ptr(), dx.data_ptr(), N, C, H, W, R, S, int(bool(causal)),
                                          dtype_code(g), dtype_code(w), stream_ptr(g.device)), "mta_conv2d_bwd_input")
     return dx
@@ -82,9 +89,9 @@ def conv2d_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, kernel_size: T
     R, S = kernel_size
     dw = torch.empty(C, R, S, device=x.device, dtype=torch.float32)
     L = lib()
-    nbytes = L.mta_conv2d_bwd_weight_workspace_bytes(N, C, H, W, R, S)
+    nbytes = _size("mta_conv2d_bwd_weight_workspace_bytes", N, C, H, W, R, S)
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         check(L.mta_conv2d_bwd_weight(x.data_ptr(), g.data_ptr(), dw.data_ptr(), ws.data_ptr(), ws.numel(), N, C, H, W, R, S,
                                       int(bool(causal)), dtype_code(x), stream_ptr(x.device)), "mta_conv2d_bwd_weight")
     return dw
@@ -97,7 +104,7 @@ def head_linear_bwd_input(grad_output: torch.Tensor, weight: torch.Tensor, causa
     assert weight.shape == (C, C), f"Weight must be a ({C},{C}) matrix, got {tuple(weight.shape)}"
     w = _weight(weight, g, "weight")
     dx = torch.empty_like(g)
-    with torch.cuda.device(g.device):
+    with on_device(g.device):
         check(lib().mta_head_linear_bwd_input(g.data_ptr(), w.data_ptr(), dx.data_ptr(), N, C, P, Q, int(bool(causal)),
                                               dtype_code(g), dtype_code(w), stream_ptr(g.device)), "mta_head_linear_bwd_input")
     return dx
@@ -114,7 +121,7 @@ def head_linear_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, causal: b
     if nbytes == 0:
         raise MTALibraryError(f"head_linear_bwd_weight: C = {C} heads is outside the supported range 1..128")
     ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         check(L.mta_head_linear_bwd_weight(x.data_ptr(), g.data_ptr(), dW.data_ptr(), ws.data_ptr(), ws.numel(), N, C, P, Q,
                                            int(bool(causal)), dtype_code(x), stream_ptr(x.device)), "mta_head_linear_bwd_weight")
     return dW
@@ -131,7 +138,7 @@ def head_linear_softmax_fwd(x: torch.Tensor, weight: torch.Tensor) -> torch.Tens
     assert weight.shape == (C, C), f"Weight must be a ({C},{C}) matrix, got {tuple(weight.shape)}"
     w = _weight(weight, x, "weight")
     y = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         check(lib().mta_head_linear_softmax_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, C, P, Q, dtype_code(x),
                                                 dtype_code(w), stream_ptr(x.device)), "mta_head_linear_softmax_fwd")
     return y
@@ -142,7 +149,7 @@ def softmax_fwd(x: torch.Tensor, causal: bool = True, out: Optional[torch.Tensor
     x = _cuda_contig(x, "input")
     N, C, P, Q = x.shape
     y = torch.empty_like(x) if out is None else out
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         check(lib().mta_softmax_fwd(x.data_ptr(), y.data_ptr(), N, C, P, Q, int(bool(causal)), dtype_code(x),
                                     stream_ptr(x.device)), "mta_softmax_fwd")
     return y
@@ -159,7 +166,7 @@ def qk_scores_fwd(q: torch.Tensor, k: torch.Tensor, scale: float, causal: bool =
         s = torch.zeros(B, H, S, S, device=q.device, dtype=q.dtype)
     else:
         s = torch.empty(B, H, S, S, device=q.device, dtype=q.dtype)
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         check(lib().mta_qk_scores_fwd(q.data_ptr(), k.data_ptr(), s.data_ptr(), B, H, S, D, float(scale),
                                       int(round_like_reference and q.dtype != torch.float32), int(bool(causal)),
                                       dtype_code(q), stream_ptr(q.device)), "mta_qk_scores_fwd")
@@ -171,7 +178,7 @@ def pv_fwd(p: torch.Tensor, v: torch.Tensor, causal: bool = True) -> torch.Tenso
     p, v = _cuda_contig(p, "p"), _cuda_contig(v, "v")
     B, H, S, D = v.shape
     o = torch.empty_like(v)
-    with torch.cuda.device(v.device):
+    with on_device(v.device):
         check(lib().mta_pv_fwd(p.data_ptr(), v.data_ptr(), o.data_ptr(), B, H, S, D, int(bool(causal)), dtype_code(v),
                                stream_ptr(v.device)), "mta_pv_fwd")
     return o
@@ -192,7 +199,7 @@ def conv_attn_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, weight: tor
     L = lib()
     nbytes = L.mta_conv_attn_workspace_bytes(B, H, S, D, cq, ck, int(bool(causal)), dtype_code(q), dtype_code(w))
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         check(L.mta_conv_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), o.data_ptr(), ws.data_ptr(),
                                   nbytes, B, H, S, D, cq, ck, int(bool(causal)), float(softmax_scale), dtype_code(q),
                                   dtype_code(w), stream_ptr(q.device)), "mta_conv_attn_fwd")
@@ -209,24 +216,21 @@ def mta_fused_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w1: torch.T
     q, k, v = _cuda_contig(q, "xq"), _cuda_contig(k, "xk"), _cuda_contig(v, "xv")
     B, H, S, D = q.shape
     assert k.shape == q.shape and v.shape == q.shape
-    w1, w2 = _weight(w1, q, "conv weight"), _weight(w2, q, "post-softmax conv weight")
-    W1, W2 = _weight(W1, q, "head-mix weight"), _weight(W2, q, "post-softmax head-mix weight")
-    wd = {w1.dtype, w2.dtype, W1.dtype, W2.dtype}
-    if len(wd) != 1:
-        w1, w2, W1, W2 = (t.float() for t in (w1, w2, W1, W2))
+    w1, W1, w2, W2 = _mta_weights(q, w1, W1, w2, W2)
     _, cq, ck = w1.shape
     _, cq2, ck2 = w2.shape
     r0, r1 = (0, S) if rows is None else rows
     if out is None:
         out = torch.empty_like(q) if (r0, r1) == (0, S) else torch.zeros_like(q)
     L = lib()
-    nbytes = L.mta_workspace_bytes(B, H, S, D, cq, ck, cq2, ck2, r0, r1, dtype_code(q))
+    code = dtype_code(q)
+    nbytes = _size("mta_workspace_bytes", B, H, S, D, cq, ck, cq2, ck2, r0, r1, code)
     if workspace is None or workspace.numel() < nbytes:
         workspace = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         check(L.mta_fused_fwd_dropout(q.data_ptr(), k.data_ptr(), v.data_ptr(), w1.data_ptr(), W1.data_ptr(), w2.data_ptr(),
                                       W2.data_ptr(), out.data_ptr(), workspace.data_ptr(), workspace.numel(), B, H, S, D, cq, ck,
-                                      cq2, ck2, r0, r1, int(bool(causal)), dtype_code(q), dtype_code(w1), float(dropout_p),
+                                      cq2, ck2, r0, r1, int(bool(causal)), code, dtype_code(w1), float(dropout_p),
                                       int(dropout_seed) & 0xFFFFFFFFFFFFFFFF, stream_ptr(q.device)),
               "mta_fused_fwd")
     return out
@@ -236,7 +240,8 @@ def _mta_weights(q, w1, W1, w2, W2):
     """The four weights as the library takes them: on the device, contiguous, of one dtype (the activations' or float32)."""
     w = [_weight(w1, q, "conv weight"), _weight(W1, q, "head-mix weight"), _weight(w2, q, "post-softmax conv weight"),
          _weight(W2, q, "post-softmax head-mix weight")]
-    return w if len({t.dtype for t in w}) == 1 else [t.float() for t in w]
+    d = w[0].dtype
+    return w if w[1].dtype == d and w[2].dtype == d and w[3].dtype == d else [t.detach().float() for t in w]
 
 
 def mta_train_fwd(q, k, v, w1, W1, w2, W2) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -247,9 +252,9 @@ def mta_train_fwd(q, k, v, w1, W1, w2, W2) -> Tuple[torch.Tensor, torch.Tensor]:
     w = _mta_weights(q, w1, W1, w2, W2)
     out = torch.empty_like(q)
     L = lib()
-    nbytes = L.mta_train_saved_bytes(B, H, S, dtype_code(q))
+    nbytes = _size("mta_train_saved_bytes", B, H, S, dtype_code(q))
     saved = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         check(L.mta_train_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), *(t.data_ptr() for t in w), out.data_ptr(), saved.data_ptr(),
                               saved.numel(), B, H, S, D, *w1.shape[1:], *w2.shape[1:], dtype_code(q), dtype_code(w[0]),
                               stream_ptr(q.device)), "mta_train_fwd")
@@ -264,9 +269,9 @@ def mta_train_bwd(grad_out, saved, q, k, v, w1, W1, w2, W2, needs) -> list:
     grads = [torch.empty_like(t) if n else None for t, n in zip((q, k, v), needs)]
     grads += [torch.empty(t.shape, dtype=torch.float32, device=q.device) if n else None for t, n in zip(w, needs[3:])]
     L = lib()
-    nbytes = L.mta_train_workspace_bytes(B, H, S, *w1.shape[1:], *w2.shape[1:], dtype_code(q))
+    nbytes = _size("mta_train_workspace_bytes", B, H, S, *w1.shape[1:], *w2.shape[1:], dtype_code(q))
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         check(L.mta_train_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), *(t.data_ptr() for t in w), g.data_ptr(), saved.data_ptr(),
                               *(None if t is None else t.data_ptr() for t in grads), ws.data_ptr(), ws.numel(), B, H, S, D,
                               *w1.shape[1:], *w2.shape[1:], dtype_code(q), dtype_code(w[0]), stream_ptr(q.device)), "mta_train_bwd")
@@ -294,7 +299,7 @@ def mta_fused_fwd_host(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w1: to
         out = torch.empty(q.shape, dtype=q.dtype, pin_memory=True)
     elif out.is_cuda or not out.is_contiguous() or out.shape != q.shape or out.dtype != q.dtype:
         raise MTALibraryError("out must be a contiguous host tensor with the shape and dtype of xq")
-    with torch.cuda.device(w1.device):
+    with on_device(w1.device):
         torch.cuda.current_stream().synchronize()            # weights written on torch's stream are read on the library's
         check(lib().mta_fused_fwd_host(q.data_ptr(), k.data_ptr(), v.data_ptr(), w1.data_ptr(), W1.data_ptr(), w2.data_ptr(),
                                        W2.data_ptr(), out.data_ptr(), B, H, S, D, cq, ck, cq2, ck2, int(bool(causal)),
