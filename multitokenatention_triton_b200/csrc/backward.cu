@@ -110,6 +110,7 @@ conv2d_bwd_weight_kernel(const T* __restrict__ x, PlaneView xv, const T* __restr
 __global__ void conv2d_bwd_weight_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int N, int C,
                                                 int tiles, int taps) {
     __shared__ double red[256];
+    pdl_wait();
     const int c = blockIdx.x / taps, tap = blockIdx.x % taps;
     double acc = 0.0;
     const long per_channel = (long)N * tiles;
@@ -212,6 +213,7 @@ head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, PlaneView xview, cons
                                   float* __restrict__ partial, int N, int C, int P, int Q, int causal) {
     constexpr int CP = 16 * MT, NV = 2 * MT;            // padded heads; 16-byte vectors per lane, side and 32-key group
     __shared__ float red[HM_WARPS][CP * CP];
+    pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     float acc[MT][2 * MT][4];                            // [16-row tile of o][8-column tile of h][fragment]
@@ -228,6 +230,8 @@ head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, PlaneView xview, cons
         const int k0 = kb * HM_KEYS;
         if (causal && k0 > p) continue;
         const int n_keys = causal ? min(p + 1, Q) : Q;   // keys of this row that carry a gradient
+        const T* g_row = dy + n * C * dyview.plane_stride + (long)p * dyview.width;
+        const T* x_row = x + n * C * xview.plane_stride + (long)p * xview.width;
         uint4 gv[4][NV], xv[4][NV];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -236,8 +240,8 @@ head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, PlaneView xview, cons
             for (int r = 0; r < NV; ++r) {
                 const int head = g + 8 * r;
                 if (head < C && kq < n_keys) {
-                    gv[j][r] = __ldg(reinterpret_cast<const uint4*>(dy + dyview.at(n * C + head, p, kq)));
-                    xv[j][r] = __ldg(reinterpret_cast<const uint4*>(x + xview.at(n * C + head, p, kq)));
+                    gv[j][r] = __ldg(reinterpret_cast<const uint4*>(g_row + head * dyview.plane_stride + kq));
+                    xv[j][r] = __ldg(reinterpret_cast<const uint4*>(x_row + head * xview.plane_stride + kq));
                 } else {
                     gv[j][r] = make_uint4(0u, 0u, 0u, 0u);
                     xv[j][r] = make_uint4(0u, 0u, 0u, 0u);
@@ -288,6 +292,7 @@ head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, PlaneView xview, cons
 __global__ void head_linear_bwd_weight_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dW, int ctas,
                                                      int pairs) {
     const int pair = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (pair >= pairs) return;
     double acc = 0.0;
     for (int i = 0; i < ctas; ++i) acc += (double)partial[(long)i * pairs + pair];

@@ -69,6 +69,13 @@ template <auto KERNEL> int ensure_smem(size_t bytes) {
     return MTA_OK;
 }
 
+// Launches KERNEL so that it may start before its predecessor in the stream has ended (programmatic dependent launch): what
+// it does before pdl_wait() - barriers, tensor memory, descriptors - then overlaps the predecessor's last blocks.  KERNEL must
+// call pdl_wait() before it reads or writes anything that another kernel may touch.
+// Measured: B1 H16 S128 forward 51 -> 37 us, B1 H16 S2048 211 -> 188.  Only up to PDL_MAX_BLOCKS blocks: every block of such a
+// launch starts later, and over the fifty waves of a long grid that cost more than the overlap gave (head mix of B8 H16 S4096,
+// 65536 blocks: 0.15 ms of 0.77).
+constexpr unsigned PDL_MAX_BLOCKS = 4096;
 template <auto KERNEL, typename... Args>
 int launch_kernel(const char* name, dim3 grid, unsigned block, size_t smem, cudaStream_t st, Args... args) {
     if (int rc = ensure_smem<KERNEL>(smem)) return rc;
@@ -77,6 +84,11 @@ int launch_kernel(const char* name, dim3 grid, unsigned block, size_t smem, cuda
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = (unsigned long long)grid.x * grid.y * grid.z <= PDL_MAX_BLOCKS ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, KERNEL, args...);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -92,6 +104,15 @@ inline bool dtype_ok(int dt) { return dt == MTA_F32 || dt == MTA_BF16 || dt == M
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---- device side -----------------------------------------------------------------------------
+// Waits until everything before this kernel in the stream is complete and visible (returns at once in an ordinary launch), then
+// lets the next kernel begin its own setup.  In this order, so that a kernel that has started knows its predecessors' predecessors
+// to be complete; and after this kernel's tensor memory is allocated: the next kernel's blocks could otherwise take columns that a
+// block of this one still needs, and wait for it.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }

@@ -26,6 +26,7 @@ conv2d_tile_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict
                    T* __restrict__ y, PlaneView yv, int C, int H, int W, int R, int S, int causal,
                    int row_begin, int row_end, int write_upper, int tiles_n, int grad_input) {
     extern __shared__ float smem[];
+    pdl_wait();
     // grad_input: the same kernel evaluates the gradient with respect to the conv's input (conv_bwd_input_kernel,
     // convolution_2d_trit.py:143-218): dx[q,k] = sum_{i,j} w[R-1-i, S-1-j] * dyh[q + i, k + j - (S-1-pad_w)], i.e. the
     // taps reversed, the rows looking forward instead of back, dyh masked like the forward's input

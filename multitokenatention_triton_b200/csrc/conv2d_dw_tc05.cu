@@ -150,6 +150,7 @@ conv2d_dw_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_const
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    pdl_wait();
 
     // Every role walks the same steps; st / use = the step's stage and how often the stage was used before.
     DwIter it;
@@ -280,6 +281,7 @@ conv2d_dw_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_const
 __global__ void conv2d_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int N, int C, int taps, int slots,
                                         int steps, long total, int ctas) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (i >= C * taps) return;
     const int c = i / taps, tap = i % taps;
     double acc = 0.0;

@@ -167,6 +167,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
     __shared__ __align__(8) uint64_t full_bar[NSTAGE], ready_bar[NSTAGE], empty_bar[NSTAGE], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
+    __shared__ float wsm[16 * 17];             // the current head's weights on their way into the Toeplitz slices
     __shared__ int tiles_loaded;               // compute tiles whose loads the producer has issued (paces the zero tiles)
     const int R = g.R, S = g.S;
     const int TH = TM + R - 1;
@@ -216,6 +217,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    pdl_wait();
 
     if (warp == 0) {
         // ---------------- producer ----------------
@@ -322,19 +324,22 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
             if (ph != head) {
                 // slice of row tap i, element (n', kk) = w[i][kk + 16 - n' - a_off]; no-swizzle K-major layout:
                 // 8 rows x 16 bytes per core matrix, the two k chunks 512 bytes apart, row groups 128 bytes apart
+                // (the head's weights are fetched from global memory once, in the order the taps use them)
+                for (int idx = ft; idx < R * S; idx += 128)
+                    wsm[idx] = load_weight(w, (long)head * R * S + (g.flip ? R * S - 1 - idx : idx), w_dtype);
+                named_barrier(2, 128);
                 const int total = R * 512;
                 for (int idx = ft; idx < total; idx += 128) {
-                    const int i = idx / 512, e = idx % 512;
-                    const int nn = e / 16, kk = e % 16;
+                    const int i = idx >> 9, e = idx & 511;
+                    const int nn = e >> 4, kk = e & 15;
                     const int j = kk + 16 - nn - a_off;
-                    const float wv = (j >= 0 && j < S) ? load_weight(w, g.flip ? ((long)head * R + (R - 1 - i)) * S + (S - 1 - j)
-                                                                             : ((long)head * R + i) * S + j, w_dtype)
-                                                       : 0.0f;
+                    const float wv = (j >= 0 && j < S) ? wsm[i * S + j] : 0.0f;
                     const T hi = from_f32<T>(wv);
                     const int off = i * 1024 + (kk / 8) * 512 + (nn / 8) * 128 + (nn % 8) * 16 + (kk % 8) * 2;
                     *reinterpret_cast<T*>(tb + off) = hi;
                     if (g.split_w) *reinterpret_cast<T*>(tb + R * 1024 + off) = from_f32<T>(wv - to_f32<T>(hi));
                 }
+                named_barrier(2, 128);            // nobody refills wsm while another warp still reads it
             }
             mbar_wait(&full_bar[st], (n / NSTAGE) & 1, err_flag);
             // staged row sr is query m0-(R-1)+sr; staged column sc is key n0-pad8+sc, in box sc/64 at byte

@@ -120,6 +120,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    pdl_wait();
 
     // Every role walks the same sequence of units.  All units, heaviest row blocks first (row block tm of every plane
     // before row block tm - 1 of any), are dealt to the CTAs in rounds that alternate direction (0 .. G-1, G-1 .. 0, ...):

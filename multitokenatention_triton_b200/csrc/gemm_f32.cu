@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(THREADS, 2)
 qk_f32_kernel(const float* __restrict__ q, const float* __restrict__ k, float* __restrict__ s, PlaneView sv, int S, int D, float scale,
               int causal, int row_begin, int row_end, int tiles_k) {
     extern __shared__ __align__(16) float smem[];
+    pdl_wait();
     const long bh = blockIdx.x;
     const int tq = blockIdx.y / tiles_k, tk = blockIdx.y % tiles_k;
     if (causal && tk * 2 * BT > min(row_begin + (tq + 1) * 2 * BT, row_end) - 1) return;
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(THREADS, 2)
 pv_f32_kernel(const float* __restrict__ p, PlaneView pv, const float* __restrict__ v, float* __restrict__ o, int planes, int S, int D,
               int causal, int row_begin, int row_end, int tiles_d, float scale) {
     extern __shared__ __align__(16) float smem[];
+    pdl_wait();
     // heaviest tiles first over groups of planes (as in gemm_tc05.cu: few enough for their V to stay in L2)
     const int n_q = (row_end - row_begin + BT - 1) / BT;
     const int per_group = n_q * tiles_d * PLANE_GROUP, in_group = (int)(blockIdx.x % per_group), p0 = (int)(blockIdx.x / per_group) * PLANE_GROUP;

@@ -265,6 +265,7 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {

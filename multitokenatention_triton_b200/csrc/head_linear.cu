@@ -25,6 +25,7 @@ head_linear_simt_kernel(const T* __restrict__ x, PlaneView xv, const void* __res
                         T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
                         int write_upper, int w_transposed) {
     extern __shared__ float ws[];   // C x C
+    pdl_wait();
     for (int i = threadIdx.x; i < C * C; i += blockDim.x)
         ws[i] = load_weight(Wm, w_transposed ? (long)(i % C) * C + i / C : i, w_dtype);
     __syncthreads();
@@ -294,6 +295,7 @@ __global__ void __launch_bounds__(MMA_WARPS * 32)
 head_linear_mma_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
                        T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
                        int row_end, int rows_per_cta, int write_upper, int w_transposed) {
+    pdl_wait();
     head_linear_mma_body<T, CP, SPLITW>(x, xv, Wm, w_dtype, y, yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,
                                         write_upper, w_transposed);
 }
@@ -303,6 +305,7 @@ __global__ void __launch_bounds__(MMA_WARPS * 32, HL_MIN_CTAS_WIDE)
 head_linear_mma_wide_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
                             T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
                             int row_end, int rows_per_cta, int write_upper, int w_transposed) {
+    pdl_wait();
     head_linear_mma_body<T, CP, SPLITW>(x, xv, Wm, w_dtype, y, yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,
                                         write_upper, w_transposed);
 }

@@ -254,6 +254,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
         for (int i = tid; i < HM_OUT_BYTES / 16; i += HM_THREADS) reinterpret_cast<uint4*>(fill_base)[i] = make_uint4(f2, f2, f2, f2);
     }
     __syncthreads();
+    pdl_wait();
     for (int i = tid; i < 128 * C; i += HM_THREADS) {
         const int m = i / C, h = i % C;
         const int r = m % R, o = m / R;

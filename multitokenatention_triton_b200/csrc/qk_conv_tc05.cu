@@ -132,6 +132,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    pdl_wait();
 
     if (warp == 0) {
         // ---------------- producer: Q tile per row of tiles, K tile per tile ----------------

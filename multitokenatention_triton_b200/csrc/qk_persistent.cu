@@ -136,6 +136,7 @@ qk_persistent_kernel(const __grid_constant__ CUtensorMap ma, const __grid_consta
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    pdl_wait();
 
     if (warp == 0) {
         // ---------------- producer ----------------

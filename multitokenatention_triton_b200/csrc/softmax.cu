@@ -35,6 +35,7 @@ softmax_rows_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y, Pl
                     int row_begin, int write_upper, int cache_elems, float pre_scale, int round_prescaled) {
     extern __shared__ float row[];
     __shared__ float red[SM_THREADS / 32];
+    pdl_wait();
     const int p = row_begin + blockIdx.x;
     const long plane = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(VT)
 softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y, PlaneView yv, int Q, int causal,
                         int row_begin, int write_upper, float pre_scale, int round_prescaled) {
     __shared__ float red[2][VT / 32];
+    pdl_wait();
     const int p = row_begin + blockIdx.x;
     const long plane = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -224,6 +226,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(SB_WARPS * 32)
 softmax_bwd_kernel(const T* __restrict__ p, PlaneView pv, const T* g, PlaneView gv, T* ds, PlaneView dv, int P, int Q, int causal) {
     struct alignas(sizeof(T) * VEC) V { T e[VEC]; };
+    pdl_wait();
     const int row = P - 1 - ((int)blockIdx.x * SB_WARPS + (threadIdx.x >> 5));     // longest rows first
     if (row < 0) return;
     const long plane = blockIdx.y;
