@@ -337,6 +337,12 @@ int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneV
     // 16-bit dtypes with aligned rows: tensor cores (mta_set_variant("conv2d", 1): CUDA cores)
     if (variant("conv2d") != 1 && conv2d_dw_tc05_supported(x, xv, dy, dyv, R, S, dtype))
         return conv2d_dw_tc05_launch(x, xv, dy, dyv, dw, workspace, N, C, H, W, R, S, causal, dtype, st);
+    if (variant("conv2d") != 1 && conv2d_fma_supported(R, S, planes)) {
+        int parts = 0;
+        if (int rc = conv2d_dw_fma_launch(x, xv, dy, dyv, partial, tiles_m * tiles_n, &parts, planes, H, W, R, S, causal, dtype, st)) return rc;
+        return launch_kernel<conv2d_bwd_weight_reduce_kernel>("conv2d_bwd_weight_reduce_kernel", (unsigned)(C * taps), 64, 0, st, partial, dw, N, C,
+                                                              parts, taps);
+    }
     // rows padded to a multiple of 4 floats, plus slack for the last window's 16-byte over-read
     const size_t smem = ((size_t)(WT_M + R - 1) * ((WT_N + S - 1 + 3) & ~3) + 8 + (size_t)(WT_THREADS / 32) * taps) * sizeof(float);
     MTA_REQUIRE(smem <= 200 * 1024, "conv2d_bwd_weight: kernel %dx%d needs %zu bytes of shared memory (max 204800)", R, S, smem);

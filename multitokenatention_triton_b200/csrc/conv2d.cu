@@ -138,6 +138,8 @@ int conv2d_launch(const void* x, PlaneView xv, long x_rows_stored, const void* w
     if (mma_ok && want != 1)
         return conv2d_mma_launch(x, xv, x_rows_stored, w, w_dtype, y, yv, planes, C, H, W, R, S, causal, row_begin,
                                  row_end, write_upper, dtype, st);
+    if (want == 0 && conv2d_fma_supported(R, S, planes))
+        return conv2d_fma_launch(x, xv, w, w_dtype, y, yv, planes, C, H, W, R, S, causal, row_begin, row_end, write_upper, false, dtype, st);
     switch (dtype) {
         case MTA_F32: return launch_tile<float>(x, xv, w, w_dtype, y, yv, planes, C, H, W, R, S, causal, row_begin, row_end, write_upper, st);
         case MTA_BF16: return launch_tile<__nv_bfloat16>(x, xv, w, w_dtype, y, yv, planes, C, H, W, R, S, causal, row_begin, row_end, write_upper, st);
@@ -153,6 +155,8 @@ int conv2d_bwd_input_launch(const void* dy, PlaneView dyv, const void* w, int w_
     // keeps it on the CUDA cores)
     if (variant("conv2d") != 1 && S % 2 == 1 && planes <= 65535 && conv2d_tc05_supported(dy, dyv, dx, dxv, W, R, S, dtype, w_dtype))
         return conv2d_tc05_launch(dy, dyv, H, w, w_dtype, dx, dxv, planes, C, H, W, R, S, causal, 0, H, write_upper, dtype, st, true);
+    if (variant("conv2d") == 0 && conv2d_fma_supported(R, S, planes))
+        return conv2d_fma_launch(dy, dyv, w, w_dtype, dx, dxv, planes, C, H, W, R, S, causal, 0, H, write_upper, true, dtype, st);
     switch (dtype) {
         case MTA_F32: return launch_tile<float>(dy, dyv, w, w_dtype, dx, dxv, planes, C, H, W, R, S, causal, 0, H, write_upper, st, true);
         case MTA_BF16: return launch_tile<__nv_bfloat16>(dy, dyv, w, w_dtype, dx, dxv, planes, C, H, W, R, S, causal, 0, H, write_upper, st, true);

@@ -1,0 +1,322 @@
+// The depthwise conv and its weight gradient on the CUDA cores for the common odd key extents: float32, and 16-bit planes whose
+// rows are not aligned for the tensor-core kernels.  Semantics: conv2d.cu (forward, and the gradient with respect to the input,
+// which is the same sum with the taps reversed and the rows looking forward) and backward.cu (weight gradient).
+//
+// Bound: the FP32 pipe, R * S multiply-adds per position.  All sums run on the packed FMA along the key axis: a pair of
+// neighbouring inputs (x[2p], x[2p+1]) meets the pair of taps that belongs to it - (w[2p], w[2p+1]) for an even output column,
+// (w[2p-1], w[2p]) for an odd one - so no input pair ever has to be re-aligned; both pair tables of a row tap sit side by side
+// in shared memory.  A thread owns 4 rows x 8 columns: per row tap it reads its taps once and four windows of 8 + S - 1 inputs,
+// 32 16-byte loads for 256 packed FMAs at 11 x 15.  The halo tile is staged as fp32 by 4-byte asynchronous copies (all in
+// flight at once) with the causal zero applied on the way; 16-byte chunks are swizzled so that lanes 32 bytes apart hit
+// different banks.
+// Measured at B1 H16 S2048 11x15 float32: 369 us (conv2d_tile_kernel: 591); the FMAs alone would take 160.
+#include "kernels.cuh"
+
+namespace mta {
+namespace {
+
+constexpr int TM = 32, TN = 128;      // output tile of a CTA
+constexpr int THREADS = 128;          // 16 column groups of 8 x 8 row groups of 4
+
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Position of column c in a staged row: 16-byte chunk c / 4 with its lowest bit flipped in every second group of 8 chunks.
+__device__ __forceinline__ int staged_col(int c) { return c ^ ((c >> 3) & 4); }
+
+// Stages rows [q_first, q_first + rows) x keys [k_first, k_first + cols) of a plane; what the conv must not see becomes 0.
+template <typename T>
+__device__ __forceinline__ void stage_tile(float* dst, int pitch, const T* plane, const PlaneView& v, int q_first, int rows, int q_lo, int q_hi,
+                                           int k_first, int cols, int W, int causal, int tid, int nthreads) {
+    const int lane = tid & 31, warp = tid >> 5, warps = nthreads >> 5;
+    for (int r = warp; r < rows; r += warps) {
+        const int q = q_first + r;
+        const bool row_ok = q >= q_lo && q < q_hi;
+        const int last = causal ? min(q, W - 1) : W - 1;
+        const T* src = plane + (long)(q - v.row0) * v.width;
+        float* d = dst + r * pitch;
+#pragma unroll 5
+        for (int c = lane; c < cols; c += 32) {
+            const int k = k_first + c;
+            const bool ok = row_ok && k >= 0 && k <= last;
+            if constexpr (sizeof(T) == 4) copy4(d + staged_col(c), ok ? src + k : plane, ok);
+            else d[staged_col(c)] = ok ? to_f32<T>(src[k]) : 0.0f;
+        }
+    }
+}
+
+template <typename T, int S>
+__global__ void __launch_bounds__(THREADS, 3)
+conv2d_fma_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ w, int w_dtype, T* __restrict__ y, PlaneView yv, int C,
+                  int H, int W, int R, int causal, int row_begin, int row_end, int write_upper, int tiles_n, int grad_input) {
+    constexpr int NP = (S + 1) / 2;                         // tap pairs per row tap
+    constexpr int WIN = 8 + S - 1;                          // inputs a thread needs per row
+    constexpr int COLS = TN + S - 1, PITCH = (COLS + 15) & ~15;
+    extern __shared__ __align__(16) float smem[];
+    pdl_wait();
+    const int th = TM + R - 1;
+    float* xs = smem;                                       // th x PITCH
+    float4* ws = reinterpret_cast<float4*>(smem + th * PITCH);   // R x NP: (even pair, odd pair)
+    const int pad_h = grad_input ? 0 : R - 1, pad_w = grad_input ? S - 1 - (S - 1) / 2 : (S - 1) / 2;
+    const long plane = blockIdx.y;
+    const int tile_m = blockIdx.x / tiles_n, tile_n = blockIdx.x % tiles_n;
+    const int m0 = row_begin + tile_m * TM, n0 = tile_n * TN;
+    const int m_end = min(m0 + TM, row_end);
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    T* yp = y + plane * yv.plane_stride;
+    const bool vec = sizeof(T) == 4 && yv.width % 4 == 0 && yv.plane_stride % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
+    if (causal && n0 > m_end - 1) {                         // tile entirely above the diagonal: nothing to read
+        if (write_upper)
+            for (int r = ty; r < TM; r += 8) {
+                const int q = m0 + r, k = n0 + tx * 8;
+                if (q >= m_end) continue;
+                T* row = yp + (long)(q - yv.row0) * yv.width + k;
+                if (vec && k + 7 < W) {
+                    reinterpret_cast<float4*>(row)[0] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    reinterpret_cast<float4*>(row)[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                } else {
+                    for (int e = 0; e < 8; ++e)
+                        if (k + e < W) row[e] = from_f32<T>(0.0f);
+                }
+            }
+        return;
+    }
+    // rows past m_end feed no output of the forward and need not be in its input view; the input gradient looks forward
+    stage_tile<T>(xs, PITCH, x + plane * xv.plane_stride, xv, m0 - pad_h, th, 0, grad_input ? H : m_end, n0 - pad_w, COLS, W, causal, tid, THREADS);
+    const long w0 = (plane % C) * (long)R * S;
+    for (int e = tid; e < R * NP; e += THREADS) {
+        const int i = e / NP, p = e % NP;
+        auto tap = [&](int j) {
+            if (j < 0 || j >= S) return 0.0f;
+            return load_weight(w, w0 + (grad_input ? R * S - 1 - (i * S + j) : i * S + j), w_dtype);
+        };
+        ws[e] = make_float4(tap(2 * p), tap(2 * p + 1), tap(2 * p - 1), tap(2 * p));
+    }
+    copy_wait_all();
+    __syncthreads();
+
+    float2 acc[4][8];
+#pragma unroll
+    for (int o = 0; o < 4; ++o)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[o][c] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+    for (int i = 0; i < R; ++i) {
+        float4 wr[NP];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) wr[p] = ws[i * NP + p];
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+            const float* row = xs + (ty * 4 + o + i) * PITCH;
+            float2 xw[(WIN + 3) / 4 * 2];
+#pragma unroll
+            for (int m = 0; m < (WIN + 3) / 4; ++m) {
+                const float4 v = *reinterpret_cast<const float4*>(row + staged_col(tx * 8 + 4 * m));
+                xw[2 * m] = make_float2(v.x, v.y);
+                xw[2 * m + 1] = make_float2(v.z, v.w);
+            }
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                const float2 we = make_float2(wr[p].x, wr[p].y), wo = make_float2(wr[p].z, wr[p].w);
+#pragma unroll
+                for (int c = 0; c < 8; c += 2) {
+                    acc[o][c] = __ffma2_rn(xw[c / 2 + p], we, acc[o][c]);
+                    acc[o][c + 1] = __ffma2_rn(xw[c / 2 + p], wo, acc[o][c + 1]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+        const int q = m0 + ty * 4 + o, k = n0 + tx * 8;
+        if (q >= m_end) continue;
+        T* row = yp + (long)(q - yv.row0) * yv.width + k;
+        const int valid = (causal ? min(q, W - 1) : W - 1) - k + 1;          // of the 8 columns, those the conv defines
+        float v[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) v[c] = c < valid ? acc[o][c].x + acc[o][c].y : 0.0f;
+        const int stored = write_upper ? W - k : valid;
+        if (vec && stored >= 8) {
+            reinterpret_cast<float4*>(row)[0] = make_float4(v[0], v[1], v[2], v[3]);
+            reinterpret_cast<float4*>(row)[1] = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (c < stored) row[c] = from_f32<T>(v[c]);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Weight gradient: a warp owns one row tap i of a share of the rows and keeps its S sums in registers over all tiles of a work
+// item, lane = (column group of 8, row parity); the only reduction is one warp sum per tap at the end of the item.  (Summing
+// per tile cost a warp reduction per tap and 4096 positions.)  The taps of odd j pair the inputs with dy shifted by one column.
+constexpr int DW_MAX_WARPS = 16;
+
+template <typename T, int S>
+__global__ void __launch_bounds__(DW_MAX_WARPS * 32)
+conv2d_dw_fma_kernel(const T* __restrict__ x, PlaneView xv, const T* __restrict__ dy, PlaneView dyv, float* __restrict__ partial, int H, int W,
+                     int R, int causal, int tiles_m, int tiles_n, int parts, int row_groups) {
+    constexpr int COLS = TN + S - 1, PITCH = (COLS + 15) & ~15;
+    constexpr int WIN = 8 + S - 1;
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float red[DW_MAX_WARPS][S];
+    pdl_wait();
+    const int th = TM + R - 1, pad_w = (S - 1) / 2;
+    float* xs = smem;                                       // th x PITCH
+    float* gs = smem + th * PITCH;                          // TM x TN
+    const int part = blockIdx.x % parts;
+    const long plane = blockIdx.x / parts;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const int tx = lane & 15, sub = lane >> 4;
+    const T* xp = x + plane * xv.plane_stride;
+    const T* gp = dy + plane * dyv.plane_stride;
+    // warp -> (row tap, row group): taps warp, warp + taps_at_once, ... are done one after the other on the staged tile
+    const int taps_at_once = warps / row_groups, group = warp / taps_at_once, first_tap = warp % taps_at_once;
+    float2 acc[2][S];                                       // at most two row taps per warp
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int j = 0; j < S; ++j) acc[u][j] = make_float2(0.0f, 0.0f);
+    const int tiles = tiles_m * tiles_n;
+    for (int t = part; t < tiles; t += parts) {
+        const int m0 = t / tiles_n * TM, n0 = t % tiles_n * TN;
+        if (causal && n0 > min(m0 + TM, H) - 1) continue;
+        __syncthreads();                                    // the previous tile has been read
+        stage_tile<T>(xs, PITCH, xp, xv, m0 - (R - 1), th, 0, H, n0 - pad_w, COLS, W, causal, tid, blockDim.x);
+        stage_tile<T>(gs, TN, gp, dyv, m0, TM, 0, H, n0, TN, W, causal, tid, blockDim.x);
+        copy_wait_all();
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = first_tap + u * taps_at_once;
+            if (i >= R) continue;
+#pragma unroll 1
+            for (int r = 2 * group + sub; r < TM; r += 2 * row_groups) {
+                const float* grow = gs + r * TN;
+                const float4 g0 = *reinterpret_cast<const float4*>(grow + staged_col(tx * 8)), g1 = *reinterpret_cast<const float4*>(grow + staged_col(tx * 8 + 4));
+                const float2 ge[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w), make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
+                const float2 go[5] = {make_float2(0.0f, g0.x), make_float2(g0.y, g0.z), make_float2(g0.w, g1.x), make_float2(g1.y, g1.z),
+                                      make_float2(g1.w, 0.0f)};
+                const float* row = xs + (r + i) * PITCH;
+                float2 xw[(WIN + 3) / 4 * 2];
+#pragma unroll
+                for (int m = 0; m < (WIN + 3) / 4; ++m) {
+                    const float4 v = *reinterpret_cast<const float4*>(row + staged_col(tx * 8 + 4 * m));
+                    xw[2 * m] = make_float2(v.x, v.y);
+                    xw[2 * m + 1] = make_float2(v.z, v.w);
+                }
+#pragma unroll
+                for (int j = 0; j < S; ++j) {
+                    if (j % 2 == 0) {
+#pragma unroll
+                        for (int p = 0; p < 4; ++p) acc[u][j] = __ffma2_rn(xw[j / 2 + p], ge[p], acc[u][j]);
+                    } else {                                // dy[c] meets x[c + j]: pairs (dy[-1], dy[0]), (dy[1], dy[2]), ...
+#pragma unroll
+                        for (int p = 0; p < 5; ++p) acc[u][j] = __ffma2_rn(xw[(j - 1) / 2 + p], go[p], acc[u][j]);
+                    }
+                }
+            }
+        }
+    }
+    float* out = partial + (plane * parts + part) * (long)R * S;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int i = first_tap + u * taps_at_once;
+        if (i < R) {
+#pragma unroll
+            for (int j = 0; j < S; ++j) {
+                float v = acc[u][j].x + acc[u][j].y;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) red[warp][j] = v;
+            }
+        }
+        __syncthreads();
+        for (int e = tid; e < taps_at_once * S; e += blockDim.x) {
+            const int tap = e / S, j = e % S, ii = tap + u * taps_at_once;
+            if (ii >= R) continue;
+            float v = 0.0f;
+            for (int gr = 0; gr < row_groups; ++gr) v += red[gr * taps_at_once + tap][j];
+            out[ii * S + j] = v;
+        }
+        __syncthreads();
+    }
+}
+
+bool extent_ok(int S) { return S % 2 == 1 && S >= 3 && S <= 15; }
+
+#define MTA_FMA_EXTENTS(CASE)                                                             \
+    switch (S) {                                                                          \
+        case 3: CASE(3); case 5: CASE(5); case 7: CASE(7); case 9: CASE(9);               \
+        case 11: CASE(11); case 13: CASE(13); default: CASE(15);                          \
+    }
+
+template <typename T>
+int launch_conv(const void* x, PlaneView xv, const void* w, int w_dtype, void* y, PlaneView yv, long planes, int C, int H, int W, int R, int S,
+                int causal, int row_begin, int row_end, bool write_upper, bool grad_input, cudaStream_t st) {
+    const int tiles_m = (row_end - row_begin + TM - 1) / TM, tiles_n = (W + TN - 1) / TN;
+    const size_t smem = ((size_t)(TM + R - 1) * ((TN + S - 1 + 15) & ~15) + (size_t)R * ((S + 1) / 2) * 4) * sizeof(float);
+    const dim3 grid((unsigned)(tiles_m * tiles_n), (unsigned)planes);
+#define MTA_CONV_CASE(SV)                                                                                                                \
+    return launch_kernel<conv2d_fma_kernel<T, SV>>("conv2d_fma_kernel", grid, THREADS, smem, st, static_cast<const T*>(x), xv, w, w_dtype, \
+                                                   static_cast<T*>(y), yv, C, H, W, R, causal, row_begin, row_end, write_upper ? 1 : 0,  \
+                                                   tiles_n, grad_input ? 1 : 0)
+    MTA_FMA_EXTENTS(MTA_CONV_CASE)
+#undef MTA_CONV_CASE
+}
+
+// Parts of a plane's tiles: about three CTAs per SM in all, at least two tiles each.
+int dw_parts(long planes, int tiles, int sms) {
+    long parts = (3L * sms + planes - 1) / planes;
+    if (parts > tiles / 2) parts = tiles / 2;
+    return parts < 1 ? 1 : (int)parts;
+}
+
+template <typename T>
+int launch_dw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, long planes, int H, int W, int R, int S, int causal,
+              int parts, cudaStream_t st) {
+    const int tiles_m = (H + TM - 1) / TM, tiles_n = (W + TN - 1) / TN;
+    // up to 8 row taps: as many row groups as fit into 16 warps; up to 16: one warp per tap; more: two taps per warp
+    const int taps_at_once = R <= DW_MAX_WARPS ? R : (R + 1) / 2, row_groups = DW_MAX_WARPS / taps_at_once;
+    const size_t smem = ((size_t)(TM + R - 1) * ((TN + S - 1 + 15) & ~15) + (size_t)TM * TN) * sizeof(float);
+#define MTA_DW_CASE(SV)                                                                                                                     \
+    return launch_kernel<conv2d_dw_fma_kernel<T, SV>>("conv2d_dw_fma_kernel", (unsigned)(planes * parts), (unsigned)(taps_at_once * row_groups * 32), \
+                                                      smem, st, static_cast<const T*>(x), xv, static_cast<const T*>(dy), dyv, partial, H, W, R, \
+                                                      causal, tiles_m, tiles_n, parts, row_groups)
+    MTA_FMA_EXTENTS(MTA_DW_CASE)
+#undef MTA_DW_CASE
+}
+
+}  // namespace
+
+bool conv2d_fma_supported(int R, int S, long planes) { return extent_ok(S) && R <= 32 && planes <= 65535; }
+
+int conv2d_fma_launch(const void* x, PlaneView xv, const void* w, int w_dtype, void* y, PlaneView yv, long planes, int C, int H, int W, int R,
+                      int S, int causal, int row_begin, int row_end, bool write_upper, bool grad_input, int dtype, cudaStream_t st) {
+#define MTA_T(TT) return launch_conv<TT>(x, xv, w, w_dtype, y, yv, planes, C, H, W, R, S, causal, row_begin, row_end, write_upper, grad_input, st)
+    if (dtype == MTA_F32) MTA_T(float);
+    if (dtype == MTA_BF16) MTA_T(__nv_bfloat16);
+    MTA_T(__half);
+#undef MTA_T
+}
+
+// Per-part sums [plane][part][R * S] in `partial`; *parts_out parts per plane, never more than `max_parts`.
+int conv2d_dw_fma_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, int max_parts, int* parts_out, long planes,
+                         int H, int W, int R, int S, int causal, int dtype, cudaStream_t st) {
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
+    const int tiles = ((H + TM - 1) / TM) * ((W + TN - 1) / TN);
+    const int parts = dw_parts(planes, tiles < max_parts ? tiles : max_parts, sms);
+    *parts_out = parts;
+#define MTA_T(TT) return launch_dw<TT>(x, xv, dy, dyv, partial, planes, H, W, R, S, causal, parts, st)
+    if (dtype == MTA_F32) MTA_T(float);
+    if (dtype == MTA_BF16) MTA_T(__nv_bfloat16);
+    MTA_T(__half);
+#undef MTA_T
+}
+
+}  // namespace mta

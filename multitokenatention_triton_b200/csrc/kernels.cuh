@@ -14,6 +14,12 @@ namespace mta {
 int conv2d_launch(const void* x, PlaneView xv, long x_rows_stored, const void* w, int w_dtype, void* y, PlaneView yv,
                   long planes, int C, int H, int W, int R, int S, int causal, int row_begin, int row_end,
                   bool write_upper, int dtype, cudaStream_t st);
+// CUDA cores, odd key extents 3 .. 15 (conv2d_fma.cu): the conv or its input gradient, and the weight gradient's per-part sums.
+bool conv2d_fma_supported(int R, int S, long planes);
+int conv2d_fma_launch(const void* x, PlaneView xv, const void* w, int w_dtype, void* y, PlaneView yv, long planes, int C, int H, int W, int R,
+                      int S, int causal, int row_begin, int row_end, bool write_upper, bool grad_input, int dtype, cudaStream_t st);
+int conv2d_dw_fma_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, int max_parts, int* parts_out, long planes,
+                         int H, int W, int R, int S, int causal, int dtype, cudaStream_t st);
 // Tensor-core version (conv2d_mma.cu): 16-bit dtypes, S <= 17, W a multiple of 8, 16-byte aligned planes.
 bool conv2d_mma_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int W, int R, int S, int dtype);
 int conv2d_mma_launch(const void* x, PlaneView xv, long x_rows_stored, const void* w, int w_dtype, void* y, PlaneView yv,
