@@ -128,57 +128,112 @@ __global__ void conv2d_bwd_weight_reduce_kernel(const float* __restrict__ partia
 }
 
 // ------------------------------------------------------------------------------------------------
+// Weight gradient of the head mix on the CUDA cores.  Bound: the FP32 pipe, C * C multiply-adds per position.  A CTA walks
+// tiles of KT keys of one row for all heads, staged as fp32 in two buffers (float32: asynchronous copies one tile ahead).  A
+// thread owns a 4 x 4 block of (o, h) and every PG-th group of 4 positions: 8 16-byte loads for 32 packed FMAs (the packed
+// halves are neighbouring positions, so both operands are pairs as they lie).  The 16-byte chunks of head r sit at chunk
+// index c ^ ((r / 4 % 4) * 2): the four head blocks of a warp read different banks.  B1 H16 S1024 fp32: 80 us (280 with one
+// (o, h) per thread).
 constexpr int HW_THREADS = 256;
 
-// PPT = (o,h) pairs per thread; KT = keys per tile.  Persistent CTAs walk the (n, row, key block) tiles.
-template <typename T, int PPT, int KT>
+__device__ __forceinline__ int hw_at(int r, int k, int KT) { return r * KT + (k ^ (((r >> 2) & 3) << 3)); }
+
+template <typename T>
 __global__ void __launch_bounds__(HW_THREADS)
 head_linear_bwd_weight_kernel(const T* __restrict__ x, PlaneView xv, const T* __restrict__ dy, PlaneView dyv,
-                              float* __restrict__ partial, int N, int C, int P, int Q, int causal) {
-    extern __shared__ __align__(16) float smem[];
-    float* xs = smem;                   // C x KT
-    float* gs = smem + (size_t)C * KT;  // C x KT
+                              float* __restrict__ partial, int N, int C, int P, int Q, int causal, int KT) {
+    extern __shared__ __align__(16) float smem[];        // two buffers of (dy, x), C4 x KT each
+    pdl_wait();
+    const int CB = (C + 3) / 4, C4 = CB * 4, blocks = CB * CB;
+    const int b_first = blockIdx.y * HW_THREADS, b_here = min(blocks - b_first, HW_THREADS);     // the (o, h) blocks of this CTA
     const int tid = threadIdx.x;
-    const int pairs = C * C;
-    float acc[PPT];
-#pragma unroll
-    for (int i = 0; i < PPT; ++i) acc[i] = 0.0f;
+    const int PG = HW_THREADS / b_here, pg = tid / b_here, blk = b_first + tid % b_here;
+    const int o0 = blk / CB * 4, h0 = blk % CB * 4;
+    const int buf = 2 * C4 * KT;
     const int kblocks = (Q + KT - 1) / KT;
     const long tiles = (long)N * P * kblocks;
-    for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int kb = (int)(tile % kblocks);
-        const int p = (int)((tile / kblocks) % P);
-        const long n = tile / ((long)kblocks * P);
-        const int k0 = kb * KT;
-        if (causal && k0 > p) continue;
-        __syncthreads();                // the previous tile's reads are done
-        for (int idx = tid; idx < C * KT; idx += HW_THREADS) {
-            const int h = idx / KT, kk = idx - h * KT, k = k0 + kk;
-            const bool ok = k < Q && (!causal || k <= p);
-            xs[idx] = ok ? to_f32<T>(x[xv.at(n * C + h, p, k)]) : 0.0f;
-            gs[idx] = ok ? to_f32<T>(dy[dyv.at(n * C + h, p, k)]) : 0.0f;
-        }
-        __syncthreads();
+    float2 acc[4][4];
 #pragma unroll
-        for (int i = 0; i < PPT; ++i) {
-            const int pair = tid + i * HW_THREADS;
-            if (pair >= pairs) break;
-            const int o = pair / C, h = pair - o * C;
-            const float4* a = reinterpret_cast<const float4*>(gs + (size_t)o * KT);
-            const float4* b = reinterpret_cast<const float4*>(xs + (size_t)h * KT);
-            float v = acc[i];
-#pragma unroll 4
-            for (int k4 = 0; k4 < KT / 4; ++k4) {
-                const float4 av = a[k4], bv = b[k4];
-                v = fmaf(av.x, bv.x, fmaf(av.y, bv.y, fmaf(av.z, bv.z, fmaf(av.w, bv.w, v))));
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+    // the next tile from t on that has a visible key (heads C .. C4 - 1 are staged as 0)
+    auto find = [&](long t) {
+        while (t < tiles && causal && (int)(t % kblocks) * KT > (int)(t / kblocks % P)) t += gridDim.x;
+        return t;
+    };
+    auto stage = [&](long t, int which) {
+        if (t >= tiles) return;
+        const int k0 = (int)(t % kblocks) * KT, p = (int)(t / kblocks % P);
+        const long n = t / ((long)kblocks * P);
+        float* gs = smem + which * buf;
+        float* xs = gs + C4 * KT;
+        const int n_keys = min(causal ? min(p + 1, Q) : Q, k0 + KT) - k0;
+        for (int idx = tid; idx < C4 * KT; idx += HW_THREADS) {
+            const int h = idx / KT, kk = idx - h * KT;
+            const bool ok = h < C && kk < n_keys;
+            const T* gp = ok ? dy + dyv.at(n * C + h, p, k0 + kk) : dy;
+            const T* xp = ok ? x + xv.at(n * C + h, p, k0 + kk) : x;
+            const int at = hw_at(h, kk, KT);
+            if constexpr (sizeof(T) == 4) {
+                const int bytes = ok ? 4 : 0;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(gs + at)), "l"(gp), "r"(bytes) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(xs + at)), "l"(xp), "r"(bytes) : "memory");
+            } else {
+                gs[at] = ok ? to_f32<T>(*gp) : 0.0f;
+                xs[at] = ok ? to_f32<T>(*xp) : 0.0f;
             }
-            acc[i] = v;
         }
-    }
+    };
+    long t = find(blockIdx.x);
+    stage(t, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int it = 0; t < tiles; ++it) {
+        const long next = find(t + gridDim.x);
+        stage(next, (it + 1) & 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const int k0 = (int)(t % kblocks) * KT, p = (int)(t / kblocks % P);
+        const int chunks = (min(causal ? min(p + 1, Q) : Q, k0 + KT) - k0 + 3) / 4;       // groups of 4 positions that hold a key
+        const float* gs = smem + (it & 1) * buf;
+        const float* xs = gs + C4 * KT;
+        if (pg < PG) {
+#pragma unroll 1
+            for (int c = pg; c < chunks; c += PG) {
+                float4 a[4], b[4];
 #pragma unroll
-    for (int i = 0; i < PPT; ++i) {
-        const int pair = tid + i * HW_THREADS;
-        if (pair < pairs) partial[(long)blockIdx.x * pairs + pair] = acc[i];
+                for (int i = 0; i < 4; ++i) {
+                    a[i] = *reinterpret_cast<const float4*>(gs + hw_at(o0 + i, c * 4, KT));
+                    b[i] = *reinterpret_cast<const float4*>(xs + hw_at(h0 + i, c * 4, KT));
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        acc[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w),
+                                               __ffma2_rn(make_float2(a[i].x, a[i].y), make_float2(b[j].x, b[j].y), acc[i][j]));
+            }
+        }
+        __syncthreads();                                 // this buffer is refilled next
+        t = next;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    // the position groups' sums, added in group order
+    float* red = smem;                                   // [PG][b_here * 16]
+    if (pg < PG) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) red[(pg * b_here + tid % b_here) * 16 + i * 4 + j] = acc[i][j].x + acc[i][j].y;
+    }
+    __syncthreads();
+    for (int e = tid; e < b_here * 16; e += HW_THREADS) {
+        const int bb = b_first + e / 16, o = bb / CB * 4 + (e & 15) / 4, h = bb % CB * 4 + (e & 3);
+        float v = 0.0f;
+        for (int gq = 0; gq < PG; ++gq) v += red[gq * b_here * 16 + e];
+        if (o < C && h < C) partial[(long)blockIdx.x * C * C + o * C + h] = v;
     }
 }
 
@@ -289,35 +344,37 @@ head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, PlaneView xview, cons
     }
 }
 
-__global__ void head_linear_bwd_weight_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dW, int ctas,
-                                                     int pairs) {
-    const int pair = blockIdx.x * blockDim.x + threadIdx.x;
+// dW = sum of the CTAs' partial sums, in a fixed order, in double: 8 threads per pair take every eighth CTA each (one thread per
+// pair was a chain of 592 dependent loads: 23 to 42 us).
+constexpr int HR_SLICES = 8;
+__global__ void __launch_bounds__(32 * HR_SLICES)
+head_linear_bwd_weight_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dW, int ctas, int pairs) {
+    __shared__ double red[HR_SLICES][32];
     pdl_wait();
-    if (pair >= pairs) return;
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, pair = blockIdx.x * 32 + lane;
     double acc = 0.0;
-    for (int i = 0; i < ctas; ++i) acc += (double)partial[(long)i * pairs + pair];
-    dW[pair] = (float)acc;
+    if (pair < pairs)
+#pragma unroll 8
+        for (int i = slice; i < ctas; i += HR_SLICES) acc += (double)partial[(long)i * pairs + pair];
+    red[slice][lane] = acc;
+    __syncthreads();
+    if (slice == 0 && pair < pairs) {
+        for (int i = 1; i < HR_SLICES; ++i) acc += red[i][lane];
+        dW[pair] = (float)acc;
+    }
 }
 
 int hw_grid(int sms) { return sms * 4; }
 
-template <typename T, int PPT, int KT>
-int launch_hw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, int N, int C, int P, int Q, int causal, int grid, cudaStream_t st) {
-    const size_t smem = 2 * (size_t)C * KT * sizeof(float);
-    if (smem > 48 * 1024)
-        MTA_CUDA_OK(cudaFuncSetAttribute(head_linear_bwd_weight_kernel<T, PPT, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    head_linear_bwd_weight_kernel<T, PPT, KT><<<grid, HW_THREADS, smem, st>>>(static_cast<const T*>(x), xv, static_cast<const T*>(dy), dyv,
-                                                                              partial, N, C, P, Q, causal);
-    MTA_LAUNCH_OK("head_linear_bwd_weight_kernel");
-    return MTA_OK;
-}
-
 template <typename T>
-int dispatch_hw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, int N, int C, int P, int Q, int causal, int grid, cudaStream_t st) {
-    if (C <= 16) return launch_hw<T, 1, 256>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
-    if (C <= 32) return launch_hw<T, 4, 256>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
-    if (C <= 64) return launch_hw<T, 16, 128>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
-    return launch_hw<T, 64, 64>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
+int launch_hw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, int N, int C, int P, int Q, int causal, int grid,
+              cudaStream_t st) {
+    const int CB = (C + 3) / 4;
+    const int KT = C <= 8 ? 512 : (C <= 16 ? 256 : (C <= 32 ? 128 : (C <= 64 ? 64 : 32)));        // 64 KB for the two buffers
+    const size_t smem = (size_t)4 * CB * 4 * KT * sizeof(float);
+    return launch_kernel<head_linear_bwd_weight_kernel<T>>("head_linear_bwd_weight_kernel", dim3((unsigned)grid, (unsigned)((CB * CB + HW_THREADS - 1) / HW_THREADS)),
+                                                           HW_THREADS, smem, st, static_cast<const T*>(x), xv, static_cast<const T*>(dy), dyv, partial, N, C,
+                                                           P, Q, causal, KT);
 }
 
 }  // namespace
@@ -398,13 +455,13 @@ int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, P
         if (dtype == MTA_BF16) { if (C <= 16) MTA_HM_CASE(__nv_bfloat16, 1); else MTA_HM_CASE(__nv_bfloat16, 2); }
         else { if (C <= 16) MTA_HM_CASE(__half, 1); else MTA_HM_CASE(__half, 2); }
 #undef MTA_HM_CASE
-    } else if (dtype == MTA_F32) rc = dispatch_hw<float>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
-    else if (dtype == MTA_BF16) rc = dispatch_hw<__nv_bfloat16>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
-    else rc = dispatch_hw<__half>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
+    } else if (dtype == MTA_F32) rc = launch_hw<float>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
+    else if (dtype == MTA_BF16) rc = launch_hw<__nv_bfloat16>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
+    else rc = launch_hw<__half>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
     if (rc) return rc;
     const int pairs = C * C;
-    return launch_kernel<head_linear_bwd_weight_reduce_kernel>("head_linear_bwd_weight_reduce_kernel", (unsigned)((pairs + 255) / 256), 256, 0, st, partial,
-                                                               dW, grid, pairs);
+    return launch_kernel<head_linear_bwd_weight_reduce_kernel>("head_linear_bwd_weight_reduce_kernel", (unsigned)((pairs + 31) / 32), 32 * HR_SLICES, 0, st,
+                                                               partial, dW, grid, pairs);
 }
 
 }  // namespace mta

@@ -87,12 +87,15 @@ softmax_rows_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y, Pl
         for (int k = n + tid; k < Q; k += SM_THREADS) yr[k] = from_f32<T>(0.0f);
 }
 
-// Vector version for 16-bit dtypes with 16-byte aligned rows: a CTA of 128 threads owns one row and keeps it
-// in registers as NCH chunks of 8 keys per thread (rows of up to NCH*1024 keys), so the row is read once with
-// 16-byte loads and written once with 16-byte stores.
+// Vector version for 16-byte aligned rows: a CTA of 128 threads owns one row and keeps it in registers as NCH 16-byte chunks
+// (8 keys, or 4 of float32) per thread, so the row is read once with 16-byte loads and written once with 16-byte stores
+// (B1 H16 S2048 float32: 67 us, 119 with the general kernel).
 constexpr int VT = 128;
 
-template <typename T> __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]);
+template <typename T> __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[16 / sizeof(T)]);
+template <> __device__ __forceinline__ void unpack8<float>(const uint4& v, float (&f)[4]) {
+    f[0] = __uint_as_float(v.x); f[1] = __uint_as_float(v.y); f[2] = __uint_as_float(v.z); f[3] = __uint_as_float(v.w);
+}
 template <> __device__ __forceinline__ void unpack8<__nv_bfloat16>(const uint4& v, float (&f)[8]) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -126,10 +129,11 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
     const long plane = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = causal ? min(p + 1, Q) : Q;
-    const int nch = (n + 7) >> 3;                       // chunks that hold at least one valid key
+    constexpr int VEC = 16 / (int)sizeof(T);            // keys per chunk
+    const int nch = (n + VEC - 1) / VEC;                // chunks that hold at least one valid key
     const uint4* xr = reinterpret_cast<const uint4*>(x + xv.at(plane, p, 0));
     uint4* yr = reinterpret_cast<uint4*>(y + yv.at(plane, p, 0));
-    float v[NCH][8];
+    float v[NCH][VEC];
     float mx = -INFINITY;
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
@@ -137,10 +141,10 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
         if (ch < nch) {
             unpack8<T>(__ldg(xr + ch), v[c]);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
+            for (int e = 0; e < VEC; ++e) {
                 float t = v[c][e] * pre_scale;
                 if (round_prescaled) t = round_to<T>(t);
-                if (ch * 8 + e >= n) t = -INFINITY;     // keys past the diagonal inside the last chunk
+                if (ch * VEC + e >= n) t = -INFINITY;     // keys past the diagonal inside the last chunk
                 v[c][e] = t;
                 mx = fmaxf(mx, t);
             }
@@ -155,7 +159,7 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
     for (int c = 0; c < NCH; ++c) {
         if (tid + c * VT < nch) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
+            for (int e = 0; e < VEC; ++e) {
                 const float ex = __expf(v[c][e] - mx);   // exp(-inf) = 0 for the masked tail
                 v[c][e] = ex;
                 sum += ex;
@@ -171,22 +175,26 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
         const int ch = tid + c * VT;
         if (ch < nch) {
             uint4 o;
-            o.x = pack2s<T>(v[c][0] * inv, v[c][1] * inv);
-            o.y = pack2s<T>(v[c][2] * inv, v[c][3] * inv);
-            o.z = pack2s<T>(v[c][4] * inv, v[c][5] * inv);
-            o.w = pack2s<T>(v[c][6] * inv, v[c][7] * inv);
-            if (!write_upper && ch * 8 + 8 > n) {       // last chunk: keys past the diagonal stay untouched
+            if constexpr (sizeof(T) == 4) {
+                o = make_uint4(__float_as_uint(v[c][0] * inv), __float_as_uint(v[c][1] * inv), __float_as_uint(v[c][2] * inv), __float_as_uint(v[c][3] * inv));
+            } else {
+                o.x = pack2s<T>(v[c][0] * inv, v[c][1] * inv);
+                o.y = pack2s<T>(v[c][2] * inv, v[c][3] * inv);
+                o.z = pack2s<T>(v[c][4] * inv, v[c][5] * inv);
+                o.w = pack2s<T>(v[c][6] * inv, v[c][7] * inv);
+            }
+            if (!write_upper && ch * VEC + VEC > n) {       // last chunk: keys past the diagonal stay untouched
                 T* dst = reinterpret_cast<T*>(yr + ch);
                 const T* src = reinterpret_cast<const T*>(&o);
-                for (int e = 0; e < 8; ++e)
-                    if (ch * 8 + e < n) dst[e] = src[e];
+                for (int e = 0; e < VEC; ++e)
+                    if (ch * VEC + e < n) dst[e] = src[e];
             } else {
                 yr[ch] = o;
             }
         }
     }
     if (write_upper)
-        for (int ch = nch + tid; ch < ((Q + 7) >> 3); ch += VT) yr[ch] = make_uint4(0u, 0u, 0u, 0u);
+        for (int ch = nch + tid; ch < (Q + VEC - 1) / VEC; ch += VT) yr[ch] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <typename T, int NCH>
@@ -200,10 +208,11 @@ int launch_vec(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, 
 template <typename T>
 int launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int Q, int causal, int row_begin,
            int row_end, bool write_upper, float pre_scale, int round_prescaled, cudaStream_t st) {
-    if constexpr (sizeof(T) == 2) if (Q <= 16 * 8 * VT && xv.plane_stride % 8 == 0 && yv.plane_stride % 8 == 0 &&
-        xv.width % 8 == 0 && yv.width % 8 == 0 && aligned16(x) && aligned16(y)) {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    if (Q <= 16 * VEC * VT && xv.plane_stride % VEC == 0 && yv.plane_stride % VEC == 0 && xv.width % VEC == 0 && yv.width % VEC == 0 && aligned16(x) &&
+        aligned16(y)) {
         const int longest = causal ? (row_end < Q ? row_end : Q) : Q;
-        const int need = (longest + 8 * VT - 1) / (8 * VT);
+        const int need = (longest + VEC * VT - 1) / (VEC * VT);
         if (need <= 1) return launch_vec<T, 1>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, st);
         if (need <= 2) return launch_vec<T, 2>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, st);
         if (need <= 4) return launch_vec<T, 4>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, st);
