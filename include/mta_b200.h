@@ -165,6 +165,17 @@ int mta_fused_fwd(const void* q, const void* k, const void* v, const void* w1, c
                   int w_dtype, void* stream);
 
 /*
+ * mta_fused_fwd (all query rows, causal) for a batch of sequences of different lengths: keys whose byte of key_mask (B,S) is 0
+ * are masked for every query, as MTAAttentionTriton.forward does with use_mask=True and a boolean (batch, keys) mask
+ * (mta_attention_triton.py:63-92, _update_mask :106-127): their scores are zero before the first conv, their probabilities
+ * zero, their weights zero before the product with V.  Needs mta_masked_workspace_bytes(...) bytes of scratch.
+ */
+size_t mta_masked_workspace_bytes(int B, int H, int S, int D, int cq, int ck, int cq2, int ck2, int dtype);
+int mta_masked_fwd(const void* q, const void* k, const void* v, const unsigned char* key_mask, const void* w1, const void* W1,
+                   const void* w2, const void* W2, void* o, void* workspace, size_t workspace_bytes, int B, int H, int S, int D,
+                   int cq, int ck, int cq2, int ck2, int dtype, int w_dtype, void* stream);
+
+/*
  * A training step's share of the MTA module (causal, no mask, no dropout): the forward that keeps what its backward reads,
  * and that backward.  They replace MTAAttentionTriton.forward under autograd (mta_attention_triton.py:61-92 with
  * convolution_2d_trit.py:143-295, triton_linear_head.py:142-278 and torch's backward of the softmax and the two products).

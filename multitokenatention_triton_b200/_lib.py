@@ -47,6 +47,8 @@ SIGNATURES = {
     "mta_conv_attn_fwd_static": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp]),
     "mta_workspace_bytes": (_sz, [_i] * 11),
     "mta_fused_fwd": (_i, [_vp] * 9 + [_sz] + [_i] * 13 + [_vp]),
+    "mta_masked_workspace_bytes": (_sz, [_i] * 9),
+    "mta_masked_fwd": (_i, [_vp] * 10 + [_sz] + [_i] * 10 + [_vp]),
     "mta_train_saved_bytes": (_sz, [_i] * 4),
     "mta_train_workspace_bytes": (_sz, [_i] * 8),
     "mta_train_fwd": (_i, [_vp] * 9 + [_sz] + [_i] * 10 + [_vp]),

@@ -66,6 +66,57 @@ int trace_end(cudaStream_t st) {
     return MTA_OK;
 }
 
+// The forward's launches over the scratch planes of `pl`.
+int run_forward(const void* q, const void* k, const void* v, const void* w1, const void* W1, const void* w2, const void* W2, void* o,
+                void* workspace, const Plan& pl, int B, int H, int S, int D, int cq, int ck, int cq2, int ck2, int causal, int dtype, int w_dtype,
+                DropoutSpec drop, DeadKeys dead, cudaStream_t st) {
+    char* ws = static_cast<char*>(workspace);
+    void* bufA = ws;
+    void* bufB = ws + pl.buf_bytes;
+    const PlaneView pv{(long)(pl.r1 - pl.ra) * pl.pitch, pl.ra, pl.pitch};
+    const long planes = (long)B * H;
+    const float scale = 1.0f / sqrtf((float)D);
+    const int round16 = dtype != MTA_F32;
+    int rc;
+    g_trace_n = 0;
+    // Default for 16-bit dtypes: the scores are computed inside the first conv's kernel and never stored
+    // (mta_set_variant("fused", 3) keeps the two kernels apart, as do the "gemm" and "conv2d" variants).
+    const bool qk_in_conv = variant("fused") == 0 && variant("gemm") == 0 && variant("conv2d") == 0 && planes <= 65535 &&
+                            qk_conv_supported(q, k, bufB, pv, S, D, cq, ck, causal, dtype, w_dtype);
+    if (qk_in_conv) {
+        if ((rc = trace_mark("qk_scores+conv1", st))) return rc;
+        if ((rc = qk_conv_launch(q, k, w1, w_dtype, bufB, pv, B, H, S, D, cq, ck, scale, pl.rb, pl.r1, dtype, st))) return rc;
+    } else {
+    if ((rc = trace_mark("qk_scores", st))) return rc;
+    if ((rc = qk_scores_launch(q, k, bufA, pv, B, H, S, D, scale, round16, causal, pl.ra, pl.r1, dtype, st))) return rc;
+    }
+    if (!qk_in_conv) {
+        if ((rc = trace_mark("conv1", st))) return rc;
+        if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w1, w_dtype, bufB, pv, planes, H, S, S, cq, ck, causal, pl.rb, pl.r1, !causal, dtype, st))) return rc;
+    }
+    // the first head mix and the softmax run as one kernel where it applies (mta_set_variant("fused", 1) keeps them apart); with dead
+    // keys only the tcgen05 one does
+    if (dead.bits && head_mix_softmax_tc05_supported(bufB, pv, bufA, pv, H, S, causal, dtype, w_dtype)) {
+        if ((rc = trace_mark("head_mix1+softmax", st))) return rc;
+        if ((rc = head_mix_softmax_tc05_launch(bufB, pv, W1, bufA, pv, B, H, S, pl.rb, pl.r1, false, dtype, st, dead))) return rc;
+    } else if (!dead.bits && variant("fused") != 1 && head_mix_softmax_supported(bufB, pv, bufA, pv, H, S, causal, dtype, w_dtype)) {
+        if ((rc = trace_mark("head_mix1+softmax", st))) return rc;
+        if ((rc = head_mix_softmax_launch(bufB, pv, W1, w_dtype, bufA, pv, B, H, S, pl.rb, pl.r1, false, dtype, st))) return rc;
+    } else {
+        if ((rc = trace_mark("head_mix1", st))) return rc;
+        if ((rc = head_linear_launch(bufB, pv, W1, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.rb, pl.r1, false, dtype, st))) return rc;
+        if ((rc = trace_mark("softmax", st))) return rc;
+        if ((rc = softmax_launch(bufA, pv, bufA, pv, planes, S, S, causal, pl.rb, pl.r1, false, 1.0f, dtype, st, dead, H))) return rc;
+    }
+    if ((rc = trace_mark("conv2", st))) return rc;
+    if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w2, w_dtype, bufB, pv, planes, H, S, S, cq2, ck2, causal, pl.r0, pl.r1, !causal, dtype, st))) return rc;
+    if ((rc = trace_mark("head_mix2", st))) return rc;
+    if ((rc = head_linear_launch(bufB, pv, W2, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.r0, pl.r1, false, dtype, st))) return rc;
+    if ((rc = trace_mark("pv", st))) return rc;
+    if ((rc = pv_launch(bufA, pv, pl.r1 - pl.ra, v, o, B, H, S, D, causal, pl.r0, pl.r1, dtype, st, drop))) return rc;
+    return trace_end(st);
+}
+
 }  // namespace
 }  // namespace mta
 
@@ -131,48 +182,45 @@ int mta_fused_fwd_dropout(const void* q, const void* k, const void* v, const voi
                 workspace_bytes, pl.total());
     MTA_REQUIRE(aligned16(workspace), "fused_fwd: workspace must be 16-byte aligned");
     if (int rc = check_device()) return rc;
+    return run_forward(q, k, v, w1, W1, w2, W2, o, workspace, pl, B, H, S, D, cq, ck, cq2, ck2, causal, dtype, w_dtype, drop, DeadKeys(),
+                       static_cast<cudaStream_t>(stream));
+}
+
+// Workspace: the two scratch planes, the masked copies of k and v, the bits of the dead keys.
+static size_t masked_copy_bytes(int B, int H, int S, int D, int dtype) { return round_up((size_t)B * H * S * D * dtype_size(dtype), 256); }
+
+size_t mta_masked_workspace_bytes(int B, int H, int S, int D, int cq, int ck, int cq2, int ck2, int dtype) {
+    const size_t planes = mta_workspace_bytes(B, H, S, D, cq, ck, cq2, ck2, 0, S, dtype);
+    if (planes == 0 || D < 1) return 0;
+    return planes + 2 * masked_copy_bytes(B, H, S, D, dtype) + round_up((size_t)B * ((S + 31) / 32) * 4, 256);
+}
+
+int mta_masked_fwd(const void* q, const void* k, const void* v, const unsigned char* key_mask, const void* w1, const void* W1, const void* w2,
+                   const void* W2, void* o, void* workspace, size_t workspace_bytes, int B, int H, int S, int D, int cq, int ck, int cq2, int ck2,
+                   int dtype, int w_dtype, void* stream) {
+    set_error("%s", "");
+    MTA_REQUIRE(dtype_ok(dtype) && dtype_ok(w_dtype), "masked_fwd: unknown dtype code (%d, %d)", dtype, w_dtype);
+    MTA_REQUIRE(B >= 0 && H >= 1 && S >= 0 && D >= 1, "masked_fwd: bad shape B=%d H=%d S=%d D=%d", B, H, S, D);
+    MTA_REQUIRE(cq >= 1 && ck >= 1 && cq2 >= 1 && ck2 >= 1 && ck % 2 == 1 && ck2 % 2 == 1,
+                "masked_fwd: kernel sizes %dx%d and %dx%d must be positive with odd key extents", cq, ck, cq2, ck2);
+    if ((long)B * S == 0) return MTA_OK;
+    MTA_REQUIRE(q && k && v && key_mask && w1 && W1 && w2 && W2 && o, "masked_fwd: null pointer");
+    MTA_REQUIRE((long)B * H <= 65535, "masked_fwd: B*H = %ld exceeds 65535", (long)B * H);
+    const size_t need = mta_masked_workspace_bytes(B, H, S, D, cq, ck, cq2, ck2, dtype);
+    MTA_REQUIRE(workspace && workspace_bytes >= need, "masked_fwd: workspace of %zu bytes is smaller than the %zu needed", workspace_bytes, need);
+    MTA_REQUIRE(aligned16(workspace), "masked_fwd: workspace must be 16-byte aligned");
+    if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    char* ws = static_cast<char*>(workspace);
-    void* bufA = ws;
-    void* bufB = ws + pl.buf_bytes;
-    const PlaneView pv{(long)(pl.r1 - pl.ra) * pl.pitch, pl.ra, pl.pitch};
-    const long planes = (long)B * H;
-    const float scale = 1.0f / sqrtf((float)D);
-    const int round16 = dtype != MTA_F32;
-    int rc;
-    g_trace_n = 0;
-    // Default for 16-bit dtypes: the scores are computed inside the first conv's kernel and never stored
-    // (mta_set_variant("fused", 3) keeps the two kernels apart, as do the "gemm" and "conv2d" variants).
-    const bool qk_in_conv = variant("fused") == 0 && variant("gemm") == 0 && variant("conv2d") == 0 && planes <= 65535 &&
-                            qk_conv_supported(q, k, bufB, pv, S, D, cq, ck, causal, dtype, w_dtype);
-    if (qk_in_conv) {
-        if ((rc = trace_mark("qk_scores+conv1", st))) return rc;
-        if ((rc = qk_conv_launch(q, k, w1, w_dtype, bufB, pv, B, H, S, D, cq, ck, scale, pl.rb, pl.r1, dtype, st))) return rc;
-    } else {
-    if ((rc = trace_mark("qk_scores", st))) return rc;
-    if ((rc = qk_scores_launch(q, k, bufA, pv, B, H, S, D, scale, round16, causal, pl.ra, pl.r1, dtype, st))) return rc;
-    }
-    if (!qk_in_conv) {
-        if ((rc = trace_mark("conv1", st))) return rc;
-        if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w1, w_dtype, bufB, pv, planes, H, S, S, cq, ck, causal, pl.rb, pl.r1, !causal, dtype, st))) return rc;
-    }
-    // the first head mix and the softmax run as one kernel where it applies (mta_set_variant("fused", 1) keeps them apart)
-    if (variant("fused") != 1 && head_mix_softmax_supported(bufB, pv, bufA, pv, H, S, causal, dtype, w_dtype)) {
-        if ((rc = trace_mark("head_mix1+softmax", st))) return rc;
-        if ((rc = head_mix_softmax_launch(bufB, pv, W1, w_dtype, bufA, pv, B, H, S, pl.rb, pl.r1, false, dtype, st))) return rc;
-    } else {
-        if ((rc = trace_mark("head_mix1", st))) return rc;
-        if ((rc = head_linear_launch(bufB, pv, W1, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.rb, pl.r1, false, dtype, st))) return rc;
-        if ((rc = trace_mark("softmax", st))) return rc;
-        if ((rc = softmax_launch(bufA, pv, bufA, pv, planes, S, S, causal, pl.rb, pl.r1, false, 1.0f, dtype, st))) return rc;
-    }
-    if ((rc = trace_mark("conv2", st))) return rc;
-    if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w2, w_dtype, bufB, pv, planes, H, S, S, cq2, ck2, causal, pl.r0, pl.r1, !causal, dtype, st))) return rc;
-    if ((rc = trace_mark("head_mix2", st))) return rc;
-    if ((rc = head_linear_launch(bufB, pv, W2, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.r0, pl.r1, false, dtype, st))) return rc;
-    if ((rc = trace_mark("pv", st))) return rc;
-    if ((rc = pv_launch(bufA, pv, pl.r1 - pl.ra, v, o, B, H, S, D, causal, pl.r0, pl.r1, dtype, st, drop))) return rc;
-    return trace_end(st);
+    const Plan pl = make_plan(B, H, S, cq, cq2, 0, S, dtype, padded_pitch(S, dtype));
+    char* extra = static_cast<char*>(workspace) + pl.total();
+    void* k_masked = extra;
+    void* v_masked = extra + masked_copy_bytes(B, H, S, D, dtype);
+    DeadKeys dead;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(extra + 2 * masked_copy_bytes(B, H, S, D, dtype));
+    dead.bits = bits;
+    dead.words = (S + 31) / 32;
+    if (int rc = mask_prepare_launch(key_mask, k, v, bits, k_masked, v_masked, B, H, S, D, dtype, st)) return rc;
+    return run_forward(q, k_masked, v_masked, w1, W1, w2, W2, o, workspace, pl, B, H, S, D, cq, ck, cq2, ck2, 1, dtype, w_dtype, DropoutSpec(), dead, st);
 }
 
 // One kernel, no scratch: 16-bit dtypes the fused kernel takes (mta_set_variant("fused", 2) keeps the three-launch path).

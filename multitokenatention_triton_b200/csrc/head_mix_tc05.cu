@@ -116,14 +116,17 @@ template <> __device__ __forceinline__ void hm_ld_round32<__half>(uint32_t taddr
 }
 #undef HM_LD_ROUND32
 
+// The first n of 32 keys, as bits.
+__device__ __forceinline__ uint32_t hm_first(int n) { return n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u); }
+
 // Pass 1 on 32 keys of a row: the logits rounded to T, their maximum folded into (m_run, s_run).
 template <typename T>
-__device__ __forceinline__ void hm_stats32(const uint32_t (&pk)[16], int nvalid, float& m_run, float& s_run) {
+__device__ __forceinline__ void hm_stats32(const uint32_t (&pk)[16], uint32_t live, float& m_run, float& s_run) {
     float2 f[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) hm_unpack2<T>(pk[i], f[i].x, f[i].y);
     float cm;
-    if (nvalid >= 32) {
+    if (live == 0xffffffffu) {
         uint32_t mx2 = pk[0];
 #pragma unroll
         for (int i = 1; i < 16; ++i) mx2 = hm_max2<T>(mx2, pk[i]);
@@ -134,8 +137,8 @@ __device__ __forceinline__ void hm_stats32(const uint32_t (&pk)[16], int nvalid,
         cm = -INFINITY;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            if (2 * i >= nvalid) f[i].x = -INFINITY;
-            if (2 * i + 1 >= nvalid) f[i].y = -INFINITY;
+            if (!(live >> (2 * i) & 1u)) f[i].x = -INFINITY;
+            if (!(live >> (2 * i + 1) & 1u)) f[i].y = -INFINITY;
             cm = fmaxf(cm, fmaxf(f[i].x, f[i].y));
         }
     }
@@ -155,12 +158,12 @@ __device__ __forceinline__ void hm_stats32(const uint32_t (&pk)[16], int nvalid,
     s_run += a0.x + a0.y;
 }
 
-// Pass 2 on 32 keys: the logits rounded to T -> probabilities in T, two per word; keys from nvalid on become 0.
+// Pass 2 on 32 keys: the logits rounded to T -> probabilities in T, two per word; keys whose bit of `live` is 0 become 0.
 template <typename T>
-__device__ __forceinline__ void hm_prob32(const uint32_t (&in)[16], int nvalid, float shift, uint32_t (&pk)[16]) {
+__device__ __forceinline__ void hm_prob32(const uint32_t (&in)[16], uint32_t live, float shift, uint32_t (&pk)[16]) {
     const float2 l2 = make_float2(HM_LOG2E, HM_LOG2E), ns = make_float2(-shift, -shift);
     // two copies of the loop: a compiler that turns the masking into selects would spend two of them on every score
-    if (nvalid >= 32) {
+    if (live == 0xffffffffu) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             float2 f;
@@ -174,22 +177,22 @@ __device__ __forceinline__ void hm_prob32(const uint32_t (&in)[16], int nvalid, 
             float2 f;
             hm_unpack2<T>(in[i], f.x, f.y);
             const float2 yv = __ffma2_rn(f, l2, ns);
-            pk[i] = hm_pack2<T>(2 * i < nvalid ? hm_ex2(yv.x) : 0.0f, 2 * i + 1 < nvalid ? hm_ex2(yv.y) : 0.0f);
+            pk[i] = hm_pack2<T>(live >> (2 * i) & 1u ? hm_ex2(yv.x) : 0.0f, live >> (2 * i + 1) & 1u ? hm_ex2(yv.y) : 0.0f);
         }
     }
 }
 
-// The plain head mix on 32 keys: the products rounded to T, two per word; keys from nvalid on become `fill`.
+// The plain head mix on 32 keys: the products rounded to T, two per word; keys whose bit of `live` is 0 become `fill`.
 template <typename T>
-__device__ __forceinline__ void hm_plain32(const uint32_t (&in)[16], int nvalid, float fill, uint32_t (&pk)[16]) {
-    if (nvalid >= 32) {
+__device__ __forceinline__ void hm_plain32(const uint32_t (&in)[16], uint32_t live, float fill, uint32_t (&pk)[16]) {
+    if (live == 0xffffffffu) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) pk[i] = in[i];
     } else {
         const uint32_t f2 = hm_pack2<T>(fill, fill);
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-            pk[i] = (2 * i < nvalid ? in[i] & 0x0000ffffu : f2 & 0x0000ffffu) | (2 * i + 1 < nvalid ? in[i] & 0xffff0000u : f2 & 0xffff0000u);
+            pk[i] = (live >> (2 * i) & 1u ? in[i] & 0x0000ffffu : f2 & 0x0000ffffu) | (live >> (2 * i + 1) & 1u ? in[i] & 0xffff0000u : f2 & 0xffff0000u);
     }
 }
 
@@ -197,6 +200,7 @@ struct HmGeom {
     int N, C, R, Q, row_begin, row_end, groups, write_upper, x_row0, causal, wt;
     float fill;          // value of the entries above the diagonal (plain head mix; the softmax writes 0 there)
     long units;
+    DeadKeys dead;       // softmax only
 };
 
 // Key tiles that the rows of the group starting at p0 reach.
@@ -393,8 +397,8 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&acc_empty[grp]);
                     }
-                    const int nvalid = n_keys - (key0 + c * 32);
-                    if (nvalid > 0) hm_stats32<T>(cur, nvalid, m_run, s_run);
+                    const uint32_t live = hm_first(n_keys - (key0 + c * 32)) & (key0 + c * 32 < g.Q ? ~g.dead.word(n, key0 + c * 32) : 0u);
+                    if (live) hm_stats32<T>(cur, live, m_run, s_run);
                 }
             }
             it += nt;
@@ -444,8 +448,8 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                     const int kb = key0 + c * 32;
                     if (kb >= g.Q || (kb >= unit_keys && !g.write_upper)) continue;
                     uint32_t pk[16];
-                    if constexpr (SOFTMAX) hm_prob32<T>(cur, n_keys - kb, shift, pk);
-                    else hm_plain32<T>(cur, n_keys - kb, g.fill, pk);
+                    if constexpr (SOFTMAX) hm_prob32<T>(cur, hm_first(n_keys - kb) & ~g.dead.word(n, kb), shift, pk);
+                    else hm_plain32<T>(cur, hm_first(n_keys - kb), g.fill, pk);
                     if (gt == 0) bulk_wait_read();                   // the previous store of this buffer has read it
                     named_barrier(2 + grp, 128);
 #pragma unroll
@@ -496,8 +500,9 @@ constexpr size_t HM_SMEM_BYTES = 1024 + HM_A_BYTES + (size_t)HM_NSTAGE * HM_STAG
 
 template <typename T, bool SOFTMAX>
 int launch_hm(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q, int causal, float fill,
-              int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st) {
+              int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st, DeadKeys dead = DeadKeys()) {
     HmGeom g{};
+    g.dead = dead;
     g.N = N; g.C = C; g.R = 128 / C; g.Q = Q; g.row_begin = row_begin; g.row_end = row_end;
     g.groups = (row_end - row_begin + g.R - 1) / g.R;
     g.write_upper = (write_upper && causal) ? 1 : 0;
@@ -542,11 +547,11 @@ bool head_mix_softmax_tc05_supported(const void* x, PlaneView xv, const void* y,
 }
 
 int head_mix_softmax_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q,
-                                 int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st) {
+                                 int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, DeadKeys dead) {
     if (N == 0 || row_end <= row_begin || Q == 0) return MTA_OK;
     if (dtype == MTA_BF16)
-        return launch_hm<__nv_bfloat16, true>(x, xv, Wm, y, yv, N, C, Q, 1, 0.0f, row_begin, row_end, write_upper, false, st);
-    return launch_hm<__half, true>(x, xv, Wm, y, yv, N, C, Q, 1, 0.0f, row_begin, row_end, write_upper, false, st);
+        return launch_hm<__nv_bfloat16, true>(x, xv, Wm, y, yv, N, C, Q, 1, 0.0f, row_begin, row_end, write_upper, false, st, dead);
+    return launch_hm<__half, true>(x, xv, Wm, y, yv, N, C, Q, 1, 0.0f, row_begin, row_end, write_upper, false, st, dead);
 }
 
 bool head_linear_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int dtype, int w_dtype) {

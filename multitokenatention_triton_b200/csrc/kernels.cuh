@@ -7,6 +7,19 @@
 
 namespace mta {
 
+// Keys that no query may see, one bit each (bit k % 32 of word k / 32), `words` words per batch element; null: every key may
+// be seen.
+struct DeadKeys {
+    const uint32_t* bits = nullptr;
+    int words = 0;
+    // The bits of keys [key, key + 32) of batch element n, key a multiple of 32.
+    __device__ uint32_t word(long n, int key) const { return bits ? __ldg(bits + n * words + (key >> 5)) : 0u; }
+};
+// Prepares them from a (B,S) byte mask (0 = dead), together with copies of k and v (B,H,S,D) whose rows of dead keys are zero
+// (mask.cu).  Zero rows of K make the scores of dead keys zero; zero rows of V drop whatever the later stages hold there.
+int mask_prepare_launch(const unsigned char* key_mask, const void* k, const void* v, uint32_t* bits, void* k_out, void* v_out, int B, int H,
+                        int S, int D, int dtype, cudaStream_t st);
+
 // Depthwise causal conv over planes; computes output rows [row_begin,row_end) of every plane.
 // When `write_upper` the entries above the diagonal of those rows are written as 0, otherwise they
 // are left untouched (internal scratch whose upper triangle nobody reads).
@@ -60,7 +73,7 @@ int head_mix_softmax_launch(const void* x, PlaneView xv, const void* Wm, int w_d
 bool head_mix_softmax_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int causal, int dtype,
                                      int w_dtype);
 int head_mix_softmax_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q,
-                                 int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st);
+                                 int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, DeadKeys dead = DeadKeys());
 
 // The plain head mix on the same kernel (one pass): y = Wm x over the head axis (Wm read transposed when `wt`), `fill`
 // above the diagonal when causal (written up to the end of the diagonal's key tile, and up to Q when `write_upper`).
@@ -68,9 +81,10 @@ bool head_linear_tc05_supported(const void* x, PlaneView xv, const void* y, Plan
 int head_linear_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q, int causal,
                             float fill, int row_begin, int row_end, bool write_upper, bool wt, int dtype, cudaStream_t st);
 
-// Causal row softmax of pre_scale * x; rows [row_begin,row_end).
+// Causal row softmax of pre_scale * x; rows [row_begin,row_end).  `dead` (planes of one batch element: `heads`): keys that get
+// probability 0, in a row with no other key too.
 int softmax_launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int P, int Q, int causal,
-                   int row_begin, int row_end, bool write_upper, float pre_scale, int dtype, cudaStream_t st);
+                   int row_begin, int row_end, bool write_upper, float pre_scale, int dtype, cudaStream_t st, DeadKeys dead = DeadKeys(), int heads = 1);
 
 // ds = p (g - sum over the row of g p), keys k <= query when causal; ds may be g.  Nothing above the diagonal is touched.
 int softmax_bwd_launch(const void* p, PlaneView pv, const void* g, PlaneView gv, void* ds, PlaneView dv, long planes, int P, int Q,

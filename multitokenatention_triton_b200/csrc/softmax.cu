@@ -32,7 +32,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 template <typename T>
 __global__ void __launch_bounds__(SM_THREADS)
 softmax_rows_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y, PlaneView yv, int Q, int causal,
-                    int row_begin, int write_upper, int cache_elems, float pre_scale, int round_prescaled) {
+                    int row_begin, int write_upper, int cache_elems, float pre_scale, int round_prescaled, DeadKeys dead, int heads) {
     extern __shared__ float row[];
     __shared__ float red[SM_THREADS / 32];
     pdl_wait();
@@ -44,10 +44,13 @@ softmax_rows_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y, Pl
     T* yr = y + yv.at(plane, p, 0);
     const bool cached = n <= cache_elems;
 
+    const long batch = plane / heads;
+    auto is_dead = [&](int k) { return dead.bits && (dead.word(batch, k) >> (k & 31) & 1u); };
     float mx = -INFINITY;
     for (int k = tid; k < n; k += SM_THREADS) {
         float v = to_f32<T>(xr[k]) * pre_scale;
         if (round_prescaled) v = round_to<T>(v);
+        if (is_dead(k)) v = -INFINITY;
         if (cached) row[k] = v;
         mx = fmaxf(mx, v);
     }
@@ -63,7 +66,7 @@ softmax_rows_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y, Pl
     for (int k = tid; k < n; k += SM_THREADS) {
         float v;
         if (cached) v = row[k];
-        else { v = to_f32<T>(xr[k]) * pre_scale; if (round_prescaled) v = round_to<T>(v); }
+        else { v = to_f32<T>(xr[k]) * pre_scale; if (round_prescaled) v = round_to<T>(v); if (is_dead(k)) v = -INFINITY; }
         const float e = (mx == -INFINITY) ? 0.0f : __expf(v - mx);
         if (cached) row[k] = e;
         sum += e;
@@ -74,13 +77,13 @@ softmax_rows_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y, Pl
     sum = 0.0f;
 #pragma unroll
     for (int i = 0; i < SM_THREADS / 32; ++i) sum += red[i];
-    const float inv = 1.0f / sum;
+    const float inv = dead.bits && sum == 0.0f ? 0.0f : 1.0f / sum;
 
     // x may alias y: every thread re-reads only the elements it writes.
     for (int k = tid; k < n; k += SM_THREADS) {
         float e;
         if (cached) e = row[k];
-        else { float v = to_f32<T>(xr[k]) * pre_scale; if (round_prescaled) v = round_to<T>(v); e = __expf(v - mx); }
+        else { float v = to_f32<T>(xr[k]) * pre_scale; if (round_prescaled) v = round_to<T>(v); e = is_dead(k) ? 0.0f : __expf(v - mx); }
         yr[k] = from_f32<T>(e * inv);
     }
     if (write_upper)
@@ -122,7 +125,7 @@ template <> __device__ __forceinline__ uint32_t pack2s<__half>(float lo, float h
 template <typename T, int NCH>
 __global__ void __launch_bounds__(VT)
 softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y, PlaneView yv, int Q, int causal,
-                        int row_begin, int write_upper, float pre_scale, int round_prescaled) {
+                        int row_begin, int write_upper, float pre_scale, int round_prescaled, DeadKeys dead, int heads) {
     __shared__ float red[2][VT / 32];
     pdl_wait();
     const int p = row_begin + blockIdx.x;
@@ -133,6 +136,7 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
     const int nch = (n + VEC - 1) / VEC;                // chunks that hold at least one valid key
     const uint4* xr = reinterpret_cast<const uint4*>(x + xv.at(plane, p, 0));
     uint4* yr = reinterpret_cast<uint4*>(y + yv.at(plane, p, 0));
+    const long batch = plane / heads;
     float v[NCH][VEC];
     float mx = -INFINITY;
 #pragma unroll
@@ -140,11 +144,12 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
         const int ch = tid + c * VT;
         if (ch < nch) {
             unpack8<T>(__ldg(xr + ch), v[c]);
+            const uint32_t dw = dead.word(batch, ch * VEC) >> (ch * VEC & 31);
 #pragma unroll
             for (int e = 0; e < VEC; ++e) {
                 float t = v[c][e] * pre_scale;
                 if (round_prescaled) t = round_to<T>(t);
-                if (ch * VEC + e >= n) t = -INFINITY;     // keys past the diagonal inside the last chunk
+                if (ch * VEC + e >= n || (dw >> e & 1u)) t = -INFINITY;     // keys past the diagonal inside the last chunk
                 v[c][e] = t;
                 mx = fmaxf(mx, t);
             }
@@ -160,7 +165,7 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
         if (tid + c * VT < nch) {
 #pragma unroll
             for (int e = 0; e < VEC; ++e) {
-                const float ex = __expf(v[c][e] - mx);   // exp(-inf) = 0 for the masked tail
+                const float ex = dead.bits && mx == -INFINITY ? 0.0f : __expf(v[c][e] - mx);   // exp(-inf) = 0 for the masked tail
                 v[c][e] = ex;
                 sum += ex;
             }
@@ -169,7 +174,8 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
     sum = warp_sum(sum);
     if (lane == 0) red[1][warp] = sum;
     __syncthreads();
-    const float inv = 1.0f / (red[1][0] + red[1][1] + red[1][2] + red[1][3]);
+    sum = red[1][0] + red[1][1] + red[1][2] + red[1][3];
+    const float inv = dead.bits && sum == 0.0f ? 0.0f : 1.0f / sum;
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
         const int ch = tid + c * VT;
@@ -199,31 +205,31 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
 
 template <typename T, int NCH>
 int launch_vec(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int Q, int causal, int row_begin,
-               int row_end, bool write_upper, float pre_scale, int round_prescaled, cudaStream_t st) {
+               int row_end, bool write_upper, float pre_scale, int round_prescaled, DeadKeys dead, int heads, cudaStream_t st) {
     dim3 grid((unsigned)(row_end - row_begin), (unsigned)planes);
     return launch_kernel<softmax_rows_vec_kernel<T, NCH>>("softmax_rows_vec_kernel", grid, VT, 0, st, static_cast<const T*>(x), xv,
-                                                          static_cast<T*>(y), yv, Q, causal, row_begin, write_upper ? 1 : 0, pre_scale, round_prescaled);
+                                                          static_cast<T*>(y), yv, Q, causal, row_begin, write_upper ? 1 : 0, pre_scale, round_prescaled, dead, heads);
 }
 
 template <typename T>
 int launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int Q, int causal, int row_begin,
-           int row_end, bool write_upper, float pre_scale, int round_prescaled, cudaStream_t st) {
+           int row_end, bool write_upper, float pre_scale, int round_prescaled, DeadKeys dead, int heads, cudaStream_t st) {
     constexpr int VEC = 16 / (int)sizeof(T);
     if (Q <= 16 * VEC * VT && xv.plane_stride % VEC == 0 && yv.plane_stride % VEC == 0 && xv.width % VEC == 0 && yv.width % VEC == 0 && aligned16(x) &&
         aligned16(y)) {
         const int longest = causal ? (row_end < Q ? row_end : Q) : Q;
         const int need = (longest + VEC * VT - 1) / (VEC * VT);
-        if (need <= 1) return launch_vec<T, 1>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, st);
-        if (need <= 2) return launch_vec<T, 2>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, st);
-        if (need <= 4) return launch_vec<T, 4>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, st);
-        if (need <= 8) return launch_vec<T, 8>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, st);
-        return launch_vec<T, 16>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, st);
+        if (need <= 1) return launch_vec<T, 1>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, dead, heads, st);
+        if (need <= 2) return launch_vec<T, 2>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, dead, heads, st);
+        if (need <= 4) return launch_vec<T, 4>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, dead, heads, st);
+        if (need <= 8) return launch_vec<T, 8>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, dead, heads, st);
+        return launch_vec<T, 16>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, round_prescaled, dead, heads, st);
     }
     const int cache = Q < ROW_CACHE ? Q : ROW_CACHE;
     const size_t smem = (size_t)cache * sizeof(float);
     const dim3 grid((unsigned)(row_end - row_begin), (unsigned)planes);
     return launch_kernel<softmax_rows_kernel<T>>("softmax_rows_kernel", grid, SM_THREADS, smem, st, static_cast<const T*>(x), xv, static_cast<T*>(y),
-                                                 yv, Q, causal, row_begin, write_upper ? 1 : 0, cache, pre_scale, round_prescaled);
+                                                 yv, Q, causal, row_begin, write_upper ? 1 : 0, cache, pre_scale, round_prescaled, dead, heads);
 }
 
 // Gradient of the causal row softmax: ds = p (g - sum_k g p) over keys k <= query, fp32 arithmetic; nothing is read or written
@@ -296,14 +302,14 @@ int softmax_bwd_launch(const void* p, PlaneView pv, const void* g, PlaneView gv,
 }
 
 int softmax_launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int P, int Q, int causal,
-                   int row_begin, int row_end, bool write_upper, float pre_scale, int dtype, cudaStream_t st) {
+                   int row_begin, int row_end, bool write_upper, float pre_scale, int dtype, cudaStream_t st, DeadKeys dead, int heads) {
     (void)P;
     if (planes == 0 || row_end <= row_begin || Q == 0) return MTA_OK;
     MTA_REQUIRE(planes <= 65535, "softmax: N*C = %ld exceeds 65535", planes);
     switch (dtype) {
-        case MTA_F32: return launch<float>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, (dtype != MTA_F32 && pre_scale != 1.0f) ? 1 : 0, st);
-        case MTA_BF16: return launch<__nv_bfloat16>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, (dtype != MTA_F32 && pre_scale != 1.0f) ? 1 : 0, st);
-        default: return launch<__half>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, (dtype != MTA_F32 && pre_scale != 1.0f) ? 1 : 0, st);
+        case MTA_F32: return launch<float>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, (dtype != MTA_F32 && pre_scale != 1.0f) ? 1 : 0, dead, heads, st);
+        case MTA_BF16: return launch<__nv_bfloat16>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, (dtype != MTA_F32 && pre_scale != 1.0f) ? 1 : 0, dead, heads, st);
+        default: return launch<__half>(x, xv, y, yv, planes, Q, causal, row_begin, row_end, write_upper, pre_scale, (dtype != MTA_F32 && pre_scale != 1.0f) ? 1 : 0, dead, heads, st);
     }
 }
 

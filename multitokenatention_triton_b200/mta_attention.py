@@ -91,6 +91,9 @@ class MTAAttentionTriton(nn.Module):
         planes, the mask applied around the two convs and before the softmax exactly where the reference applies it.
         The convs, head mixes, softmax and the two contractions are this library's kernels; the mask arithmetic
         (masked_fill, add, where) is elementwise torch."""
+        out = self._forward_with_key_mask(xq, xk, xv, mask)
+        if out is not None:
+            return out
         mask = self._update_mask(mask=mask, bsz=xq.size(0), xq=xq, xk_size=xk.size(-2))
         dead = mask == float("-inf")
         head_dim = xq.size(-1)
@@ -105,6 +108,25 @@ class MTAAttentionTriton(nn.Module):
         scores = F.dropout(scores, p=self.dropout, training=self.training)
         output = ops.pv_fwd(scores, xv, causal=False)
         return output.transpose(1, 2)
+
+    def _forward_with_key_mask(self, xq, xk, xv, mask):
+        """The two masks that leave the causal triangle as it is - None and a boolean (bsz, keys) one - take the fused causal
+        forward, the second with its dead keys; None when the call needs the general path (another mask, a gradient,
+        dropout, non-causal modules, cross attention, even key extents)."""
+        w1, w2 = self.mta_conv_triton.effective_weight(), self.mta_conv_after_sm_triton.effective_weight()
+        if not (self.causal and self.fused and xq.is_cuda and xk.shape == xq.shape and xv.shape == xq.shape and w1.size(-1) % 2 and w2.size(-1) % 2):
+            return None
+        if (self.training and self.dropout > 0.0) or (torch.is_grad_enabled() and any(t.requires_grad for t in (xq, xk, xv, *self.parameters()))):
+            return None
+        weights = (w1, self.wpsm_triton.weight, w2, self.wposm_triton.weight)
+        if not isinstance(mask, torch.Tensor):
+            return ops.mta_fused_fwd(xq, xk, xv, *weights, causal=True).transpose(1, 2)
+        if mask.dtype != torch.bool or mask.dim() != 2:
+            return None
+        assert mask.size(0) == xq.size(0)
+        if mask.size(1) != xq.size(-2):
+            return None
+        return ops.mta_masked_fwd(xq, xk, xv, mask.to(xq.device), *weights).transpose(1, 2)
 
     def _update_mask(self, mask, bsz: int, xq, xk_size: int):
         """The reference's mask normalisation (mta_attention_triton.py:106-127): None -> the causal mask; bool -> 0 / -inf;
@@ -124,8 +146,8 @@ class MTAAttentionTriton(nn.Module):
                 # (bsz, keys) -> (bsz, heads, queries, keys); the reference's repeat on the 2-D tensor is only
                 # shape-correct for bsz == 1, this is the same mask for that case and the evident intent otherwise
                 mask = mask[:, None, None, :].repeat(1, self.n_heads, xq.size(-2), 1)
-                mask_i, mask_j = torch.triu_indices(xq.size(-2), xk_size, offset=1)
-                mask[:, :, mask_i, mask_j] = float("-inf")
+                above = torch.ones(xq.size(-2), xk_size, dtype=torch.bool, device=mask.device).triu(1)
+                mask.masked_fill_(above, float("-inf"))
             else:
                 if mask.size(0) == 1 and mask.size(1) == 1:
                     mask = mask.repeat(bsz, self.n_heads, 1, 1)

@@ -244,6 +244,23 @@ def _mta_weights(q, w1, W1, w2, W2):
     return w if w[1].dtype == d and w[2].dtype == d and w[3].dtype == d else [t.detach().float() for t in w]
 
 
+def mta_masked_fwd(q, k, v, key_mask, w1, W1, w2, W2) -> torch.Tensor:
+    """The causal MTA forward with a boolean (B, keys) mask (False = masked for every query): (B,H,S,D)."""
+    q, k, v, key_mask = _cuda_contig(q, "xq"), _cuda_contig(k, "xk"), _cuda_contig(v, "xv"), _cuda_contig(key_mask, "mask")
+    B, H, S, D = q.shape
+    assert k.shape == q.shape and v.shape == q.shape and key_mask.shape == (B, S) and key_mask.dtype == torch.bool
+    w = _mta_weights(q, w1, W1, w2, W2)
+    out = torch.empty_like(q)
+    code = dtype_code(q)
+    nbytes = _size("mta_masked_workspace_bytes", B, H, S, D, *w1.shape[1:], *w2.shape[1:], code)
+    ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
+    with on_device(q.device):
+        check(lib().mta_masked_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), key_mask.data_ptr(), *(t.data_ptr() for t in w), out.data_ptr(),
+                                   ws.data_ptr(), ws.numel(), B, H, S, D, *w1.shape[1:], *w2.shape[1:], code, dtype_code(w[0]),
+                                   stream_ptr(q.device)), "mta_masked_fwd")
+    return out
+
+
 def mta_train_fwd(q, k, v, w1, W1, w2, W2) -> Tuple[torch.Tensor, torch.Tensor]:
     """The causal MTA forward of a training step: (output (B,H,S,D), the score planes that mta_train_bwd reads)."""
     q, k, v = _cuda_contig(q, "xq"), _cuda_contig(k, "xk"), _cuda_contig(v, "xv")
