@@ -237,113 +237,6 @@ head_linear_bwd_weight_kernel(const T* __restrict__ x, PlaneView xv, const T* __
     }
 }
 
-// Tensor-core version for 16-bit dtypes and C <= 32: dW = dY X^T with the positions as the contraction index of
-// mma.sync m16n8k16 (A = dy, rows = output heads; B = x, columns = input heads).  The contraction index may be
-// assigned to positions in any order as long as A and B agree, so lane (g,t) reads 16 bytes (8 consecutive keys
-// 8t .. 8t+7 of a 32-key group) from planes g and g+8 of dy and of x, and word w of those vectors feeds k-slots
-// {2t,2t+1} (w even) or {2t+8,2t+9} (w odd) of MMA w/2.  A warp owns (batch element, row, 128-key block) items and
-// accumulates over all of them in registers; MT = 16-head tiles per side.
-template <typename T> struct MmaK16;
-template <> struct MmaK16<__nv_bfloat16> {
-    static __device__ __forceinline__ void run(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    }
-};
-template <> struct MmaK16<__half> {
-    static __device__ __forceinline__ void run(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    }
-};
-
-constexpr int HM_WARPS = 4;
-constexpr int HM_KEYS = 128;       // keys per item
-
-template <typename T, int MT>
-__global__ void __launch_bounds__(HM_WARPS * 32)
-head_linear_bwd_weight_mma_kernel(const T* __restrict__ x, PlaneView xview, const T* __restrict__ dy, PlaneView dyview,
-                                  float* __restrict__ partial, int N, int C, int P, int Q, int causal) {
-    constexpr int CP = 16 * MT, NV = 2 * MT;            // padded heads; 16-byte vectors per lane, side and 32-key group
-    __shared__ float red[HM_WARPS][CP * CP];
-    pdl_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    float acc[MT][2 * MT][4];                            // [16-row tile of o][8-column tile of h][fragment]
-#pragma unroll
-    for (int a = 0; a < MT; ++a)
-#pragma unroll
-        for (int b = 0; b < 2 * MT; ++b) acc[a][b][0] = acc[a][b][1] = acc[a][b][2] = acc[a][b][3] = 0.0f;
-    const int kblocks = (Q + HM_KEYS - 1) / HM_KEYS;
-    const long items = (long)N * P * kblocks;
-    for (long item = (long)blockIdx.x * HM_WARPS + warp; item < items; item += (long)gridDim.x * HM_WARPS) {
-        const int kb = (int)(item % kblocks);
-        const int p = (int)((item / kblocks) % P);
-        const long n = item / ((long)kblocks * P);
-        const int k0 = kb * HM_KEYS;
-        if (causal && k0 > p) continue;
-        const int n_keys = causal ? min(p + 1, Q) : Q;   // keys of this row that carry a gradient
-        const T* g_row = dy + n * C * dyview.plane_stride + (long)p * dyview.width;
-        const T* x_row = x + n * C * xview.plane_stride + (long)p * xview.width;
-        uint4 gv[4][NV], xv[4][NV];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int kq = k0 + 32 * j + 8 * t;
-#pragma unroll
-            for (int r = 0; r < NV; ++r) {
-                const int head = g + 8 * r;
-                if (head < C && kq < n_keys) {
-                    gv[j][r] = __ldg(reinterpret_cast<const uint4*>(g_row + head * dyview.plane_stride + kq));
-                    xv[j][r] = __ldg(reinterpret_cast<const uint4*>(x_row + head * xview.plane_stride + kq));
-                } else {
-                    gv[j][r] = make_uint4(0u, 0u, 0u, 0u);
-                    xv[j][r] = make_uint4(0u, 0u, 0u, 0u);
-                }
-                if (kq + 8 > n_keys && kq < n_keys) {     // the vector that holds the last valid key: zero what lies beyond it
-                    uint32_t* wd = &gv[j][r].x;
-                    uint32_t* wx = &xv[j][r].x;
-#pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        if (kq + e >= n_keys) {
-                            wd[e >> 1] &= (e & 1) ? 0x0000ffffu : 0xffff0000u;
-                            wx[e >> 1] &= (e & 1) ? 0x0000ffffu : 0xffff0000u;
-                        }
-                }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int a = 0; a < MT; ++a)
-#pragma unroll
-                    for (int b = 0; b < 2 * MT; ++b) {
-                        const uint32_t* ga = &gv[j][2 * a].x;       // dy of head 16a + g
-                        const uint32_t* gb = &gv[j][2 * a + 1].x;   // dy of head 16a + g + 8
-                        const uint32_t* xb = &xv[j][b].x;           // x of head 8b + g
-                        MmaK16<T>::run(acc[a][b], ga[2 * m], gb[2 * m], ga[2 * m + 1], gb[2 * m + 1], xb[2 * m], xb[2 * m + 1]);
-                    }
-    }
-    // fragment (a, b): c0 c1 = (o = 16a + g, h = 8b + 2t, + 1), c2 c3 = (o + 8, same h)
-#pragma unroll
-    for (int a = 0; a < MT; ++a)
-#pragma unroll
-        for (int b = 0; b < 2 * MT; ++b)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int o = 16 * a + g + ((r & 2) ? 8 : 0), h = 8 * b + 2 * t + (r & 1);
-                red[warp][o * CP + h] = acc[a][b][r];
-            }
-    __syncthreads();
-    for (int i = threadIdx.x; i < CP * CP; i += HM_WARPS * 32) {
-        const int o = i / CP, h = i % CP;
-        if (o < C && h < C) partial[(long)blockIdx.x * C * C + o * C + h] = red[0][i] + red[1][i] + red[2][i] + red[3][i];
-    }
-}
-
 // dW = sum of the CTAs' partial sums, in a fixed order, in double: 8 threads per pair take every eighth CTA each (one thread per
 // pair was a chain of 592 dependent loads: 23 to 42 us).
 constexpr int HR_SLICES = 8;
@@ -446,22 +339,17 @@ int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, P
     const int grid = hw_grid(sms);
     float* partial = static_cast<float*>(workspace);
     int rc;
-    const bool vec_ok = dtype != MTA_F32 && C <= 32 && aligned16(x) && aligned16(dy) && xv.width % 8 == 0 && dyv.width % 8 == 0 &&
-                        xv.plane_stride % 8 == 0 && dyv.plane_stride % 8 == 0;
-    if (vec_ok && variant("head_linear") != 1) {         // tensor cores (mta_set_variant("head_linear", 1): CUDA cores)
-#define MTA_HM_CASE(TT, MTV)                                                                                                            \
-    rc = launch_kernel<head_linear_bwd_weight_mma_kernel<TT, MTV>>("head_linear_bwd_weight_mma_kernel", (unsigned)grid, HM_WARPS * 32, 0, st, \
-                                                                   static_cast<const TT*>(x), xv, static_cast<const TT*>(dy), dyv, partial, N, C, P, Q, causal)
-        if (dtype == MTA_BF16) { if (C <= 16) MTA_HM_CASE(__nv_bfloat16, 1); else MTA_HM_CASE(__nv_bfloat16, 2); }
-        else { if (C <= 16) MTA_HM_CASE(__half, 1); else MTA_HM_CASE(__half, 2); }
-#undef MTA_HM_CASE
+    int slots = grid;                                     // sums of C * C floats in `partial`
+    // 16-bit dtypes with aligned rows: tensor cores (mta_set_variant("head_linear", 1): CUDA cores)
+    if (variant("head_linear") != 1 && head_dw_tc05_supported(x, xv, dy, dyv, C, dtype)) {
+        rc = head_dw_tc05_launch(x, xv, dy, dyv, partial, &slots, N, C, P, Q, causal, dtype, st);
     } else if (dtype == MTA_F32) rc = launch_hw<float>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
     else if (dtype == MTA_BF16) rc = launch_hw<__nv_bfloat16>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
     else rc = launch_hw<__half>(x, xv, dy, dyv, partial, N, C, P, Q, causal, grid, st);
     if (rc) return rc;
     const int pairs = C * C;
     return launch_kernel<head_linear_bwd_weight_reduce_kernel>("head_linear_bwd_weight_reduce_kernel", (unsigned)((pairs + 31) / 32), 32 * HR_SLICES, 0, st,
-                                                               partial, dW, grid, pairs);
+                                                               partial, dW, slots, pairs);
 }
 
 }  // namespace mta

@@ -61,6 +61,11 @@ size_t head_linear_bwd_weight_workspace(int C);
 int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dW, void* workspace, int N, int C,
                                   int P, int Q, int causal, int dtype, cudaStream_t st);
 
+// The head mix's weight gradient on tcgen05 (head_dw_tc05.cu).
+bool head_dw_tc05_supported(const void* x, PlaneView xv, const void* dy, PlaneView dyv, int C, int dtype);
+int head_dw_tc05_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, int* slots_out, int N, int C, int P, int Q,
+                        int causal, int dtype, cudaStream_t st);
+
 // Head mix followed by the causal row softmax of the mixed logits, in one pass (16-bit dtypes, C <= 32, causal);
 // entries above the diagonal of y are written as 0 when `write_upper`, else left untouched.
 bool head_mix_softmax_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int causal, int dtype,
