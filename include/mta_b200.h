@@ -140,6 +140,12 @@ int mta_conv2d_bwd_input(const void* dy, const void* w, void* dx, int N, int C, 
 size_t mta_conv2d_bwd_weight_workspace_bytes(int N, int C, int H, int W, int R, int S);
 int mta_conv2d_bwd_weight(const void* x, const void* dy, float* dw, void* workspace, size_t workspace_bytes, int N, int C,
                           int H, int W, int R, int S, int causal, int dtype, void* stream);
+/* The two weight gradients with the result in a dtype of the caller's choice (rounded once, from the double sum through
+ * float32). */
+int mta_conv2d_bwd_weight_as(const void* x, const void* dy, void* dw, int dw_dtype, void* workspace, size_t workspace_bytes, int N,
+                             int C, int H, int W, int R, int S, int causal, int dtype, void* stream);
+int mta_head_linear_bwd_weight_as(const void* x, const void* dy, void* dW, int dw_dtype, void* workspace, size_t workspace_bytes,
+                                  int N, int C, int P, int Q, int causal, int dtype, void* stream);
 int mta_head_linear_bwd_input(const void* dy, const void* Wm, void* dx, int N, int C, int P, int Q, int causal, int dtype,
                               int w_dtype, void* stream);
 size_t mta_head_linear_bwd_weight_workspace_bytes(int C);
@@ -182,19 +188,20 @@ int mta_masked_fwd(const void* q, const void* k, const void* v, const unsigned c
  *   saved      mta_train_saved_bytes(...) bytes: five score planes (scores, conv 1, probabilities, conv 2, head mix 2) with
  *              padded rows, written by mta_train_fwd, only read by mta_train_bwd; the part above the diagonal is undefined
  *   workspace  mta_train_workspace_bytes(...) bytes of scratch
- *   dout       gradient of o, (B,H,S,D) contiguous in `dtype`; dq, dk, dv: the same; dw1 (H,cq,ck), dW1 (H,H),
- *              dw2 (H,cq2,ck2), dW2 (H,H): float32.  A gradient whose pointer is NULL is not computed.
+ *   dout       gradient of o in `dtype`: (B,H,S,D) contiguous, or (B,S,H,D) contiguous with dout_heads_inner != 0;
+ *              dq, dk, dv: (B,H,S,D) in `dtype`; dw1 (H,cq,ck), dW1 (H,H), dw2 (H,cq2,ck2), dW2 (H,H): `w_dtype`.  A gradient
+ *              whose pointer is NULL is not computed.
  * ck and ck2 must be odd, H at most 128.  Accumulation is fp32 (weight gradients: fp32 per block, double across blocks).
  */
 size_t mta_train_saved_bytes(int B, int H, int S, int dtype);
-size_t mta_train_workspace_bytes(int B, int H, int S, int cq, int ck, int cq2, int ck2, int dtype);
+size_t mta_train_workspace_bytes(int B, int H, int S, int D, int cq, int ck, int cq2, int ck2, int dtype);
 int mta_train_fwd(const void* q, const void* k, const void* v, const void* w1, const void* W1, const void* w2,
                   const void* W2, void* o, void* saved, size_t saved_bytes, int B, int H, int S, int D, int cq, int ck,
                   int cq2, int ck2, int dtype, int w_dtype, void* stream);
 int mta_train_bwd(const void* q, const void* k, const void* v, const void* w1, const void* W1, const void* w2,
-                  const void* W2, const void* dout, const void* saved, void* dq, void* dk, void* dv, float* dw1,
-                  float* dW1, float* dw2, float* dW2, void* workspace, size_t workspace_bytes, int B, int H, int S, int D,
-                  int cq, int ck, int cq2, int ck2, int dtype, int w_dtype, void* stream);
+                  const void* W2, const void* dout, const void* saved, void* dq, void* dk, void* dv, void* dw1,
+                  void* dW1, void* dw2, void* dW2, void* workspace, size_t workspace_bytes, int B, int H, int S, int D,
+                  int cq, int ck, int cq2, int ck2, int dout_heads_inner, int dtype, int w_dtype, void* stream);
 
 /*
  * mta_fused_fwd with dropout on the attention weights between the second head mix and the product with V, where

@@ -50,9 +50,11 @@ SIGNATURES = {
     "mta_masked_workspace_bytes": (_sz, [_i] * 9),
     "mta_masked_fwd": (_i, [_vp] * 10 + [_sz] + [_i] * 10 + [_vp]),
     "mta_train_saved_bytes": (_sz, [_i] * 4),
-    "mta_train_workspace_bytes": (_sz, [_i] * 8),
+    "mta_train_workspace_bytes": (_sz, [_i] * 9),
     "mta_train_fwd": (_i, [_vp] * 9 + [_sz] + [_i] * 10 + [_vp]),
-    "mta_train_bwd": (_i, [_vp] * 17 + [_sz] + [_i] * 10 + [_vp]),
+    "mta_train_bwd": (_i, [_vp] * 17 + [_sz] + [_i] * 11 + [_vp]),
+    "mta_conv2d_bwd_weight_as": (_i, [_vp, _vp, _vp, _i, _vp, _sz] + [_i] * 8 + [_vp]),
+    "mta_head_linear_bwd_weight_as": (_i, [_vp, _vp, _vp, _i, _vp, _sz] + [_i] * 6 + [_vp]),
     "mta_fused_fwd_dropout": (_i, [_vp] * 9 + [_sz] + [_i] * 13 + [_f, ctypes.c_ulonglong, _vp]),
     "mta_fused_fwd_host": (_i, [_vp] * 8 + [_i] * 12),
     "mta_host_pipeline_release": (_i, []),

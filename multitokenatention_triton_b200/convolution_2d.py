@@ -29,7 +29,7 @@ class Conv2dTritonFunction(Function):
         if ctx.needs_input_grad[0]:
             grad_input = ops.conv2d_bwd_input(grad_output, weight, ctx.causal)
         if ctx.needs_input_grad[1]:
-            grad_weight = ops.conv2d_bwd_weight(input, grad_output, tuple(weight.shape[1:]), ctx.causal).to(weight.dtype)
+            grad_weight = ops.conv2d_bwd_weight(input, grad_output, tuple(weight.shape[1:]), ctx.causal, weight.dtype)
         return grad_input, grad_weight, None
 
 

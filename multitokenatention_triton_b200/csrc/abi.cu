@@ -173,22 +173,27 @@ size_t mta_conv2d_bwd_weight_workspace_bytes(int N, int C, int H, int W, int R, 
 
 int mta_conv2d_bwd_weight(const void* x, const void* dy, float* dw, void* workspace, size_t workspace_bytes, int N, int C,
                           int H, int W, int R, int S, int causal, int dtype, void* stream) {
+    return mta_conv2d_bwd_weight_as(x, dy, dw, MTA_F32, workspace, workspace_bytes, N, C, H, W, R, S, causal, dtype, stream);
+}
+
+int mta_conv2d_bwd_weight_as(const void* x, const void* dy, void* dw, int dw_dtype, void* workspace, size_t workspace_bytes, int N,
+                             int C, int H, int W, int R, int S, int causal, int dtype, void* stream) {
     g_error[0] = 0;
-    MTA_REQUIRE(dtype_ok(dtype), "conv2d_bwd_weight: unknown dtype code %d", dtype);
+    MTA_REQUIRE(dtype_ok(dtype) && dtype_ok(dw_dtype), "conv2d_bwd_weight: unknown dtype code (x %d, dw %d)", dtype, dw_dtype);
     MTA_REQUIRE(N >= 0 && C >= 1 && H >= 0 && W >= 0, "conv2d_bwd_weight: bad shape N=%d C=%d H=%d W=%d", N, C, H, W);
     MTA_REQUIRE(R >= 1 && S >= 1, "conv2d_bwd_weight: kernel size %dx%d must be positive", R, S);
     MTA_REQUIRE(dw, "conv2d_bwd_weight: null pointer");
     if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if ((long)N * H * W == 0) {
-        MTA_CUDA_OK(cudaMemsetAsync(dw, 0, (size_t)C * R * S * sizeof(float), st));
+        MTA_CUDA_OK(cudaMemsetAsync(dw, 0, (size_t)C * R * S * dtype_size(dw_dtype), st));
         return MTA_OK;
     }
     MTA_REQUIRE(x && dy, "conv2d_bwd_weight: null pointer");
     const size_t need = conv2d_bwd_weight_workspace(N, C, H, W, R, S);
     MTA_REQUIRE(workspace && workspace_bytes >= need, "conv2d_bwd_weight: workspace of %zu bytes is smaller than the %zu needed",
                 workspace_bytes, need);
-    return conv2d_bwd_weight_launch(x, full_view(H, W), dy, full_view(H, W), dw, workspace, N, C, H, W, R, S, causal ? 1 : 0, dtype, st);
+    return conv2d_bwd_weight_launch(x, full_view(H, W), dy, full_view(H, W), dw, dw_dtype, workspace, N, C, H, W, R, S, causal ? 1 : 0, dtype, st);
 }
 
 int mta_head_linear_bwd_input(const void* dy, const void* Wm, void* dx, int N, int C, int P, int Q, int causal, int dtype,
@@ -212,21 +217,26 @@ size_t mta_head_linear_bwd_weight_workspace_bytes(int C) {
 
 int mta_head_linear_bwd_weight(const void* x, const void* dy, float* dW, void* workspace, size_t workspace_bytes, int N,
                                int C, int P, int Q, int causal, int dtype, void* stream) {
+    return mta_head_linear_bwd_weight_as(x, dy, dW, MTA_F32, workspace, workspace_bytes, N, C, P, Q, causal, dtype, stream);
+}
+
+int mta_head_linear_bwd_weight_as(const void* x, const void* dy, void* dW, int dw_dtype, void* workspace, size_t workspace_bytes,
+                                  int N, int C, int P, int Q, int causal, int dtype, void* stream) {
     g_error[0] = 0;
-    MTA_REQUIRE(dtype_ok(dtype), "head_linear_bwd_weight: unknown dtype code %d", dtype);
+    MTA_REQUIRE(dtype_ok(dtype) && dtype_ok(dw_dtype), "head_linear_bwd_weight: unknown dtype code (x %d, dW %d)", dtype, dw_dtype);
     MTA_REQUIRE(N >= 0 && C >= 1 && C <= 128 && P >= 0 && Q >= 0, "head_linear_bwd_weight: bad shape N=%d C=%d P=%d Q=%d", N, C, P, Q);
     MTA_REQUIRE(dW, "head_linear_bwd_weight: null pointer");
     if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if ((long)N * P * Q == 0) {
-        MTA_CUDA_OK(cudaMemsetAsync(dW, 0, (size_t)C * C * sizeof(float), st));
+        MTA_CUDA_OK(cudaMemsetAsync(dW, 0, (size_t)C * C * dtype_size(dw_dtype), st));
         return MTA_OK;
     }
     MTA_REQUIRE(x && dy, "head_linear_bwd_weight: null pointer");
     const size_t need = head_linear_bwd_weight_workspace(C);
     MTA_REQUIRE(workspace && workspace_bytes >= need, "head_linear_bwd_weight: workspace of %zu bytes is smaller than the %zu needed",
                 workspace_bytes, need);
-    return head_linear_bwd_weight_launch(x, full_view(P, Q), dy, full_view(P, Q), dW, workspace, N, C, P, Q, causal ? 1 : 0, dtype, st);
+    return head_linear_bwd_weight_launch(x, full_view(P, Q), dy, full_view(P, Q), dW, dw_dtype, workspace, N, C, P, Q, causal ? 1 : 0, dtype, st);
 }
 
 int mta_qk_scores_fwd(const void* q, const void* k, void* s, int B, int H, int S, int D, float scale, int round_scale,

@@ -107,7 +107,7 @@ conv2d_bwd_weight_kernel(const T* __restrict__ x, PlaneView xv, const T* __restr
 }
 
 // dw[c, tap] = sum over the planes of channel c and their tiles, in a fixed order, in double.
-__global__ void conv2d_bwd_weight_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int N, int C,
+__global__ void conv2d_bwd_weight_reduce_kernel(const float* __restrict__ partial, void* __restrict__ dw, int dw_dtype, int N, int C,
                                                 int tiles, int taps) {
     __shared__ double red[256];
     pdl_wait();
@@ -124,7 +124,7 @@ __global__ void conv2d_bwd_weight_reduce_kernel(const float* __restrict__ partia
         if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
         __syncthreads();
     }
-    if (threadIdx.x == 0) dw[blockIdx.x] = (float)red[0];
+    if (threadIdx.x == 0) store_weight(dw, blockIdx.x, dw_dtype, (float)red[0]);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -241,7 +241,7 @@ head_linear_bwd_weight_kernel(const T* __restrict__ x, PlaneView xv, const T* __
 // pair was a chain of 592 dependent loads: 23 to 42 us).
 constexpr int HR_SLICES = 8;
 __global__ void __launch_bounds__(32 * HR_SLICES)
-head_linear_bwd_weight_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dW, int ctas, int pairs) {
+head_linear_bwd_weight_reduce_kernel(const float* __restrict__ partial, void* __restrict__ dW, int dw_dtype, int ctas, int pairs) {
     __shared__ double red[HR_SLICES][32];
     pdl_wait();
     const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, pair = blockIdx.x * 32 + lane;
@@ -253,7 +253,7 @@ head_linear_bwd_weight_reduce_kernel(const float* __restrict__ partial, float* _
     __syncthreads();
     if (slice == 0 && pair < pairs) {
         for (int i = 1; i < HR_SLICES; ++i) acc += red[i][lane];
-        dW[pair] = (float)acc;
+        store_weight(dW, pair, dw_dtype, (float)acc);
     }
 }
 
@@ -277,8 +277,8 @@ size_t conv2d_bwd_weight_workspace(int N, int C, int H, int W, int R, int S) {
     return std::max((size_t)N * C * tiles * R * S * sizeof(float), conv2d_dw_tc05_workspace(N, C, H, W, R, S));
 }
 
-int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dw, void* workspace, int N, int C, int H,
-                             int W, int R, int S, int causal, int dtype, cudaStream_t st) {
+int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dw, int dw_dtype, void* workspace, int N, int C,
+                             int H, int W, int R, int S, int causal, int dtype, cudaStream_t st) {
     const int tiles_m = (H + WT_M - 1) / WT_M, tiles_n = (W + WT_N - 1) / WT_N;
     const long planes = (long)N * C;
     MTA_REQUIRE(planes <= 65535, "conv2d_bwd_weight: N*C = %ld exceeds 65535", planes);
@@ -286,11 +286,11 @@ int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneV
     float* partial = static_cast<float*>(workspace);
     // 16-bit dtypes with aligned rows: tensor cores (mta_set_variant("conv2d", 1): CUDA cores)
     if (variant("conv2d") != 1 && conv2d_dw_tc05_supported(x, xv, dy, dyv, R, S, dtype))
-        return conv2d_dw_tc05_launch(x, xv, dy, dyv, dw, workspace, N, C, H, W, R, S, causal, dtype, st);
+        return conv2d_dw_tc05_launch(x, xv, dy, dyv, dw, dw_dtype, workspace, N, C, H, W, R, S, causal, dtype, st);
     if (variant("conv2d") != 1 && conv2d_fma_supported(R, S, planes)) {
         int parts = 0;
         if (int rc = conv2d_dw_fma_launch(x, xv, dy, dyv, partial, tiles_m * tiles_n, &parts, planes, H, W, R, S, causal, dtype, st)) return rc;
-        return launch_kernel<conv2d_bwd_weight_reduce_kernel>("conv2d_bwd_weight_reduce_kernel", (unsigned)(C * taps), 64, 0, st, partial, dw, N, C,
+        return launch_kernel<conv2d_bwd_weight_reduce_kernel>("conv2d_bwd_weight_reduce_kernel", (unsigned)(C * taps), 64, 0, st, partial, dw, dw_dtype, N, C,
                                                               parts, taps);
     }
     // rows padded to a multiple of 4 floats, plus slack for the last window's 16-byte over-read
@@ -321,7 +321,7 @@ int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneV
 #undef MTA_BW_CASE
 #undef MTA_BW_LAUNCH
     MTA_LAUNCH_OK("conv2d_bwd_weight_kernel");
-    return launch_kernel<conv2d_bwd_weight_reduce_kernel>("conv2d_bwd_weight_reduce_kernel", (unsigned)(C * taps), 256, 0, st, partial, dw, N, C,
+    return launch_kernel<conv2d_bwd_weight_reduce_kernel>("conv2d_bwd_weight_reduce_kernel", (unsigned)(C * taps), 256, 0, st, partial, dw, dw_dtype, N, C,
                                                           tiles_m * tiles_n, taps);
 }
 
@@ -331,7 +331,7 @@ size_t head_linear_bwd_weight_workspace(int C) {
     return (size_t)hw_grid(sms) * C * C * sizeof(float);
 }
 
-int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dW, void* workspace, int N, int C,
+int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dW, int dw_dtype, void* workspace, int N, int C,
                                   int P, int Q, int causal, int dtype, cudaStream_t st) {
     int sms = 0;
     if (int bad = sm_count(&sms)) return bad;
@@ -349,7 +349,7 @@ int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, P
     if (rc) return rc;
     const int pairs = C * C;
     return launch_kernel<head_linear_bwd_weight_reduce_kernel>("head_linear_bwd_weight_reduce_kernel", (unsigned)((pairs + 31) / 32), 32 * HR_SLICES, 0, st,
-                                                               partial, dW, slots, pairs);
+                                                               partial, dW, dw_dtype, slots, pairs);
 }
 
 }  // namespace mta

@@ -133,6 +133,13 @@ __device__ __forceinline__ float load_weight(const void* w, long i, int w_dtype)
     return __half2float(reinterpret_cast<const __half*>(w)[i]);
 }
 
+// Stores v as element `i` of an array whose dtype is only known at run time (weight gradients are tiny).
+__device__ __forceinline__ void store_weight(void* w, long i, int w_dtype, float v) {
+    if (w_dtype == MTA_F32) reinterpret_cast<float*>(w)[i] = v;
+    else if (w_dtype == MTA_BF16) reinterpret_cast<__nv_bfloat16*>(w)[i] = __float2bfloat16_rn(v);
+    else reinterpret_cast<__half*>(w)[i] = __float2half_rn(v);
+}
+
 template <typename T> struct DTypeOf;
 template <> struct DTypeOf<float> { static constexpr int value = MTA_F32; };
 template <> struct DTypeOf<__nv_bfloat16> { static constexpr int value = MTA_BF16; };

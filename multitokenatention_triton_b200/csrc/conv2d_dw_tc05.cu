@@ -278,7 +278,7 @@ conv2d_dw_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_const
 }
 
 // dw[c, tap] = sum over the planes of channel c and the slots of each, in a fixed order, in double.
-__global__ void conv2d_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int N, int C, int taps, int slots,
+__global__ void conv2d_dw_reduce_kernel(const float* __restrict__ partial, void* __restrict__ dw, int dw_dtype, int N, int C, int taps, int slots,
                                         int steps, long total, int ctas) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_wait();
@@ -290,7 +290,7 @@ __global__ void conv2d_dw_reduce_kernel(const float* __restrict__ partial, float
         const int used = dw_owner(total, (plane + 1) * steps - 1, ctas) - dw_owner(total, plane * steps, ctas) + 1;
         for (int s = 0; s < used; ++s) acc += (double)partial[(plane * slots + s) * taps + tap];
     }
-    dw[i] = (float)acc;
+    store_weight(dw, i, dw_dtype, (float)acc);
 }
 
 DwGeom dw_geom(long planes, int H, int W, int R, int S, int causal, int sms, int* ctas) {
@@ -308,7 +308,7 @@ DwGeom dw_geom(long planes, int H, int W, int R, int S, int causal, int sms, int
 }
 
 template <typename T>
-int launch_dw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, float* dw, int N, int C, DwGeom g, int ctas,
+int launch_dw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, void* dw, int dw_dtype, int N, int C, DwGeom g, int ctas,
               cudaStream_t st) {
     CUtensorMap mx, mdy;
     int rc;
@@ -323,7 +323,7 @@ int launch_dw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float*
     const size_t smem = 1024 + g.nstage * stage;
     if ((rc = launch_kernel<conv2d_dw_tc05_kernel<T>>("conv2d_dw_tc05_kernel", (unsigned)ctas, DW_THREADS, smem, st, mx, mdy, partial, g, flag))) return rc;
     const int taps = g.R * g.S;
-    return launch_kernel<conv2d_dw_reduce_kernel>("conv2d_dw_reduce_kernel", (unsigned)((C * taps + 63) / 64), 64, 0, st, partial, dw, N, C, taps,
+    return launch_kernel<conv2d_dw_reduce_kernel>("conv2d_dw_reduce_kernel", (unsigned)((C * taps + 63) / 64), 64, 0, st, partial, dw, dw_dtype, N, C, taps,
                                                   g.slots, g.steps, g.total, ctas);
 }
 
@@ -345,14 +345,14 @@ size_t conv2d_dw_tc05_workspace(int N, int C, int H, int W, int R, int S) {
     return most;
 }
 
-int conv2d_dw_tc05_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dw, void* workspace, int N, int C, int H, int W,
-                          int R, int S, int causal, int dtype, cudaStream_t st) {
+int conv2d_dw_tc05_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dw, int dw_dtype, void* workspace, int N, int C, int H,
+                          int W, int R, int S, int causal, int dtype, cudaStream_t st) {
     int sms = 0, ctas = 0;
     if (int rc = sm_count(&sms)) return rc;
     const DwGeom g = dw_geom((long)N * C, H, W, R, S, causal, sms, &ctas);
     float* partial = static_cast<float*>(workspace);
-    if (dtype == MTA_BF16) return launch_dw<__nv_bfloat16>(x, xv, dy, dyv, partial, dw, N, C, g, ctas, st);
-    return launch_dw<__half>(x, xv, dy, dyv, partial, dw, N, C, g, ctas, st);
+    if (dtype == MTA_BF16) return launch_dw<__nv_bfloat16>(x, xv, dy, dyv, partial, dw, dw_dtype, N, C, g, ctas, st);
+    return launch_dw<__half>(x, xv, dy, dyv, partial, dw, dw_dtype, N, C, g, ctas, st);
 }
 
 }  // namespace mta

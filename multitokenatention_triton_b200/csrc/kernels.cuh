@@ -15,6 +15,8 @@ struct DeadKeys {
     // The bits of keys [key, key + 32) of batch element n, key a multiple of 32.
     __device__ uint32_t word(long n, int key) const { return bits ? __ldg(bits + n * words + (key >> 5)) : 0u; }
 };
+// out (B,H,S,D) contiguous = in (B,S,H,D) contiguous (mask.cu).
+int swap_heads_launch(const void* in, void* out, int B, int H, int S, int D, int dtype, cudaStream_t st);
 // Prepares them from a (B,S) byte mask (0 = dead), together with copies of k and v (B,H,S,D) whose rows of dead keys are zero
 // (mask.cu).  Zero rows of K make the scores of dead keys zero; zero rows of V drop whatever the later stages hold there.
 int mask_prepare_launch(const unsigned char* key_mask, const void* k, const void* v, uint32_t* bits, void* k_out, void* v_out, int B, int H,
@@ -46,19 +48,19 @@ int head_linear_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype,
                        int dtype, cudaStream_t st, bool w_transposed = false);
 
 // Gradients of the two stand-alone ops (backward.cu, conv2d.cu).  dx of the conv: zeros above the diagonal when causal and
-// `write_upper`.  The weight gradients are float32, reduced in a fixed order through a caller workspace of the given size.
+// `write_upper`.  The weight gradients come in `dw_dtype`, reduced in a fixed order through a caller workspace.
 int conv2d_bwd_input_launch(const void* dy, PlaneView dyv, const void* w, int w_dtype, void* dx, PlaneView dxv, long planes, int C, int H,
                             int W, int R, int S, int causal, bool write_upper, int dtype, cudaStream_t st);
 size_t conv2d_bwd_weight_workspace(int N, int C, int H, int W, int R, int S);
-int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dw, void* workspace, int N, int C, int H,
-                             int W, int R, int S, int causal, int dtype, cudaStream_t st);
+int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dw, int dw_dtype, void* workspace, int N, int C,
+                             int H, int W, int R, int S, int causal, int dtype, cudaStream_t st);
 // The conv's weight gradient on tcgen05 (conv2d_dw_tc05.cu).
 bool conv2d_dw_tc05_supported(const void* x, PlaneView xv, const void* dy, PlaneView dyv, int R, int S, int dtype);
 size_t conv2d_dw_tc05_workspace(int N, int C, int H, int W, int R, int S);
-int conv2d_dw_tc05_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dw, void* workspace, int N, int C, int H, int W,
-                          int R, int S, int causal, int dtype, cudaStream_t st);
+int conv2d_dw_tc05_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dw, int dw_dtype, void* workspace, int N, int C, int H,
+                          int W, int R, int S, int causal, int dtype, cudaStream_t st);
 size_t head_linear_bwd_weight_workspace(int C);
-int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* dW, void* workspace, int N, int C,
+int head_linear_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dW, int dw_dtype, void* workspace, int N, int C,
                                   int P, int Q, int causal, int dtype, cudaStream_t st);
 
 // The head mix's weight gradient on tcgen05 (head_dw_tc05.cu).

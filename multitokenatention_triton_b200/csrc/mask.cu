@@ -44,7 +44,31 @@ int launch(const unsigned char* key_mask, const void* k, const void* v, uint32_t
                                                      row_pieces, (S + 31) / 32);
 }
 
+// One 16-byte piece (or element) per thread; consecutive threads along a row of D.
+template <typename PIECE>
+__global__ void __launch_bounds__(MP_THREADS)
+swap_heads_kernel(const PIECE* __restrict__ in, PIECE* __restrict__ out, int H, int S, int row_pieces) {
+    pdl_wait();
+    const int i = (int)(blockIdx.x * MP_THREADS + threadIdx.x);
+    if (i >= S * row_pieces) return;
+    const int s = i / row_pieces, e = i - s * row_pieces, b = (int)blockIdx.y / H, h = (int)blockIdx.y % H;
+    out[(long)blockIdx.y * S * row_pieces + i] = in[(((long)b * S + s) * H + h) * row_pieces + e];
+}
+
+template <typename PIECE> int launch_swap(const void* in, void* out, int B, int H, int S, int row_pieces, cudaStream_t st) {
+    const dim3 grid((unsigned)((S * row_pieces + MP_THREADS - 1) / MP_THREADS), (unsigned)(B * H));
+    return launch_kernel<swap_heads_kernel<PIECE>>("swap_heads_kernel", grid, MP_THREADS, 0, st, static_cast<const PIECE*>(in), static_cast<PIECE*>(out), H, S,
+                                                   row_pieces);
+}
+
 }  // namespace
+
+int swap_heads_launch(const void* in, void* out, int B, int H, int S, int D, int dtype, cudaStream_t st) {
+    const size_t row = (size_t)D * dtype_size(dtype);
+    if (row % 16 == 0 && aligned16(in) && aligned16(out)) return launch_swap<uint4>(in, out, B, H, S, (int)(row / 16), st);
+    if (dtype == MTA_F32) return launch_swap<uint32_t>(in, out, B, H, S, D, st);
+    return launch_swap<uint16_t>(in, out, B, H, S, D, st);
+}
 
 int mask_prepare_launch(const unsigned char* key_mask, const void* k, const void* v, uint32_t* bits, void* k_out, void* v_out, int B, int H,
                         int S, int D, int dtype, cudaStream_t st) {

@@ -65,9 +65,9 @@ size_t mta_train_saved_bytes(int B, int H, int S, int dtype) {
     return SAVED * train_plan(B, H, S, dtype).plane_bytes;
 }
 
-size_t mta_train_workspace_bytes(int B, int H, int S, int cq, int ck, int cq2, int ck2, int dtype) {
-    if (B <= 0 || H <= 0 || S <= 0 || cq < 1 || ck < 1 || cq2 < 1 || ck2 < 1 || !dtype_ok(dtype)) return 0;
-    return 2 * train_plan(B, H, S, dtype).plane_bytes + partial_bytes(B, H, S, cq, ck, cq2, ck2);
+size_t mta_train_workspace_bytes(int B, int H, int S, int D, int cq, int ck, int cq2, int ck2, int dtype) {
+    if (B <= 0 || H <= 0 || S <= 0 || D <= 0 || cq < 1 || ck < 1 || cq2 < 1 || ck2 < 1 || !dtype_ok(dtype)) return 0;
+    return 2 * train_plan(B, H, S, dtype).plane_bytes + partial_bytes(B, H, S, cq, ck, cq2, ck2) + (size_t)B * H * S * D * dtype_size(dtype);
 }
 
 int mta_train_fwd(const void* q, const void* k, const void* v, const void* w1, const void* W1, const void* w2, const void* W2, void* o,
@@ -101,14 +101,14 @@ int mta_train_fwd(const void* q, const void* k, const void* v, const void* w1, c
 }
 
 int mta_train_bwd(const void* q, const void* k, const void* v, const void* w1, const void* W1, const void* w2, const void* W2,
-                  const void* dout, const void* saved, void* dq, void* dk, void* dv, float* dw1, float* dW1, float* dw2, float* dW2,
-                  void* workspace, size_t workspace_bytes, int B, int H, int S, int D, int cq, int ck, int cq2, int ck2, int dtype,
-                  int w_dtype, void* stream) {
+                  const void* dout, const void* saved, void* dq, void* dk, void* dv, void* dw1, void* dW1, void* dw2, void* dW2,
+                  void* workspace, size_t workspace_bytes, int B, int H, int S, int D, int cq, int ck, int cq2, int ck2, int dout_heads_inner,
+                  int dtype, int w_dtype, void* stream) {
     set_error("%s", "");
     if (int rc = check_shape("train_bwd", B, H, S, D, cq, ck, cq2, ck2, dtype, w_dtype)) return rc;
     MTA_REQUIRE((long)B * S > 0, "train_bwd: empty problem");
     MTA_REQUIRE(q && k && v && w1 && W1 && w2 && W2 && dout && saved && workspace, "train_bwd: null pointer");
-    const size_t need = mta_train_workspace_bytes(B, H, S, cq, ck, cq2, ck2, dtype);
+    const size_t need = mta_train_workspace_bytes(B, H, S, D, cq, ck, cq2, ck2, dtype);
     MTA_REQUIRE(workspace_bytes >= need, "train_bwd: workspace of %zu bytes is smaller than the %zu needed", workspace_bytes, need);
     MTA_REQUIRE(aligned16(saved) && aligned16(workspace), "train_bwd: saved planes and workspace must be 16-byte aligned");
     if (int rc = check_device()) return rc;
@@ -123,23 +123,28 @@ int mta_train_bwd(const void* q, const void* k, const void* v, const void* w1, c
     void* partial = ws + 2 * t.plane_bytes;
     const float scale = 1.0f / sqrtf((float)D);
     int rc;
+    if (dout_heads_inner) {                               // (B,S,H,D), as autograd hands it over: the products want (B,H,S,D)
+        void* swapped = ws + 2 * t.plane_bytes + partial_bytes(B, H, S, cq, ck, cq2, ck2);
+        if ((rc = swap_heads_launch(dout, swapped, B, H, S, D, dtype, st))) return rc;
+        dout = swapped;
+    }
     if (dv && (rc = ptx_launch(pl[MIX2], t.v, dout, dv, B, H, S, D, 1, 1.0f, dtype, st))) return rc;
     // how far back the chain of plane gradients has to go
     const bool to_scores = dq || dk, to_conv1 = to_scores || dw1, to_mix1 = to_conv1 || dW1, to_conv2 = to_mix1 || dw2;
     if (!to_conv2 && !dW2) return MTA_OK;
     // d(head mix 2) = dO V^T
     if ((rc = qk_scores_launch(dout, v, ga, t.v, B, H, S, D, 1.0f, 0, 1, 0, S, dtype, st))) return rc;
-    if (dW2 && (rc = head_linear_bwd_weight_launch(pl[CONV2], t.v, ga, t.v, dW2, partial, B, H, S, S, 1, dtype, st))) return rc;
+    if (dW2 && (rc = head_linear_bwd_weight_launch(pl[CONV2], t.v, ga, t.v, dW2, w_dtype, partial, B, H, S, S, 1, dtype, st))) return rc;
     if (!to_conv2) return MTA_OK;
     if ((rc = head_linear_launch(ga, t.v, W2, w_dtype, gb, t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st, true))) return rc;      // d(conv 2)
-    if (dw2 && (rc = conv2d_bwd_weight_launch(pl[PROBS], t.v, gb, t.v, dw2, partial, B, H, S, S, cq2, ck2, 1, dtype, st))) return rc;
+    if (dw2 && (rc = conv2d_bwd_weight_launch(pl[PROBS], t.v, gb, t.v, dw2, w_dtype, partial, B, H, S, S, cq2, ck2, 1, dtype, st))) return rc;
     if (!to_mix1) return MTA_OK;
     if ((rc = conv2d_bwd_input_launch(gb, t.v, w2, w_dtype, ga, t.v, t.planes, H, S, S, cq2, ck2, 1, false, dtype, st))) return rc;  // d(probabilities)
     if ((rc = softmax_bwd_launch(pl[PROBS], t.v, ga, t.v, ga, t.v, t.planes, S, S, 1, dtype, st))) return rc;                       // d(head mix 1)
-    if (dW1 && (rc = head_linear_bwd_weight_launch(pl[CONV1], t.v, ga, t.v, dW1, partial, B, H, S, S, 1, dtype, st))) return rc;
+    if (dW1 && (rc = head_linear_bwd_weight_launch(pl[CONV1], t.v, ga, t.v, dW1, w_dtype, partial, B, H, S, S, 1, dtype, st))) return rc;
     if (!to_conv1) return MTA_OK;
     if ((rc = head_linear_launch(ga, t.v, W1, w_dtype, gb, t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st, true))) return rc;      // d(conv 1)
-    if (dw1 && (rc = conv2d_bwd_weight_launch(pl[SCORES], t.v, gb, t.v, dw1, partial, B, H, S, S, cq, ck, 1, dtype, st))) return rc;
+    if (dw1 && (rc = conv2d_bwd_weight_launch(pl[SCORES], t.v, gb, t.v, dw1, w_dtype, partial, B, H, S, S, cq, ck, 1, dtype, st))) return rc;
     if (!to_scores) return MTA_OK;
     if ((rc = conv2d_bwd_input_launch(gb, t.v, w1, w_dtype, ga, t.v, t.planes, H, S, S, cq, ck, 1, false, dtype, st))) return rc;    // d(scores)
     if (dq && (rc = pv_launch(ga, t.v, S, k, dq, B, H, S, D, 1, 0, S, dtype, st, DropoutSpec(), scale))) return rc;

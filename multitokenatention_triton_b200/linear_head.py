@@ -27,7 +27,7 @@ class TritonLinearHeadFunction(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             grad_input = ops.head_linear_bwd_input(grad_output, weight, ctx.causal)
         if ctx.needs_input_grad[1]:
-            grad_weight = ops.head_linear_bwd_weight(input, grad_output, ctx.causal).to(weight.dtype)
+            grad_weight = ops.head_linear_bwd_weight(input, grad_output, ctx.causal, weight.dtype)
         return grad_input, grad_weight, None, None
 
 

@@ -81,20 +81,21 @@ def conv2d_bwd_input(grad_output: torch.Tensor, weight: torch.Tensor, causal: bo
     return dx
 
 
-def conv2d_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, kernel_size: Tuple[int, int], causal: bool) -> torch.Tensor:
-    """Gradient of conv2d_fwd with respect to its weight: (C,R,S) float32."""
+def conv2d_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, kernel_size: Tuple[int, int], causal: bool,
+                      dtype: torch.dtype = torch.float32) -> torch.Tensor:
+    """Gradient of conv2d_fwd with respect to its weight: (C,R,S) in `dtype`."""
     x, g = _cuda_contig(x, "input"), _cuda_contig(grad_output, "grad_output")
     assert x.shape == g.shape and x.dtype == g.dtype
     N, C, H, W = x.shape
     R, S = kernel_size
-    dw = torch.empty(C, R, S, device=x.device, dtype=torch.float32)
+    dw = torch.empty(C, R, S, device=x.device, dtype=dtype if dtype in _lib.DTYPE_CODE else torch.float32)
     L = lib()
     nbytes = _size("mta_conv2d_bwd_weight_workspace_bytes", N, C, H, W, R, S)
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
     with on_device(x.device):
-        check(L.mta_conv2d_bwd_weight(x.data_ptr(), g.data_ptr(), dw.data_ptr(), ws.data_ptr(), ws.numel(), N, C, H, W, R, S,
-                                      int(bool(causal)), dtype_code(x), stream_ptr(x.device)), "mta_conv2d_bwd_weight")
-    return dw
+        check(L.mta_conv2d_bwd_weight_as(x.data_ptr(), g.data_ptr(), dw.data_ptr(), dtype_code(dw), ws.data_ptr(), ws.numel(), N, C, H, W,
+                                         R, S, int(bool(causal)), dtype_code(x), stream_ptr(x.device)), "mta_conv2d_bwd_weight")
+    return dw.to(dtype)
 
 
 def head_linear_bwd_input(grad_output: torch.Tensor, weight: torch.Tensor, causal: bool = True) -> torch.Tensor:
@@ -110,21 +111,22 @@ def head_linear_bwd_input(grad_output: torch.Tensor, weight: torch.Tensor, causa
     return dx
 
 
-def head_linear_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, causal: bool = True) -> torch.Tensor:
-    """Gradient of head_linear_fwd with respect to its weight: (C,C) float32."""
+def head_linear_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, causal: bool = True,
+                           dtype: torch.dtype = torch.float32) -> torch.Tensor:
+    """Gradient of head_linear_fwd with respect to its weight: (C,C) in `dtype`."""
     x, g = _cuda_contig(x, "input"), _cuda_contig(grad_output, "grad_output")
     assert x.shape == g.shape and x.dtype == g.dtype
     N, C, P, Q = x.shape
-    dW = torch.empty(C, C, device=x.device, dtype=torch.float32)
+    dW = torch.empty(C, C, device=x.device, dtype=dtype if dtype in _lib.DTYPE_CODE else torch.float32)
     L = lib()
-    nbytes = L.mta_head_linear_bwd_weight_workspace_bytes(C)
+    nbytes = _size("mta_head_linear_bwd_weight_workspace_bytes", C)
     if nbytes == 0:
         raise MTALibraryError(f"head_linear_bwd_weight: C = {C} heads is outside the supported range 1..128")
     ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     with on_device(x.device):
-        check(L.mta_head_linear_bwd_weight(x.data_ptr(), g.data_ptr(), dW.data_ptr(), ws.data_ptr(), ws.numel(), N, C, P, Q,
-                                           int(bool(causal)), dtype_code(x), stream_ptr(x.device)), "mta_head_linear_bwd_weight")
-    return dW
+        check(L.mta_head_linear_bwd_weight_as(x.data_ptr(), g.data_ptr(), dW.data_ptr(), dtype_code(dW), ws.data_ptr(), ws.numel(), N, C,
+                                              P, Q, int(bool(causal)), dtype_code(x), stream_ptr(x.device)), "mta_head_linear_bwd_weight")
+    return dW.to(dtype)
 
 
 def head_linear_softmax_fwd(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -279,19 +281,22 @@ def mta_train_fwd(q, k, v, w1, W1, w2, W2) -> Tuple[torch.Tensor, torch.Tensor]:
 
 
 def mta_train_bwd(grad_out, saved, q, k, v, w1, W1, w2, W2, needs) -> list:
-    """Gradients of (q, k, v, w1, W1, w2, W2) where `needs` says so (None elsewhere); those of the weights are float32."""
-    q, k, v, g = (_cuda_contig(q, "xq"), _cuda_contig(k, "xk"), _cuda_contig(v, "xv"), _cuda_contig(grad_out, "grad_output"))
+    """Gradients of (q, k, v, w1, W1, w2, W2) where `needs` says so (None elsewhere), those of the weights in the dtype the
+    library read them in."""
+    q, k, v = _cuda_contig(q, "xq"), _cuda_contig(k, "xk"), _cuda_contig(v, "xv")
+    inner = grad_out.transpose(1, 2).is_contiguous()         # the gradient of the (B,S,H,D) view the module returns
+    g = grad_out if inner else _cuda_contig(grad_out, "grad_output")
     B, H, S, D = q.shape
     w = _mta_weights(q, w1, W1, w2, W2)
     grads = [torch.empty_like(t) if n else None for t, n in zip((q, k, v), needs)]
-    grads += [torch.empty(t.shape, dtype=torch.float32, device=q.device) if n else None for t, n in zip(w, needs[3:])]
+    grads += [torch.empty_like(t) if n else None for t, n in zip(w, needs[3:])]
     L = lib()
-    nbytes = _size("mta_train_workspace_bytes", B, H, S, *w1.shape[1:], *w2.shape[1:], dtype_code(q))
+    nbytes = _size("mta_train_workspace_bytes", B, H, S, D, *w1.shape[1:], *w2.shape[1:], dtype_code(q))
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
     with on_device(q.device):
         check(L.mta_train_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), *(t.data_ptr() for t in w), g.data_ptr(), saved.data_ptr(),
                               *(None if t is None else t.data_ptr() for t in grads), ws.data_ptr(), ws.numel(), B, H, S, D,
-                              *w1.shape[1:], *w2.shape[1:], dtype_code(q), dtype_code(w[0]), stream_ptr(q.device)), "mta_train_bwd")
+                              *w1.shape[1:], *w2.shape[1:], int(inner), dtype_code(q), dtype_code(w[0]), stream_ptr(q.device)), "mta_train_bwd")
     return grads
 
 
