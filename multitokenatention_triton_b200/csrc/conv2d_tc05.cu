@@ -82,6 +82,7 @@ __device__ __forceinline__ uint64_t smem_desc_plain(uint32_t saddr, uint32_t lbo
 
 struct ConvGeom {
     int C, W, R, S, causal, row_begin, row_end, tiles_n, tiles_m, x_row0, write_upper, split_w;
+    int nout;          // output staging tiles (1 or 2)
     int lead;          // staged rows start `lead` rows before the tile: R-1 for the conv (row taps look back), 0 for its
                        // input gradient (taps reversed, looking forward)
     int flip;          // input gradient: tap (i, j) uses w[R-1-i][S-1-j]
@@ -177,7 +178,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
     const int tb_off = NBOX * box_bytes + box3_bytes;         // Toeplitz slices follow the boxes
     const int stage_bytes = tb_off + tb_bytes;
     uint8_t* out_base = smem;                                  // 1024-byte aligned, as the swizzled TMA store needs
-    uint8_t* zero_box = smem + 2 * OUT_BYTES;                 // 16 KB of zeros: source of the zero tiles above the diagonal
+    uint8_t* zero_box = smem + g.nout * OUT_BYTES;                 // 16 KB of zeros: source of the zero tiles above the diagonal
     uint8_t* stage_base = zero_box + TM * 128;                // then the stage ring
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int pad_w = (S - 1) / 2;
@@ -383,12 +384,15 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
         for (int n = 0; n < my_tiles; ++n, it.next(g, g.tiles_m)) {
             const int ab = n & 1;
             const int plane = it.plane, m0 = it.m0(g), n0 = it.n0();
-            uint8_t* obuf = out_base + ab * OUT_BYTES;       // staging tile n % 2: two 64-column boxes
+            uint8_t* obuf = out_base + (g.nout == 2 ? ab : 0) * OUT_BYTES;       // staging tile n % nout: two 64-column boxes
             uint8_t* orow = obuf + half * (TM * 128) + row * 128;
             mbar_wait(&acc_full[ab], (n >> 1) & 1, err_flag);
             __syncwarp();
             fence_after_sync();
-            if (issuer) bulk_wait_read_1();                  // the store of tile n-2 has finished reading this staging tile
+            if (issuer) {                                    // the store of tile n - nout has finished reading this staging tile
+                if (g.nout == 2) bulk_wait_read_1();
+                else bulk_wait_read();
+            }
             named_barrier(1, 256);
             const int q = m0 + row;
 #pragma unroll
@@ -435,12 +439,15 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
     if (warp == 0) tmem_dealloc(tmem, 2 * TN);
 }
 
-size_t conv2d_tc05_smem_bytes(int R, bool split_w) {
+constexpr size_t CONV_SMEM_LIMIT = 225 * 1024;         // what the static arrays leave
+
+// With two output staging tiles, or with one (which takes up to 16 row taps).
+size_t conv2d_tc05_smem_bytes(int R, bool split_w, int nout) {
     const int TH = TM + R - 1;
     const size_t box = (size_t)((TH * 128 + 1023) & ~1023);
     const size_t tb = (size_t)((R * 1024 * (split_w ? 2 : 1) + 1023) & ~1023);
     const size_t box3 = (size_t)((TH * 32 + 1023) & ~1023);
-    return 1024 + 2 * OUT_BYTES + TM * 128 + NSTAGE * (NBOX * box + box3 + tb);
+    return 1024 + nout * OUT_BYTES + TM * 128 + NSTAGE * (NBOX * box + box3 + tb);
 }
 
 template <typename T>
@@ -482,8 +489,9 @@ int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, 
     g.zero_total = g.zero_per_plane * planes;
     int sms = 0;
     if (int bad = sm_count(&sms)) return bad;
-    const size_t smem = conv2d_tc05_smem_bytes(R, g.split_w != 0);
-    MTA_REQUIRE(smem <= 227 * 1024, "conv2d (tcgen05): kernel with %d row taps needs %zu bytes of shared memory", R, smem);
+    g.nout = conv2d_tc05_smem_bytes(R, g.split_w != 0, 2) <= CONV_SMEM_LIMIT ? 2 : 1;
+    const size_t smem = conv2d_tc05_smem_bytes(R, g.split_w != 0, g.nout);
+    MTA_REQUIRE(smem <= CONV_SMEM_LIMIT, "conv2d (tcgen05): kernel with %d row taps needs %zu bytes of shared memory", R, smem);
     const unsigned grid = (unsigned)std::min<long>(g.total_tiles, sms);
     return launch_kernel<conv2d_tc05_kernel<T>>("conv2d_tc05_kernel", grid, THREADS, smem, st, mx, mx3, my, w, w_dtype, yv.row0, g, flag);
 }
@@ -493,7 +501,7 @@ int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, 
 
 bool conv2d_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int W, int R, int S, int dtype,
                            int w_dtype) {
-    return dtype != MTA_F32 && S <= 17 && R <= 16 && conv2d_tc05_smem_bytes(R, w_dtype == MTA_F32) <= 227 * 1024 && xv.width % 8 == 0 && yv.width % 8 == 0 &&
+    return dtype != MTA_F32 && S <= 17 && R <= 16 && conv2d_tc05_smem_bytes(R, w_dtype == MTA_F32, 1) <= CONV_SMEM_LIMIT && xv.width % 8 == 0 && yv.width % 8 == 0 &&
            xv.plane_stride % 8 == 0 && yv.plane_stride % 8 == 0 && aligned16(x) && aligned16(y);
 }
 

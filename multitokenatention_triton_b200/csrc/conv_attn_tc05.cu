@@ -33,7 +33,6 @@ using namespace tc05;
 using namespace qc;
 
 constexpr int CA_THREADS = 16 * 32;
-constexpr int NSTAGE = 3;                   // staged score tiles in flight
 constexpr uint32_t C_COL = 0, S_COL = 128, P_COL = 272, O_COL = 384;
 constexpr int VBOX_BYTES = TN * 128;         // one box of the V tile: 128 keys x 64 elements
 constexpr float LOG2E = 1.4426950408889634f;
@@ -57,7 +56,8 @@ __device__ __forceinline__ int ca_key_tiles(const CaGeom& g, int tm) {
     return (q_last + TN - 1) / TN;
 }
 
-template <typename T, int D>
+// NSTAGE: staged score tiles in flight, three where they fit into shared memory, else two (more than six row taps at D = 128).
+template <typename T, int D, int NSTAGE>
 __global__ void __launch_bounds__(CA_THREADS, 1)
 conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                       const __grid_constant__ CUtensorMap mv, T* __restrict__ o, const void* __restrict__ w, int w_dtype,
@@ -383,8 +383,11 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-size_t conv_attn_smem_bytes(int D, int R, bool split_w) {
-    return 1024 + (size_t)(D / 64) * (BOX_BYTES + KBOX_BYTES + VBOX_BYTES) + (size_t)NSTAGE * TB_OFF + 2 * (size_t)toeplitz_bytes(R, split_w ? 1 : 0);
+constexpr size_t CA_STATIC_SMEM = 4608;     // barriers, the exchange arrays and the weight buffer, rounded up
+constexpr size_t CA_SMEM_LIMIT = 227 * 1024;
+
+size_t conv_attn_smem_bytes(int D, int R, bool split_w, int nstage) {
+    return 1024 + (size_t)(D / 64) * (BOX_BYTES + KBOX_BYTES + VBOX_BYTES) + (size_t)nstage * TB_OFF + 2 * (size_t)toeplitz_bytes(R, split_w ? 1 : 0);
 }
 
 template <typename T, int D>
@@ -408,19 +411,20 @@ int launch_ca(const void* q, const void* k, const void* v, const void* w, int w_
     if ((rc = wait_flag_ptr(&flag))) return rc;
     int sms = 0;
     if (int bad = sm_count(&sms)) return bad;
-    const size_t smem = conv_attn_smem_bytes(D, R, g.split_w != 0);
     const unsigned grid = (unsigned)std::min<long>(g.units, sms);
-    return launch_kernel<conv_attn_tc05_kernel<T, D>>("conv_attn_tc05_kernel", grid, CA_THREADS, smem, st, mq, mk, mv, static_cast<T*>(o), w, w_dtype, g, flag);
+    const size_t smem3 = conv_attn_smem_bytes(D, R, g.split_w != 0, 3), smem2 = conv_attn_smem_bytes(D, R, g.split_w != 0, 2);
+    if (smem3 + CA_STATIC_SMEM <= CA_SMEM_LIMIT)
+        return launch_kernel<conv_attn_tc05_kernel<T, D, 3>>("conv_attn_tc05_kernel", grid, CA_THREADS, smem3, st, mq, mk, mv, static_cast<T*>(o), w,
+                                                             w_dtype, g, flag);
+    return launch_kernel<conv_attn_tc05_kernel<T, D, 2>>("conv_attn_tc05_kernel", grid, CA_THREADS, smem2, st, mq, mk, mv, static_cast<T*>(o), w,
+                                                         w_dtype, g, flag);
 }
-
-constexpr size_t CA_STATIC_SMEM = 4608;     // barriers, the exchange arrays and the weight buffer, rounded up
-constexpr size_t CA_SMEM_LIMIT = 227 * 1024;
 
 }  // namespace
 
 bool conv_attn_fused_shape_ok(int S, int D, int R, int KS, int causal, int dtype, int w_dtype) {
     return causal && dtype != MTA_F32 && (D == 64 || D == 128) && S >= 1 && KS % 2 == 1 && KS <= 17 && R >= 1 && R <= 16 &&
-           conv_attn_smem_bytes(D, R, w_dtype == MTA_F32) + CA_STATIC_SMEM <= CA_SMEM_LIMIT;
+           conv_attn_smem_bytes(D, R, w_dtype == MTA_F32, 2) + CA_STATIC_SMEM <= CA_SMEM_LIMIT;
 }
 
 bool conv_attn_fused_supported(const void* q, const void* k, const void* v, const void* o, int S, int D, int R, int KS, int causal,

@@ -24,7 +24,6 @@ using namespace tc05;
 using namespace qc;
 
 constexpr int OUT_BYTES = 2 * TM * 128;           // output staging: two 64-column boxes
-constexpr int NSTAGE = 3;                         // staged score tiles in flight
 // Four drain warps (warps 4-7): a thread converts its whole staged row.  Measured at B8 H16 S4096 D128, 6 x 11: 1.26 ms;
 // eight warps with spinning waits 1.35 ms - the kernel is bound by shared-memory bandwidth (the conv MMAs' operand
 // reads, ~300 KB per tile, plus ~200 KB of tile traffic), and extra polling and extra warps only add to it.
@@ -69,7 +68,9 @@ struct QcIter {
     __device__ int n0() const { return tn * TN; }
 };
 
-template <typename T, int D>
+// NSTAGE: staged score tiles in flight.  Three where they fit into shared memory, else two (B8 H16 S4096 6x11: 1.28 against
+// 1.26 ms), which takes up to 16 row taps at D = 128.
+template <typename T, int D, int NSTAGE>
 __global__ void __launch_bounds__(THREADS, 1)
 qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                     const __grid_constant__ CUtensorMap my, const void* __restrict__ w, int w_dtype, QcGeom g, int* err_flag) {
@@ -308,8 +309,10 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-size_t qk_conv_smem_bytes(int D, int R, bool split_w) {
-    return 1024 + OUT_BYTES + (size_t)(D / 64) * (BOX_BYTES + KBOX_BYTES) + (size_t)NSTAGE * TB_OFF +
+constexpr size_t QC_SMEM_LIMIT = 225 * 1024;
+
+size_t qk_conv_smem_bytes(int D, int R, bool split_w, int nstage) {
+    return 1024 + OUT_BYTES + (size_t)(D / 64) * (BOX_BYTES + KBOX_BYTES) + (size_t)nstage * TB_OFF +
            2 * (size_t)toeplitz_bytes(R, split_w ? 1 : 0);
 }
 
@@ -342,9 +345,11 @@ int launch_qc(const void* q, const void* k, const void* w, int w_dtype, void* y,
     if ((rc = wait_flag_ptr(&flag))) return rc;
     int sms = 0;
     if (int bad = sm_count(&sms)) return bad;
-    const size_t smem = qk_conv_smem_bytes(D, R, g.split_w != 0);
     const unsigned grid = (unsigned)std::min<long>(g.total_tiles, sms);
-    return launch_kernel<qk_conv_tc05_kernel<T, D>>("qk_conv_tc05_kernel", grid, THREADS, smem, st, mq, mk, my, w, w_dtype, g, flag);
+    const size_t smem3 = qk_conv_smem_bytes(D, R, g.split_w != 0, 3), smem2 = qk_conv_smem_bytes(D, R, g.split_w != 0, 2);
+    if (smem3 <= QC_SMEM_LIMIT)
+        return launch_kernel<qk_conv_tc05_kernel<T, D, 3>>("qk_conv_tc05_kernel", grid, THREADS, smem3, st, mq, mk, my, w, w_dtype, g, flag);
+    return launch_kernel<qk_conv_tc05_kernel<T, D, 2>>("qk_conv_tc05_kernel", grid, THREADS, smem2, st, mq, mk, my, w, w_dtype, g, flag);
 }
 
 }  // namespace
@@ -352,7 +357,7 @@ int launch_qc(const void* q, const void* k, const void* w, int w_dtype, void* y,
 bool qk_conv_supported(const void* q, const void* k, const void* y, PlaneView yv, int S, int D, int R, int KS, int causal, int dtype,
                        int w_dtype) {
     return causal && dtype != MTA_F32 && (D == 64 || D == 128) && KS % 2 == 1 && KS <= 17 && R >= 1 && R <= 16 &&
-           qk_conv_smem_bytes(D, R, w_dtype == MTA_F32) <= 225 * 1024 && yv.width >= S && yv.width % 8 == 0 && yv.plane_stride % 8 == 0 && aligned16(q) &&
+           qk_conv_smem_bytes(D, R, w_dtype == MTA_F32, 2) <= QC_SMEM_LIMIT && yv.width >= S && yv.width % 8 == 0 && yv.plane_stride % 8 == 0 && aligned16(q) &&
            aligned16(k) && aligned16(y);
 }
 

@@ -1,0 +1,49 @@
+"""Up to 16 row taps on the tensor-core convs (one output staging tile, two staged score tiles): each against the CUDA-core path."""
+import pytest
+import torch
+
+from multitokenatention_triton_b200 import _lib, ops
+from util import npf, rel_fro, rel_max
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("S,R,Sk,causal,dtype", [(264, 9, 9, True, torch.bfloat16), (520, 11, 15, True, torch.float16), (136, 16, 17, True, torch.bfloat16),
+                                                 (384, 13, 3, False, torch.float16)])
+def test_conv2d(S, R, Sk, causal, dtype):
+    g = torch.Generator(device=DEV).manual_seed(S)
+    x, gr = (torch.randn(3, 5, S, S, device=DEV, generator=g).to(dtype) for _ in range(2))
+    w = (torch.randn(5, R, Sk, device=DEV, generator=g) * (R * Sk) ** -0.5).to(dtype)
+    if causal:
+        x, gr = (t.masked_fill(torch.ones(S, S, dtype=torch.bool, device=DEV).triu(1), float("nan")) for t in (x, gr))
+    got = {}
+    for variant in (0, 1):
+        _lib.set_variant("conv2d", variant)
+        try:
+            got[variant] = ops.conv2d_fwd(x, w, causal), ops.conv2d_bwd_input(gr, w, causal)
+        finally:
+            _lib.set_variant("conv2d", 0)
+    _lib.device_status()
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, b in zip(got[0], got[1]):
+        assert float((a.float() - b.float()).abs().max()) <= 2 * ulp * float(b.float().abs().max())
+
+
+@pytest.mark.parametrize("S,D,R,Sk", [(257, 128, 7, 9), (130, 128, 11, 15), (400, 128, 16, 17), (200, 64, 14, 11)])
+def test_conv_attention_and_scores_in_the_conv(S, D, R, Sk):
+    g = torch.Generator(device=DEV).manual_seed(S + R)
+    q, k, v = (torch.randn(2, 8, S, D, device=DEV, generator=g).to(torch.bfloat16) for _ in range(3))
+    w = (torch.randn(8, R, Sk, device=DEV, generator=g) * (R * Sk) ** -0.5).to(torch.bfloat16)
+    mix = [(torch.eye(8, device=DEV) + 0.1 * torch.randn(8, 8, device=DEV, generator=g)).to(torch.bfloat16) for _ in range(2)]
+    one = ops.conv_attn_fwd(q, k, v, w, True, D ** -0.5), ops.mta_fused_fwd(q, k, v, w, mix[0], w, mix[1])
+    _lib.set_variant("gemm", 1)
+    _lib.set_variant("conv2d", 1)
+    try:
+        ref = ops.conv_attn_fwd(q, k, v, w, True, D ** -0.5), ops.mta_fused_fwd(q, k, v, w, mix[0], w, mix[1])
+    finally:
+        _lib.set_variant("gemm", 0)
+        _lib.set_variant("conv2d", 0)
+    _lib.device_status()
+    for a, b in zip(one, ref):
+        assert rel_fro(npf(a), npf(b)) <= 1e-2 and rel_max(npf(a), npf(b)) <= 3e-2
