@@ -5,51 +5,113 @@
 //   y[n,o,p,q] = fill                          for q >  p when causal (fill may be -inf)
 //
 // Kernels:
-//   head_linear_simt_kernel  any dtype, any C <= 128, any Q.  One thread per (row, key); the C inputs of
-//                            that position sit in registers, the weight in shared memory.
+//   head_linear_simt_kernel  any dtype, any C <= 128, any Q, on the CUDA cores.
 //   head_linear_mma_kernel   16-bit dtypes, C <= 32, Q a multiple of 8 and 16-byte aligned rows.  One warp
 //                            owns 64 consecutive keys of a row: every lane reads 16 bytes (8 keys) of
 //                            CP/4 head planes, the mix runs as m16n8k8 TF32 tensor-core MMAs (16-bit values
 //                            are exact in TF32, accumulation is fp32, so the result equals fp32 FMA up to
 //                            summation order), and every lane writes 16-byte vectors.  Key blocks above the
 //                            diagonal are never read: they are only filled.
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace mta {
 namespace {
 
 // ------------------------------------------------------------------------------------------------
-template <typename T, int CP>
-__global__ void __launch_bounds__(256)
+// Bound: HBM up to 16 heads, the FP32 pipe above (C * C multiply-adds per position).  A thread owns V neighbouring keys of a
+// row: the C inputs of each sit in registers, all loads in flight at once.  The outputs are made eight heads at a time as
+// packed pairs of heads: the weights lie head-minor in shared memory, so two 16-byte broadcasts feed 4 V packed FMAs.  A warp
+// takes rows_per_warp rows so that a CTA reads the weights once for several rows.
+// Measured, float32: B1 H16 S2048 90 -> PENDING us; B3 H64 S553 540 -> PENDING us (one position per thread, one weight per load).
+constexpr int HS_WARPS = 8;
+constexpr int HS_OG = 8;
+
+template <typename T, int V> struct alignas(sizeof(T) * V) HsVec { T e[V]; };
+
+constexpr int hs_min_ctas(int cp) { return cp <= 32 ? 2 : 1; }
+
+template <typename T, int CP, int V>
+__global__ void __launch_bounds__(HS_WARPS * 32, hs_min_ctas(CP))
 head_linear_simt_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
-                        T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
-                        int write_upper, int w_transposed) {
-    extern __shared__ float ws[];   // C x C
+                        T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin, int row_end,
+                        int rows_per_warp, int write_upper, int w_transposed, int vec) {
+    extern __shared__ __align__(16) float ws[];   // [h][o], o padded to a multiple of HS_OG
     pdl_wait();
-    for (int i = threadIdx.x; i < C * C; i += blockDim.x)
-        ws[i] = load_weight(Wm, w_transposed ? (long)(i % C) * C + i / C : i, w_dtype);
-    __syncthreads();
-    const int p = row_begin + blockIdx.y;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    const long n = blockIdx.z;
-    if (q >= Q) return;
-    if (causal && q > p) {
-        if (write_upper) {
-            const T f = from_f32<T>(fill);
-            for (int o = 0; o < C; ++o) y[yv.at(n * C + o, p, q)] = f;
-        }
-        return;
+    const int OP = (C + HS_OG - 1) / HS_OG * HS_OG;
+    for (int i = threadIdx.x; i < CP * OP; i += HS_WARPS * 32) {
+        const int h = i / OP, o = i - h * OP;
+        ws[i] = h < C && o < C ? load_weight(Wm, w_transposed ? (long)h * C + o : (long)o * C + h, w_dtype) : 0.0f;
     }
-    float xr[CP];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long n = blockIdx.z;
+    const int k = ((int)blockIdx.x * 32 + lane) * V;
+    const int k_warp = (int)blockIdx.x * 32 * V;
+    const T* xn = x + n * C * xv.plane_stride + k;
+    T* yn = y + n * C * yv.plane_stride + k;
+#pragma unroll 1
+    for (int r = 0; r < rows_per_warp; ++r) {
+        const int p = row_begin + ((int)blockIdx.y * rows_per_warp + r) * HS_WARPS + warp;
+        if (p >= row_end) return;
+        const int mixed = min(max((causal ? min(p, Q - 1) : Q - 1) - k + 1, 0), V);      // of the thread's keys: mixed, then filled
+        const int stored = write_upper ? min(max(Q - k, 0), V) : mixed;
+        const T* xr = xn + (long)(p - xv.row0) * xv.width;
+        T* yr = yn + (long)(p - yv.row0) * yv.width;
+        const bool none = causal && k_warp > p;             // the whole warp lies above the diagonal
+        if (none && !write_upper) continue;
+        float xs[CP][V];
+        if (!none) {
 #pragma unroll
-    for (int h = 0; h < CP; ++h) xr[h] = h < C ? to_f32<T>(x[xv.at(n * C + h, p, q)]) : 0.0f;
-    for (int o = 0; o < C; ++o) {
-        float acc = 0.0f;
-        const float* wr = ws + o * C;
+            for (int h = 0; h < CP; ++h) {
+                const T* src = xr + h * xv.plane_stride;
+                if (vec && mixed == V && h < C) {
+                    const HsVec<T, V> t = *reinterpret_cast<const HsVec<T, V>*>(src);
 #pragma unroll
-        for (int h = 0; h < CP; ++h)
-            if (h < C) acc = fmaf(wr[h], xr[h], acc);
-        y[yv.at(n * C + o, p, q)] = from_f32<T>(acc);
+                    for (int e = 0; e < V; ++e) xs[h][e] = to_f32<T>(t.e[e]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < V; ++e) xs[h][e] = e < mixed && h < C ? to_f32<T>(src[e]) : 0.0f;
+                }
+            }
+        }
+#pragma unroll 1
+        for (int o0 = 0; o0 < OP; o0 += HS_OG) {
+            float2 acc[V][HS_OG / 2];
+#pragma unroll
+            for (int e = 0; e < V; ++e)
+#pragma unroll
+                for (int j = 0; j < HS_OG / 2; ++j) acc[e][j] = make_float2(0.0f, 0.0f);
+            if (!none) {
+#pragma unroll
+                for (int h = 0; h < CP; ++h) {
+                    const float4 w0 = *reinterpret_cast<const float4*>(ws + h * OP + o0), w1 = *reinterpret_cast<const float4*>(ws + h * OP + o0 + 4);
+                    const float2 wv[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
+#pragma unroll
+                    for (int e = 0; e < V; ++e) {
+                        const float2 x2 = make_float2(xs[h][e], xs[h][e]);
+#pragma unroll
+                        for (int j = 0; j < HS_OG / 2; ++j) acc[e][j] = __ffma2_rn(wv[j], x2, acc[e][j]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < HS_OG; ++j) {
+                if (o0 + j >= C) break;
+                T* dst = yr + (o0 + j) * yv.plane_stride;
+                HsVec<T, V> t;
+#pragma unroll
+                for (int e = 0; e < V; ++e) t.e[e] = from_f32<T>(e < mixed ? (j & 1 ? acc[e][j / 2].y : acc[e][j / 2].x) : fill);
+                if (vec && stored == V) {
+                    *reinterpret_cast<HsVec<T, V>*>(dst) = t;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < V; ++e)
+                        if (e < stored) dst[e] = t.e[e];
+                }
+            }
+        }
     }
 }
 
@@ -697,25 +759,38 @@ int launch_mix_softmax(const void* x, PlaneView xv, const void* Wm, int w_dtype,
     return MTA_OK;
 }
 
-template <typename T, int CP>
+template <typename T, int CP, int V>
 int launch_simt(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C, int Q,
                 int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st) {
-    dim3 grid((unsigned)((Q + 255) / 256), (unsigned)(row_end - row_begin), (unsigned)N);
-    const size_t smem = (size_t)C * C * sizeof(float);
-    return launch_kernel<head_linear_simt_kernel<T, CP>>("head_linear_simt_kernel", grid, 256, smem, st, static_cast<const T*>(x), xv, Wm, w_dtype,
-                                                         static_cast<T*>(y), yv, C, Q, causal, fill, row_begin, write_upper ? 1 : 0, wt ? 1 : 0);
+    auto vec_ok = [](const void* p, const PlaneView& v) {
+        return v.width % V == 0 && v.plane_stride % V == 0 && reinterpret_cast<uintptr_t>(p) % (V * sizeof(T)) == 0;
+    };
+    const int rows = row_end - row_begin, blocks_x = (Q + 32 * V - 1) / (32 * V);
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
+    // several rows per warp once there are enough warps for two full loads of the chip
+    const long warps = (long)N * rows * blocks_x;
+    const int rows_per_warp = (int)std::min<long>(8, std::max<long>(1, warps / (2L * 16 * sms)));
+    const int rows_per_cta = HS_WARPS * rows_per_warp;
+    const dim3 grid((unsigned)blocks_x, (unsigned)((rows + rows_per_cta - 1) / rows_per_cta), (unsigned)N);
+    const size_t smem = (size_t)CP * ((C + HS_OG - 1) / HS_OG * HS_OG) * sizeof(float);
+    return launch_kernel<head_linear_simt_kernel<T, CP, V>>("head_linear_simt_kernel", grid, HS_WARPS * 32, smem, st, static_cast<const T*>(x), xv, Wm,
+                                                            w_dtype, static_cast<T*>(y), yv, C, Q, causal, fill, row_begin, row_end, rows_per_warp,
+                                                            write_upper ? 1 : 0, wt ? 1 : 0, vec_ok(x, xv) && vec_ok(y, yv) ? 1 : 0);
 }
 
 template <typename T>
 int dispatch_simt(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C, int Q,
                   int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st) {
-#define MTA_SIMT_CASE(CPV) \
-    return launch_simt<T, CPV>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st)
-    if (C <= 8) MTA_SIMT_CASE(8);
-    if (C <= 16) MTA_SIMT_CASE(16);
-    if (C <= 32) MTA_SIMT_CASE(32);
-    if (C <= 64) MTA_SIMT_CASE(64);
-    MTA_SIMT_CASE(128);
+// keys per thread: what C inputs of each leave of the registers
+#define MTA_SIMT_CASE(CPV, VV) \
+    return launch_simt<T, CPV, VV>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st)
+    if (C <= 8) MTA_SIMT_CASE(8, 4);
+    if (C <= 12) MTA_SIMT_CASE(12, 4);
+    if (C <= 16) MTA_SIMT_CASE(16, 4);
+    if (C <= 32) MTA_SIMT_CASE(32, 2);
+    if (C <= 64) MTA_SIMT_CASE(64, 2);
+    MTA_SIMT_CASE(128, 1);
 #undef MTA_SIMT_CASE
 }
 
