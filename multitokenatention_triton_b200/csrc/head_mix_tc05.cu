@@ -211,7 +211,8 @@ __device__ __forceinline__ int hm_tiles(const HmGeom& g, int p0) {
 
 // SOFTMAX: the two-pass kernel described at the top.  Otherwise the plain head mix (linear_head_kernel_forward,
 // triton_linear_head.py:76-139): one pass, the rounded products go out as they are, `fill` above the diagonal.
-template <typename T, bool SOFTMAX>
+// MASKED: some keys are dead (softmax only).
+template <typename T, bool SOFTMAX, bool MASKED>
 __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const CUtensorMap& my, const T* __restrict__ Wm, int y_row0,
                                                    const HmGeom& g, int* err_flag) {
     extern __shared__ uint8_t smem_raw[];
@@ -397,7 +398,8 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&acc_empty[grp]);
                     }
-                    const uint32_t live = hm_first(n_keys - (key0 + c * 32)) & (key0 + c * 32 < g.Q ? ~g.dead.word(n, key0 + c * 32) : 0u);
+                    uint32_t live = hm_first(n_keys - (key0 + c * 32));
+                    if (MASKED && key0 + c * 32 < g.Q) live &= ~g.dead.word(n, key0 + c * 32);
                     if (live) hm_stats32<T>(cur, live, m_run, s_run);
                 }
             }
@@ -448,7 +450,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                     const int kb = key0 + c * 32;
                     if (kb >= g.Q || (kb >= unit_keys && !g.write_upper)) continue;
                     uint32_t pk[16];
-                    if constexpr (SOFTMAX) hm_prob32<T>(cur, hm_first(n_keys - kb) & ~g.dead.word(n, kb), shift, pk);
+                    if constexpr (SOFTMAX) hm_prob32<T>(cur, hm_first(n_keys - kb) & (MASKED ? ~g.dead.word(n, kb) : 0xffffffffu), shift, pk);
                     else hm_plain32<T>(cur, hm_first(n_keys - kb), g.fill, pk);
                     if (gt == 0) bulk_wait_read();                   // the previous store of this buffer has read it
                     named_barrier(2 + grp, 128);
@@ -483,17 +485,17 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-template <typename T>
+template <typename T, bool MASKED>
 __global__ void __launch_bounds__(HM_THREADS, 1)
 head_mix_softmax_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap my, const T* __restrict__ Wm,
                              int y_row0, HmGeom g, int* err_flag) {
-    head_mix_tc05_body<T, true>(mx, my, Wm, y_row0, g, err_flag);
+    head_mix_tc05_body<T, true, MASKED>(mx, my, Wm, y_row0, g, err_flag);
 }
 template <typename T>
 __global__ void __launch_bounds__(HM_THREADS, 1)
 head_mix_plain_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap my, const T* __restrict__ Wm,
                            int y_row0, HmGeom g, int* err_flag) {
-    head_mix_tc05_body<T, false>(mx, my, Wm, y_row0, g, err_flag);
+    head_mix_tc05_body<T, false, false>(mx, my, Wm, y_row0, g, err_flag);
 }
 
 constexpr size_t HM_SMEM_BYTES = 1024 + HM_A_BYTES + (size_t)HM_NSTAGE * HM_STAGE_BYTES + (size_t)(HM_NACC + 1) * HM_OUT_BYTES;
@@ -526,11 +528,16 @@ int launch_hm(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv
     int sms = 0;
     if (int bad = sm_count(&sms)) return bad;
     const unsigned grid = (unsigned)std::min<long>(g.units, sms);
-    if constexpr (SOFTMAX)
-        return launch_kernel<head_mix_softmax_tc05_kernel<T>>("head_mix_softmax_tc05_kernel", grid, HM_THREADS, HM_SMEM_BYTES, st, mx, my,
-                                                              static_cast<const T*>(Wm), yv.row0, g, flag);
+    const T* wm = static_cast<const T*>(Wm);
+    if constexpr (SOFTMAX) {
+        if (dead.bits)
+            return launch_kernel<head_mix_softmax_tc05_kernel<T, true>>("head_mix_softmax_tc05_kernel", grid, HM_THREADS, HM_SMEM_BYTES, st, mx, my, wm,
+                                                                        yv.row0, g, flag);
+        return launch_kernel<head_mix_softmax_tc05_kernel<T, false>>("head_mix_softmax_tc05_kernel", grid, HM_THREADS, HM_SMEM_BYTES, st, mx, my, wm,
+                                                                     yv.row0, g, flag);
+    }
     return launch_kernel<head_mix_plain_tc05_kernel<T>>("head_mix_plain_tc05_kernel", grid, HM_THREADS, HM_SMEM_BYTES, st, mx, my,
-                                                        static_cast<const T*>(Wm), yv.row0, g, flag);
+                                                        wm, yv.row0, g, flag);
 }
 
 bool hm_tc05_ok(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int dtype, int w_dtype) {
