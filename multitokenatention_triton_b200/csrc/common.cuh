@@ -108,6 +108,9 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // lets the next kernel begin its own setup.  In this order, so that a kernel that has started knows its predecessors' predecessors
 // to be complete; and after this kernel's tensor memory is allocated: the next kernel's blocks could otherwise take columns that a
 // block of this one still needs, and wait for it.
+// A kernel launched with `early_weights` reads its weights before it calls this, while its predecessor still runs.  Only kernels
+// that are not the first of a library call may: the call's first kernel waits for everything before the call, the weights'
+// writers among it, and no later kernel of the call starts before that.
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

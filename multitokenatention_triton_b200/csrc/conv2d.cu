@@ -124,7 +124,7 @@ int launch_tile(const void* x, PlaneView xv, const void* w, int w_dtype, void* y
 
 int conv2d_launch(const void* x, PlaneView xv, long x_rows_stored, const void* w, int w_dtype, void* y, PlaneView yv,
                   long planes, int C, int H, int W, int R, int S, int causal, int row_begin, int row_end,
-                  bool write_upper, int dtype, cudaStream_t st) {
+                  bool write_upper, int dtype, cudaStream_t st, bool early_weights) {
     if (planes == 0 || row_end <= row_begin || W == 0) return MTA_OK;
     const int want = variant("conv2d");      // 0 auto, 1 CUDA cores, 2 mma.sync tensor cores, 3 tcgen05 tensor cores
     const bool mma_ok = planes <= 65535 && conv2d_mma_supported(x, xv, y, yv, W, R, S, dtype);
@@ -134,7 +134,7 @@ int conv2d_launch(const void* x, PlaneView xv, long x_rows_stored, const void* w
     // Measured on the 6 x 11 bf16 case (B4 H16 S2048): tcgen05 kernel 183 us, mma.sync kernel 274 us, CUDA cores 1289 us.
     if (tc05_ok && (want == 0 || want == 3))
         return conv2d_tc05_launch(x, xv, x_rows_stored, w, w_dtype, y, yv, planes, C, H, W, R, S, causal, row_begin,
-                                  row_end, write_upper, dtype, st);
+                                  row_end, write_upper, dtype, st, false, early_weights);
     if (mma_ok && want != 1)
         return conv2d_mma_launch(x, xv, x_rows_stored, w, w_dtype, y, yv, planes, C, H, W, R, S, causal, row_begin,
                                  row_end, write_upper, dtype, st);
@@ -149,12 +149,12 @@ int conv2d_launch(const void* x, PlaneView xv, long x_rows_stored, const void* w
 
 // Gradient with respect to the conv's input, whole planes; zeros above the diagonal when causal and `write_upper`.
 int conv2d_bwd_input_launch(const void* dy, PlaneView dyv, const void* w, int w_dtype, void* dx, PlaneView dxv, long planes, int C, int H,
-                            int W, int R, int S, int causal, bool write_upper, int dtype, cudaStream_t st) {
+                            int W, int R, int S, int causal, bool write_upper, int dtype, cudaStream_t st, bool early_weights) {
     if (planes == 0 || H == 0 || W == 0) return MTA_OK;
     // 16-bit dtypes, small odd key extents: the tcgen05 conv kernel with the taps reversed (mta_set_variant("conv2d", 1)
     // keeps it on the CUDA cores)
     if (variant("conv2d") != 1 && S % 2 == 1 && planes <= 65535 && conv2d_tc05_supported(dy, dyv, dx, dxv, W, R, S, dtype, w_dtype))
-        return conv2d_tc05_launch(dy, dyv, H, w, w_dtype, dx, dxv, planes, C, H, W, R, S, causal, 0, H, write_upper, dtype, st, true);
+        return conv2d_tc05_launch(dy, dyv, H, w, w_dtype, dx, dxv, planes, C, H, W, R, S, causal, 0, H, write_upper, dtype, st, true, early_weights);
     if (variant("conv2d") == 0 && conv2d_fma_supported(R, S, planes))
         return conv2d_fma_launch(dy, dyv, w, w_dtype, dx, dxv, planes, C, H, W, R, S, causal, 0, H, write_upper, true, dtype, st);
     switch (dtype) {

@@ -83,6 +83,7 @@ __device__ __forceinline__ uint64_t smem_desc_plain(uint32_t saddr, uint32_t lbo
 struct ConvGeom {
     int C, W, R, S, causal, row_begin, row_end, tiles_n, tiles_m, x_row0, write_upper, split_w;
     int nout;          // output staging tiles (1 or 2)
+    int early_weights; // see pdl_wait()
     int lead;          // staged rows start `lead` rows before the tile: R-1 for the conv (row taps look back), 0 for its
                        // input gradient (taps reversed, looking forward)
     int flip;          // input gradient: tap (i, j) uses w[R-1-i][S-1-j]
@@ -218,7 +219,8 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
-    pdl_wait();
+    // the fix-up warps and the MMA issuers touch no other kernel's memory but the weights
+    if (!g.early_weights || !(warp == 1 || warp == 2 || warp == 3 || warp == 8 || warp >= 14)) pdl_wait();
 
     if (warp == 0) {
         // ---------------- producer ----------------
@@ -227,7 +229,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
             it.init(g, t_begin);
             for (int n = 0; n < my_tiles; ++n, it.next(g, g.tiles_m)) {
                 const int st = n % NSTAGE;
-                mbar_wait(&empty_bar[st], ((n / NSTAGE) & 1) ^ 1, err_flag);
+                mbar_wait_spin(&empty_bar[st], ((n / NSTAGE) & 1) ^ 1, err_flag);
                 uint8_t* xa = stage_base + st * stage_bytes;
                 mbar_expect_tx(&full_bar[st], (uint32_t)(NBOX * TH * 128 + TH * 32));
 #pragma unroll
@@ -291,8 +293,8 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
         const uint32_t el = elect_one();
         for (int n = 0; n < my_tiles; ++n) {
             const int st = n % NSTAGE, ab = n & 1;
-            mbar_wait(&ready_bar[st], (n / NSTAGE) & 1, err_flag);
-            mbar_wait(&acc_empty[ab], ((n >> 1) & 1) ^ 1, err_flag);
+            mbar_wait_spin(&ready_bar[st], (n / NSTAGE) & 1, err_flag);
+            mbar_wait_spin(&acc_empty[ab], ((n >> 1) & 1) ^ 1, err_flag);
             __syncwarp();
             fence_after_sync();
             const uint32_t xa_addr = smem_u32(stage_base + st * stage_bytes);
@@ -317,7 +319,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
             uint8_t* xa = stage_base + st * stage_bytes;
             uint8_t* tb = xa + tb_off;
             // the stage (and its Toeplitz slices) is free once the MMAs of tile n - NSTAGE are done
-            mbar_wait(&empty_bar[st], ((n / NSTAGE) & 1) ^ 1, err_flag);
+            mbar_wait_spin(&empty_bar[st], ((n / NSTAGE) & 1) ^ 1, err_flag);
             int ph;
             if (st == 0) { ph = ph0; ph0 = head; }
             else if (st == 1) { ph = ph1; ph1 = head; }
@@ -342,7 +344,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
                 }
                 named_barrier(2, 128);            // nobody refills wsm while another warp still reads it
             }
-            mbar_wait(&full_bar[st], (n / NSTAGE) & 1, err_flag);
+            mbar_wait_spin(&full_bar[st], (n / NSTAGE) & 1, err_flag);
             // staged row sr is query m0-(R-1)+sr; staged column sc is key n0-pad8+sc, in box sc/64 at byte
             // sr*128 + (((sc%64)/8) ^ (sr%8))*16 + (sc%8)*2.  Zero the keys above the query.
             if (g.causal && n0 - pad8 + NCH * 8 - 1 > m0 - g.lead) {
@@ -386,7 +388,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
             const int plane = it.plane, m0 = it.m0(g), n0 = it.n0();
             uint8_t* obuf = out_base + (g.nout == 2 ? ab : 0) * OUT_BYTES;       // staging tile n % nout: two 64-column boxes
             uint8_t* orow = obuf + half * (TM * 128) + row * 128;
-            mbar_wait(&acc_full[ab], (n >> 1) & 1, err_flag);
+            mbar_wait_spin(&acc_full[ab], (n >> 1) & 1, err_flag);
             __syncwarp();
             fence_after_sync();
             if (issuer) {                                    // the store of tile n - nout has finished reading this staging tile
@@ -453,7 +455,7 @@ size_t conv2d_tc05_smem_bytes(int R, bool split_w, int nout) {
 template <typename T>
 int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, int w_dtype, void* y, PlaneView yv,
                 long planes, int C, int W, int R, int S, int causal, int row_begin, int row_end, bool write_upper,
-                bool grad_input, cudaStream_t st) {
+                bool grad_input, bool early_weights, cudaStream_t st) {
     CUtensorMap mx;
     int rc;
     const int TH = TM + R - 1;
@@ -476,6 +478,7 @@ int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, 
     g.split_w = w_dtype == MTA_F32 ? 1 : 0;
     g.lead = grad_input ? 0 : R - 1;
     g.flip = grad_input ? 1 : 0;
+    g.early_weights = early_weights ? 1 : 0;
     const int tiles_m = (row_end - row_begin + TM - 1) / TM;
     g.tiles_m = tiles_m;
     long per_plane = 0;
@@ -507,14 +510,14 @@ bool conv2d_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView
 
 int conv2d_tc05_launch(const void* x, PlaneView xv, long x_rows_stored, const void* w, int w_dtype, void* y, PlaneView yv,
                        long planes, int C, int H, int W, int R, int S, int causal, int row_begin, int row_end,
-                       bool write_upper, int dtype, cudaStream_t st, bool grad_input) {
+                       bool write_upper, int dtype, cudaStream_t st, bool grad_input, bool early_weights) {
     (void)H;
     MTA_REQUIRE(!grad_input || S % 2 == 1, "conv2d (tcgen05): the input gradient needs an odd key extent");
     if (dtype == MTA_BF16)
         return launch_tc05<__nv_bfloat16>(x, xv, x_rows_stored, w, w_dtype, y, yv, planes, C, W, R, S, causal, row_begin,
-                                          row_end, write_upper, grad_input, st);
+                                          row_end, write_upper, grad_input, early_weights, st);
     return launch_tc05<__half>(x, xv, x_rows_stored, w, w_dtype, y, yv, planes, C, W, R, S, causal, row_begin, row_end,
-                               write_upper, grad_input, st);
+                               write_upper, grad_input, early_weights, st);
 }
 
 }  // namespace mta

@@ -92,26 +92,26 @@ int run_forward(const void* q, const void* k, const void* v, const void* w1, con
     }
     if (!qk_in_conv) {
         if ((rc = trace_mark("conv1", st))) return rc;
-        if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w1, w_dtype, bufB, pv, planes, H, S, S, cq, ck, causal, pl.rb, pl.r1, !causal, dtype, st))) return rc;
+        if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w1, w_dtype, bufB, pv, planes, H, S, S, cq, ck, causal, pl.rb, pl.r1, !causal, dtype, st, true))) return rc;
     }
     // the first head mix and the softmax run as one kernel where it applies (mta_set_variant("fused", 1) keeps them apart); with dead
     // keys only the tcgen05 one does
     if (dead.bits && head_mix_softmax_tc05_supported(bufB, pv, bufA, pv, H, S, causal, dtype, w_dtype)) {
         if ((rc = trace_mark("head_mix1+softmax", st))) return rc;
-        if ((rc = head_mix_softmax_tc05_launch(bufB, pv, W1, bufA, pv, B, H, S, pl.rb, pl.r1, false, dtype, st, dead))) return rc;
+        if ((rc = head_mix_softmax_tc05_launch(bufB, pv, W1, bufA, pv, B, H, S, pl.rb, pl.r1, false, dtype, st, dead, true))) return rc;
     } else if (!dead.bits && variant("fused") != 1 && head_mix_softmax_supported(bufB, pv, bufA, pv, H, S, causal, dtype, w_dtype)) {
         if ((rc = trace_mark("head_mix1+softmax", st))) return rc;
-        if ((rc = head_mix_softmax_launch(bufB, pv, W1, w_dtype, bufA, pv, B, H, S, pl.rb, pl.r1, false, dtype, st))) return rc;
+        if ((rc = head_mix_softmax_launch(bufB, pv, W1, w_dtype, bufA, pv, B, H, S, pl.rb, pl.r1, false, dtype, st, true))) return rc;
     } else {
         if ((rc = trace_mark("head_mix1", st))) return rc;
-        if ((rc = head_linear_launch(bufB, pv, W1, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.rb, pl.r1, false, dtype, st))) return rc;
+        if ((rc = head_linear_launch(bufB, pv, W1, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.rb, pl.r1, false, dtype, st, false, true))) return rc;
         if ((rc = trace_mark("softmax", st))) return rc;
         if ((rc = softmax_launch(bufA, pv, bufA, pv, planes, S, S, causal, pl.rb, pl.r1, false, 1.0f, dtype, st, dead, H))) return rc;
     }
     if ((rc = trace_mark("conv2", st))) return rc;
-    if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w2, w_dtype, bufB, pv, planes, H, S, S, cq2, ck2, causal, pl.r0, pl.r1, !causal, dtype, st))) return rc;
+    if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w2, w_dtype, bufB, pv, planes, H, S, S, cq2, ck2, causal, pl.r0, pl.r1, !causal, dtype, st, true))) return rc;
     if ((rc = trace_mark("head_mix2", st))) return rc;
-    if ((rc = head_linear_launch(bufB, pv, W2, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.r0, pl.r1, false, dtype, st))) return rc;
+    if ((rc = head_linear_launch(bufB, pv, W2, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.r0, pl.r1, false, dtype, st, false, true))) return rc;
     if ((rc = trace_mark("pv", st))) return rc;
     if ((rc = pv_launch(bufA, pv, pl.r1 - pl.ra, v, o, B, H, S, D, causal, pl.r0, pl.r1, dtype, st, drop))) return rc;
     return trace_end(st);

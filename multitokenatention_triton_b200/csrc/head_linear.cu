@@ -36,14 +36,15 @@ template <typename T, int CP, int V>
 __global__ void __launch_bounds__(HS_WARPS * 32, hs_min_ctas(CP))
 head_linear_simt_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
                         T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin, int row_end,
-                        int rows_per_warp, int write_upper, int w_transposed, int vec) {
+                        int rows_per_warp, int write_upper, int w_transposed, int vec, int early_weights) {
     extern __shared__ __align__(16) float ws[];   // [h][o], o padded to a multiple of HS_OG
-    pdl_wait();
+    if (!early_weights) pdl_wait();
     const int OP = (C + HS_OG - 1) / HS_OG * HS_OG;
     for (int i = threadIdx.x; i < CP * OP; i += HS_WARPS * 32) {
         const int h = i / OP, o = i - h * OP;
         ws[i] = h < C && o < C ? load_weight(Wm, w_transposed ? (long)h * C + o : (long)o * C + h, w_dtype) : 0.0f;
     }
+    if (early_weights) pdl_wait();
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long n = blockIdx.z;
@@ -200,7 +201,7 @@ template <typename T, int CP, bool SPLITW>
 __device__ __forceinline__ void
 head_linear_mma_body(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
                      T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
-                     int row_end, int rows_per_cta, int write_upper, int w_transposed) {
+                     int row_end, int rows_per_cta, int write_upper, int w_transposed, int early_weights) {
     constexpr int KSTEPS = CP / 8;
     constexpr int MT = (CP + 15) / 16;
     constexpr int NLOAD = CP / 4;            // head planes read per lane: t, t+4, ...
@@ -208,6 +209,7 @@ head_linear_mma_body(const T* __restrict__ x, PlaneView xv, const void* __restri
     const int g = lane >> 2, t = lane & 3;
     const long n = blockIdx.z;
 
+    if (!early_weights) pdl_wait();
     // A fragments of the weight: a0 (g, t) a1 (g+8, t) a2 (g, t+4) a3 (g+8, t+4) of each 16x8 block.
     uint32_t wa[MT][KSTEPS][4];
     uint32_t wl[SPLITW ? MT : 1][SPLITW ? KSTEPS : 1][4];
@@ -229,6 +231,7 @@ head_linear_mma_body(const T* __restrict__ x, PlaneView xv, const void* __restri
                 }
             }
 
+    if (early_weights) pdl_wait();
     const int key0 = (blockIdx.x * MMA_WARPS + warp) * MMA_KEYS_PER_WARP;
     if (key0 >= Q) return;
     const uint32_t fill2 = pack2<T>(fill, fill);
@@ -356,20 +359,18 @@ template <typename T, int CP, bool SPLITW>
 __global__ void __launch_bounds__(MMA_WARPS * 32)
 head_linear_mma_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
                        T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
-                       int row_end, int rows_per_cta, int write_upper, int w_transposed) {
-    pdl_wait();
+                       int row_end, int rows_per_cta, int write_upper, int w_transposed, int early_weights) {
     head_linear_mma_body<T, CP, SPLITW>(x, xv, Wm, w_dtype, y, yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,
-                                        write_upper, w_transposed);
+                                        write_upper, w_transposed, early_weights);
 }
 // More than 16 heads: twice the accumulators and weight fragments; bounded so that HL_MIN_CTAS_WIDE CTAs stay resident.
 template <typename T, int CP, bool SPLITW>
 __global__ void __launch_bounds__(MMA_WARPS * 32, HL_MIN_CTAS_WIDE)
 head_linear_mma_wide_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
                             T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
-                            int row_end, int rows_per_cta, int write_upper, int w_transposed) {
-    pdl_wait();
+                            int row_end, int rows_per_cta, int write_upper, int w_transposed, int early_weights) {
     head_linear_mma_body<T, CP, SPLITW>(x, xv, Wm, w_dtype, y, yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,
-                                        write_upper, w_transposed);
+                                        write_upper, w_transposed, early_weights);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -761,7 +762,7 @@ int launch_mix_softmax(const void* x, PlaneView xv, const void* Wm, int w_dtype,
 
 template <typename T, int CP, int V>
 int launch_simt(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C, int Q,
-                int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st) {
+                int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, bool early, cudaStream_t st) {
     auto vec_ok = [](const void* p, const PlaneView& v) {
         return v.width % V == 0 && v.plane_stride % V == 0 && reinterpret_cast<uintptr_t>(p) % (V * sizeof(T)) == 0;
     };
@@ -776,15 +777,15 @@ int launch_simt(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* 
     const size_t smem = (size_t)CP * ((C + HS_OG - 1) / HS_OG * HS_OG) * sizeof(float);
     return launch_kernel<head_linear_simt_kernel<T, CP, V>>("head_linear_simt_kernel", grid, HS_WARPS * 32, smem, st, static_cast<const T*>(x), xv, Wm,
                                                             w_dtype, static_cast<T*>(y), yv, C, Q, causal, fill, row_begin, row_end, rows_per_warp,
-                                                            write_upper ? 1 : 0, wt ? 1 : 0, vec_ok(x, xv) && vec_ok(y, yv) ? 1 : 0);
+                                                            write_upper ? 1 : 0, wt ? 1 : 0, vec_ok(x, xv) && vec_ok(y, yv) ? 1 : 0, early ? 1 : 0);
 }
 
 template <typename T>
 int dispatch_simt(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C, int Q,
-                  int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st) {
+                  int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, bool early, cudaStream_t st) {
 // keys per thread: what C inputs of each leave of the registers
 #define MTA_SIMT_CASE(CPV, VV) \
-    return launch_simt<T, CPV, VV>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st)
+    return launch_simt<T, CPV, VV>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, early, st)
     if (C <= 8) MTA_SIMT_CASE(8, 4);
     if (C <= 12) MTA_SIMT_CASE(12, 4);
     if (C <= 16) MTA_SIMT_CASE(16, 4);
@@ -796,7 +797,7 @@ int dispatch_simt(const void* x, PlaneView xv, const void* Wm, int w_dtype, void
 
 template <typename T, int CP>
 int launch_mma(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C, int Q,
-               int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st) {
+               int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, bool early, cudaStream_t st) {
     const int rows = row_end - row_begin;
     const int rows_per_cta = rows >= 2048 ? 8 : (rows >= 256 ? 4 : 1);
     dim3 grid((unsigned)((Q + MMA_WARPS * MMA_KEYS_PER_WARP - 1) / (MMA_WARPS * MMA_KEYS_PER_WARP)),
@@ -804,7 +805,7 @@ int launch_mma(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y
 #define MTA_HL_LAUNCH(KERNEL, SPLIT)                                                                                                   \
     return launch_kernel<KERNEL<T, CP, SPLIT>>("head_linear_mma_kernel", grid, MMA_WARPS * 32, 0, st, static_cast<const T*>(x), xv, Wm,   \
                                                w_dtype, static_cast<T*>(y), yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,    \
-                                               write_upper ? 1 : 0, wt ? 1 : 0)
+                                               write_upper ? 1 : 0, wt ? 1 : 0, early ? 1 : 0)
     if constexpr (CP > 16) {
         if (w_dtype == MTA_F32) MTA_HL_LAUNCH(head_linear_mma_wide_kernel, true);
         else MTA_HL_LAUNCH(head_linear_mma_wide_kernel, false);
@@ -817,9 +818,9 @@ int launch_mma(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y
 
 template <typename T>
 int dispatch_mma(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C, int Q,
-                 int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st) {
+                 int causal, float fill, int row_begin, int row_end, bool write_upper, bool wt, bool early, cudaStream_t st) {
 #define MTA_MMA_CASE(CPV) \
-    return launch_mma<T, CPV>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st)
+    return launch_mma<T, CPV>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, early, st)
     if (C <= 8) MTA_MMA_CASE(8);
     if (C <= 16) MTA_MMA_CASE(16);
     MTA_MMA_CASE(32);
@@ -845,7 +846,7 @@ bool head_mix_softmax_supported(const void* x, PlaneView xv, const void* y, Plan
 }
 
 int head_mix_softmax_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C,
-                            int Q, int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st) {
+                            int Q, int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, bool early_weights) {
     if (N == 0 || row_end <= row_begin || Q == 0) return MTA_OK;
     // variant "mix_softmax": 0 auto (tcgen05 where it applies), 1 the mma.sync kernel, 2 tcgen05 or an error
     const int want = variant("mix_softmax");
@@ -856,7 +857,7 @@ int head_mix_softmax_launch(const void* x, PlaneView xv, const void* Wm, int w_d
     // at every shape tried (B8 H16 S4096: 1.39 against 2.05 ms; B4 H32 S4096: 1.40 against 2.21; B1 H32 S8192: 1.48 against
     // 2.21; B32 H16 S512: 0.16 against 0.39), so it runs wherever it applies.
     if (tc05_able && want != 1)
-        return head_mix_softmax_tc05_launch(x, xv, Wm, y, yv, N, C, Q, row_begin, row_end, write_upper, dtype, st);
+        return head_mix_softmax_tc05_launch(x, xv, Wm, y, yv, N, C, Q, row_begin, row_end, write_upper, dtype, st, DeadKeys(), early_weights);
     MTA_REQUIRE(mix_softmax_mma_ok(x, xv, y, yv, C, Q, 1, dtype),
                 "head_mix_softmax: needs a 16-bit dtype, C <= 32, Q %% 8 == 0, 16-byte aligned rows and x != y");
     MTA_REQUIRE(N <= 65535, "head_mix_softmax: N = %d exceeds 65535", N);
@@ -874,7 +875,7 @@ int head_mix_softmax_launch(const void* x, PlaneView xv, const void* Wm, int w_d
 
 int head_linear_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C,
                        int P, int Q, int causal, float fill, int row_begin, int row_end, bool write_upper, int dtype,
-                       cudaStream_t st, bool wt) {
+                       cudaStream_t st, bool wt, bool early) {
     (void)P;
     if (N == 0 || row_end <= row_begin || Q == 0) return MTA_OK;
     MTA_REQUIRE(C >= 1 && C <= 128, "head_linear: C = %d heads is outside the supported range 1..128", C);
@@ -890,15 +891,15 @@ int head_linear_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype,
     // of the copy bandwidth and the tcgen05 kernel takes 0.95 to 1.16 of its time (B4 H16 S2048: 0.173 against 0.160 ms),
     // so tcgen05 is the default only for 64 and 128 heads, which the mma.sync kernel does not take.
     if (tc05_able && (want == 3 || (want == 0 && !mma_able)))
-        return head_linear_tc05_launch(x, xv, Wm, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, dtype, st);
+        return head_linear_tc05_launch(x, xv, Wm, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, dtype, st, early);
     const bool use_mma = mma_able && want != 1;
     if (dtype == MTA_F32)
-        return dispatch_simt<float>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st);
+        return dispatch_simt<float>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, early, st);
     if (dtype == MTA_BF16)
-        return use_mma ? dispatch_mma<__nv_bfloat16>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st)
-                       : dispatch_simt<__nv_bfloat16>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st);
-    return use_mma ? dispatch_mma<__half>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st)
-                   : dispatch_simt<__half>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st);
+        return use_mma ? dispatch_mma<__nv_bfloat16>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, early, st)
+                       : dispatch_simt<__nv_bfloat16>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, early, st);
+    return use_mma ? dispatch_mma<__half>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, early, st)
+                   : dispatch_simt<__half>(x, xv, Wm, w_dtype, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, early, st);
 }
 
 }  // namespace mta

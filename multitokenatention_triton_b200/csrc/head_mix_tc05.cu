@@ -201,6 +201,7 @@ struct HmGeom {
     float fill;          // value of the entries above the diagonal (plain head mix; the softmax writes 0 there)
     long units;
     DeadKeys dead;       // softmax only
+    int early_weights;
 };
 
 // Key tiles that the rows of the group starting at p0 reach.
@@ -259,7 +260,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
         for (int i = tid; i < HM_OUT_BYTES / 16; i += HM_THREADS) reinterpret_cast<uint4*>(fill_base)[i] = make_uint4(f2, f2, f2, f2);
     }
     __syncthreads();
-    pdl_wait();
+    if (!g.early_weights) pdl_wait();
     for (int i = tid; i < 128 * C; i += HM_THREADS) {
         const int m = i / C, h = i % C;
         const int r = m % R, o = m / R;
@@ -271,6 +272,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    if (g.early_weights) pdl_wait();
 
     // Every role walks the same sequence of units and, within a unit, of 2 * nt tiles: pass 1 upwards, pass 2 downwards.
     // Units, heaviest first, are dealt to the CTAs in rounds of alternating direction (equal tile counts per CTA, as in
@@ -502,9 +504,10 @@ constexpr size_t HM_SMEM_BYTES = 1024 + HM_A_BYTES + (size_t)HM_NSTAGE * HM_STAG
 
 template <typename T, bool SOFTMAX>
 int launch_hm(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q, int causal, float fill,
-              int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st, DeadKeys dead = DeadKeys()) {
+              int row_begin, int row_end, bool write_upper, bool wt, cudaStream_t st, DeadKeys dead, bool early_weights) {
     HmGeom g{};
     g.dead = dead;
+    g.early_weights = early_weights ? 1 : 0;
     g.N = N; g.C = C; g.R = 128 / C; g.Q = Q; g.row_begin = row_begin; g.row_end = row_end;
     g.groups = (row_end - row_begin + g.R - 1) / g.R;
     g.write_upper = (write_upper && causal) ? 1 : 0;
@@ -554,11 +557,11 @@ bool head_mix_softmax_tc05_supported(const void* x, PlaneView xv, const void* y,
 }
 
 int head_mix_softmax_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q,
-                                 int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, DeadKeys dead) {
+                                 int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, DeadKeys dead, bool early_weights) {
     if (N == 0 || row_end <= row_begin || Q == 0) return MTA_OK;
     if (dtype == MTA_BF16)
-        return launch_hm<__nv_bfloat16, true>(x, xv, Wm, y, yv, N, C, Q, 1, 0.0f, row_begin, row_end, write_upper, false, st, dead);
-    return launch_hm<__half, true>(x, xv, Wm, y, yv, N, C, Q, 1, 0.0f, row_begin, row_end, write_upper, false, st, dead);
+        return launch_hm<__nv_bfloat16, true>(x, xv, Wm, y, yv, N, C, Q, 1, 0.0f, row_begin, row_end, write_upper, false, st, dead, early_weights);
+    return launch_hm<__half, true>(x, xv, Wm, y, yv, N, C, Q, 1, 0.0f, row_begin, row_end, write_upper, false, st, dead, early_weights);
 }
 
 bool head_linear_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int dtype, int w_dtype) {
@@ -566,11 +569,11 @@ bool head_linear_tc05_supported(const void* x, PlaneView xv, const void* y, Plan
 }
 
 int head_linear_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q, int causal,
-                            float fill, int row_begin, int row_end, bool write_upper, bool wt, int dtype, cudaStream_t st) {
+                            float fill, int row_begin, int row_end, bool write_upper, bool wt, int dtype, cudaStream_t st, bool early_weights) {
     if (N == 0 || row_end <= row_begin || Q == 0) return MTA_OK;
     if (dtype == MTA_BF16)
-        return launch_hm<__nv_bfloat16, false>(x, xv, Wm, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st);
-    return launch_hm<__half, false>(x, xv, Wm, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st);
+        return launch_hm<__nv_bfloat16, false>(x, xv, Wm, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st, DeadKeys(), early_weights);
+    return launch_hm<__half, false>(x, xv, Wm, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, st, DeadKeys(), early_weights);
 }
 
 }  // namespace mta

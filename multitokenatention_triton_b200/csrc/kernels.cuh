@@ -22,13 +22,15 @@ int swap_heads_launch(const void* in, void* out, int B, int H, int S, int D, int
 int mask_prepare_launch(const unsigned char* key_mask, const void* k, const void* v, uint32_t* bits, void* k_out, void* v_out, int B, int H,
                         int S, int D, int dtype, cudaStream_t st);
 
+// `early_weights` below: this is not the first kernel of the library call (see pdl_wait() in common.cuh).
+//
 // Depthwise causal conv over planes; computes output rows [row_begin,row_end) of every plane.
 // When `write_upper` the entries above the diagonal of those rows are written as 0, otherwise they
 // are left untouched (internal scratch whose upper triangle nobody reads).
 // `x_rows_stored` = rows each plane of x holds (from xv.row0 on).
 int conv2d_launch(const void* x, PlaneView xv, long x_rows_stored, const void* w, int w_dtype, void* y, PlaneView yv,
                   long planes, int C, int H, int W, int R, int S, int causal, int row_begin, int row_end,
-                  bool write_upper, int dtype, cudaStream_t st);
+                  bool write_upper, int dtype, cudaStream_t st, bool early_weights = false);
 // CUDA cores, odd key extents 3 .. 15 (conv2d_fma.cu): the conv or its input gradient, and the weight gradient's per-part sums.
 bool conv2d_fma_supported(int R, int S, long planes);
 int conv2d_fma_launch(const void* x, PlaneView xv, const void* w, int w_dtype, void* y, PlaneView yv, long planes, int C, int H, int W, int R,
@@ -45,12 +47,12 @@ int conv2d_mma_launch(const void* x, PlaneView xv, long x_rows_stored, const voi
 // `w_transposed`: y[o] = sum_h Wm[h,o] x[h] (the gradient with respect to the head mix's input).
 int head_linear_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N,
                        int C, int P, int Q, int causal, float fill, int row_begin, int row_end, bool write_upper,
-                       int dtype, cudaStream_t st, bool w_transposed = false);
+                       int dtype, cudaStream_t st, bool w_transposed = false, bool early_weights = false);
 
 // Gradients of the two stand-alone ops (backward.cu, conv2d.cu).  dx of the conv: zeros above the diagonal when causal and
 // `write_upper`.  The weight gradients come in `dw_dtype`, reduced in a fixed order through a caller workspace.
 int conv2d_bwd_input_launch(const void* dy, PlaneView dyv, const void* w, int w_dtype, void* dx, PlaneView dxv, long planes, int C, int H,
-                            int W, int R, int S, int causal, bool write_upper, int dtype, cudaStream_t st);
+                            int W, int R, int S, int causal, bool write_upper, int dtype, cudaStream_t st, bool early_weights = false);
 size_t conv2d_bwd_weight_workspace(int N, int C, int H, int W, int R, int S);
 int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dw, int dw_dtype, void* workspace, int N, int C,
                              int H, int W, int R, int S, int causal, int dtype, cudaStream_t st);
@@ -73,20 +75,21 @@ int head_dw_tc05_launch(const void* x, PlaneView xv, const void* dy, PlaneView d
 bool head_mix_softmax_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int causal, int dtype,
                                 int w_dtype);
 int head_mix_softmax_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C,
-                            int Q, int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st);
+                            int Q, int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, bool early_weights = false);
 
 // The same on tcgen05 (head_mix_tc05.cu): C a power of two in 8..128, weights in the activations' 16-bit dtype; entries
 // above the diagonal are written as 0 up to the end of the diagonal's 128-key tile, and up to Q when `write_upper`.
 bool head_mix_softmax_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int causal, int dtype,
                                      int w_dtype);
 int head_mix_softmax_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q,
-                                 int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, DeadKeys dead = DeadKeys());
+                                 int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, DeadKeys dead = DeadKeys(),
+                                 bool early_weights = false);
 
 // The plain head mix on the same kernel (one pass): y = Wm x over the head axis (Wm read transposed when `wt`), `fill`
 // above the diagonal when causal (written up to the end of the diagonal's key tile, and up to Q when `write_upper`).
 bool head_linear_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int dtype, int w_dtype);
 int head_linear_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q, int causal,
-                            float fill, int row_begin, int row_end, bool write_upper, bool wt, int dtype, cudaStream_t st);
+                            float fill, int row_begin, int row_end, bool write_upper, bool wt, int dtype, cudaStream_t st, bool early_weights = false);
 
 // Causal row softmax of pre_scale * x; rows [row_begin,row_end).  `dead` (planes of one batch element: `heads`): keys that get
 // probability 0, in a row with no other key too.
@@ -131,7 +134,7 @@ bool conv2d_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView
 // looking forward - with x = dy and y = dx.
 int conv2d_tc05_launch(const void* x, PlaneView xv, long x_rows_stored, const void* w, int w_dtype, void* y, PlaneView yv,
                        long planes, int C, int H, int W, int R, int S, int causal, int row_begin, int row_end,
-                       bool write_upper, int dtype, cudaStream_t st, bool grad_input = false);
+                       bool write_upper, int dtype, cudaStream_t st, bool grad_input = false, bool early_weights = false);
 
 // tcgen05 tensor-core versions (gemm_tc05.cu): 16-bit dtypes, D in {64,128}, S a multiple of 8.
 bool tc05_contractions_supported(int S, int D, int dtype, const void* a, const void* b, const void* c, PlaneView view);

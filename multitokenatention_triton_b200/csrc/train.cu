@@ -88,15 +88,15 @@ int mta_train_fwd(const void* q, const void* k, const void* v, const void* w1, c
     for (int i = 0; i < SAVED; ++i) pl[i] = base + i * t.plane_bytes;
     int rc;
     if ((rc = qk_scores_launch(q, k, pl[SCORES], t.v, B, H, S, D, 1.0f / sqrtf((float)D), dtype != MTA_F32, 1, 0, S, dtype, st))) return rc;
-    if ((rc = conv2d_launch(pl[SCORES], t.v, S, w1, w_dtype, pl[CONV1], t.v, t.planes, H, S, S, cq, ck, 1, 0, S, false, dtype, st))) return rc;
+    if ((rc = conv2d_launch(pl[SCORES], t.v, S, w1, w_dtype, pl[CONV1], t.v, t.planes, H, S, S, cq, ck, 1, 0, S, false, dtype, st, true))) return rc;
     if (head_mix_softmax_supported(pl[CONV1], t.v, pl[PROBS], t.v, H, S, 1, dtype, w_dtype)) {
-        if ((rc = head_mix_softmax_launch(pl[CONV1], t.v, W1, w_dtype, pl[PROBS], t.v, B, H, S, 0, S, false, dtype, st))) return rc;
+        if ((rc = head_mix_softmax_launch(pl[CONV1], t.v, W1, w_dtype, pl[PROBS], t.v, B, H, S, 0, S, false, dtype, st, true))) return rc;
     } else {
-        if ((rc = head_linear_launch(pl[CONV1], t.v, W1, w_dtype, pl[PROBS], t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st))) return rc;
+        if ((rc = head_linear_launch(pl[CONV1], t.v, W1, w_dtype, pl[PROBS], t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st, false, true))) return rc;
         if ((rc = softmax_launch(pl[PROBS], t.v, pl[PROBS], t.v, t.planes, S, S, 1, 0, S, false, 1.0f, dtype, st))) return rc;
     }
-    if ((rc = conv2d_launch(pl[PROBS], t.v, S, w2, w_dtype, pl[CONV2], t.v, t.planes, H, S, S, cq2, ck2, 1, 0, S, false, dtype, st))) return rc;
-    if ((rc = head_linear_launch(pl[CONV2], t.v, W2, w_dtype, pl[MIX2], t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st))) return rc;
+    if ((rc = conv2d_launch(pl[PROBS], t.v, S, w2, w_dtype, pl[CONV2], t.v, t.planes, H, S, S, cq2, ck2, 1, 0, S, false, dtype, st, true))) return rc;
+    if ((rc = head_linear_launch(pl[CONV2], t.v, W2, w_dtype, pl[MIX2], t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st, false, true))) return rc;
     return pv_launch(pl[MIX2], t.v, S, v, o, B, H, S, D, 1, 0, S, dtype, st);
 }
 
@@ -136,17 +136,17 @@ int mta_train_bwd(const void* q, const void* k, const void* v, const void* w1, c
     if ((rc = qk_scores_launch(dout, v, ga, t.v, B, H, S, D, 1.0f, 0, 1, 0, S, dtype, st))) return rc;
     if (dW2 && (rc = head_linear_bwd_weight_launch(pl[CONV2], t.v, ga, t.v, dW2, w_dtype, partial, B, H, S, S, 1, dtype, st))) return rc;
     if (!to_conv2) return MTA_OK;
-    if ((rc = head_linear_launch(ga, t.v, W2, w_dtype, gb, t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st, true))) return rc;      // d(conv 2)
+    if ((rc = head_linear_launch(ga, t.v, W2, w_dtype, gb, t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st, true, true))) return rc;      // d(conv 2)
     if (dw2 && (rc = conv2d_bwd_weight_launch(pl[PROBS], t.v, gb, t.v, dw2, w_dtype, partial, B, H, S, S, cq2, ck2, 1, dtype, st))) return rc;
     if (!to_mix1) return MTA_OK;
-    if ((rc = conv2d_bwd_input_launch(gb, t.v, w2, w_dtype, ga, t.v, t.planes, H, S, S, cq2, ck2, 1, false, dtype, st))) return rc;  // d(probabilities)
+    if ((rc = conv2d_bwd_input_launch(gb, t.v, w2, w_dtype, ga, t.v, t.planes, H, S, S, cq2, ck2, 1, false, dtype, st, true))) return rc;  // d(probabilities)
     if ((rc = softmax_bwd_launch(pl[PROBS], t.v, ga, t.v, ga, t.v, t.planes, S, S, 1, dtype, st))) return rc;                       // d(head mix 1)
     if (dW1 && (rc = head_linear_bwd_weight_launch(pl[CONV1], t.v, ga, t.v, dW1, w_dtype, partial, B, H, S, S, 1, dtype, st))) return rc;
     if (!to_conv1) return MTA_OK;
-    if ((rc = head_linear_launch(ga, t.v, W1, w_dtype, gb, t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st, true))) return rc;      // d(conv 1)
+    if ((rc = head_linear_launch(ga, t.v, W1, w_dtype, gb, t.v, B, H, S, S, 1, 0.0f, 0, S, false, dtype, st, true, true))) return rc;      // d(conv 1)
     if (dw1 && (rc = conv2d_bwd_weight_launch(pl[SCORES], t.v, gb, t.v, dw1, w_dtype, partial, B, H, S, S, cq, ck, 1, dtype, st))) return rc;
     if (!to_scores) return MTA_OK;
-    if ((rc = conv2d_bwd_input_launch(gb, t.v, w1, w_dtype, ga, t.v, t.planes, H, S, S, cq, ck, 1, false, dtype, st))) return rc;    // d(scores)
+    if ((rc = conv2d_bwd_input_launch(gb, t.v, w1, w_dtype, ga, t.v, t.planes, H, S, S, cq, ck, 1, false, dtype, st, true))) return rc;    // d(scores)
     if (dq && (rc = pv_launch(ga, t.v, S, k, dq, B, H, S, D, 1, 0, S, dtype, st, DropoutSpec(), scale))) return rc;
     if (dk && (rc = ptx_launch(ga, t.v, q, dk, B, H, S, D, 1, scale, dtype, st))) return rc;
     return MTA_OK;
