@@ -887,10 +887,14 @@ int head_linear_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype,
     MTA_REQUIRE(want != 2 || mma_able, "head_linear: the mma.sync variant needs a 16-bit dtype, C <= 32, Q %% 8 == 0 and 16-byte aligned rows");
     MTA_REQUIRE(want != 3 || tc05_able,
                 "head_linear: the tcgen05 variant needs 16-bit activations and weights of one dtype, 8, 16, 32, 64 or 128 heads and x != y");
-    // Measured on B200 (bf16, causal, upper triangle written): up to 32 heads the mma.sync kernel already runs at 78 to 87 %
-    // of the copy bandwidth and the tcgen05 kernel takes 0.95 to 1.16 of its time (B4 H16 S2048: 0.173 against 0.160 ms),
-    // so tcgen05 is the default only for 64 and 128 heads, which the mma.sync kernel does not take.
-    if (tc05_able && (want == 3 || (want == 0 && !mma_able)))
+    // Measured on B200 (bf16, mma.sync / tcgen05, us).  More than 16 heads: B1 H32 S4096 269 / 206, S256 11.7 / 7.8, S128 5.2 / 7.2.
+    // Up to 16 heads on the lower triangle only: B8 H16 S1024 68 / 53, B8 H8 S1024 38 / 28, B1 H16 S2048 forward 182 / 174; shorter
+    // rows keep the mma.sync kernel, whose blocks start faster (S512 5.6 / 7.7), and so do longer ones and whole planes, where
+    // HBM is the limit and it is the better streamer (B8 H16 S4096 forward 4640 / 4800, B4 H16 S2048 alone 158 / 173).  The choice
+    // depends on the heads, the row length and the output's form only, so that a row range or a part of the batch gets the same
+    // bits as the whole.
+    const bool tc05_better = C > 16 ? Q >= 256 : (causal && !write_upper && Q >= 1024 && Q < 4096);
+    if (tc05_able && (want == 3 || (want == 0 && (!mma_able || tc05_better))))
         return head_linear_tc05_launch(x, xv, Wm, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, dtype, st, early);
     const bool use_mma = mma_able && want != 1;
     if (dtype == MTA_F32)
