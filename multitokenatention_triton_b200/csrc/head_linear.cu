@@ -197,11 +197,11 @@ constexpr int MMA_KEYS_PER_WARP = 64;       // keys of one row handled per warp 
 constexpr int HL_MIN_CTAS_WIDE = 3;    // resident CTAs per SM asked for when there are more than 16 heads (B1 H32 S8192 bf16:
                                        // 1.015 ms unconstrained at 182 registers, 0.891 with 3, 1.869 with 4, which spills)
 // The kernel body; the two __global__ entry points below differ only in their register bound.
-template <typename T, int CP, bool SPLITW>
+template <typename T, int CP, bool SPLITW, bool EARLY>
 __device__ __forceinline__ void
 head_linear_mma_body(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
                      T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
-                     int row_end, int rows_per_cta, int write_upper, int w_transposed, int early_weights) {
+                     int row_end, int rows_per_cta, int write_upper, int w_transposed) {
     constexpr int KSTEPS = CP / 8;
     constexpr int MT = (CP + 15) / 16;
     constexpr int NLOAD = CP / 4;            // head planes read per lane: t, t+4, ...
@@ -209,7 +209,7 @@ head_linear_mma_body(const T* __restrict__ x, PlaneView xv, const void* __restri
     const int g = lane >> 2, t = lane & 3;
     const long n = blockIdx.z;
 
-    if (!early_weights) pdl_wait();
+    if (!EARLY) pdl_wait();
     // A fragments of the weight: a0 (g, t) a1 (g+8, t) a2 (g, t+4) a3 (g+8, t+4) of each 16x8 block.
     uint32_t wa[MT][KSTEPS][4];
     uint32_t wl[SPLITW ? MT : 1][SPLITW ? KSTEPS : 1][4];
@@ -231,7 +231,7 @@ head_linear_mma_body(const T* __restrict__ x, PlaneView xv, const void* __restri
                 }
             }
 
-    if (early_weights) pdl_wait();
+    if (EARLY) pdl_wait();
     const int key0 = (blockIdx.x * MMA_WARPS + warp) * MMA_KEYS_PER_WARP;
     if (key0 >= Q) return;
     const uint32_t fill2 = pack2<T>(fill, fill);
@@ -353,24 +353,26 @@ head_linear_mma_body(const T* __restrict__ x, PlaneView xv, const void* __restri
     }
 }
 
+// EARLY: the weights are read before the wait on the predecessor (see pdl_wait()); a run-time test of it cost 16 registers and
+// one resident CTA of five (B8 H16 S4096: 0.85 against 0.76 ms).
 // Up to 16 heads: no bound on resident CTAs (the compiler settles at 96 to 120 registers; stating a bound of one CTA
 // made it take far more and the kernel slower: 0.84 ms against 0.76 ms at B8 H16 S4096).
-template <typename T, int CP, bool SPLITW>
+template <typename T, int CP, bool SPLITW, bool EARLY>
 __global__ void __launch_bounds__(MMA_WARPS * 32)
 head_linear_mma_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
                        T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
-                       int row_end, int rows_per_cta, int write_upper, int w_transposed, int early_weights) {
-    head_linear_mma_body<T, CP, SPLITW>(x, xv, Wm, w_dtype, y, yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,
-                                        write_upper, w_transposed, early_weights);
+                       int row_end, int rows_per_cta, int write_upper, int w_transposed) {
+    head_linear_mma_body<T, CP, SPLITW, EARLY>(x, xv, Wm, w_dtype, y, yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,
+                                        write_upper, w_transposed);
 }
 // More than 16 heads: twice the accumulators and weight fragments; bounded so that HL_MIN_CTAS_WIDE CTAs stay resident.
-template <typename T, int CP, bool SPLITW>
+template <typename T, int CP, bool SPLITW, bool EARLY>
 __global__ void __launch_bounds__(MMA_WARPS * 32, HL_MIN_CTAS_WIDE)
 head_linear_mma_wide_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ Wm, int w_dtype,
                             T* __restrict__ y, PlaneView yv, int C, int Q, int causal, float fill, int row_begin,
-                            int row_end, int rows_per_cta, int write_upper, int w_transposed, int early_weights) {
-    head_linear_mma_body<T, CP, SPLITW>(x, xv, Wm, w_dtype, y, yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,
-                                        write_upper, w_transposed, early_weights);
+                            int row_end, int rows_per_cta, int write_upper, int w_transposed) {
+    head_linear_mma_body<T, CP, SPLITW, EARLY>(x, xv, Wm, w_dtype, y, yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,
+                                        write_upper, w_transposed);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -802,17 +804,23 @@ int launch_mma(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y
     const int rows_per_cta = rows >= 2048 ? 8 : (rows >= 256 ? 4 : 1);
     dim3 grid((unsigned)((Q + MMA_WARPS * MMA_KEYS_PER_WARP - 1) / (MMA_WARPS * MMA_KEYS_PER_WARP)),
               (unsigned)((rows + rows_per_cta - 1) / rows_per_cta), (unsigned)N);
-#define MTA_HL_LAUNCH(KERNEL, SPLIT)                                                                                                   \
-    return launch_kernel<KERNEL<T, CP, SPLIT>>("head_linear_mma_kernel", grid, MMA_WARPS * 32, 0, st, static_cast<const T*>(x), xv, Wm,   \
-                                               w_dtype, static_cast<T*>(y), yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta,    \
-                                               write_upper ? 1 : 0, wt ? 1 : 0, early ? 1 : 0)
+#define MTA_HL_RUN(KERNEL, SPLIT, EARLY)                                                                                                   \
+    return launch_kernel<KERNEL<T, CP, SPLIT, EARLY>>("head_linear_mma_kernel", grid, MMA_WARPS * 32, 0, st, static_cast<const T*>(x), xv, Wm, \
+                                                      w_dtype, static_cast<T*>(y), yv, C, Q, causal, fill, row_begin, row_end, rows_per_cta, \
+                                                      write_upper ? 1 : 0, wt ? 1 : 0)
+#define MTA_HL_LAUNCH(KERNEL, SPLIT)                       \
+    do {                                                   \
+        if (early) MTA_HL_RUN(KERNEL, SPLIT, true);        \
+        MTA_HL_RUN(KERNEL, SPLIT, false);                  \
+    } while (0)
     if constexpr (CP > 16) {
         if (w_dtype == MTA_F32) MTA_HL_LAUNCH(head_linear_mma_wide_kernel, true);
-        else MTA_HL_LAUNCH(head_linear_mma_wide_kernel, false);
+        MTA_HL_LAUNCH(head_linear_mma_wide_kernel, false);
     } else {
         if (w_dtype == MTA_F32) MTA_HL_LAUNCH(head_linear_mma_kernel, true);
-        else MTA_HL_LAUNCH(head_linear_mma_kernel, false);
+        MTA_HL_LAUNCH(head_linear_mma_kernel, false);
     }
+#undef MTA_HL_RUN
 #undef MTA_HL_LAUNCH
 }
 
