@@ -895,13 +895,12 @@ int head_linear_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype,
     MTA_REQUIRE(want != 2 || mma_able, "head_linear: the mma.sync variant needs a 16-bit dtype, C <= 32, Q %% 8 == 0 and 16-byte aligned rows");
     MTA_REQUIRE(want != 3 || tc05_able,
                 "head_linear: the tcgen05 variant needs 16-bit activations and weights of one dtype, 8, 16, 32, 64 or 128 heads and x != y");
-    // Measured on B200 (bf16, mma.sync / tcgen05, us).  More than 16 heads: B1 H32 S4096 269 / 206, S256 11.7 / 7.8, S128 5.2 / 7.2.
-    // Up to 16 heads on the lower triangle only: B8 H16 S1024 68 / 53, B8 H8 S1024 38 / 28, B1 H16 S2048 forward 182 / 174; shorter
-    // rows keep the mma.sync kernel, whose blocks start faster (S512 5.6 / 7.7), and so do longer ones and whole planes, where
-    // HBM is the limit and it is the better streamer (B8 H16 S4096 forward 4640 / 4800, B4 H16 S2048 alone 158 / 173).  The choice
-    // depends on the heads, the row length and the output's form only, so that a row range or a part of the batch gets the same
-    // bits as the whole.
-    const bool tc05_better = C > 16 ? Q >= 256 : (causal && !write_upper && Q >= 1024 && Q < 4096);
+    // Measured on B200 (bf16, lower triangle, mma.sync / tcgen05, us).  More than 16 heads: B4 H32 S1024 91 / 56, S256 11.7 / 7.8,
+    // S128 5.2 / 7.2.  9 to 16 heads: B8 S1024 62 / 54, B2 S2048 58 / 52, B4 S3072 226 / 239, B8 S4096 785 / 849 (where HBM is the
+    // limit the mma.sync kernel streams better, and on whole planes too).  8 heads: B8 S4096 497 / 421, B8 S2048 134 / 108, B1 S1024
+    // 11 / 17.  Shorter rows keep the mma.sync kernel, whose blocks start faster.  The choice depends on the heads, the row length
+    // and the output's form only, so that a row range or a part of the batch gets the same bits as the whole.
+    const bool tc05_better = C > 16 ? Q >= 256 : (C > 8 ? causal && !write_upper && Q >= 1024 && Q <= 2048 : Q >= 1536);
     if (tc05_able && (want == 3 || (want == 0 && (!mma_able || tc05_better))))
         return head_linear_tc05_launch(x, xv, Wm, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, dtype, st, early);
     const bool use_mma = mma_able && want != 1;
