@@ -149,6 +149,22 @@ int mta_head_linear_bwd_weight_as(const void* x, const void* dy, void* dW, int d
 int mta_head_linear_bwd_input(const void* dy, const void* Wm, void* dx, int N, int C, int P, int Q, int causal, int dtype,
                               int w_dtype, void* stream);
 size_t mta_head_linear_bwd_weight_workspace_bytes(int C);
+/* mta_conv2d_fwd, mta_head_linear_fwd and the two input gradients with a workspace (NULL: none).  16-bit planes whose rows are not
+ * 16-byte aligned then run on the tensor cores, on copies with padded rows; mta_planes_workspace_bytes says how much the copies
+ * take (0: nothing to gain). */
+size_t mta_planes_workspace_bytes(int N, int C, int P, int Q, int dtype);
+int mta_conv2d_fwd_ws(const void* x, const void* w, void* y, void* workspace, size_t workspace_bytes, int N, int C, int H, int W, int R,
+                      int S, int causal, int x_dtype, int w_dtype, void* stream);
+int mta_head_linear_fwd_ws(const void* x, const void* Wm, void* y, void* workspace, size_t workspace_bytes, int N, int C, int P, int Q,
+                           int causal, float fill, int x_dtype, int w_dtype, void* stream);
+int mta_conv2d_bwd_input_ws(const void* dy, const void* w, void* dx, void* workspace, size_t workspace_bytes, int N, int C, int H, int W,
+                            int R, int S, int causal, int dtype, int w_dtype, void* stream);
+int mta_head_linear_bwd_input_ws(const void* dy, const void* Wm, void* dx, void* workspace, size_t workspace_bytes, int N, int C, int P,
+                                 int Q, int causal, int dtype, int w_dtype, void* stream);
+/* The sizes with which 16-bit planes whose rows are not 16-byte aligned run on the tensor cores too: room for copies of x and dy
+ * with padded rows behind the partial sums.  Never less than the *_bytes size, equal to it for other planes. */
+size_t mta_conv2d_bwd_weight_workspace_for(int N, int C, int H, int W, int R, int S, int dtype);
+size_t mta_head_linear_bwd_weight_workspace_for(int N, int C, int P, int Q, int dtype);
 int mta_head_linear_bwd_weight(const void* x, const void* dy, float* dW, void* workspace, size_t workspace_bytes, int N,
                                int C, int P, int Q, int causal, int dtype, void* stream);
 

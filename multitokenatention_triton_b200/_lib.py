@@ -30,6 +30,11 @@ SIGNATURES = {
     "mta_device_status": (_i, [_vp]),
     "mta_conv2d_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "mta_head_linear_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _vp]),
+    "mta_planes_workspace_bytes": (_sz, [_i] * 5),
+    "mta_conv2d_fwd_ws": (_i, [_vp] * 4 + [_sz] + [_i] * 9 + [_vp]),
+    "mta_head_linear_fwd_ws": (_i, [_vp] * 4 + [_sz] + [_i] * 5 + [_f, _i, _i, _vp]),
+    "mta_conv2d_bwd_input_ws": (_i, [_vp] * 4 + [_sz] + [_i] * 9 + [_vp]),
+    "mta_head_linear_bwd_input_ws": (_i, [_vp] * 4 + [_sz] + [_i] * 7 + [_vp]),
     "mta_softmax_fwd": (_i, [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp]),
     "mta_head_linear_softmax_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp]),
     "mta_conv2d_bwd_input": (_i, [_vp, _vp, _vp] + [_i] * 9 + [_vp]),
@@ -37,6 +42,8 @@ SIGNATURES = {
     "mta_conv2d_bwd_weight": (_i, [_vp, _vp, _vp, _vp, _sz] + [_i] * 8 + [_vp]),
     "mta_head_linear_bwd_input": (_i, [_vp, _vp, _vp] + [_i] * 7 + [_vp]),
     "mta_head_linear_bwd_weight_workspace_bytes": (_sz, [_i]),
+    "mta_head_linear_bwd_weight_workspace_for": (_sz, [_i] * 5),
+    "mta_conv2d_bwd_weight_workspace_for": (_sz, [_i] * 7),
     "mta_head_linear_bwd_weight": (_i, [_vp, _vp, _vp, _vp, _sz] + [_i] * 6 + [_vp]),
     "mta_qk_scores_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _f, _i, _i, _i, _vp]),
     "mta_pv_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp]),

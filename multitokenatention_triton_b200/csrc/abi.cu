@@ -69,6 +69,33 @@ int sm_count(int* out) {
 
 PlaneView full_view(int rows, int cols) { return PlaneView{(long)rows * cols, 0, cols}; }
 
+namespace {
+// `op(copy of x, copy of y)` on padded copies in the workspace; y's is copied back.
+template <typename OP>
+int on_padded(const void* x, void* y, PlaneView v, const PadPlan& p, void* workspace, long planes, int H, int W, int causal, float fill, int dtype,
+              cudaStream_t st, OP op) {
+    char* xp = static_cast<char*>(workspace);
+    char* yp = xp + p.bytes;
+    if (int rc = pad_planes(x, v, xp, p, planes, H, W, causal, dtype, st)) return rc;
+    if (int rc = op(xp, yp)) return rc;
+    return unpad_planes(yp, p, y, v, planes, H, W, causal, fill, dtype, st);
+}
+
+int head_mix_maybe_padded(const void* x, const void* Wm, int w_dtype, void* y, void* workspace, size_t workspace_bytes, int N, int C, int P, int Q,
+                          int causal, float fill, bool w_transposed, int dtype, cudaStream_t st) {
+    const PlaneView v = full_view(P, Q);
+    const PadPlan p = pad_plan((long)N * C, P, Q, dtype);
+    // B1 H12 S601 (4M scores) 21 us without copies, 26 with; B1 H16 S1022 48 / 42; B3 H12 S1739 251 / 189; 64 heads, B2 S1001: 914 / 226
+    const bool pays = C > 32 || (long)N * C * P * Q >= 8L << 20;
+    if (p.use && pays && workspace && workspace_bytes >= 2 * p.bytes && variant("head_linear") == 0 && aligned16(workspace) &&
+        (C <= 32 || head_linear_tc05_supported(workspace, p.view, static_cast<char*>(workspace) + p.bytes, p.view, C, Q, dtype, w_dtype)))
+        return on_padded(x, y, v, p, workspace, (long)N * C, P, Q, causal, fill, dtype, st, [&](const void* xp, void* yp) {
+            return head_linear_launch(xp, p.view, Wm, w_dtype, yp, p.view, N, C, P, Q, causal, fill, 0, P, false, dtype, st, w_transposed);
+        });
+    return head_linear_launch(x, v, Wm, w_dtype, y, v, N, C, P, Q, causal, fill, 0, P, true, dtype, st, w_transposed);
+}
+}  // namespace
+
 }  // namespace mta
 
 using namespace mta;
@@ -93,8 +120,19 @@ int mta_set_variant(const char* key, int value) {
     return MTA_OK;
 }
 
+size_t mta_planes_workspace_bytes(int N, int C, int P, int Q, int dtype) {
+    if (N <= 0 || C <= 0 || P <= 0 || Q <= 0 || !dtype_ok(dtype)) return 0;
+    const PadPlan p = pad_plan((long)N * C, P, Q, dtype);
+    return p.use ? 2 * p.bytes : 0;
+}
+
 int mta_conv2d_fwd(const void* x, const void* w, void* y, int N, int C, int H, int W, int R, int S, int causal,
                    int x_dtype, int w_dtype, void* stream) {
+    return mta_conv2d_fwd_ws(x, w, y, nullptr, 0, N, C, H, W, R, S, causal, x_dtype, w_dtype, stream);
+}
+
+int mta_conv2d_fwd_ws(const void* x, const void* w, void* y, void* workspace, size_t workspace_bytes, int N, int C, int H, int W, int R,
+                      int S, int causal, int x_dtype, int w_dtype, void* stream) {
     g_error[0] = 0;
     MTA_REQUIRE(dtype_ok(x_dtype) && dtype_ok(w_dtype), "conv2d: unknown dtype code (x %d, w %d)", x_dtype, w_dtype);
     MTA_REQUIRE(N >= 0 && C >= 1 && H >= 0 && W >= 0, "conv2d: bad shape N=%d C=%d H=%d W=%d", N, C, H, W);
@@ -104,12 +142,23 @@ int mta_conv2d_fwd(const void* x, const void* w, void* y, int N, int C, int H, i
     MTA_REQUIRE(x != y, "conv2d: in-place operation is not supported");
     if (int rc = check_device()) return rc;
     const PlaneView v = full_view(H, W);
-    return conv2d_launch(x, v, H, w, w_dtype, y, v, (long)N * C, C, H, W, R, S, causal ? 1 : 0, 0, H, true, x_dtype,
-                         static_cast<cudaStream_t>(stream));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const PadPlan p = pad_plan((long)N * C, H, W, x_dtype);
+    if (p.use && workspace && workspace_bytes >= 2 * p.bytes && variant("conv2d") == 0 &&
+        conv2d_tc05_supported(workspace, p.view, workspace, p.view, W, R, S, x_dtype, w_dtype))
+        return on_padded(x, y, v, p, workspace, (long)N * C, H, W, causal ? 1 : 0, 0.0f, x_dtype, st, [&](const void* xp, void* yp) {
+            return conv2d_launch(xp, p.view, H, w, w_dtype, yp, p.view, (long)N * C, C, H, W, R, S, causal ? 1 : 0, 0, H, false, x_dtype, st);
+        });
+    return conv2d_launch(x, v, H, w, w_dtype, y, v, (long)N * C, C, H, W, R, S, causal ? 1 : 0, 0, H, true, x_dtype, st);
 }
 
 int mta_head_linear_fwd(const void* x, const void* Wm, void* y, int N, int C, int P, int Q, int causal, float fill,
                         int x_dtype, int w_dtype, void* stream) {
+    return mta_head_linear_fwd_ws(x, Wm, y, nullptr, 0, N, C, P, Q, causal, fill, x_dtype, w_dtype, stream);
+}
+
+int mta_head_linear_fwd_ws(const void* x, const void* Wm, void* y, void* workspace, size_t workspace_bytes, int N, int C, int P, int Q,
+                           int causal, float fill, int x_dtype, int w_dtype, void* stream) {
     g_error[0] = 0;
     MTA_REQUIRE(dtype_ok(x_dtype) && dtype_ok(w_dtype), "head_linear: unknown dtype code (x %d, w %d)", x_dtype, w_dtype);
     MTA_REQUIRE(N >= 0 && C >= 1 && P >= 0 && Q >= 0, "head_linear: bad shape N=%d C=%d P=%d Q=%d", N, C, P, Q);
@@ -117,9 +166,8 @@ int mta_head_linear_fwd(const void* x, const void* Wm, void* y, int N, int C, in
     MTA_REQUIRE(x && Wm && y, "head_linear: null pointer");
     MTA_REQUIRE(x != y, "head_linear: in-place operation is not supported");
     if (int rc = check_device()) return rc;
-    const PlaneView v = full_view(P, Q);
-    return head_linear_launch(x, v, Wm, w_dtype, y, v, N, C, P, Q, causal ? 1 : 0, fill, 0, P, true, x_dtype,
-                              static_cast<cudaStream_t>(stream));
+    return head_mix_maybe_padded(x, Wm, w_dtype, y, workspace, workspace_bytes, N, C, P, Q, causal ? 1 : 0, fill, false, x_dtype,
+                                 static_cast<cudaStream_t>(stream));
 }
 
 int mta_softmax_fwd(const void* x, void* y, int N, int C, int P, int Q, int causal, int dtype, void* stream) {
@@ -154,6 +202,11 @@ int mta_head_linear_softmax_fwd(const void* x, const void* Wm, void* y, int N, i
 
 int mta_conv2d_bwd_input(const void* dy, const void* w, void* dx, int N, int C, int H, int W, int R, int S, int causal,
                          int dtype, int w_dtype, void* stream) {
+    return mta_conv2d_bwd_input_ws(dy, w, dx, nullptr, 0, N, C, H, W, R, S, causal, dtype, w_dtype, stream);
+}
+
+int mta_conv2d_bwd_input_ws(const void* dy, const void* w, void* dx, void* workspace, size_t workspace_bytes, int N, int C, int H, int W,
+                            int R, int S, int causal, int dtype, int w_dtype, void* stream) {
     g_error[0] = 0;
     MTA_REQUIRE(dtype_ok(dtype) && dtype_ok(w_dtype), "conv2d_bwd_input: unknown dtype code (dy %d, w %d)", dtype, w_dtype);
     MTA_REQUIRE(N >= 0 && C >= 1 && H >= 0 && W >= 0, "conv2d_bwd_input: bad shape N=%d C=%d H=%d W=%d", N, C, H, W);
@@ -162,13 +215,25 @@ int mta_conv2d_bwd_input(const void* dy, const void* w, void* dx, int N, int C, 
     MTA_REQUIRE(dy && w && dx, "conv2d_bwd_input: null pointer");
     MTA_REQUIRE(dy != dx, "conv2d_bwd_input: in-place operation is not supported");
     if (int rc = check_device()) return rc;
-    return conv2d_bwd_input_launch(dy, full_view(H, W), w, w_dtype, dx, full_view(H, W), (long)N * C, C, H, W, R, S, causal ? 1 : 0, true,
-                                   dtype, static_cast<cudaStream_t>(stream));
+    const PlaneView v = full_view(H, W);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const PadPlan p = pad_plan((long)N * C, H, W, dtype);
+    if (p.use && workspace && workspace_bytes >= 2 * p.bytes && variant("conv2d") == 0 && S % 2 == 1 &&
+        conv2d_tc05_supported(workspace, p.view, workspace, p.view, W, R, S, dtype, w_dtype))
+        return on_padded(dy, dx, v, p, workspace, (long)N * C, H, W, causal ? 1 : 0, 0.0f, dtype, st, [&](const void* xp, void* yp) {
+            return conv2d_bwd_input_launch(xp, p.view, w, w_dtype, yp, p.view, (long)N * C, C, H, W, R, S, causal ? 1 : 0, false, dtype, st);
+        });
+    return conv2d_bwd_input_launch(dy, v, w, w_dtype, dx, v, (long)N * C, C, H, W, R, S, causal ? 1 : 0, true, dtype, st);
 }
 
 size_t mta_conv2d_bwd_weight_workspace_bytes(int N, int C, int H, int W, int R, int S) {
     if (N <= 0 || C <= 0 || H <= 0 || W <= 0 || R < 1 || S < 1) return 0;
     return conv2d_bwd_weight_workspace(N, C, H, W, R, S);
+}
+
+size_t mta_conv2d_bwd_weight_workspace_for(int N, int C, int H, int W, int R, int S, int dtype) {
+    if (N <= 0 || C <= 0 || H <= 0 || W <= 0 || R < 1 || S < 1 || !dtype_ok(dtype)) return 0;
+    return conv2d_bwd_weight_padded_workspace(N, C, H, W, R, S, dtype);
 }
 
 int mta_conv2d_bwd_weight(const void* x, const void* dy, float* dw, void* workspace, size_t workspace_bytes, int N, int C,
@@ -193,11 +258,16 @@ int mta_conv2d_bwd_weight_as(const void* x, const void* dy, void* dw, int dw_dty
     const size_t need = conv2d_bwd_weight_workspace(N, C, H, W, R, S);
     MTA_REQUIRE(workspace && workspace_bytes >= need, "conv2d_bwd_weight: workspace of %zu bytes is smaller than the %zu needed",
                 workspace_bytes, need);
-    return conv2d_bwd_weight_launch(x, full_view(H, W), dy, full_view(H, W), dw, dw_dtype, workspace, N, C, H, W, R, S, causal ? 1 : 0, dtype, st);
+    return conv2d_bwd_weight_padded(x, full_view(H, W), dy, full_view(H, W), dw, dw_dtype, workspace, workspace_bytes, N, C, H, W, R, S, causal ? 1 : 0, dtype, st);
 }
 
 int mta_head_linear_bwd_input(const void* dy, const void* Wm, void* dx, int N, int C, int P, int Q, int causal, int dtype,
                               int w_dtype, void* stream) {
+    return mta_head_linear_bwd_input_ws(dy, Wm, dx, nullptr, 0, N, C, P, Q, causal, dtype, w_dtype, stream);
+}
+
+int mta_head_linear_bwd_input_ws(const void* dy, const void* Wm, void* dx, void* workspace, size_t workspace_bytes, int N, int C, int P,
+                                 int Q, int causal, int dtype, int w_dtype, void* stream) {
     g_error[0] = 0;
     MTA_REQUIRE(dtype_ok(dtype) && dtype_ok(w_dtype), "head_linear_bwd_input: unknown dtype code (dy %d, w %d)", dtype, w_dtype);
     MTA_REQUIRE(N >= 0 && C >= 1 && P >= 0 && Q >= 0, "head_linear_bwd_input: bad shape N=%d C=%d P=%d Q=%d", N, C, P, Q);
@@ -205,14 +275,18 @@ int mta_head_linear_bwd_input(const void* dy, const void* Wm, void* dx, int N, i
     MTA_REQUIRE(dy && Wm && dx, "head_linear_bwd_input: null pointer");
     MTA_REQUIRE(dy != dx, "head_linear_bwd_input: in-place operation is not supported");
     if (int rc = check_device()) return rc;
-    const PlaneView v = full_view(P, Q);
-    return head_linear_launch(dy, v, Wm, w_dtype, dx, v, N, C, P, Q, causal ? 1 : 0, 0.0f, 0, P, true, dtype,
-                              static_cast<cudaStream_t>(stream), true);
+    return head_mix_maybe_padded(dy, Wm, w_dtype, dx, workspace, workspace_bytes, N, C, P, Q, causal ? 1 : 0, 0.0f, true, dtype,
+                                 static_cast<cudaStream_t>(stream));
 }
 
 size_t mta_head_linear_bwd_weight_workspace_bytes(int C) {
     if (C < 1 || C > 128) return 0;
     return head_linear_bwd_weight_workspace(C);
+}
+
+size_t mta_head_linear_bwd_weight_workspace_for(int N, int C, int P, int Q, int dtype) {
+    if (C < 1 || C > 128 || N < 0 || P < 0 || Q < 0 || !dtype_ok(dtype)) return 0;
+    return head_linear_bwd_weight_padded_workspace(N, C, P, Q, dtype);
 }
 
 int mta_head_linear_bwd_weight(const void* x, const void* dy, float* dW, void* workspace, size_t workspace_bytes, int N,
@@ -236,7 +310,7 @@ int mta_head_linear_bwd_weight_as(const void* x, const void* dy, void* dW, int d
     const size_t need = head_linear_bwd_weight_workspace(C);
     MTA_REQUIRE(workspace && workspace_bytes >= need, "head_linear_bwd_weight: workspace of %zu bytes is smaller than the %zu needed",
                 workspace_bytes, need);
-    return head_linear_bwd_weight_launch(x, full_view(P, Q), dy, full_view(P, Q), dW, dw_dtype, workspace, N, C, P, Q, causal ? 1 : 0, dtype, st);
+    return head_linear_bwd_weight_padded(x, full_view(P, Q), dy, full_view(P, Q), dW, dw_dtype, workspace, workspace_bytes, N, C, P, Q, causal ? 1 : 0, dtype, st);
 }
 
 int mta_qk_scores_fwd(const void* q, const void* k, void* s, int B, int H, int S, int D, float scale, int round_scale,

@@ -272,6 +272,54 @@ int launch_hw(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float*
 
 }  // namespace
 
+// Weight gradients with a workspace that may hold padded copies of x and dy (pad.cu) behind the partial sums: 16-bit planes with unaligned
+// rows then run on the tensor cores.  The CUDA-core kernels read element by element; bf16, us without / with copies: 6 x 11 conv
+// N1 C8 S401 25 / 28, N1 C16 S515 40 / 32, N3 C12 S1739 435 / 192; head mix 42 / 32, 67 / 46, 650 / 204.
+namespace {
+// x and dy at `ws` in padded form; returns an MTA_* status.
+int pad_both(const void*& x, PlaneView& xv, const void*& dy, PlaneView& dyv, const PadPlan& p, char* ws, long planes, int H, int W, int causal,
+             int dtype, cudaStream_t st) {
+    int rc;
+    if ((rc = pad_planes(x, xv, ws, p, planes, H, W, causal, dtype, st))) return rc;
+    if ((rc = pad_planes(dy, dyv, ws + p.bytes, p, planes, H, W, causal, dtype, st))) return rc;
+    x = ws;
+    dy = ws + p.bytes;
+    xv = dyv = p.view;
+    return MTA_OK;
+}
+}  // namespace
+
+size_t conv2d_bwd_weight_padded_workspace(int N, int C, int H, int W, int R, int S, int dtype) {
+    const PadPlan p = pad_plan((long)N * C, H, W, dtype);
+    return ((conv2d_bwd_weight_workspace(N, C, H, W, R, S) + 255) & ~size_t(255)) + (p.use ? 2 * p.bytes : 0);
+}
+
+int conv2d_bwd_weight_padded(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dw, int dw_dtype, void* workspace,
+                             size_t workspace_bytes, int N, int C, int H, int W, int R, int S, int causal, int dtype, cudaStream_t st) {
+    const PadPlan p = pad_plan((long)N * C, H, W, dtype);
+    if (p.use && (long)N * C * H * W >= 2L << 20 && variant("conv2d") != 1 && workspace_bytes >= conv2d_bwd_weight_padded_workspace(N, C, H, W, R, S, dtype) &&
+        conv2d_dw_tc05_supported(workspace, p.view, workspace, p.view, R, S, dtype)) {
+        char* ws = static_cast<char*>(workspace) + ((conv2d_bwd_weight_workspace(N, C, H, W, R, S) + 255) & ~size_t(255));
+        if (int rc = pad_both(x, xv, dy, dyv, p, ws, (long)N * C, H, W, causal, dtype, st)) return rc;
+    }
+    return conv2d_bwd_weight_launch(x, xv, dy, dyv, dw, dw_dtype, workspace, N, C, H, W, R, S, causal, dtype, st);
+}
+
+size_t head_linear_bwd_weight_padded_workspace(int N, int C, int P, int Q, int dtype) {
+    const PadPlan p = pad_plan((long)N * C, P, Q, dtype);
+    return ((head_linear_bwd_weight_workspace(C) + 255) & ~size_t(255)) + (p.use ? 2 * p.bytes : 0);
+}
+
+int head_linear_bwd_weight_padded(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dW, int dw_dtype, void* workspace,
+                                  size_t workspace_bytes, int N, int C, int P, int Q, int causal, int dtype, cudaStream_t st) {
+    const PadPlan p = pad_plan((long)N * C, P, Q, dtype);
+    if (p.use && variant("head_linear") != 1 && workspace_bytes >= head_linear_bwd_weight_padded_workspace(N, C, P, Q, dtype)) {
+        char* ws = static_cast<char*>(workspace) + ((head_linear_bwd_weight_workspace(C) + 255) & ~size_t(255));
+        if (int rc = pad_both(x, xv, dy, dyv, p, ws, (long)N * C, P, Q, causal, dtype, st)) return rc;
+    }
+    return head_linear_bwd_weight_launch(x, xv, dy, dyv, dW, dw_dtype, workspace, N, C, P, Q, causal, dtype, st);
+}
+
 size_t conv2d_bwd_weight_workspace(int N, int C, int H, int W, int R, int S) {
     const long tiles = (long)((H + WT_M - 1) / WT_M) * ((W + WT_N - 1) / WT_N);
     return std::max((size_t)N * C * tiles * R * S * sizeof(float), conv2d_dw_tc05_workspace(N, C, H, W, R, S));

@@ -15,6 +15,17 @@ struct DeadKeys {
     // The bits of keys [key, key + 32) of batch element n, key a multiple of 32.
     __device__ uint32_t word(long n, int key) const { return bits ? __ldg(bits + n * words + (key >> 5)) : 0u; }
 };
+// Copies of unaligned 16-bit planes in padded rows (pad.cu): `use` says whether they pay, `bytes` is the size of one.
+struct PadPlan {
+    bool use;
+    PlaneView view;
+    size_t bytes;
+};
+PadPlan pad_plan(long planes, int H, int W, int dtype);
+// The lower triangle only when causal; unpad_planes writes the whole of `out`, `fill` above the diagonal.
+int pad_planes(const void* in, PlaneView iv, void* copy, const PadPlan& p, long planes, int H, int W, int causal, int dtype, cudaStream_t st);
+int unpad_planes(const void* copy, const PadPlan& p, void* out, PlaneView ov, long planes, int H, int W, int causal, float fill, int dtype,
+                 cudaStream_t st);
 // out (B,H,S,D) contiguous = in (B,S,H,D) contiguous (mask.cu).
 int swap_heads_launch(const void* in, void* out, int B, int H, int S, int D, int dtype, cudaStream_t st);
 // Prepares them from a (B,S) byte mask (0 = dead), together with copies of k and v (B,H,S,D) whose rows of dead keys are zero
@@ -56,6 +67,13 @@ int conv2d_bwd_input_launch(const void* dy, PlaneView dyv, const void* w, int w_
 size_t conv2d_bwd_weight_workspace(int N, int C, int H, int W, int R, int S);
 int conv2d_bwd_weight_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dw, int dw_dtype, void* workspace, int N, int C,
                              int H, int W, int R, int S, int causal, int dtype, cudaStream_t st);
+// The same with a workspace that may also hold padded copies of x and dy (the size is what makes them possible).
+size_t conv2d_bwd_weight_padded_workspace(int N, int C, int H, int W, int R, int S, int dtype);
+int conv2d_bwd_weight_padded(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dw, int dw_dtype, void* workspace,
+                             size_t workspace_bytes, int N, int C, int H, int W, int R, int S, int causal, int dtype, cudaStream_t st);
+size_t head_linear_bwd_weight_padded_workspace(int N, int C, int P, int Q, int dtype);
+int head_linear_bwd_weight_padded(const void* x, PlaneView xv, const void* dy, PlaneView dyv, void* dW, int dw_dtype, void* workspace,
+                                  size_t workspace_bytes, int N, int C, int P, int Q, int causal, int dtype, cudaStream_t st);
 // The conv's weight gradient on tcgen05 (conv2d_dw_tc05.cu).
 bool conv2d_dw_tc05_supported(const void* x, PlaneView xv, const void* dy, PlaneView dyv, int R, int S, int dtype);
 size_t conv2d_dw_tc05_workspace(int N, int C, int H, int W, int R, int S);

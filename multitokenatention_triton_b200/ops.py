@@ -33,6 +33,18 @@ def _size(name: str, *args: int) -> int:
     return getattr(lib(), name)(*args)
 
 
+def _row_copies(x: torch.Tensor) -> Optional[torch.Tensor]:
+    """Workspace for copies of 16-bit planes whose rows are not 16-byte aligned."""
+    if x.shape[3] % 8 == 0 or x.dtype == torch.float32:
+        return None
+    nbytes = _size("mta_planes_workspace_bytes", *x.shape, dtype_code(x))
+    return torch.empty(nbytes, dtype=torch.uint8, device=x.device) if nbytes else None
+
+
+def _buffer(ws: Optional[torch.Tensor]) -> Tuple[Optional[int], int]:
+    return (None, 0) if ws is None else (ws.data_ptr(), ws.numel())
+
+
 def conv2d_fwd(x: torch.Tensor, weight: torch.Tensor, causal: bool) -> torch.Tensor:
     """Depthwise causal conv: x (N,C,H,W), weight (C,R,S) -> (N,C,H,W)."""
     x = _cuda_contig(x, "input")
@@ -43,8 +55,9 @@ def conv2d_fwd(x: torch.Tensor, weight: torch.Tensor, causal: bool) -> torch.Ten
     assert C == Cw, "This implementation assumes depthwise convolution (C_in == C_out)"
     w = _weight(weight, x, "weight")
     y = torch.empty_like(x)
+    ws = _row_copies(x)
     with on_device(x.device):
-        check(lib().mta_conv2d_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, C, H, W, R, S, int(bool(causal)),
+        check(lib().mta_conv2d_fwd_ws(x.data_ptr(), w.data_ptr(), y.data_ptr(), *_buffer(ws), N, C, H, W, R, S, int(bool(causal)),
                                    dtype_code(x), dtype_code(w), stream_ptr(x.device)), "mta_conv2d_fwd")
     return y
 
@@ -60,8 +73,9 @@ def head_linear_fwd(x: torch.Tensor, weight: torch.Tensor, causal: bool = True, 
     assert C == L, f"Channel dimension {C} must match weight dimension {L}"
     w = _weight(weight, x, "weight")
     y = torch.empty_like(x)
+    ws = _row_copies(x)
     with on_device(x.device):
-        check(lib().mta_head_linear_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, C, P, Q, int(bool(causal)),
+        check(lib().mta_head_linear_fwd_ws(x.data_ptr(), w.data_ptr(), y.data_ptr(), *_buffer(ws), N, C, P, Q, int(bool(causal)),
                                         float(output_value), dtype_code(x), dtype_code(w), stream_ptr(x.device)),
               "mta_head_linear_fwd")
     return y
@@ -75,8 +89,9 @@ def conv2d_bwd_input(grad_output: torch.Tensor, weight: torch.Tensor, causal: bo
     assert C == Cw, "This implementation assumes depthwise convolution (C_in == C_out)"
     w = _weight(weight, g, "weight")
     dx = torch.empty_like(g)
+    ws = _row_copies(g)
     with on_device(g.device):
-        check(lib().mta_conv2d_bwd_input(g.data_ptr(), w.data_ptr(), dx.data_ptr(), N, C, H, W, R, S, int(bool(causal)),
+        check(lib().mta_conv2d_bwd_input_ws(g.data_ptr(), w.data_ptr(), dx.data_ptr(), *_buffer(ws), N, C, H, W, R, S, int(bool(causal)),
                                          dtype_code(g), dtype_code(w), stream_ptr(g.device)), "mta_conv2d_bwd_input")
     return dx
 
@@ -90,7 +105,7 @@ def conv2d_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, kernel_size: T
     R, S = kernel_size
     dw = torch.empty(C, R, S, device=x.device, dtype=dtype if dtype in _lib.DTYPE_CODE else torch.float32)
     L = lib()
-    nbytes = _size("mta_conv2d_bwd_weight_workspace_bytes", N, C, H, W, R, S)
+    nbytes = _size("mta_conv2d_bwd_weight_workspace_for", N, C, H, W, R, S, dtype_code(x))
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
     with on_device(x.device):
         check(L.mta_conv2d_bwd_weight_as(x.data_ptr(), g.data_ptr(), dw.data_ptr(), dtype_code(dw), ws.data_ptr(), ws.numel(), N, C, H, W,
@@ -105,8 +120,9 @@ def head_linear_bwd_input(grad_output: torch.Tensor, weight: torch.Tensor, causa
     assert weight.shape == (C, C), f"Weight must be a ({C},{C}) matrix, got {tuple(weight.shape)}"
     w = _weight(weight, g, "weight")
     dx = torch.empty_like(g)
+    ws = _row_copies(g)
     with on_device(g.device):
-        check(lib().mta_head_linear_bwd_input(g.data_ptr(), w.data_ptr(), dx.data_ptr(), N, C, P, Q, int(bool(causal)),
+        check(lib().mta_head_linear_bwd_input_ws(g.data_ptr(), w.data_ptr(), dx.data_ptr(), *_buffer(ws), N, C, P, Q, int(bool(causal)),
                                               dtype_code(g), dtype_code(w), stream_ptr(g.device)), "mta_head_linear_bwd_input")
     return dx
 
@@ -119,7 +135,7 @@ def head_linear_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, causal: b
     N, C, P, Q = x.shape
     dW = torch.empty(C, C, device=x.device, dtype=dtype if dtype in _lib.DTYPE_CODE else torch.float32)
     L = lib()
-    nbytes = _size("mta_head_linear_bwd_weight_workspace_bytes", C)
+    nbytes = _size("mta_head_linear_bwd_weight_workspace_for", N, C, P, Q, dtype_code(x))
     if nbytes == 0:
         raise MTALibraryError(f"head_linear_bwd_weight: C = {C} heads is outside the supported range 1..128")
     ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)

@@ -7,7 +7,7 @@ import torch
 from multitokenatention_triton_b200 import _lib, ops
 from multitokenatention_triton_b200.synthetic import MTAWorkload, make_mta_inputs
 from oracle import mta_oracle as orc
-from util import ROUND, assert_parity, npf
+from util import ROUND, assert_parity, npf, rel_fro
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -26,3 +26,38 @@ def test_forward_ragged(S, H, D, cq, ck, dtype):
     _lib.device_status()
     a = [npf(inp[k]) for k in ("q", "k", "v", "w1", "W1", "w2", "W2")]
     assert_parity(npf(out), orc.mta_fwd(*a, True, ROUND[dtype]), dtype, f"S{S} H{H} D{D} {cq}x{ck}")
+
+
+# The stand-alone ops on rows that are not 16-byte aligned, from the size on at which they work on copies with padded rows (1M to 8M scores),
+# against the CUDA-core kernels; the first and last elements of the tensors lie inside a 16-byte piece.
+@pytest.mark.parametrize("S,H,causal,dtype,offset", [
+    (1025, 4, True, torch.bfloat16, 0), (839, 6, False, torch.float16, 3), (1502, 2, True, torch.float16, 0), (1023, 16, True, torch.bfloat16, 1),
+    (515, 64, True, torch.bfloat16, 0), (390, 14, False, torch.bfloat16, 5)])
+def test_stand_alone_ops_on_unaligned_rows(S, H, causal, dtype, offset):
+    g = torch.Generator(device=DEV).manual_seed(S)
+    x, gr = (torch.randn(H * S * S + offset, device=DEV, generator=g).to(dtype)[offset:].view(1, H, S, S) for _ in range(2))
+    upper = torch.ones(S, S, dtype=torch.bool, device=DEV).triu(1)
+    if causal:
+        for t in (x, gr):
+            t.masked_fill_(upper, float("nan"))
+    w = (torch.randn(H, 6, 11, device=DEV, generator=g) / 8).to(dtype)
+    mix = torch.randn(H, H, device=DEV, generator=g).to(dtype)
+    got = {}
+    for variant in (0, 1):
+        _lib.set_variant("conv2d", variant)
+        _lib.set_variant("head_linear", variant)
+        try:
+            got[variant] = (ops.conv2d_fwd(x, w, causal), ops.conv2d_bwd_input(gr, w, causal), ops.head_linear_fwd(x, mix, causal, -3.3),
+                            ops.head_linear_bwd_input(gr, mix, causal), ops.conv2d_bwd_weight(x, gr, (6, 11), causal),
+                            ops.head_linear_bwd_weight(x, gr, causal))
+        finally:
+            _lib.set_variant("conv2d", 0)
+            _lib.set_variant("head_linear", 0)
+    _lib.device_status()
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, b in zip(got[0][:4], got[1][:4]):
+        assert float((a.float() - b.float()).abs().max()) <= 2 * ulp * float(b.float().abs().max())
+        if causal:
+            assert torch.equal(a.masked_select(upper), b.masked_select(upper))
+    for a, b in zip(got[0][4:], got[1][4:]):
+        assert rel_fro(npf(a), npf(b)) <= 1e-4
