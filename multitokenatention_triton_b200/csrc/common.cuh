@@ -77,7 +77,7 @@ template <auto KERNEL> int ensure_smem(size_t bytes) {
 // 65536 blocks: 0.15 ms of 0.77).
 constexpr unsigned PDL_MAX_BLOCKS = 4096;
 template <auto KERNEL, typename... Args>
-int launch_kernel(const char* name, dim3 grid, unsigned block, size_t smem, cudaStream_t st, Args... args) {
+int launch_kernel_early(bool early, const char* name, dim3 grid, unsigned block, size_t smem, cudaStream_t st, Args... args) {
     if (int rc = ensure_smem<KERNEL>(smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -88,7 +88,7 @@ int launch_kernel(const char* name, dim3 grid, unsigned block, size_t smem, cuda
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = (unsigned long long)grid.x * grid.y * grid.z <= PDL_MAX_BLOCKS ? 1 : 0;
+    cfg.numAttrs = early ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, KERNEL, args...);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -97,6 +97,10 @@ int launch_kernel(const char* name, dim3 grid, unsigned block, size_t smem, cuda
     }
     count_launch();
     return MTA_OK;
+}
+template <auto KERNEL, typename... Args>
+int launch_kernel(const char* name, dim3 grid, unsigned block, size_t smem, cudaStream_t st, Args... args) {
+    return launch_kernel_early<KERNEL>((unsigned long long)grid.x * grid.y * grid.z <= PDL_MAX_BLOCKS, name, grid, block, smem, st, args...);
 }
 
 inline size_t dtype_size(int dt) { return dt == MTA_F32 ? 4 : 2; }

@@ -70,7 +70,15 @@ struct QcIter {
 
 // NSTAGE: staged score tiles in flight.  Three where they fit into shared memory, else two (B8 H16 S4096 6x11: 1.28 against
 // 1.26 ms), which takes up to 16 row taps at D = 128.
-template <typename T, int D, int NSTAGE>
+//
+// PACED: the MMAs are issued from a branch that one lane enters, a third as fast as from warp-uniform code (mma_f16_ss).  Where a launch
+// is long enough for the chip to run at its power limit the faster issue gains nothing and costs energy: B8 H16 S4096 6x11, forwards
+// back to back, this kernel 1.57 ms with uniform issue, 1.54 paced.  Such a launch also does without the early start of launch_kernel:
+// its blocks then land on the SMs in order, and neighbours share K tiles in L2 (whole forward 4.67 ms with, 4.60 without; B8 S2048
+// 1.252 / 1.240 ms, B4 S1024, 18 tiles a block, 182 / 185 us).
+constexpr int QC_LONG = 64;                       // tiles per block from which on a launch counts as long
+
+template <typename T, int D, int NSTAGE, bool PACED>
 __global__ void __launch_bounds__(THREADS, 1)
 qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                     const __grid_constant__ CUtensorMap my, const void* __restrict__ w, int w_dtype, QcGeom g, int* err_flag) {
@@ -161,7 +169,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
     } else if (warp == 1) {
         // ---------------- score MMAs: S[128 x 144] = Q K^T into TMEM columns S_COL.. ----------------
         constexpr uint32_t idesc = instr_desc_f16(AbFmtQ<T>::value, 0, 0, TM, SN);
-        const uint32_t el = elect_one();
+        const uint32_t el = PACED ? 1u : elect_one();           // PACED: one lane enters the branch below
         QcIter it;
         it.init(g, t_begin);
         bool new_q = true;
@@ -176,22 +184,25 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
             __syncwarp();
             fence_after_sync();
             new_q = it.next(g);
-            const uint32_t qa = smem_u32(q_base), ka = smem_u32(k_base);
+            if (!PACED || lane == 0) {
+                const uint32_t qa = smem_u32(q_base), ka = smem_u32(k_base);
 #pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-                const uint32_t qoff = (kk / 4) * BOX_BYTES + (kk % 4) * 32, koff = (kk / 4) * KBOX_BYTES + (kk % 4) * 32;
-                mma_f16_ss(tmem + S_COL, smem_desc_sw128(qa + qoff, 16, 1024), smem_desc_sw128(ka + koff, 16, 1024), idesc,
-                           kk > 0 ? 1u : 0u, el);
+                for (int kk = 0; kk < D / 16; ++kk) {
+                    const uint32_t qoff = (kk / 4) * BOX_BYTES + (kk % 4) * 32, koff = (kk / 4) * KBOX_BYTES + (kk % 4) * 32;
+                    mma_f16_ss(tmem + S_COL, smem_desc_sw128(qa + qoff, 16, 1024), smem_desc_sw128(ka + koff, 16, 1024), idesc,
+                               kk > 0 ? 1u : 0u, el);
+                }
+                mma_commit(&k_free, el);
+                mma_commit(&s_full, el);
+                if (new_q || n == my_tiles - 1) mma_commit(&q_free, el);     // last tile of this row of tiles
             }
-            mma_commit(&k_free, el);
-            mma_commit(&s_full, el);
-            if (new_q || n == my_tiles - 1) mma_commit(&q_free, el);     // last tile of this row of tiles
+            if constexpr (PACED) __syncwarp();
         }
     } else if (warp == 2 || warp == 3) {
         // ---------------- conv MMAs ----------------
         QcIter it;
         it.init(g, t_begin);
-        const uint32_t el = elect_one();
+        const uint32_t el = PACED ? 1u : elect_one();           // PACED: one lane enters the branch below
         int cur_head = -1, hn = -1;                          // the running head and how many times it has changed
         for (int n = 0; n < my_tiles; ++n, it.next(g)) {
             const int st = n % NSTAGE, ab = n & 1;
@@ -201,13 +212,16 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
             mbar_wait(&acc_empty[ab], ((n >> 1) & 1) ^ 1, err_flag);
             __syncwarp();
             fence_after_sync();
-            const uint32_t xa_addr = smem_u32(stage_base + st * TB_OFF);
-            const uint32_t tb_addr = smem_u32(tb_base + (hn & 1) * tb_bytes);
-            const uint32_t d0 = tmem + (uint32_t)(ab * TN);
-            if (warp == 2) issue_conv<T, 0>(xa_addr, tb_addr, d0, R, g.split_w, el);
-            else issue_conv<T, 1>(xa_addr, tb_addr, d0, R, g.split_w, el);
-            mma_commit(&empty_bar[st], el);
-            mma_commit(&acc_full[ab], el);
+            if (!PACED || lane == 0) {
+                const uint32_t xa_addr = smem_u32(stage_base + st * TB_OFF);
+                const uint32_t tb_addr = smem_u32(tb_base + (hn & 1) * tb_bytes);
+                const uint32_t d0 = tmem + (uint32_t)(ab * TN);
+                if (warp == 2) issue_conv<T, 0>(xa_addr, tb_addr, d0, R, g.split_w, el);
+                else issue_conv<T, 1>(xa_addr, tb_addr, d0, R, g.split_w, el);
+                mma_commit(&empty_bar[st], el);
+                mma_commit(&acc_full[ab], el);
+            }
+            if constexpr (PACED) __syncwarp();
         }
     } else if (warp < 8) {
         // ---------------- drain: score tile TMEM -> rounded, scaled, masked -> staged tile; Toeplitz slices ----------------
@@ -347,9 +361,12 @@ int launch_qc(const void* q, const void* k, const void* w, int w_dtype, void* y,
     if (int bad = sm_count(&sms)) return bad;
     const unsigned grid = (unsigned)std::min<long>(g.total_tiles, sms);
     const size_t smem3 = qk_conv_smem_bytes(D, R, g.split_w != 0, 3), smem2 = qk_conv_smem_bytes(D, R, g.split_w != 0, 2);
-    if (smem3 <= QC_SMEM_LIMIT)
-        return launch_kernel<qk_conv_tc05_kernel<T, D, 3>>("qk_conv_tc05_kernel", grid, THREADS, smem3, st, mq, mk, my, w, w_dtype, g, flag);
-    return launch_kernel<qk_conv_tc05_kernel<T, D, 2>>("qk_conv_tc05_kernel", grid, THREADS, smem2, st, mq, mk, my, w, w_dtype, g, flag);
+    const bool three = smem3 <= QC_SMEM_LIMIT, is_long = g.total_tiles >= (long)QC_LONG * sms;
+#define MTA_QC_LAUNCH(NST, PACED) \
+    launch_kernel_early<qk_conv_tc05_kernel<T, D, NST, PACED>>(!PACED, "qk_conv_tc05_kernel", grid, THREADS, three ? smem3 : smem2, st, mq, mk, my, w, w_dtype, g, flag)
+    if (is_long) return three ? MTA_QC_LAUNCH(3, true) : MTA_QC_LAUNCH(2, true);
+    return three ? MTA_QC_LAUNCH(3, false) : MTA_QC_LAUNCH(2, false);
+#undef MTA_QC_LAUNCH
 }
 
 }  // namespace
