@@ -47,3 +47,16 @@ def test_conv_attention_and_scores_in_the_conv(S, D, R, Sk):
     _lib.device_status()
     for a, b in zip(one, ref):
         assert rel_fro(npf(a), npf(b)) <= 1e-2 and rel_max(npf(a), npf(b)) <= 3e-2
+
+
+# 64 score tiles per block and more take the long-launch form of the score + conv kernel: bit-identical to the short one.
+@pytest.mark.parametrize("R,Sk", [(6, 11), (11, 15)])
+def test_long_launches_equal_short_ones(R, Sk):
+    g = torch.Generator(device=DEV).manual_seed(R)
+    q, k, v = (torch.randn(16, 16, 1030, 128, device=DEV, generator=g).to(torch.bfloat16) for _ in range(3))
+    w = (torch.randn(16, R, Sk, device=DEV, generator=g) * (R * Sk) ** -0.5).to(torch.bfloat16)
+    mix = [(torch.eye(16, device=DEV) + 0.1 * torch.randn(16, 16, device=DEV, generator=g)).to(torch.bfloat16) for _ in range(2)]
+    whole = ops.mta_fused_fwd(q, k, v, w, mix[0], w, mix[1])
+    for b in (0, 7, 15):
+        assert torch.equal(whole[b:b + 1], ops.mta_fused_fwd(q[b:b + 1], k[b:b + 1], v[b:b + 1], w, mix[0], w, mix[1]))
+    _lib.device_status()
