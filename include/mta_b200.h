@@ -266,9 +266,12 @@ int mta_stage_times_ms(float* ms, const char** names, int capacity);
 int mta_device_status(void* stream);
 
 /* Fault injection on the host, for tests of the path above: marks the current device exactly as a kernel's timed-out
- * wait would (no kernel is made to wait).  Until mta_device_status() clears it, kernels of this library return without
- * computing and every compute entry point returns 4 (MTA_ERR_TIMEOUT) without launching. */
+ * wait would (no kernel is made to wait).  Until mta_device_status() clears it, kernels with bounded waits store nothing
+ * and every compute entry point returns 4 (MTA_ERR_TIMEOUT) without launching. */
 int mta_inject_wait_timeout(void* stream);
+/* The same from the device and later: enqueues a kernel whose bounded wait, with a limit of a few milliseconds, runs out.  Calls
+ * enqueued meanwhile are accepted, and their kernels with bounded waits store nothing. */
+int mta_inject_late_wait_timeout(void* stream);
 
 /* Number of kernel launches issued by this library on the calling thread since the last reset
  * (what a benchmark reports as its launch count). */

@@ -27,6 +27,7 @@ SIGNATURES = {
     "mta_reset_launch_count": (None, []),
     "mta_set_variant": (_i, [ctypes.c_char_p, _i]),
     "mta_inject_wait_timeout": (_i, [_vp]),
+    "mta_inject_late_wait_timeout": (_i, [_vp]),
     "mta_device_status": (_i, [_vp]),
     "mta_conv2d_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "mta_head_linear_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _vp]),

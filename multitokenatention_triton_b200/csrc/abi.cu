@@ -47,8 +47,8 @@ int check_device() {
         return MTA_ERR_ARCH;
     }
     if (wait_flag_raised()) {
-        set_error("a bounded wait of an earlier kernel on device %d gave up: every kernel since then has returned without "
-                  "computing; mta_device_status() reports and clears the condition", dev);
+        set_error("a bounded wait of an earlier kernel on device %d gave up: results since then are invalid; "
+                  "mta_device_status() reports and clears the condition", dev);
         return MTA_ERR_TIMEOUT;
     }
     return MTA_OK;
@@ -351,6 +351,12 @@ int mta_device_status(void* stream) {
 int mta_inject_wait_timeout(void* stream) {
     g_error[0] = 0;
     return wait_flag_inject(static_cast<cudaStream_t>(stream));
+}
+
+int mta_inject_late_wait_timeout(void* stream) {
+    g_error[0] = 0;
+    if (int rc = check_device()) return rc;
+    return wait_flag_inject_late(static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

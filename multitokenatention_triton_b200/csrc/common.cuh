@@ -71,7 +71,8 @@ template <auto KERNEL> int ensure_smem(size_t bytes) {
 
 // Launches KERNEL so that it may start before its predecessor in the stream has ended (programmatic dependent launch): what
 // it does before pdl_wait() - barriers, tensor memory, descriptors - then overlaps the predecessor's last blocks.  KERNEL must
-// call pdl_wait() before it reads or writes anything that another kernel may touch.
+// call pdl_wait() before it reads or writes anything that another kernel may touch; the one exception, the flag of a wait that gave up,
+// is read again after it (flag_down() in tc05.cuh).
 // Measured: B1 H16 S128 forward 51 -> 37 us, B1 H16 S2048 211 -> 188.  Only up to PDL_MAX_BLOCKS blocks: every block of such a
 // launch starts later, and over the fifty waves of a long grid that cost more than the overlap gave (head mix of B8 H16 S4096,
 // 65536 blocks: 0.15 ms of 0.77).

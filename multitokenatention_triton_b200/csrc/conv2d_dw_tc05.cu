@@ -125,9 +125,7 @@ conv2d_dw_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_const
     const int nacc = 2 * g.pairs * DW_KEYS <= 512 ? 2 : 1;    // sets of accumulators
     const uint32_t acc_cols = (uint32_t)(g.pairs * DW_KEYS);
 
-    if (tid == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
-    __syncthreads();
-    if (abort_flag != 0) return;
+    if (gave_up_before(err_flag, &abort_flag)) return;
     if (warp == 0) {
         if (lane == 0) {
             for (int i = 0; i < DW_MAX_STAGES; ++i) {
@@ -220,6 +218,7 @@ conv2d_dw_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_const
         // lane j of the warp collects key tap j, which column n holds in the warp's lane n + j + 8 - pad - 32 half ----
         const int quarter = warp & 3, half = quarter & 1;
         const int from = lane + 8 - (g.S - 1) / 2 - 32 * half;
+        const int n_out = flag_down(err_flag) ? g.R * g.S : 0;
         int f = 0;
         long done = 0;                                        // steps of this CTA before the segment
         const long all = it.left;
@@ -264,7 +263,7 @@ conv2d_dw_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_const
             named_barrier(1, 128);
             const int slot = (int)blockIdx.x - dw_owner(g.total, (long)plane * g.steps, gridDim.x);
             float* out = partial + ((long)plane * g.slots + slot) * g.R * g.S;
-            for (int i = tid - 256; i < g.R * g.S; i += 128) out[i] = (float)(red[0][i] + red[1][i]);
+            for (int i = tid - 256; i < n_out; i += 128) out[i] = (float)(red[0][i] + red[1][i]);
             named_barrier(1, 128);                            // nobody overwrites red while another thread still reads it
             done += seg;
             it.left -= seg;

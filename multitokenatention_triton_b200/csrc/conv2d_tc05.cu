@@ -193,9 +193,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
     const int my_tiles = t_end > t_begin ? (int)(t_end - t_begin) : 0;
 
     if (tid == 0) tiles_loaded = 0;
-    if (tid == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
-    __syncthreads();
-    if (abort_flag != 0 || my_tiles == 0) return;
+    if (gave_up_before(err_flag, &abort_flag) || my_tiles == 0) return;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -254,7 +252,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
             fence_proxy_async();
         }
         __syncwarp();
-        if (lane == 0 && my_zero > 0) {
+        if (lane == 0 && my_zero > 0 && flag_down(err_flag)) {
             // walker over (plane, row tile, column tile) with column tiles conv_key_tiles(tm) .. tiles_n - 1
             int zp = (int)(z_begin / g.zero_per_plane), ztm = 0;
             long r = z_begin - (long)zp * g.zero_per_plane;
@@ -379,7 +377,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
         // ---------------- epilogue: warps 4-7 drain columns 0..63, warps 10-13 columns 64..127 ----------------
         const int quarter = warp & 3;                        // the TMEM lanes a warp may read depend on its index mod 4
         const int half = warp >= 10 ? 1 : 0;
-        const bool issuer = (warp == 4 && lane == 0);
+        const bool issuer = warp == 4 && lane == 0 && flag_down(err_flag);
         const int row = quarter * 32 + lane;                 // row of the tile this thread owns
         TileIter it;
         it.init(g, t_begin);

@@ -87,9 +87,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     const int a_off = 8 - (KS - 1) / 2;
     const int lead = R - 1;
 
-    if (tid == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
-    __syncthreads();
-    if (abort_flag != 0) return;
+    if (gave_up_before(err_flag, &abort_flag)) return;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -245,6 +243,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
         const int half = warp >= 12 ? 1 : 0;
         const int row = quarter * 32 + lane;                 // row of the tile = TMEM lane of this thread
         const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16);
+        const int store_rows = flag_down(err_flag) ? g.tmo : 0;
         const float c2 = g.sm_scale * LOG2E;
         const bool neg = c2 < 0.0f;                          // a negative scale turns the row maximum into a minimum
         const float masked = neg ? INFINITY : -INFINITY;     // raw value whose logit is -inf
@@ -329,7 +328,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
             xch_sum[half][row] = l_part;
             named_barrier(1 + quarter, 64);
             const float inv = 1.0f / (l_part + xch_sum[half ^ 1][row]);
-            const bool store = row < g.tmo && q < g.row_end;
+            const bool store = row < store_rows && q < g.row_end;
             T* orow = o + ((long)plane * g.S + (store ? q : 0)) * D + half * OH;
 #pragma unroll 1
             for (int c = 0; c < OH / 32; ++c) {

@@ -92,6 +92,25 @@ int wait_flag_inject(cudaStream_t st) {
     return MTA_OK;
 }
 
+// A kernel whose bounded wait runs out, with a limit of a few milliseconds: nothing arrives on its barrier.  It lets its
+// successor start first, as every kernel does.
+__global__ void wait_runs_out_kernel(int* err_flag) {
+    __shared__ __align__(8) uint64_t bar;
+    if (threadIdx.x == 0) {
+        tc05::mbar_init(&bar, 1);
+        tc05::fence_mbar_init();
+    }
+    __syncwarp();
+    pdl_wait();
+    if (threadIdx.x == 0) tc05::mbar_wait(&bar, 0, err_flag, 2048);
+}
+
+int wait_flag_inject_late(cudaStream_t st) {
+    int* flag = nullptr;
+    if (int rc = wait_flag_ptr(&flag)) return rc;
+    return launch_kernel<wait_runs_out_kernel>("wait_runs_out_kernel", dim3(1), 32, 0, st, flag);
+}
+
 int make_tensor_map_3d(CUtensorMap* out, const void* base, uint64_t planes, uint64_t rows, uint64_t cols,
                        uint64_t row_pitch_elems, uint64_t plane_pitch_elems, uint32_t box_cols, uint32_t box_rows,
                        bool swizzle128) {
@@ -218,10 +237,8 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
         acc_bar;
     __shared__ uint32_t tmem_slot;
 
-    __shared__ int abort_flag;      // an earlier bounded wait on this device gave up: the whole CTA does nothing
-    if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
-    __syncthreads();
-    if (abort_flag != 0) return;
+    __shared__ int abort_flag;
+    if (gave_up_before(err_flag, &abort_flag)) return;
     // Heaviest tiles first (the last query tile has all keys, or the first key tile all queries), over groups of planes: plane by
     // plane, the last planes' heavy tiles start when little else is left (B1 H16 S2048: 30 us against 25); all planes at once,
     // the V tiles of 128 planes do not stay in L2 (B8 H16 S4096: 549 us against 441).
@@ -314,6 +331,7 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
         }
     } else {
         const int et = (int)threadIdx.x - 64;                // 0..127
+        const int store_end = flag_down(err_flag) ? q_end : 0;
         for (int it = DROP ? 0 : d0 - kt0; it < (DROP ? nk : d1 - kt0); ++it) {
             const int kt = kt0 + it, st = it % PV_STAGES, use = it / PV_STAGES;
             uint8_t* sp = smem + st * STAGE_BYTES;
@@ -367,7 +385,7 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
             uint32_t r[32];
             tmem_ld_32x32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c * 32), r);
             tmem_ld_wait();
-            if (q >= q_end) continue;
+            if (q >= store_end) continue;
 #pragma unroll
             for (int v8 = 0; v8 < 4; ++v8) {
                 float f[8];

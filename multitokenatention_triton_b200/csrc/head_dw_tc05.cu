@@ -73,7 +73,6 @@ head_dw_tc05_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_consta
     __shared__ HdIter first;
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int C = g.C, R = g.R;
-    if (tid == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
     if (tid == 32) {
         const long begin = blockIdx.x * g.total / gridDim.x;
         first.left = (blockIdx.x + 1) * g.total / gridDim.x - begin;
@@ -84,8 +83,7 @@ head_dw_tc05_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_consta
         first.step = r;
         first.count = cnt;
     }
-    __syncthreads();
-    if (abort_flag != 0) return;
+    if (gave_up_before(err_flag, &abort_flag)) return;
     if (warp == 0) {
         if (lane == 0) {
             for (int i = 0; i < HD_MAX_STAGES; ++i) {
@@ -180,11 +178,12 @@ head_dw_tc05_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_consta
     } else {
         const int quarter = warp & 3, et = tid - 192;     // TMEM lanes this warp may read; thread index 0..127
         const int l = quarter * 32 + lane, r = l & (R - 1);
+        const int n_out = flag_down(err_flag) ? C * C : 0;
         int filled = 0;
         for (int seg = 0; seg < HD_SEGMENTS; ++seg) {
             float* out = partial + ((long)blockIdx.x * HD_SEGMENTS + seg) * C * C;
             if (all * seg / HD_SEGMENTS == all * (seg + 1) / HD_SEGMENTS) {
-                for (int i = et; i < C * C; i += 128) out[i] = 0.0f;
+                for (int i = et; i < n_out; i += 128) out[i] = 0.0f;
                 continue;
             }
             const int ab = filled & 1;
@@ -207,7 +206,7 @@ head_dw_tc05_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_consta
             if (lane == 0) mbar_arrive(&acc_empty[ab]);
             ++filled;
             named_barrier(1, 128);
-            for (int i = et; i < C * C; i += 128) {
+            for (int i = et; i < n_out; i += 128) {
                 const int o = i / C, h = i - o * C;
                 float sum = 0.0f;
                 for (int rr = 0; rr < R; ++rr) sum += picked[(o * R + rr) * C + h];

@@ -230,9 +230,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int C = g.C, R = g.R;
 
-    if (tid == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
-    __syncthreads();
-    if (abort_flag != 0) return;
+    if (gave_up_before(err_flag, &abort_flag)) return;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -373,7 +371,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
         const int r = m % R;
         const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(grp * HM_KEYS);
         uint8_t* out_buf = out_base + grp * HM_OUT_BYTES;
-        const int gt = (sw & 3) * 32 + lane;                 // thread index within the group; thread 0 issues the group's stores
+        const bool issuer = (sw & 3) == 0 && lane == 0 && flag_down(err_flag);   // the thread that issues the group's stores
         int it = 0;
         int ub = 0;
         bool ok = true;
@@ -454,7 +452,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                     uint32_t pk[16];
                     if constexpr (SOFTMAX) hm_prob32<T>(cur, hm_first(n_keys - kb) & (MASKED ? ~g.dead.word(n, kb) : 0xffffffffu), shift, pk);
                     else hm_plain32<T>(cur, hm_first(n_keys - kb), g.fill, pk);
-                    if (gt == 0) bulk_wait_read();                   // the previous store of this buffer has read it
+                    if (issuer) bulk_wait_read();                   // the previous store of this buffer has read it
                     named_barrier(2 + grp, 128);
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4)
@@ -462,14 +460,14 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                             make_uint4(pk[4 * q4], pk[4 * q4 + 1], pk[4 * q4 + 2], pk[4 * q4 + 3]);
                     fence_proxy_async();
                     named_barrier(2 + grp, 128);
-                    if (gt == 0) {
+                    if (issuer) {
                         tma_store_3d(&my, out_buf, kb, p0 - y_row0, n * C);
                         bulk_commit();
                     }
                 }
             }
             it += nt;
-            if (g.write_upper && gt == 0) {
+            if (g.write_upper && issuer) {
                 // Everything past the unit's last tile is `fill` (0 for the softmax): boxes of the constant buffer, the
                 // groups taking turns.  Nobody waits for these stores before the kernel ends.
                 for (int kb = nt * HM_KEYS + grp * 32; kb < g.Q; kb += HM_NACC * 32) {

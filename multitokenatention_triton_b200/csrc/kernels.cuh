@@ -188,5 +188,7 @@ int device_wait_status(cudaStream_t st, int* timed_out);
 bool wait_flag_raised();
 // Raises the flag from the host as a timed-out wait would.
 int wait_flag_inject(cudaStream_t st);
+// Launches a kernel whose bounded wait gives up after a few milliseconds.
+int wait_flag_inject_late(cudaStream_t st);
 
 }  // namespace mta

@@ -109,9 +109,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
     const long t_end = min(t_begin + per, g.total_tiles);
     const int my_tiles = t_end > t_begin ? (int)(t_end - t_begin) : 0;
 
-    if (tid == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
-    __syncthreads();
-    if (abort_flag != 0 || my_tiles == 0) return;
+    if (gave_up_before(err_flag, &abort_flag) || my_tiles == 0) return;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -265,7 +263,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
         // ---------------- epilogue: warps 8-11 take columns 0..63, warps 12-15 columns 64..127 ----------------
         const int quarter = warp & 3;
         const int half = warp >= 12 ? 1 : 0;
-        const bool issuer = (warp == 8 && lane == 0);
+        const bool issuer = warp == 8 && lane == 0 && flag_down(err_flag);
         const int row = quarter * 32 + lane;
         QcIter it;
         it.init(g, t_begin);

@@ -110,9 +110,7 @@ qk_persistent_kernel(const __grid_constant__ CUtensorMap ma, const __grid_consta
     const long t_end = min(t_begin + per, g.total);
     const int my_tiles = t_end > t_begin ? (int)(t_end - t_begin) : 0;
 
-    if (tid == 0) abort_flag = *reinterpret_cast<volatile int*>(err_flag);
-    __syncthreads();
-    if (abort_flag != 0 || my_tiles == 0) return;
+    if (gave_up_before(err_flag, &abort_flag) || my_tiles == 0) return;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -189,7 +187,7 @@ qk_persistent_kernel(const __grid_constant__ CUtensorMap ma, const __grid_consta
         const int e = warp - 2;
         const int quarter = warp & 3;                        // the TMEM lanes a warp may read depend on its index mod 4
         const int half = e >> 2;
-        const bool issuer = (warp == 2 && lane == 0);
+        const bool issuer = warp == 2 && lane == 0 && flag_down(err_flag);
         const int row = quarter * 32 + lane;
         uint8_t* orow = out_base + half * BOX_BYTES + row * 128;
         const float sc = g.round_scale ? round_to<T>(g.scale) : g.scale;

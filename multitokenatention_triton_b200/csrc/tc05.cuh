@@ -53,7 +53,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// A wait gave up: raise the device flag (later kernels return at once) and its mirror in host memory, whose address sits
+// A wait gave up: raise the device flag (later kernels store nothing) and its mirror in host memory, whose address sits
 // two ints after the flag (the host then sees the timeout without synchronising).
 __device__ __forceinline__ void raise_wait_flag(int* err_flag) {
     if (atomicExch(err_flag, 1) == 0) {
@@ -65,8 +65,8 @@ __device__ __forceinline__ void raise_wait_flag(int* err_flag) {
     }
 }
 // Bounded wait for the phase with the given parity.  Returns false (and raises *err_flag) on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err_flag) {
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err_flag, uint32_t limit = WAIT_LIMIT) {
+    for (uint32_t i = 0; i < limit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         // Back off: hundreds of threads polling barriers in shared memory slow down the tensor core's operand reads.
         if (i >= 4) __nanosleep(i < 64 ? 64 : 256);
@@ -87,6 +87,20 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, i
     raise_wait_flag(err_flag);
     return false;
 }
+
+// The flag is looked at twice.  gave_up_before(): at a kernel's start, by the whole block; when it is up the block returns at once -
+// but not before its predecessors are complete, or its successors would overtake them.
+__device__ __forceinline__ bool gave_up_before(int* err_flag, int* slot) {
+    if (threadIdx.x == 0) *slot = *reinterpret_cast<volatile int*>(err_flag);
+    __syncthreads();
+    if (*slot == 0) return false;
+    pdl_wait();
+    return true;
+}
+// flag_down(): after pdl_wait(), by the threads that store results: a kernel that started early may have read the flag before its
+// predecessor raised it.  Such a kernel runs to its end without storing.  These threads wait for their first accumulator anyway; read
+// where the producer starts, the flag cost 0.6 us a kernel (B1 H16 S2048 7x7 forward 171.6 -> 175.6 us).
+__device__ __forceinline__ bool flag_down(const int* err_flag) { return *reinterpret_cast<const volatile int*>(err_flag) == 0; }
 
 // ---- TMA -----------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
