@@ -37,8 +37,18 @@ def _row_copies(x: torch.Tensor) -> Optional[torch.Tensor]:
     """Workspace for copies of 16-bit planes whose rows are not 16-byte aligned."""
     if x.shape[3] % 8 == 0 or x.dtype == torch.float32:
         return None
-    nbytes = _size("mta_planes_workspace_bytes", *x.shape, dtype_code(x))
-    return torch.empty(nbytes, dtype=torch.uint8, device=x.device) if nbytes else None
+    return _scratch(x.device, _size("mta_planes_workspace_bytes", *x.shape, dtype_code(x)), 0)
+
+
+def _scratch(device: torch.device, nbytes: int, least: int) -> Optional[torch.Tensor]:
+    """nbytes of workspace, or the least the call can do with where there is no room for more: without copies in padded rows the
+    kernels work, slower, on the planes as they are."""
+    if nbytes > least:
+        try:
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+        except torch.cuda.OutOfMemoryError:
+            pass
+    return torch.empty(least, dtype=torch.uint8, device=device) if least else None
 
 
 def _buffer(ws: Optional[torch.Tensor]) -> Tuple[Optional[int], int]:
@@ -106,7 +116,7 @@ def conv2d_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, kernel_size: T
     dw = torch.empty(C, R, S, device=x.device, dtype=dtype if dtype in _lib.DTYPE_CODE else torch.float32)
     L = lib()
     nbytes = _size("mta_conv2d_bwd_weight_workspace_for", N, C, H, W, R, S, dtype_code(x))
-    ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
+    ws = _scratch(x.device, nbytes, max(_size("mta_conv2d_bwd_weight_workspace_bytes", N, C, H, W, R, S), 16))
     with on_device(x.device):
         check(L.mta_conv2d_bwd_weight_as(x.data_ptr(), g.data_ptr(), dw.data_ptr(), dtype_code(dw), ws.data_ptr(), ws.numel(), N, C, H, W,
                                          R, S, int(bool(causal)), dtype_code(x), stream_ptr(x.device)), "mta_conv2d_bwd_weight")
@@ -138,7 +148,7 @@ def head_linear_bwd_weight(x: torch.Tensor, grad_output: torch.Tensor, causal: b
     nbytes = _size("mta_head_linear_bwd_weight_workspace_for", N, C, P, Q, dtype_code(x))
     if nbytes == 0:
         raise MTALibraryError(f"head_linear_bwd_weight: C = {C} heads is outside the supported range 1..128")
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    ws = _scratch(x.device, nbytes, _size("mta_head_linear_bwd_weight_workspace_bytes", C))
     with on_device(x.device):
         check(L.mta_head_linear_bwd_weight_as(x.data_ptr(), g.data_ptr(), dW.data_ptr(), dtype_code(dW), ws.data_ptr(), ws.numel(), N, C,
                                               P, Q, int(bool(causal)), dtype_code(x), stream_ptr(x.device)), "mta_head_linear_bwd_weight")

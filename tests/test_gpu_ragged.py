@@ -61,3 +61,36 @@ def test_stand_alone_ops_on_unaligned_rows(S, H, causal, dtype, offset):
             assert torch.equal(a.masked_select(upper), b.masked_select(upper))
     for a, b in zip(got[0][4:], got[1][4:]):
         assert rel_fro(npf(a), npf(b)) <= 1e-4
+
+
+def test_stand_alone_ops_without_room_for_copies(monkeypatch):
+    """Two more planes than the result needs are not to be had: the ops run as they do without copies."""
+    S, H = 1025, 16
+    x, g = (torch.randn(1, H, S, S, device=DEV).to(torch.bfloat16) for _ in range(2))
+    w, mix = torch.randn(H, 6, 11, device=DEV).to(torch.bfloat16), torch.randn(H, H, device=DEV).to(torch.bfloat16)
+    L, st, shape, bf16 = _lib.lib(), torch.cuda.current_stream().cuda_stream, (1, H, S, S), _lib.MTA_BF16
+    want = [torch.empty_like(x) for _ in range(4)] + [torch.empty(H, 6, 11, device=DEV), torch.empty(H, H, device=DEV)]
+    conv_ws, mix_ws = L.mta_conv2d_bwd_weight_workspace_bytes(*shape, 6, 11), L.mta_head_linear_bwd_weight_workspace_bytes(H)
+    ws = torch.empty(max(conv_ws, mix_ws), dtype=torch.uint8, device=DEV)
+    y = [t.data_ptr() for t in want]
+    for rc in (L.mta_conv2d_fwd(x.data_ptr(), w.data_ptr(), y[0], *shape, 6, 11, 1, bf16, bf16, st),
+               L.mta_conv2d_bwd_input(x.data_ptr(), w.data_ptr(), y[1], *shape, 6, 11, 1, bf16, bf16, st),
+               L.mta_head_linear_fwd(x.data_ptr(), mix.data_ptr(), y[2], *shape, 1, -3.5, bf16, bf16, st),
+               L.mta_head_linear_bwd_input(x.data_ptr(), mix.data_ptr(), y[3], *shape, 1, bf16, bf16, st),
+               L.mta_conv2d_bwd_weight(x.data_ptr(), g.data_ptr(), y[4], ws.data_ptr(), conv_ws, *shape, 6, 11, 1, bf16, st),
+               L.mta_head_linear_bwd_weight(x.data_ptr(), g.data_ptr(), y[5], ws.data_ptr(), mix_ws, *shape, 1, bf16, st)):
+        _lib.check(rc, "without a workspace")
+    real = torch.empty
+
+    def empty(*a, **k):
+        if k.get("dtype") == torch.uint8 and a[0] >= 2 * x.numel() * 2:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return real(*a, **k)
+
+    monkeypatch.setattr(torch, "empty", empty)
+    got = [ops.conv2d_fwd(x, w, True), ops.conv2d_bwd_input(x, w, True), ops.head_linear_fwd(x, mix, True, -3.5),
+           ops.head_linear_bwd_input(x, mix, True), ops.conv2d_bwd_weight(x, g, (6, 11), True), ops.head_linear_bwd_weight(x, g, True)]
+    monkeypatch.undo()
+    _lib.device_status()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
