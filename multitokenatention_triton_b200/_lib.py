@@ -106,10 +106,14 @@ def dtype_code(t: torch.Tensor) -> int:
         raise MTALibraryError(f"unsupported dtype {t.dtype}: expected float32, bfloat16 or float16") from None
 
 
+# What torch.cuda.current_stream() wraps in an object, where this version of torch has it.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr(device: torch.device) -> int:
-    if device.index is None:
+    if device.index is None or _raw_stream is None:
         return torch.cuda.current_stream(device).cuda_stream
-    return torch._C._cuda_getCurrentRawStream(device.index)      # what current_stream() wraps in an object
+    return _raw_stream(device.index)
 
 
 class _Here:
