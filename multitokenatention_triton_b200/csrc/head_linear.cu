@@ -896,11 +896,22 @@ int head_linear_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype,
     MTA_REQUIRE(want != 3 || tc05_able,
                 "head_linear: the tcgen05 variant needs 16-bit activations and weights of one dtype, 8, 16, 32, 64 or 128 heads and x != y");
     // Measured on B200 (bf16, lower triangle, mma.sync / tcgen05, us).  More than 16 heads: B4 H32 S1024 91 / 56, S256 11.7 / 7.8,
-    // S128 5.2 / 7.2.  9 to 16 heads: B8 S1024 62 / 54, B2 S2048 58 / 52, B4 S3072 226 / 239, B8 S4096 785 / 849 (where HBM is the
-    // limit the mma.sync kernel streams better, and on whole planes too).  8 heads: B8 S4096 497 / 421, B8 S2048 134 / 108, B1 S1024
-    // 11 / 17.  Shorter rows keep the mma.sync kernel, whose blocks start faster.  The choice depends on the heads, the row length
-    // and the output's form only, so that a row range or a part of the batch gets the same bits as the whole.
-    const bool tc05_better = C > 16 ? Q >= 256 : (C > 8 ? causal && !write_upper && Q >= 1024 && Q <= 2048 : Q >= 1536);
+    // S128 5.2 / 7.2.  8 heads: B8 S4096 497 / 421, B8 S2048 134 / 108, B1 S1024 11 / 17.  Shorter rows keep the mma.sync kernel,
+    // whose blocks start faster.  The choice depends on the heads, the row length and the output's form only, so that a row range
+    // or a part of the batch gets the same bits as the whole.
+    // 16 heads, the stage inside the forward:
+    //         S512       S768       S896       S1021      S1536     S2048      S2304      S2688      S3072      S4096
+    //   B1    10 / 14    12 / 14    13 / 16    14 / 16    19 / 19   31 / 27    37 / 31    51 / 44    63 / 57    101 / 101
+    //   B2    12 / 14    14 / 14    16 / 16    18 / 17    34 / 30   56 / 51    68 / 66    92 / 91    115 / 118  196 / 204
+    //   B4    14 / 14    21 / 20    25 / 23    31 / 27    65 / 59   107 / 105  131 / 135  176 / 186  227 / 241  390 / 425
+    //   B8    21 / 19    37 / 31    48 / 41    59 / 53    124 / 121 205 / 213  258 / 275  353 / 380  457 / 492  785 / 855
+    // So the times cross where a launch has about 2M scores a head (below, blocks that start faster count) and again at 16M to 30M
+    // (beyond, HBM is the limit and the mma.sync kernel streams better; on whole planes too), and a line by length alone is a
+    // compromise over the batch: the ratios' mean over B1 to B8 is 0.95 at 1021 and at 2048 keys, within 2 % of 1 from 700 to 900 and
+    // from 2560 to 3072, where moving the line would slow one batch as much as it gains on another.  By the length of the padded
+    // rows, which is what the kernels walk: 1021 keys cost what 1024 do.
+    const int row = (Q + 63) / 64 * 64;
+    const bool tc05_better = C > 16 ? Q >= 256 : (C > 8 ? causal && !write_upper && row >= 1024 && row <= 2048 : Q >= 1536);
     if (tc05_able && (want == 3 || (want == 0 && (!mma_able || tc05_better))))
         return head_linear_tc05_launch(x, xv, Wm, y, yv, N, C, Q, causal, fill, row_begin, row_end, write_upper, wt, dtype, st, early);
     const bool use_mma = mma_able && want != 1;

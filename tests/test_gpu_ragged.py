@@ -94,3 +94,21 @@ def test_stand_alone_ops_without_room_for_copies(monkeypatch):
     _lib.device_status()
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("S,variant", [(960, 2), (961, 3), (1021, 3), (1024, 3), (2048, 3), (2049, 2)])
+def test_lengths_of_one_padded_row_take_one_head_mix(S, variant):
+    """The second head mix of 16 heads is chosen by the padded row: bit for bit what the kernel of that row gives, not the other's."""
+    g = torch.Generator(device=DEV).manual_seed(S)
+    q, k, v = (torch.randn(1, 16, S, 64, device=DEV, generator=g).to(torch.bfloat16) for _ in range(3))
+    w = torch.randn(16, 3, 3, device=DEV, generator=g).to(torch.bfloat16)
+    mix = torch.randn(16, 16, device=DEV, generator=g).to(torch.bfloat16)
+    out = {}
+    for n in (0, 2, 3):
+        _lib.set_variant("head_linear", n)
+        try:
+            out[n] = ops.mta_fused_fwd(q, k, v, w, mix, w, mix)
+        finally:
+            _lib.set_variant("head_linear", 0)
+    _lib.device_status()
+    assert torch.equal(out[0], out[variant]) and not torch.equal(out[2], out[3])
