@@ -7,7 +7,7 @@ import torch
 from multitokenatention_triton_b200 import _lib, ops
 from multitokenatention_triton_b200.synthetic import MTAWorkload, make_mta_inputs
 from oracle import mta_oracle as orc
-from util import ROUND, assert_parity, npf, rel_fro
+from util import ROUND, assert_parity, conv64, conv64_bwd_input, npf, rel_fro
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -61,6 +61,38 @@ def test_stand_alone_ops_on_unaligned_rows(S, H, causal, dtype, offset):
             assert torch.equal(a.masked_select(upper), b.masked_select(upper))
     for a, b in zip(got[0][4:], got[1][4:]):
         assert rel_fro(npf(a), npf(b)) <= 1e-4
+
+
+@pytest.mark.parametrize("S,H,causal,dtype,offset", [
+    (1025, 4, True, torch.bfloat16, 0), (839, 6, False, torch.float16, 3), (1502, 2, True, torch.float16, 0), (1023, 16, True, torch.bfloat16, 1),
+    (515, 64, True, torch.bfloat16, 0), (390, 14, False, torch.bfloat16, 5)])
+def test_stand_alone_ops_on_unaligned_rows_against_float64(S, H, causal, dtype, offset):
+    """A result plane may be off by its own rounding (half a unit in the last of 8 or 11 significant bits, so 2^-8 or 2^-11 of it)
+    and by a float32 sum of up to 66 products; a weight gradient by float32 sums of a block, whose errors do not add up over the
+    blocks."""
+    g = torch.Generator(device=DEV).manual_seed(S)
+    x, gr = (torch.randn(H * S * S + offset, device=DEV, generator=g).to(dtype)[offset:].view(1, H, S, S) for _ in range(2))
+    w = (torch.randn(H, 6, 11, device=DEV, generator=g) / 8).to(dtype)
+    mix = (torch.randn(H, H, device=DEV, generator=g) * H ** -0.5).to(dtype)
+    got = (ops.conv2d_fwd(x, w, causal), ops.conv2d_bwd_input(gr, w, causal), ops.head_linear_fwd(x, mix, causal, -3.5),
+           ops.head_linear_bwd_input(gr, mix, causal))
+    dw, dmix = ops.conv2d_bwd_weight(x, gr, (6, 11), causal), ops.head_linear_bwd_weight(x, gr, causal)
+    _lib.device_status()
+    dead = torch.ones(S, S, dtype=torch.bool, device=DEV).triu(1)
+    xd, gd = x.double(), gr.double()
+    if causal:
+        xd, gd = xd.masked_fill(dead, 0.0), gd.masked_fill(dead, 0.0)
+    mixed = torch.einsum("oh,bhpq->bopq", mix.double(), xd), torch.einsum("oh,bopq->bhpq", mix.double(), gd)
+    if causal:
+        mixed[0].masked_fill_(dead, -3.5)
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, b in zip(got, (conv64(xd, w, causal), conv64_bwd_input(gd, w, causal), *mixed)):
+        assert bool(((a.double() - b).abs() <= u * b.abs() + 1e-4).all())
+    xp = torch.nn.functional.pad(xd, (5, 5, 5, 0))
+    want = torch.stack([torch.stack([(xp[:, :, i:i + S, j:j + S] * gd).sum((0, 2, 3)) for j in range(11)], -1) for i in range(6)], -2)
+    assert float((dw.double() - want).norm() / want.norm()) <= 1e-5
+    want = torch.einsum("bopq,bhpq->oh", gd, xd)
+    assert float((dmix.double() - want).norm() / want.norm()) <= 1e-5
 
 
 def test_stand_alone_ops_without_room_for_copies(monkeypatch):

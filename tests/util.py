@@ -46,3 +46,29 @@ def assert_parity(a: np.ndarray, ref: np.ndarray, dtype: torch.dtype, what: str 
     else:
         f, m = rel_fro(a, ref), rel_max(a, ref)
         assert f <= BF16_REL and m <= BF16_REL, f"{what}: rel fro {f:.3e}, rel max {m:.3e} > {BF16_REL}"
+
+
+def conv64(x: torch.Tensor, w: torch.Tensor, causal: bool) -> torch.Tensor:
+    """The depthwise conv in float64, tap by tap: rows look back, keys are centred; zeros above the diagonal when causal."""
+    x, w = x.double(), w.double()
+    H, W, (C, R, S) = x.shape[2], x.shape[3], w.shape
+    dead = torch.arange(W, device=x.device)[None, :] > torch.arange(H, device=x.device)[:, None]
+    if causal:
+        x = x.masked_fill(dead, 0.0)
+    pad = (S - 1) // 2
+    xp = torch.nn.functional.pad(x, (pad, S - 1 - pad, R - 1, 0))
+    y = torch.zeros_like(x)
+    for i in range(R):
+        for j in range(S):
+            y += w[None, :, i, j, None, None] * xp[:, :, i:i + H, j:j + W]
+    return y.masked_fill(dead, 0.0) if causal else y
+
+
+def conv64_bwd_input(dy: torch.Tensor, w: torch.Tensor, causal: bool) -> torch.Tensor:
+    """Its gradient with respect to x (odd key extents): the key taps reversed, rows looking forward."""
+    H, W = dy.shape[2:]
+    if causal:
+        dead = torch.arange(W, device=dy.device)[None, :] > torch.arange(H, device=dy.device)[:, None]
+        dy = dy.masked_fill(dead, 0.0)
+    dx = conv64(dy.flip(2), w.flip(2), False).flip(2)
+    return dx.masked_fill(dead, 0.0) if causal else dx
