@@ -144,8 +144,8 @@ int qk_f32_launch(const void* q, const void* k, void* s, PlaneView sv, int B, in
 int pv_f32_launch(const void* p, PlaneView pview, const void* v, void* o, int B, int H, int S, int D, int causal, int row_begin, int row_end,
                   bool trans, float scale, cudaStream_t st);
 
-// tcgen05 version of the conv (conv2d_tc05.cu): 16-bit dtypes, S <= 17, W a multiple of 8, R small enough for its
-// shared-memory rings (R <= 13 with 16-bit weights).
+// tcgen05 version of the conv (conv2d_tc05.cu): 16-bit dtypes, S <= 17, any W on rows whose pitch is a multiple of 8 elements, R <= 16
+// and small enough for its shared-memory rings (float32 weights take two sets of slices: R <= 9).
 bool conv2d_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int W, int R, int S, int dtype,
                            int w_dtype);
 // `grad_input` (odd S): the same kernel evaluates the gradient with respect to the conv's input - taps reversed, rows
@@ -154,7 +154,7 @@ int conv2d_tc05_launch(const void* x, PlaneView xv, long x_rows_stored, const vo
                        long planes, int C, int H, int W, int R, int S, int causal, int row_begin, int row_end,
                        bool write_upper, int dtype, cudaStream_t st, bool grad_input = false, bool early_weights = false);
 
-// tcgen05 tensor-core versions (gemm_tc05.cu): 16-bit dtypes, D in {64,128}, S a multiple of 8.
+// tcgen05 tensor-core versions (gemm_tc05.cu): 16-bit dtypes, D in {64,128}, any S on planes whose row pitch is a multiple of 8 elements.
 bool tc05_contractions_supported(int S, int D, int dtype, const void* a, const void* b, const void* c, PlaneView view);
 int pv_tc05_launch(const void* p, PlaneView pview, long p_rows_stored, const void* v, void* o, int B, int H, int S, int D,
                    int causal, int row_begin, int row_end, int dtype, cudaStream_t st, DropoutSpec drop = DropoutSpec(),

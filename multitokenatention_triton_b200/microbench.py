@@ -1,12 +1,14 @@
 """Micro-benchmarks of the stand-alone kernels on the configurations their roofline targets are quoted on.
 
-    python -m multitokenatention_triton_b200.microbench [conv2d|head_linear|softmax|mix_softmax|qk|pv|backward|conv_attn|graph|all] [--variant V]
-                                                        [--batch N] [--seq S] [--iters K]
+    python -m multitokenatention_triton_b200.microbench [conv2d|head_linear|softmax|mix_softmax|qk|pv|backward|conv_attn|graph|train|write|all]
+                                                        [--variant V] [--batch N] [--seq S] [--taps R S] [--iters K]
 
   conv2d       causal depthwise conv 6x11 on a (B=4, H=16, S=2048, S) bf16 score plane
   head_linear  16x16 head mix on post-softmax probabilities of the same shape
   graph        the whole forward (five launches) at --batch/--heads/--seq/--dim, launched call by call and replayed
                from a CUDA graph: what stream capture saves where the forward is launch-bound (not part of "all")
+  train        the module's forward and backward, both convs with --taps (not part of "all")
+  write        what memory takes when it is only written: torch's fill of a plane of the shape (not part of "all")
 
 Each kernel is timed alone with CUDA events on the launching stream (3 warm-up launches, then K timed ones;
 input + output of one launch exceed the 126 MB L2).  One JSON line per kernel:
@@ -65,12 +67,13 @@ def _line(name, ms, nbytes=None, flops=None, **extra):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("which", nargs="?", default="all", choices=["conv2d", "head_linear", "softmax", "mix_softmax", "qk", "pv", "backward", "conv_attn", "graph", "all"])
+    ap.add_argument("which", nargs="?", default="all", choices=["conv2d", "head_linear", "softmax", "mix_softmax", "qk", "pv", "backward", "conv_attn", "graph", "train", "write", "all"])
     ap.add_argument("--variant", type=int, default=0)
     ap.add_argument("--batch", type=int, default=4)
     ap.add_argument("--heads", type=int, default=16)
     ap.add_argument("--seq", type=int, default=2048)
     ap.add_argument("--dim", type=int, default=128)
+    ap.add_argument("--taps", type=int, nargs=2, default=(6, 11))
     ap.add_argument("--iters", type=int, default=20)
     ap.add_argument("--dtype", default="bfloat16", choices=["bfloat16", "float16", "float32"])
     a = ap.parse_args()
@@ -79,20 +82,21 @@ def main():
     es = torch.empty(0, dtype=dtype).element_size()
     N, C, S, D = a.batch, a.heads, a.seq, a.dim
     tri = S * (S + 1) // 2
+    cq, ck = a.taps
     shape = f"B{N} H{C} S{S} {a.dtype}"
     for key in ("conv2d", "head_linear", "gemm"):
         _lib.set_variant(key, a.variant)
 
     if a.which in ("conv2d", "all"):
-        inp = make_conv_inputs(N, C, S, D, 6, 11, dtype, seed=1)
+        inp = make_conv_inputs(N, C, S, D, cq, ck, dtype, seed=1)
         x, w = inp["x"].to(dev), inp["w"].to(dev)
         y = torch.empty_like(x)
 
         def run():
-            _lib.check(_lib.lib().mta_conv2d_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, C, S, S, 6, 11, 1,
+            _lib.check(_lib.lib().mta_conv2d_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, C, S, S, cq, ck, 1,
                                                  _lib.dtype_code(x), _lib.dtype_code(w), _lib.stream_ptr(dev)), "conv2d")
         ms = _time(run, a.iters)
-        _line("conv2d 6x11 causal", ms, nbytes=es * N * C * (tri + S * S), shape=shape, variant=a.variant,
+        _line(f"conv2d {cq}x{ck} causal", ms, nbytes=es * N * C * (tri + S * S), shape=shape, variant=a.variant,
               lower_only_bytes=2 * es * N * C * tri)
         del x, y
     if a.which in ("head_linear", "softmax", "mix_softmax", "all"):
@@ -123,13 +127,13 @@ def main():
         # gradients of the two stand-alone ops: dx moves read-lower + write-full like the forward; a weight gradient
         # reads the lower triangle of x and of dy
         from .synthetic import make_upstream_grad
-        inp = make_conv_inputs(N, C, S, D, 6, 11, dtype, seed=1)
+        inp = make_conv_inputs(N, C, S, D, cq, ck, dtype, seed=1)
         x, w = inp["x"].to(dev), inp["w"].to(dev)
         g = make_upstream_grad((N, C, S, S), dtype, 1001).to(dev)
         ms = _time(lambda: ops.conv2d_bwd_input(g, w, True), a.iters)
-        _line("conv2d 6x11 causal, input gradient", ms, nbytes=es * N * C * (tri + S * S), shape=shape, variant=a.variant)
-        ms = _time(lambda: ops.conv2d_bwd_weight(x, g, (6, 11), True), a.iters)
-        _line("conv2d 6x11 causal, weight gradient", ms, nbytes=2 * es * N * C * tri, shape=shape)
+        _line(f"conv2d {cq}x{ck} causal, input gradient", ms, nbytes=es * N * C * (tri + S * S), shape=shape, variant=a.variant)
+        ms = _time(lambda: ops.conv2d_bwd_weight(x, g, (cq, ck), True), a.iters)
+        _line(f"conv2d {cq}x{ck} causal, weight gradient", ms, nbytes=2 * es * N * C * tri, shape=shape)
         hl = make_head_linear_inputs(N, C, S, dtype, seed=2)
         W = hl["W"].to(dev)
         x = hl["x"].to(dev)
@@ -185,6 +189,28 @@ def main():
         print(json.dumps({"kernel": "full forward, call by call against CUDA-graph replay", "shape": shape + f" D{D}",
                           "ms_eager": eager, "ms_graph": replay, "bit_identical": bool(torch.equal(out, ref)),
                           "tokens_per_s_graph": N * S / (replay * 1e-3)}), flush=True)
+    if a.which == "write":
+        y = torch.empty(N, C, S, S, dtype=dtype, device=dev)
+        ms = _time(lambda: y.fill_(1.0), a.iters)
+        _line("fill", ms, nbytes=es * N * C * S * S, shape=shape)
+    if a.which == "train":
+        import types
+        from . import MTAAttentionTriton
+        cfg = types.SimpleNamespace(use_mta=True, query_kernel_size=cq, key_kernel_size=ck, after_sm_query_kernel_size=cq, after_sm_key_kernel_size=ck,
+                                    pre_sm_linear_head=True, post_sm_linear_head=True, pad_key="both", init_method="identity", dim=C * D)
+        m = MTAAttentionTriton(C, cfg, dropout=0.0, causal=True).to(dev, dtype)
+        m.reset_mta_parameters()
+        q, k, v = (torch.randn(N, C, S, D, device=dev).to(dtype).requires_grad_() for _ in range(3))
+        up = torch.randn(N, S, C, D, device=dev).to(dtype)
+        leaves = [q, k, v, *m.parameters()]
+
+        def run():
+            for t in leaves:
+                t.grad = None
+            m(q, k, v).backward(up)
+        ms = _time(run, a.iters)
+        # every product and its two gradients, per lower-triangle score: Q K^T and P V, two convs, two head mixes
+        _line(f"training step {cq}x{ck}", ms, flops=3 * (4.0 * D + 4 * cq * ck + 4 * C) * N * C * tri, shape=shape + f" D{D}")
     _lib.device_status()
 
 

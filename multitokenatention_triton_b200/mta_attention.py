@@ -8,8 +8,9 @@ chunk_start_ids) returning the (B,S,H,D) transpose view of a (B,H,S,D) tensor.
 `fused=True` (default) runs the whole forward through mta_fused_fwd, or through mta_train_fwd / mta_train_bwd when a
 gradient is needed (without dropout).  `fused=False` runs the reference's
 seven steps one by one through the stand-alone entry points, which keeps every 16-bit rounding point of
-the reference.  `use_mask=True` runs the reference's explicit-mask path (None, boolean, additive, padding or
-(1,1,S,S) masks) stage by stage over full score planes.
+the reference.  `use_mask=True` takes the reference's explicit masks (None, boolean, additive, padding or (1,1,S,S)): None
+and a boolean (batch, keys) mask without a gradient or dropout run as the fused causal forward, the second through
+mta_masked_fwd; the others run stage by stage over full score planes.
 """
 import torch
 import torch.nn as nn
@@ -73,8 +74,8 @@ class MTAAttentionTriton(nn.Module):
         w1, w2 = self.mta_conv_triton.effective_weight(), self.mta_conv_after_sm_triton.effective_weight()
         if self.fused and not dropping and xk.shape == xq.shape and xv.shape == xq.shape and w1.size(-1) % 2 and w2.size(-1) % 2:
             return MTAFunction.apply(xq, xk, xv, w1, self.wpsm_triton.weight, w2, self.wposm_triton.weight).transpose(1, 2)
-        # stage by stage; every stage is differentiable (the conv and the head mix through their backward kernels, the
-        # scores, the softmax and the product with V through autograd_ops), so this is the path a training step uses
+        # Stage by stage: `fused=False`, a gradient with dropout, cross attention, even key extents.  Every stage is differentiable,
+        # the conv and the head mix through their backward kernels, the scores, the softmax and the product with V through autograd_ops.
         head_dim = xq.size(-1)
         scores = QKScoresFunction.apply(xq, xk, head_dim ** -0.5, True)
         scores = self.mta_conv_triton(scores)
