@@ -74,6 +74,9 @@ conv2d_mma_kernel(const __grid_constant__ CUtensorMap mx, const void* __restrict
     const int a_off = pad8 - pad_w;            // staged column of tap j for output column x: x + a_off + j
     T* yp = y + plane * yv.plane_stride;
 
+    __shared__ int abort_flag;
+    if (gave_up_before(err_flag, &abort_flag)) return;
+
     if (causal && n0 > m_end - 1) {            // tile entirely above the diagonal
         if (write_upper) {
             const uint4 z = make_uint4(0u, 0u, 0u, 0u);

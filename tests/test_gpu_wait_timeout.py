@@ -29,6 +29,7 @@ def _calls():
     fused_ws = L.mta_workspace_bytes(N, H, S, D, R, K, R, K, 0, S, BF16)
     calls = {
         "conv2d": (lambda y, st: L.mta_conv2d_fwd(a["x"], a["w"], y, N, H, S, S, R, K, 1, BF16, BF16, st), plane),
+        "conv2d_mma": (lambda y, st: L.mta_conv2d_fwd(a["x"], a["w"], y, N, H, S, S, R, K, 1, BF16, BF16, st), plane),
         "conv2d_bwd_input": (lambda y, st: L.mta_conv2d_bwd_input(a["x"], a["w"], y, N, H, S, S, R, K, 1, BF16, BF16, st), plane),
         "head_linear": (lambda y, st: L.mta_head_linear_fwd(a["x"], a["W"], y, N, H, S, S, 1, 0.0, BF16, BF16, st), plane),
         "head_linear_softmax": (lambda y, st: L.mta_head_linear_softmax_fwd(a["x"], a["W"], y, N, H, S, S, BF16, BF16, st), plane),
@@ -47,7 +48,7 @@ def _calls():
     return p, calls
 
 
-@pytest.mark.parametrize("name", ["conv2d", "conv2d_bwd_input", "head_linear", "head_linear_softmax", "qk_scores", "pv", "conv_attn",
+@pytest.mark.parametrize("name", ["conv2d", "conv2d_mma", "conv2d_bwd_input", "head_linear", "head_linear_softmax", "qk_scores", "pv", "conv_attn",
                                   "conv2d_bwd_weight", "head_linear_bwd_weight", "fused"])
 def test_the_successor_of_a_kernel_that_gave_up_writes_nothing(name):
     keep, calls = _calls()
@@ -58,6 +59,7 @@ def test_the_successor_of_a_kernel_that_gave_up_writes_nothing(name):
     buf = torch.full((room,), 0x5A, dtype=torch.uint8, device=DEV)
     # the kernels without bounded waits, such as the mma.sync head mix, carry on
     _lib.set_variant("head_linear", 3 if name in ("head_linear", "fused") else 0)
+    _lib.set_variant("conv2d", 2 if name == "conv2d_mma" else 0)
     try:
         _lib.check(call(good.data_ptr(), st), name)          # a first call also does what only a first call does
         _lib.device_status()
@@ -66,6 +68,7 @@ def test_the_successor_of_a_kernel_that_gave_up_writes_nothing(name):
         assert L.mta_device_status(st) == 4
     finally:
         _lib.set_variant("head_linear", 0)
+        _lib.set_variant("conv2d", 0)
         L.mta_device_status(st)
     assert bool((buf[:nbytes] == 0x5A).all()), "written after the predecessor gave up"
     _lib.check(call(buf.data_ptr(), st), name)               # and afterwards the call works again
