@@ -331,7 +331,7 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
         }
     } else {
         const int et = (int)threadIdx.x - 64;                // 0..127
-        const int store_end = flag_down(err_flag) ? q_end : 0;
+        const int flag = read_flag(err_flag);                // looked at after the loop: these warps clear the diagonal tiles first
         for (int it = DROP ? 0 : d0 - kt0; it < (DROP ? nk : d1 - kt0); ++it) {
             const int kt = kt0 + it, st = it % PV_STAGES, use = it / PV_STAGES;
             uint8_t* sp = smem + st * STAGE_BYTES;
@@ -385,7 +385,7 @@ pv_tc05_kernel(const __grid_constant__ CUtensorMap mp, const __grid_constant__ C
             uint32_t r[32];
             tmem_ld_32x32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c * 32), r);
             tmem_ld_wait();
-            if (q >= store_end) continue;
+            if (q >= q_end || flag != 0) continue;
 #pragma unroll
             for (int v8 = 0; v8 < 4; ++v8) {
                 float f[8];

@@ -99,8 +99,9 @@ __device__ __forceinline__ bool gave_up_before(int* err_flag, int* slot) {
 }
 // flag_down(): after pdl_wait(), by the threads that store results: a kernel that started early may have read the flag before its
 // predecessor raised it.  Such a kernel runs to its end without storing.  These threads wait for their first accumulator anyway; read
-// where the producer starts, the flag cost 0.6 us a kernel (B1 H16 S2048 7x7 forward 171.6 -> 175.6 us).
-__device__ __forceinline__ bool flag_down(const int* err_flag) { return *reinterpret_cast<const volatile int*>(err_flag) == 0; }
+// where the producer starts, the flag cost 0.8 us a kernel (B1 H16 S2048 7x7 forward 171.6 -> 175.6 us; like this 170.7).
+__device__ __forceinline__ int read_flag(const int* err_flag) { return *reinterpret_cast<const volatile int*>(err_flag); }
+__device__ __forceinline__ bool flag_down(const int* err_flag) { return read_flag(err_flag) == 0; }
 
 // ---- TMA -----------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
