@@ -63,9 +63,13 @@ def test_the_successor_of_a_kernel_that_gave_up_writes_nothing(name):
     try:
         _lib.check(call(good.data_ptr(), st), name)          # a first call also does what only a first call does
         _lib.device_status()
-        _lib.check(L.mta_inject_late_wait_timeout(st), "inject")
-        _lib.check(call(buf.data_ptr(), st), name)
-        assert L.mta_device_status(st) == 4
+        for _ in range(5):                                   # a host that pauses longer than the wait has its call refused
+            _lib.check(L.mta_inject_late_wait_timeout(st), "inject")
+            rc = call(buf.data_ptr(), st)
+            assert L.mta_device_status(st) == 4
+            if rc != 4:
+                break
+        _lib.check(rc, name)
     finally:
         _lib.set_variant("head_linear", 0)
         _lib.set_variant("conv2d", 0)
