@@ -90,32 +90,6 @@ __device__ __forceinline__ float hm_ex2(float x) {
     return y;
 }
 
-// 32 fp32 columns of this thread's TMEM lane, rounded to T and packed two per word (word i = columns 2i, 2i+1), as ONE
-// asm statement: the 32 loaded values never become C++ variables, only the 16 packed words do.
-template <typename T> __device__ __forceinline__ void hm_ld_round32(uint32_t taddr, uint32_t (&pk)[16]);
-#define HM_LD_ROUND32(CVT)                                                                                              \
-    asm volatile(                                                                                                       \
-        "{\n\t.reg .b32 t<32>;\n\t"                                                                                    \
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "                                                                       \
-        "{t0, t1, t2, t3, t4, t5, t6, t7, t8, t9, t10, t11, t12, t13, t14, t15, "                                       \
-        "t16, t17, t18, t19, t20, t21, t22, t23, t24, t25, t26, t27, t28, t29, t30, t31}, [%16];\n\t"                   \
-        "tcgen05.wait::ld.sync.aligned;\n\t"                                                                            \
-        CVT " %0, t1, t0;\n\t" CVT " %1, t3, t2;\n\t" CVT " %2, t5, t4;\n\t" CVT " %3, t7, t6;\n\t"                      \
-        CVT " %4, t9, t8;\n\t" CVT " %5, t11, t10;\n\t" CVT " %6, t13, t12;\n\t" CVT " %7, t15, t14;\n\t"                \
-        CVT " %8, t17, t16;\n\t" CVT " %9, t19, t18;\n\t" CVT " %10, t21, t20;\n\t" CVT " %11, t23, t22;\n\t"            \
-        CVT " %12, t25, t24;\n\t" CVT " %13, t27, t26;\n\t" CVT " %14, t29, t28;\n\t" CVT " %15, t31, t30;\n\t}\n"       \
-        : "=r"(pk[0]), "=r"(pk[1]), "=r"(pk[2]), "=r"(pk[3]), "=r"(pk[4]), "=r"(pk[5]), "=r"(pk[6]), "=r"(pk[7]), "=r"(pk[8]), \
-          "=r"(pk[9]), "=r"(pk[10]), "=r"(pk[11]), "=r"(pk[12]), "=r"(pk[13]), "=r"(pk[14]), "=r"(pk[15])                 \
-        : "r"(taddr)                                                                                                    \
-        : "memory")
-template <> __device__ __forceinline__ void hm_ld_round32<__nv_bfloat16>(uint32_t taddr, uint32_t (&pk)[16]) {
-    HM_LD_ROUND32("cvt.rn.bf16x2.f32");
-}
-template <> __device__ __forceinline__ void hm_ld_round32<__half>(uint32_t taddr, uint32_t (&pk)[16]) {
-    HM_LD_ROUND32("cvt.rn.f16x2.f32");
-}
-#undef HM_LD_ROUND32
-
 // The first n of 32 keys, as bits.
 __device__ __forceinline__ uint32_t hm_first(int n) { return n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u); }
 
@@ -392,7 +366,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                 uint32_t cur[16];
 #pragma unroll 1
                 for (int c = 0; c < 4; ++c) {
-                    hm_ld_round32<T>(t_base + (uint32_t)(c * 32), cur);
+                    tmem_ld_round32<T>(t_base + (uint32_t)(c * 32), cur);
                     if (c == 3) {
                         fence_before_sync();
                         __syncwarp();
@@ -436,7 +410,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                 uint32_t cur[16];
 #pragma unroll 1
                 for (int c = 0; c < 4; ++c) {
-                    hm_ld_round32<T>(t_base + (uint32_t)(c * 32), cur);
+                    tmem_ld_round32<T>(t_base + (uint32_t)(c * 32), cur);
                     if (c == 3) {
                         fence_before_sync();
                         __syncwarp();

@@ -55,7 +55,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 // A wait gave up: raise the device flag (later kernels store nothing) and its mirror in host memory, whose address sits
 // two ints after the flag (the host then sees the timeout without synchronising).
-__device__ __forceinline__ void raise_wait_flag(int* err_flag) {
+// Not inlined: a kernel has a dozen waits, and the instructions of the roles that share a scheduler compete for its instruction cache.
+inline __device__ __noinline__ void raise_wait_flag(int* err_flag) {
     if (atomicExch(err_flag, 1) == 0) {
         int* mirror = *reinterpret_cast<int* volatile*>(err_flag + 2);
         if (mirror) {
@@ -85,6 +86,19 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, i
         if ((i & 8191u) == 8191u && *reinterpret_cast<volatile int*>(err_flag) != 0) return false;
     }
     raise_wait_flag(err_flag);
+    return false;
+}
+
+// Whole-warp wait for several barriers at once: every lane with `active` polls its own barrier, the warp goes on when all are through.
+// One after the other the waits of an MMA-issuing warp cost some 50 cycles each, with nothing left to wait for.
+__device__ __forceinline__ bool mbar_wait_lanes(uint64_t* bar, uint32_t parity, bool active, int* err_flag) {
+    bool ok = !active;
+    for (uint32_t i = 0; i < WAIT_LIMIT * 8u; ++i) {
+        if (!ok) ok = mbar_try_wait(bar, parity);
+        if (__all_sync(0xffffffffu, ok)) return true;
+        if ((i & 8191u) == 8191u && __any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(err_flag) != 0)) return false;
+    }
+    if (!ok) raise_wait_flag(err_flag);
     return false;
 }
 
@@ -204,8 +218,12 @@ __host__ __device__ constexpr uint32_t instr_desc_f16(int ab_format, int a_mn_ma
            ((uint32_t)b_mn_major << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// Index of the calling warp in its CTA, in a form the compiler knows to be the same for the whole warp.
-__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// A value that is the same in the whole warp, in a form the compiler knows to be.  What decides whether and how MMAs are issued has to
+// pass through here unless it comes from kernel arguments and constants alone: behind a branch that could diverge the operands of
+// every MMA are moved from vector to uniform registers one by one.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+// Index of the calling warp in its CTA.
+__device__ __forceinline__ int warp_index() { return uniform((int)(threadIdx.x >> 5)); }
 
 // D[tmem] (+)= A[smem] * B[smem].  Called by a whole warp, executed by the thread whose `el` is 1 (from elect_one(), the same
 // thread for everything that one commit covers).  The instruction takes its descriptors from uniform registers: when it sits
@@ -230,6 +248,18 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uin
         "setp.ne.b32 p, %4, 0;\n\t"
         "setp.ne.b32 q, %5, 0;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(el));
+}
+// The same, after which the MMA leaves A one row up: lane r of the 8 columns holds what lane r + 1 held, within each group of 32
+// lanes (lane 31 of a group keeps its value).  The next MMA from the same A then sees its rows shifted by one, which is what the
+// row taps of a conv need.  Measured: the shift is free from N = 32 on (16 cycles per MMA of M 128, N 32, K 16; 40 with A in shared
+// memory, whose 4 KB have to be fetched for every tap).
+__device__ __forceinline__ void mma_f16_ts_shift(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t el) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16.ashift [%0], [%1], %2, %3, p;\n\t}\n"
         ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(el));
 }
 // Arrive on `bar` once every MMA issued so far by the elected thread has completed.
@@ -272,6 +302,31 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
         : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+// 32 fp32 columns of this thread's TMEM lane, rounded to T and packed two per word (word i = columns 2i, 2i+1), as ONE
+// asm statement: the 32 loaded values never become C++ variables, only the 16 packed words do.
+template <typename T> __device__ __forceinline__ void tmem_ld_round32(uint32_t taddr, uint32_t (&pk)[16]);
+#define MTA_LD_ROUND32(CVT)                                                                                              \
+    asm volatile(                                                                                                       \
+        "{\n\t.reg .b32 t<32>;\n\t"                                                                                    \
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "                                                                       \
+        "{t0, t1, t2, t3, t4, t5, t6, t7, t8, t9, t10, t11, t12, t13, t14, t15, "                                       \
+        "t16, t17, t18, t19, t20, t21, t22, t23, t24, t25, t26, t27, t28, t29, t30, t31}, [%16];\n\t"                   \
+        "tcgen05.wait::ld.sync.aligned;\n\t"                                                                            \
+        CVT " %0, t1, t0;\n\t" CVT " %1, t3, t2;\n\t" CVT " %2, t5, t4;\n\t" CVT " %3, t7, t6;\n\t"                      \
+        CVT " %4, t9, t8;\n\t" CVT " %5, t11, t10;\n\t" CVT " %6, t13, t12;\n\t" CVT " %7, t15, t14;\n\t"                \
+        CVT " %8, t17, t16;\n\t" CVT " %9, t19, t18;\n\t" CVT " %10, t21, t20;\n\t" CVT " %11, t23, t22;\n\t"            \
+        CVT " %12, t25, t24;\n\t" CVT " %13, t27, t26;\n\t" CVT " %14, t29, t28;\n\t" CVT " %15, t31, t30;\n\t}\n"       \
+        : "=r"(pk[0]), "=r"(pk[1]), "=r"(pk[2]), "=r"(pk[3]), "=r"(pk[4]), "=r"(pk[5]), "=r"(pk[6]), "=r"(pk[7]), "=r"(pk[8]), \
+          "=r"(pk[9]), "=r"(pk[10]), "=r"(pk[11]), "=r"(pk[12]), "=r"(pk[13]), "=r"(pk[14]), "=r"(pk[15])                 \
+        : "r"(taddr)                                                                                                    \
+        : "memory")
+template <> __device__ __forceinline__ void tmem_ld_round32<__nv_bfloat16>(uint32_t taddr, uint32_t (&pk)[16]) {
+    MTA_LD_ROUND32("cvt.rn.bf16x2.f32");
+}
+template <> __device__ __forceinline__ void tmem_ld_round32<__half>(uint32_t taddr, uint32_t (&pk)[16]) {
+    MTA_LD_ROUND32("cvt.rn.f16x2.f32");
+}
+#undef MTA_LD_ROUND32
 // Store of 32 lanes x 32 consecutive fp32 columns: lane i of the warp writes row (lane base + i).
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
@@ -282,6 +337,14 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
           "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
           "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
           "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+// The same for 16 consecutive columns.
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }

@@ -50,7 +50,7 @@ def test_conv_attention_and_scores_in_the_conv(S, D, R, Sk):
         assert rel_fro(npf(a), npf(b)) <= 1e-2 and rel_max(npf(a), npf(b)) <= 3e-2
 
 
-# 64 score tiles per block and more take the long-launch form of the score + conv kernel: bit-identical to the short one.
+# A long launch of the score + conv kernel works through its planes in groups: bit-identical to launches of one group.
 @pytest.mark.parametrize("R,Sk", [(6, 11), (11, 15)])
 def test_long_launches_equal_short_ones(R, Sk):
     g = torch.Generator(device=DEV).manual_seed(R)
