@@ -108,12 +108,27 @@ int run_forward(const void* q, const void* k, const void* v, const void* w1, con
         if ((rc = trace_mark("softmax", st))) return rc;
         if ((rc = softmax_launch(bufA, pv, bufA, pv, planes, S, S, causal, pl.rb, pl.r1, false, 1.0f, dtype, st, dead, H))) return rc;
     }
-    if ((rc = trace_mark("conv2", st))) return rc;
-    if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w2, w_dtype, bufB, pv, planes, H, S, S, cq2, ck2, causal, pl.r0, pl.r1, !causal, dtype, st, true))) return rc;
-    if ((rc = trace_mark("head_mix2", st))) return rc;
-    if ((rc = head_linear_launch(bufB, pv, W2, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.r0, pl.r1, false, dtype, st, false, true))) return rc;
+    // The second conv and the second head mix: one kernel where the conv is small.  one / two kernels, us, 3 x 3: H16 B1 S64 14 / 20,
+    // B1 S512 18 / 25, B4 S1024 49 / 66, B1 S4096 139 / 215; H8 B1 S1024 18 / 26; H32 B1 S512 27 / 37, B1 S2048 100 / 113; H64 B1 S256
+    // 26 / 35, B1 S1024 83 / 82, B4 S1024 249 / 240, B1 S4096 800 / 903 (two heads' rows of a group are two thirds of what it reads).
+    // 2 x 3 gains more everywhere.  3 x 5 was level with two kernels (B4 H16 S2048 212 / 215) and 3 x 7 and more cost FMAs in proportion.
+    // Two forms keep the two kernels because of what is promised for them, not for speed: 8 heads up to 128 keys (the number of launches)
+    // and 16 heads of 64 (bit for bit the head mix kernel that head_linear_launch picks by the row).
+    const void* weights = bufA;
+    const bool one = variant("fused") != 1 && variant("conv2d") == 0 && variant("head_linear") == 0 && (H > 8 || S > 128) && (H != 16 || D != 64) &&
+                     conv_mix_supported(bufA, pv, bufB, pv, H, cq2, ck2, causal, dtype, w_dtype);
+    if (one) {
+        if ((rc = trace_mark("conv2+head_mix2", st))) return rc;
+        if ((rc = conv_mix_launch(bufA, pv, w2, W2, bufB, pv, B, H, S, cq2, ck2, pl.r0, pl.r1, dtype, st))) return rc;
+        weights = bufB;
+    } else {
+        if ((rc = trace_mark("conv2", st))) return rc;
+        if ((rc = conv2d_launch(bufA, pv, pl.r1 - pl.ra, w2, w_dtype, bufB, pv, planes, H, S, S, cq2, ck2, causal, pl.r0, pl.r1, !causal, dtype, st, true))) return rc;
+        if ((rc = trace_mark("head_mix2", st))) return rc;
+        if ((rc = head_linear_launch(bufB, pv, W2, w_dtype, bufA, pv, B, H, S, S, causal, 0.0f, pl.r0, pl.r1, false, dtype, st, false, true))) return rc;
+    }
     if ((rc = trace_mark("pv", st))) return rc;
-    if ((rc = pv_launch(bufA, pv, pl.r1 - pl.ra, v, o, B, H, S, D, causal, pl.r0, pl.r1, dtype, st, drop))) return rc;
+    if ((rc = pv_launch(weights, pv, pl.r1 - pl.ra, v, o, B, H, S, D, causal, pl.r0, pl.r1, dtype, st, drop))) return rc;
     return trace_end(st);
 }
 

@@ -109,6 +109,12 @@ bool head_linear_tc05_supported(const void* x, PlaneView xv, const void* y, Plan
 int head_linear_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q, int causal,
                             float fill, int row_begin, int row_end, bool write_upper, bool wt, int dtype, cudaStream_t st, bool early_weights = false);
 
+// A small causal conv (2 or 3 row taps, 3 or 5 key taps) and the head mix that follows it in one kernel (conv_mix_tc05.cu): the conv's
+// output never reaches memory.  16-bit dtypes, weights in the same one, C = 8, 16, 32 or 64, rows [row_begin,row_end).
+bool conv_mix_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int CQ, int CK, int causal, int dtype, int w_dtype);
+int conv_mix_launch(const void* x, PlaneView xv, const void* w, const void* Wm, void* y, PlaneView yv, int N, int C, int Q, int CQ, int CK, int row_begin,
+                    int row_end, int dtype, cudaStream_t st);
+
 // Causal row softmax of pre_scale * x; rows [row_begin,row_end).  `dead` (planes of one batch element: `heads`): keys that get
 // probability 0, in a row with no other key too.
 int softmax_launch(const void* x, PlaneView xv, void* y, PlaneView yv, long planes, int P, int Q, int causal,
