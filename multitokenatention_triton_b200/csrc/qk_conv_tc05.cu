@@ -14,7 +14,7 @@
 // each), 12-15 epilogue.  TMEM: score buffers at columns 0 and 128, conv accumulators at 256 and 368.
 // Bound: the tensor pipe (per tile 512 cycles of score MMAs, 120 per row tap of conv MMAs: 1232 of the 1850 that a tile takes for 6 x 11)
 // and the hand-overs from MMA to drain to MMA.  Before, with the conv's operand in shared memory (a tile of 123 x 128 took 4700 cycles,
-// 3000 of them the conv MMAs' operand reads): B8 H16 S4096 6x11 1.27 -> 0.84 ms, B1 H16 S2048 7x7 72 -> 53 us, B2 H16 S1021 44 -> 29 us.
+// 3000 of them the conv MMAs' operand reads): B8 H16 S4096 6x11 1.27 -> 0.80 ms, B1 H16 S2048 7x7 72 -> 51 us, B2 H16 S1021 44 -> 29 us.
 // 16-bit dtypes, D in {64, 128}, odd key extent <= 17, causal.
 #include "toeplitz_ts.cuh"
 
@@ -23,12 +23,9 @@ namespace {
 using namespace tc05;
 using namespace qc;
 
-constexpr int OUT_COLS = TN / 2;                  // keys of one staging tile: two make an output tile
-constexpr int OUT_PITCH = OUT_COLS * 2;           // bytes between rows of its staging tile: 28 words, so the 16-byte stores of eight
-                                                  // consecutive rows fall into different banks without a swizzle
-// One staging tile.
-__host__ __device__ inline int out_bytes(int R) { return (tile_rows(R) * OUT_PITCH + 127) & ~127; }
-constexpr long GROUP_BYTES = 32 << 20;            // K of the planes that are worked on at a time
+// K of the planes that are worked on at a time stays in L2 (B8 H16 S4096: with one group 148 planes were in work, 155 MB of K; the kernel
+// 0.93 ms, 0.84 with groups).
+constexpr long GROUP_BYTES = 32 << 20;
 constexpr int DRAIN_WARPS = 8;
 constexpr int THREADS = 512;
 constexpr uint32_t C_COL = 2 * SN;                // TMEM column of the first conv accumulator
@@ -36,76 +33,9 @@ constexpr uint32_t C_COL = 2 * SN;                // TMEM column of the first co
 // the walk over the tiles.
 enum : int { ODD_TILE = 1, SECOND_SET = 2 };
 
-struct QcGeom {
-    int C, S, R, KS, row_begin, row_end, tiles_n, tiles_m, tmo, split_w, y_row0;
+struct QcGeom : TileGeom {
+    int S, R, KS, split_w, y_row0;
     float scale;
-    int tiles_per_plane, planes;
-    int groups, group_planes;                     // planes are worked through in groups
-};
-
-__device__ __forceinline__ int qc_key_tiles(const QcGeom& g, int tm) {
-    const int q_last = min(g.row_begin + (tm + 1) * g.tmo, g.row_end);
-    return min((q_last + TN - 1) / TN, g.tiles_n);
-}
-
-// A CTA's tiles: of every group of planes a contiguous range, so that all CTAs work on the same few planes at a time and K stays in L2
-// (B8 H16 S4096: with one range over all planes 148 of them were in work, 155 MB of K; 0.93 -> 0.84 ms).
-struct QcIter {
-    int plane, head, tm, tn, nk, left, group;
-    // The range of this CTA in group gr: returns its length.
-    __device__ int range(const QcGeom& g, int gr, unsigned* first) const {
-        const int p0 = gr * g.group_planes, np = min(g.group_planes, g.planes - p0);
-        const unsigned tiles = (unsigned)np * (unsigned)g.tiles_per_plane;
-        const unsigned c = (blockIdx.x + (unsigned)gr * (gridDim.x / 2 + 1)) % gridDim.x;      // who gets one tile more changes
-        const unsigned t0 = tiles * c / gridDim.x;
-        *first = t0;
-        return (int)(tiles * (c + 1) / gridDim.x - t0);
-    }
-    __device__ int total(const QcGeom& g) const {
-        int n = 0;
-        unsigned t;
-        for (int gr = 0; gr < g.groups; ++gr) n += range(g, gr, &t);
-        return n;
-    }
-    __device__ void enter(const QcGeom& g) {
-        unsigned t = 0;
-        do left = group < g.groups ? range(g, group++, &t) : 1 << 30;
-        while (left == 0);
-        const unsigned p = t / (unsigned)g.tiles_per_plane;
-        int r = (int)(t - p * (unsigned)g.tiles_per_plane);
-        plane = (group - 1) * g.group_planes + (int)p;
-        head = plane % g.C;
-        for (tm = 0;; ++tm) {
-            nk = qc_key_tiles(g, tm);
-            if (r < nk) break;
-            r -= nk;
-        }
-        tn = r;
-    }
-    __device__ void init(const QcGeom& g) {
-        group = 0;
-        enter(g);
-    }
-    // returns true when the walk moved on to another row of tiles (another Q tile)
-    __device__ bool next(const QcGeom& g) {
-        if (--left == 0) {
-            enter(g);
-            return true;
-        }
-        if (++tn == nk) {
-            tn = 0;
-            if (++tm == g.tiles_m) {
-                tm = 0;
-                ++plane;
-                if (++head == g.C) head = 0;
-            }
-            nk = qc_key_tiles(g, tm);
-            return true;
-        }
-        return false;
-    }
-    __device__ int m0(const QcGeom& g) const { return g.row_begin + tm * g.tmo; }
-    __device__ int n0() const { return tn * TN; }
 };
 
 template <typename T, int D>
@@ -126,13 +56,13 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
     uint8_t* q_base = smem;
     uint8_t* k_base = q_base + 2 * QK_BYTES;
     uint8_t* tb_base = k_base + 2 * QK_BYTES;                   // two sets of Toeplitz slices: successive heads alternate
-    uint8_t* out_base = tb_base + 2 * tb_bytes;                // two output tiles of two staging tiles
+    uint8_t* out_base = tb_base + 2 * tb_bytes;                // two staging tiles
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int pad_w = (KS - 1) / 2;
     const int a_off = 8 - pad_w;
     const int lead = R - 1, gr = group_rows(R);
 
-    QcIter it;
+    TileIter it;
     const int my_tiles = uniform(it.total(g));
 
     if (gave_up_before(err_flag, &abort_flag) || my_tiles == 0) return;
@@ -238,6 +168,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
                 cur_head = head;
                 ++hn;
                 // this set of slices was read last by the conv MMAs of the head before the previous one: tiles <= n - 2
+                // (that of tile n - 3 is over: the scores of tile n - 1, seen above, followed it)
                 if (n >= 2) mbar_wait_spin(&acc_full[b], ((n - 2) >> 1) & 1, err_flag);
                 float taps[TAPS_PER_THREAD];
                 fetch_taps(taps, w, w_dtype, head, R, KS, ft);
@@ -262,7 +193,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
         for (int n = 0; n < my_tiles; ++n, it.next(g)) {
             const int b = n & 1;
             const int plane = it.plane, m0 = it.m0(g), n0 = it.n0();
-            uint8_t* obuf = out_base + 2 * b * stage;
+            uint8_t* obuf = out_base + b * stage;
             uint8_t* orow = obuf + row * OUT_PITCH;
             if (issuer) bulk_wait_read_1();                  // the store of tile n - 2 has finished reading this staging tile
             mbar_wait_spin(&acc_full[b], (n >> 1) & 1, err_flag);
@@ -271,26 +202,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
             const uint32_t tacc = tmem + ((uint32_t)(quarter * 32) << 16) + C_COL + (uint32_t)(b * TN);
             const int live = m0 + row - n0 + 1;              // columns on or below the diagonal
             const bool diag = n0 + TN - 1 > m0;
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {                    // one staging tile each
-                uint32_t r[OUT_COLS], pk[OUT_COLS / 2];
-                tmem_ld_32x32(tacc + (uint32_t)(h * OUT_COLS), *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-                tmem_ld_32x16(tacc + (uint32_t)(h * OUT_COLS + 32), *reinterpret_cast<uint32_t(*)[16]>(&r[32]));
-                tmem_ld_32x8(tacc + (uint32_t)(h * OUT_COLS + 48), *reinterpret_cast<uint32_t(*)[8]>(&r[48]));
-                tmem_ld_wait();
-#pragma unroll
-                for (int e = 0; e < OUT_COLS / 2; ++e) pk[e] = pack2q<T>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
-                if (diag) {
-                    const int nl = live - h * OUT_COLS;
-#pragma unroll
-                    for (int e = 0; e < OUT_COLS / 2; ++e) pk[e] &= (2 * e < nl ? 0x0000ffffu : 0u) | (2 * e + 1 < nl ? 0xffff0000u : 0u);
-                }
-                if (inside) {
-#pragma unroll
-                    for (int c = 0; c < OUT_COLS / 8; ++c)
-                        *reinterpret_cast<uint4*>(orow + h * stage + c * 16) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-                }
-            }
+            stage_row<T>(tacc, orow, live, diag, inside);
             fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[b]);
@@ -299,7 +211,6 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
             if (issuer) {
                 // the box has the tile's rows; rows past row_end and columns past S are clipped by the tensor map
                 tma_store_3d(&my, obuf, n0, m0 - g.y_row0, plane);
-                if (n0 + OUT_COLS < g.S) tma_store_3d(&my, obuf + stage, n0 + OUT_COLS, m0 - g.y_row0, plane);
                 bulk_commit();
             }
         }
@@ -313,7 +224,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
 constexpr size_t QC_SMEM_LIMIT = 225 * 1024;
 
 size_t qk_conv_smem_bytes(int D, int R, bool split_w) {
-    return 1024 + 4 * (size_t)out_bytes(R) + 4 * (size_t)(D / 64) * BOX_BYTES + 2 * (size_t)toeplitz_bytes(R, split_w ? 1 : 0);
+    return 1024 + 2 * (size_t)out_bytes(R) + 4 * (size_t)(D / 64) * BOX_BYTES + 2 * (size_t)toeplitz_bytes(R, split_w ? 1 : 0);
 }
 
 template <typename T, int D>
@@ -321,35 +232,24 @@ int launch_qc(const void* q, const void* k, const void* w, int w_dtype, void* y,
               float scale, int row_begin, int row_end, cudaStream_t st) {
     const long planes = (long)B * H;
     QcGeom g{};
-    g.C = H; g.S = S; g.R = R; g.KS = KS; g.row_begin = row_begin; g.row_end = row_end; g.scale = scale;
-    g.tmo = tile_rows(R);
-    g.tiles_n = (S + TN - 1) / TN;
-    g.tiles_m = (row_end - row_begin + g.tmo - 1) / g.tmo;
+    set_tiles(g, planes, H, S, R, 1, row_begin, row_end);
+    set_groups(g, (planes * S * D * 2 + GROUP_BYTES - 1) / GROUP_BYTES);
+    g.S = S; g.R = R; g.KS = KS; g.scale = scale;
     g.split_w = w_dtype == MTA_F32 ? 1 : 0;
     g.y_row0 = yv.row0;
-    long per_plane = 0;
-    for (int tm = 0; tm < g.tiles_m; ++tm) {
-        const int q_last = std::min(row_begin + (tm + 1) * g.tmo, row_end);
-        per_plane += std::min((q_last + TN - 1) / TN, g.tiles_n);
-    }
-    g.tiles_per_plane = (int)per_plane;
-    g.planes = (int)planes;
-    g.groups = (int)std::max<long>(1, std::min<long>(planes, ((long)planes * S * D * 2 + GROUP_BYTES - 1) / GROUP_BYTES));
-    g.group_planes = (int)((planes + g.groups - 1) / g.groups);
-    g.groups = (int)((planes + g.group_planes - 1) / g.group_planes);
     CUtensorMap mq, mk, my;
     int rc;
     if ((rc = make_tensor_map_3d(&mq, q, (uint64_t)planes, S, D, D, (uint64_t)S * D, 64, 32, true))) return rc;
     if ((rc = make_tensor_map_3d(&mk, k, (uint64_t)planes, S, D, D, (uint64_t)S * D, 64, SN, true))) return rc;
     if ((rc = make_tensor_map_3d(&my, y, (uint64_t)planes, (uint64_t)(row_end - yv.row0), S, (uint64_t)yv.width,
-                                 (uint64_t)yv.plane_stride, OUT_COLS, (uint32_t)g.tmo, false)))
+                                 (uint64_t)yv.plane_stride, TN, (uint32_t)g.tmo, false)))
         return rc;
     int* flag = nullptr;
     if ((rc = wait_flag_ptr(&flag))) return rc;
     int sms = 0;
     if (int bad = sm_count(&sms)) return bad;
-    const unsigned grid = (unsigned)std::min<long>(per_plane * planes, sms);
-    MTA_REQUIRE(per_plane * g.group_planes * (sms + 1) < (1l << 32), "qk_conv: planes of %d x %d are too large", row_end - row_begin, S);
+    MTA_REQUIRE(tiles_countable(g, sms), "qk_conv: planes of %d x %d are too large", row_end - row_begin, S);
+    const unsigned grid = (unsigned)std::min<long>((long)g.tiles_per_plane * planes, sms);
     return launch_kernel<qk_conv_tc05_kernel<T, D>>("qk_conv_tc05_kernel", grid, THREADS, qk_conv_smem_bytes(D, R, g.split_w != 0), st, mq, mk, my, w,
                                                     w_dtype, g, flag);
 }

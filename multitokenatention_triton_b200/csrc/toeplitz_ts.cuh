@@ -1,5 +1,5 @@
-// Pieces shared by the kernels that compute a score tile Q K^T into tensor memory (TMEM) and run the conv's Toeplitz MMAs over it
-// (qk_conv_tc05.cu, conv_attn_tc05.cu): tile geometry, the drain that turns the fp32 scores into the 16-bit operand in place, the
+// Pieces shared by the kernels that run the conv as Toeplitz MMAs with its input in tensor memory (TMEM): conv2d_tc05.cu, and with the
+// scores Q K^T computed on the spot qk_conv_tc05.cu and conv_attn_tc05.cu.  Tile geometry, the drain that turns the fp32 scores into the 16-bit operand in place, the
 // conv MMA schedule and the Toeplitz slices.
 //
 // The score tile never leaves TMEM.  S[128 x 128] comes out of the score MMAs as fp32, the drain warps round it to 16 bits in place
@@ -140,12 +140,12 @@ __device__ __forceinline__ void clear_taps(float* wsm, int ft, int bar_id) {
     named_barrier(bar_id, 128);
 }
 // A caller that knows its next head ahead of time fetches its weights (thread ft holds taps ft, ft + 128, ...) before it needs them,
-// which hides the latency of global memory behind whatever it does next.
-__device__ __forceinline__ void fetch_taps(float (&reg)[TAPS_PER_THREAD], const void* w, int w_dtype, int head, int R, int KS, int ft) {
+// which hides the latency of global memory behind whatever it does next.  `flip`: taps in reverse order.
+__device__ __forceinline__ void fetch_taps(float (&reg)[TAPS_PER_THREAD], const void* w, int w_dtype, int head, int R, int KS, int ft, bool flip = false) {
 #pragma unroll
     for (int i = 0; i < TAPS_PER_THREAD; ++i) {
         const int idx = ft + 128 * i;
-        reg[i] = idx < R * KS ? load_weight(w, (long)head * R * KS + idx, w_dtype) : 0.0f;
+        reg[i] = idx < R * KS ? load_weight(w, (long)head * R * KS + (flip ? R * KS - 1 - idx : idx), w_dtype) : 0.0f;
     }
 }
 template <typename T>
@@ -195,6 +195,130 @@ __device__ __forceinline__ void drain_half(uint32_t tcol, uint32_t sc2, int live
     }
     tmem_st_32x32(tcol, pk);
     tmem_st_wait();
+}
+
+// The output tiles of a launch: `planes` planes, rows [row_begin,row_end) in tiles_m rows of tiles of tmo rows, tiles_n tiles of TN keys
+// (causal: only those that reach a key <= query).
+struct TileGeom {
+    int C, row_begin, row_end, tiles_n, tiles_m, tmo, causal;
+    int planes, tiles_per_plane;
+    int groups, group_planes;                     // planes are worked through in groups
+};
+__host__ __device__ __forceinline__ int key_tiles(const TileGeom& g, int tm) {
+    if (!g.causal) return g.tiles_n;
+    const int q_last = g.row_begin + (tm + 1) * g.tmo < g.row_end ? g.row_begin + (tm + 1) * g.tmo : g.row_end;
+    const int n = (q_last + TN - 1) / TN;
+    return n < g.tiles_n ? n : g.tiles_n;
+}
+// All but the groups, which are up to the kernel (set_groups).
+inline void set_tiles(TileGeom& g, long planes, int C, int W, int R, int causal, int row_begin, int row_end) {
+    g.C = C; g.row_begin = row_begin; g.row_end = row_end; g.causal = causal ? 1 : 0;
+    g.tmo = tile_rows(R);
+    g.tiles_n = (W + TN - 1) / TN;
+    g.tiles_m = (row_end - row_begin + g.tmo - 1) / g.tmo;
+    g.planes = (int)planes;
+    g.tiles_per_plane = 0;
+    for (int tm = 0; tm < g.tiles_m; ++tm) g.tiles_per_plane += key_tiles(g, tm);
+}
+inline void set_groups(TileGeom& g, long groups) {
+    g.groups = (int)(groups < 1 ? 1 : (groups > g.planes ? g.planes : groups));
+    g.group_planes = (g.planes + g.groups - 1) / g.groups;
+    g.groups = (g.planes + g.group_planes - 1) / g.group_planes;
+}
+// The walk below counts the tiles of a group times the CTAs in 32 bits.
+inline bool tiles_countable(const TileGeom& g, int sms) { return (double)g.tiles_per_plane * g.group_planes * (sms + 1) < 4294967296.0; }
+
+// A CTA's tiles: of every group of planes a contiguous range, so that all CTAs work on the same few planes at a time.
+struct TileIter {
+    int plane, head, tm, tn, nk, left, group;
+    // The range of this CTA in group gr: returns its length.
+    __device__ int range(const TileGeom& g, int gr, unsigned* first) const {
+        const int p0 = gr * g.group_planes, np = min(g.group_planes, g.planes - p0);
+        const unsigned tiles = (unsigned)np * (unsigned)g.tiles_per_plane;
+        const unsigned c = (blockIdx.x + (unsigned)gr * (gridDim.x / 2 + 1)) % gridDim.x;      // who gets one tile more changes
+        const unsigned t0 = tiles * c / gridDim.x;
+        *first = t0;
+        return (int)(tiles * (c + 1) / gridDim.x - t0);
+    }
+    __device__ int total(const TileGeom& g) const {
+        int n = 0;
+        unsigned t;
+        for (int gr = 0; gr < g.groups; ++gr) n += range(g, gr, &t);
+        return n;
+    }
+    __device__ void enter(const TileGeom& g) {
+        unsigned t = 0;
+        do left = group < g.groups ? range(g, group++, &t) : 1 << 30;
+        while (left == 0);
+        const unsigned p = t / (unsigned)g.tiles_per_plane;
+        int r = (int)(t - p * (unsigned)g.tiles_per_plane);
+        plane = (group - 1) * g.group_planes + (int)p;
+        head = plane % g.C;
+        for (tm = 0;; ++tm) {
+            nk = key_tiles(g, tm);
+            if (r < nk) break;
+            r -= nk;
+        }
+        tn = r;
+    }
+    __device__ void init(const TileGeom& g) {
+        group = 0;
+        enter(g);
+    }
+    // returns true when the walk moved on to another row of tiles (another Q tile)
+    __device__ bool next(const TileGeom& g) {
+        if (--left == 0) {
+            enter(g);
+            return true;
+        }
+        if (++tn == nk) {
+            tn = 0;
+            if (++tm == g.tiles_m) {
+                tm = 0;
+                ++plane;
+                if (++head == g.C) head = 0;
+            }
+            nk = key_tiles(g, tm);
+            return true;
+        }
+        return false;
+    }
+    __device__ int m0(const TileGeom& g) const { return g.row_begin + tm * g.tmo; }
+    __device__ int n0() const { return tn * TN; }
+};
+
+// ---- output ------------------------------------------------------------------------------------------
+// Bytes between rows of a staging tile: one box of 112 columns, whole 32-byte sectors in memory.  (Two boxes of 56, without the two-way
+// bank conflict of this pitch: score + conv kernel at B8 H16 S4096 845 us, 805 like this.)
+constexpr int OUT_PITCH = TN * 2;
+__host__ __device__ inline int out_bytes(int R) { return (tile_rows(R) * OUT_PITCH + 127) & ~127; }
+
+// A thread's row of a finished accumulator at `tacc` -> 16 bits -> its row of a staging tile at `orow`.  `live`:
+// columns on or below the diagonal, the others become 0 (`diag`: there are others, for some thread of the warp); `inside`: the lane
+// carries an output row.  Whole-warp call; on return the accumulator has been read.
+template <typename T>
+__device__ __forceinline__ void stage_row(uint32_t tacc, uint8_t* orow, int live, bool diag, bool inside) {
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        constexpr int OUT_COLS = TN / 2;
+        uint32_t r[OUT_COLS], pk[OUT_COLS / 2];
+        tmem_ld_32x32(tacc + (uint32_t)(h * OUT_COLS), *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+        tmem_ld_32x16(tacc + (uint32_t)(h * OUT_COLS + 32), *reinterpret_cast<uint32_t(*)[16]>(&r[32]));
+        tmem_ld_32x8(tacc + (uint32_t)(h * OUT_COLS + 48), *reinterpret_cast<uint32_t(*)[8]>(&r[48]));
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < OUT_COLS / 2; ++e) pk[e] = pack2q<T>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+        if (diag) {
+            const int nl = live - h * OUT_COLS;
+#pragma unroll
+            for (int e = 0; e < OUT_COLS / 2; ++e) pk[e] &= (2 * e < nl ? 0x0000ffffu : 0u) | (2 * e + 1 < nl ? 0xffff0000u : 0u);
+        }
+        if (inside) {
+#pragma unroll
+            for (int c = 0; c < OUT_COLS / 8; ++c)
+                *reinterpret_cast<uint4*>(orow + h * OUT_COLS * 2 + c * 16) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+        }
+    }
 }
 
 }  // namespace qc

@@ -1,10 +1,10 @@
-"""The score + conv kernel at the edges of its tiles: 4 (33 - R) query rows in four groups of 33 - R, 112 keys."""
+"""The convs with their input in tensor memory at the edges of their tiles: 4 (33 - R) query rows in four groups of 33 - R, 112 keys."""
 import pytest
 import torch
 
 from multitokenatention_triton_b200 import _lib, ops
 from oracle import mta_oracle as orc
-from util import ROUND, assert_parity, npf
+from util import ROUND, assert_parity, conv64, conv64_bwd_input, npf
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -28,3 +28,24 @@ def test_tile_edges(S, R, Sk, D, dtype, w32):
     got = npf(ops.mta_fused_fwd(*[t.to(DEV) for t in args]))
     _lib.device_status()
     assert_parity(got, orc.mta_fwd(*[npf(t) for t in args], True, ROUND[dtype]), dtype, f"S={S} {R}x{Sk}")
+
+
+# the conv alone and its input gradient: a result may be off by half a unit in its last place (2^-8 or 2^-11 of it) and by the float32 sum of
+# up to 272 products, 272 * 2^-24 of their magnitudes, which add up to about 11
+@pytest.mark.parametrize("S,R,Sk,causal,dtype,w32", [(107, 6, 11, True, torch.bfloat16, False), (108, 6, 11, False, torch.float16, False),
+                                                     (113, 6, 11, True, torch.float16, True), (225, 6, 11, False, torch.bfloat16, False),
+                                                     (129, 1, 1, True, torch.bfloat16, False), (112, 2, 4, True, torch.bfloat16, False),
+                                                     (69, 16, 17, True, torch.bfloat16, True), (137, 16, 17, False, torch.float16, True),
+                                                     (233, 11, 15, True, torch.bfloat16, False)])
+def test_conv2d_tile_edges(S, R, Sk, causal, dtype, w32):
+    g = torch.Generator(device=DEV).manual_seed(S * 100 + R)
+    x = torch.randn(2, 3, S, S, device=DEV, generator=g).to(dtype)
+    w = (torch.randn(3, R, Sk, device=DEV, generator=g) * (R * Sk) ** -0.5).to(torch.float32 if w32 else dtype)
+    nan = x.masked_fill(torch.ones(S, S, dtype=torch.bool, device=DEV).triu(1), float("nan")) if causal else x
+    pairs = [(ops.conv2d_fwd(nan, w, causal), conv64(x, w, causal))]
+    if Sk % 2 == 1:
+        pairs.append((ops.conv2d_bwd_input(nan, w, causal), conv64_bwd_input(x, w, causal)))
+    _lib.device_status()
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, b in pairs:
+        assert bool(((a.double() - b).abs() <= u * b.abs() + 2e-4).all())
