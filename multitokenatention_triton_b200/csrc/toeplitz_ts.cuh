@@ -71,7 +71,7 @@ __device__ __forceinline__ uint64_t desc_plain(uint32_t saddr, uint32_t lbo_byte
 // Shared-memory bytes of one head's Toeplitz slices.
 __host__ __device__ inline int toeplitz_bytes(int R, int split_w) { return (R * 1024 * (split_w ? 2 : 1) + 1023) & ~1023; }
 
-// The conv MMAs of one row tap (or of the high or low part of its weights): A in the score buffer at a0, k-step s = staged
+// The conv MMAs of one row tap (or of the high or low part of its weights): A in a buffer of 16 NK columns at a0, k-step s = staged
 // columns 16 s .. 16 s + 15, which reach the 16-column output blocks s - 1 and s of the accumulator at d0 (the first and the last
 // k-step reach one block only: N = 16, half of the slice).  Every other k-step comes first: those touch each block once, so the first
 // batch of a tile (ACC false) needs no cleared accumulator.  All from one thread, in this order, so the result does not depend on
@@ -80,41 +80,41 @@ __host__ __device__ inline int toeplitz_bytes(int R, int split_w) { return (R * 
 // SHIFT: A is left one row up, for the next tap.
 // An MMA takes 16 cycles on the tensor pipe and only so many instructions may come with it: with the accumulate flag or the order of
 // the k-steps as run-time values it was 22 to 28 cycles an MMA.
-template <typename T, int FIRST, bool SHIFT, bool ACC>
+template <typename T, int NK, int FIRST, bool SHIFT, bool ACC>
 __device__ __forceinline__ void issue_tap(uint32_t a0, uint64_t db, uint32_t d0, uint32_t el) {
     constexpr uint32_t idesc32 = instr_desc_f16(AbFmtQ<T>::value, 0, 0, TM, 32);
     constexpr uint32_t idesc16 = instr_desc_f16(AbFmtQ<T>::value, 0, 0, TM, 16);
 #pragma unroll
     for (int pass = 0; pass < 2; ++pass)
 #pragma unroll
-        for (int s = pass ^ FIRST; s < SN / 16; s += 2) {
-            const bool upper = s == 0, lower = s == SN / 16 - 1;
+        for (int s = pass ^ FIRST; s < NK; s += 2) {
+            const bool upper = s == 0, lower = s == NK - 1;
             const uint64_t b = db + (upper ? 16u : 0u);
-            const uint32_t a = a0 + 8u * (uint32_t)s + (s >= 4 ? 32u : 0u);             // k-steps 4 .. 7 in the buffer's second half
+            const uint32_t a = a0 + 8u * (uint32_t)s + (s >= NK / 2 ? 4u * NK : 0u);     // in the buffer's second half
             const uint32_t d = d0 + (upper ? 0u : 16u * (uint32_t)(s - 1)), idesc = (upper || lower) ? idesc16 : idesc32;
             if (SHIFT) mma_f16_ts_shift(d, a, b, idesc, (pass > 0 || ACC) ? 1u : 0u, el);
             else mma_f16_ts(d, a, b, idesc, (pass > 0 || ACC) ? 1u : 0u, el);
         }
 }
-template <typename T, int FIRST>
+template <typename T, int NK, int FIRST>
 __device__ __forceinline__ void issue_taps(uint32_t a0, uint64_t db, uint32_t d0, int R, int split_w, uint32_t el) {
     // (the shift after the last tap is of no use to anybody and costs nothing)
     if (split_w) {                                                        // float32 weights: every tap in two parts
         const uint64_t low = (uint64_t)(R * 64);
-        issue_tap<T, FIRST, false, false>(a0, db, d0, el);
-        issue_tap<T, FIRST, true, true>(a0, db + low, d0, el);
+        issue_tap<T, NK, FIRST, false, false>(a0, db, d0, el);
+        issue_tap<T, NK, FIRST, true, true>(a0, db + low, d0, el);
 #pragma unroll 1
         for (int i = 1; i < R; ++i) {
             db += 64;
-            issue_tap<T, FIRST, false, true>(a0, db, d0, el);
-            issue_tap<T, FIRST, true, true>(a0, db + low, d0, el);
+            issue_tap<T, NK, FIRST, false, true>(a0, db, d0, el);
+            issue_tap<T, NK, FIRST, true, true>(a0, db + low, d0, el);
         }
     } else {
-        issue_tap<T, FIRST, true, false>(a0, db, d0, el);
+        issue_tap<T, NK, FIRST, true, false>(a0, db, d0, el);
 #pragma unroll 1
         for (int i = 1; i < R; ++i) {
             db += 64;
-            issue_tap<T, FIRST, true, true>(a0, db, d0, el);
+            issue_tap<T, NK, FIRST, true, true>(a0, db, d0, el);
         }
     }
 }
@@ -122,8 +122,8 @@ __device__ __forceinline__ void issue_taps(uint32_t a0, uint64_t db, uint32_t d0
 template <typename T>
 __device__ __forceinline__ void issue_conv(uint32_t a0, uint32_t tb_addr, uint32_t d0, int odd, int R, int split_w, uint32_t el) {
     const uint64_t db = desc_plain(tb_addr, 512, 128);
-    if (odd) issue_taps<T, 0>(a0, db, d0, R, split_w, el);
-    else issue_taps<T, 1>(a0, db, d0, R, split_w, el);
+    if (odd) issue_taps<T, SN / 16, 0>(a0, db, d0, R, split_w, el);
+    else issue_taps<T, SN / 16, 1>(a0, db, d0, R, split_w, el);
 }
 
 // The Toeplitz slices of a head (row tap i, element (n', kk) = w[i][kk + 16 - n' - a_off]; with `split_w` a second set holding what

@@ -49,3 +49,19 @@ def test_conv2d_tile_edges(S, R, Sk, causal, dtype, w32):
     u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     for a, b in pairs:
         assert bool(((a.double() - b).abs() <= u * b.abs() + 2e-4).all())
+
+
+# the conv attention: tiles of 80 keys, units of 4 (33 - R) rows
+@pytest.mark.parametrize("S,R,Sk,D,dtype,w32", [(1, 6, 11, 64, torch.bfloat16, False), (27, 6, 11, 128, torch.float16, False), (79, 6, 11, 128, torch.bfloat16, False),
+                                                (81, 6, 11, 64, torch.bfloat16, True), (109, 6, 11, 128, torch.bfloat16, False), (161, 1, 1, 128, torch.float16, False),
+                                                (129, 2, 3, 64, torch.bfloat16, False), (137, 16, 17, 128, torch.bfloat16, True), (241, 16, 17, 64, torch.float16, False),
+                                                (321, 11, 15, 128, torch.bfloat16, False)])
+def test_conv_attention_tile_edges(S, R, Sk, D, dtype, w32):
+    g = torch.Generator().manual_seed(S * 100 + R)
+    q, k, v = (torch.randn(2, 4, S, D, generator=g).to(dtype) for _ in range(3))
+    w = (torch.randn(4, R, Sk, generator=g) * (R * Sk) ** -0.5).to(torch.float32 if w32 else dtype)
+    _lib.reset_launch_count()
+    got = npf(ops.conv_attn_fwd(*[t.to(DEV) for t in (q, k, v, w)], True, D ** -0.5))
+    assert _lib.launch_count() == 1
+    _lib.device_status()
+    assert_parity(got, orc.conv_attn_fwd(*[npf(t) for t in (q, k, v, w)], True, None, orc.ROUND_NONE), dtype, f"S={S} {R}x{Sk}")
