@@ -10,7 +10,8 @@
 // FMAs).  The halo tile is staged as fp32 by 4-byte asynchronous copies (all in
 // flight at once) with the causal zero applied on the way; 16-byte chunks are swizzled so that lanes 32 bytes apart hit
 // different banks.
-// Measured at B1 H16 S2048 11x15 float32: 308 us (conv2d_tile_kernel: 591), the FMA pipe 65 % busy.
+// Measured at B1 H16 S2048 11x15 float32: 295 us (conv2d_tile_kernel: 591); four CTAs an SM, which 15 key taps only get when the compiler is
+// held to 128 registers (305 us with 129 and three).
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -67,7 +68,7 @@ __device__ __forceinline__ void stage_tile(float* dst, int pitch, const T* plane
 }
 
 template <typename T, int S>
-__global__ void __launch_bounds__(THREADS, 3)
+__global__ void __launch_bounds__(THREADS, S == 15 ? 4 : 3)
 conv2d_fma_kernel(const T* __restrict__ x, PlaneView xv, const void* __restrict__ w, int w_dtype, T* __restrict__ y, PlaneView yv, int C,
                   int H, int W, int R, int causal, int row_begin, int row_end, int write_upper, int tiles_n, int grad_input) {
     constexpr int NP = (S + 1) / 2;                         // tap pairs per row tap

@@ -850,12 +850,14 @@ bool mix_softmax_mma_ok(const void* x, PlaneView xv, const void* y, PlaneView yv
 bool head_mix_softmax_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int causal, int dtype,
                                 int w_dtype) {
     return mix_softmax_mma_ok(x, xv, y, yv, C, Q, causal, dtype) ||
-           head_mix_softmax_tc05_supported(x, xv, y, yv, C, Q, causal, dtype, w_dtype);
+           head_mix_softmax_tc05_supported(x, xv, y, yv, C, Q, causal, dtype, w_dtype) ||
+           head_mix_softmax_f32_supported(x, xv, y, yv, C, Q, causal, dtype);
 }
 
 int head_mix_softmax_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C,
                             int Q, int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, bool early_weights) {
     if (N == 0 || row_end <= row_begin || Q == 0) return MTA_OK;
+    if (dtype == MTA_F32) return head_mix_softmax_f32_launch(x, xv, Wm, w_dtype, y, yv, N, C, Q, row_begin, row_end, write_upper, st, early_weights);
     // variant "mix_softmax": 0 auto (tcgen05 where it applies), 1 the mma.sync kernel, 2 tcgen05 or an error
     const int want = variant("mix_softmax");
     const bool tc05_able = head_mix_softmax_tc05_supported(x, xv, y, yv, C, Q, 1, dtype, w_dtype);

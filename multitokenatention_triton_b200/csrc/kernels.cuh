@@ -88,12 +88,17 @@ bool head_dw_tc05_supported(const void* x, PlaneView xv, const void* dy, PlaneVi
 int head_dw_tc05_launch(const void* x, PlaneView xv, const void* dy, PlaneView dyv, float* partial, int* slots_out, int N, int C, int P, int Q,
                         int causal, int dtype, cudaStream_t st);
 
-// Head mix followed by the causal row softmax of the mixed logits, in one pass (16-bit dtypes, C <= 32, causal);
+// Head mix followed by the causal row softmax of the mixed logits, in one pass (causal; 16-bit dtypes with C <= 32, float32 with rows that fit);
 // entries above the diagonal of y are written as 0 when `write_upper`, else left untouched.
 bool head_mix_softmax_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int causal, int dtype,
                                 int w_dtype);
 int head_mix_softmax_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C,
                             int Q, int row_begin, int row_end, bool write_upper, int dtype, cudaStream_t st, bool early_weights = false);
+
+// The same in float32 (head_mix_softmax_f32.cu), rows whose C logits fit into shared memory, 16-byte aligned.
+bool head_mix_softmax_f32_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int Q, int causal, int dtype);
+int head_mix_softmax_f32_launch(const void* x, PlaneView xv, const void* Wm, int w_dtype, void* y, PlaneView yv, int N, int C, int Q, int row_begin,
+                                int row_end, bool write_upper, cudaStream_t st, bool early_weights);
 
 // The same on tcgen05 (head_mix_tc05.cu): C a power of two in 8..128, weights in the activations' 16-bit dtype; entries
 // above the diagonal are written as 0 up to the end of the diagonal's 128-key tile, and up to Q when `write_upper`.
