@@ -15,8 +15,8 @@
 // A work unit = (batch element n, group of R rows).  Two passes over the unit's key tiles:
 //   pass 1  tiles 0 .. diagonal: MMA -> TMEM -> round to the 16-bit dtype (the reference's rounding point) -> running
 //           (maximum, sum of exponentials) per thread; nothing is written;
-//   pass 2  the same tiles from the diagonal back to 0 (the input comes from L2: a unit's rows are at most 1 MB):
-//           MMA again -> round -> 2^(x log2 e - shift) -> 16-bit -> a staging buffer per softmax group -> one TMA store
+//   pass 2  the same tiles from the diagonal back to 0: the last four are still in the accumulators, the others come from L2 (a unit's
+//           rows are at most 1 MB) and are mixed again -> round -> 2^(x log2 e - shift) -> 16-bit -> a staging buffer per softmax group -> one TMA store
 //           per 32 keys x 128 rows (a box of 32 keys x R rows x C planes, the mirror image of the input box).
 // Recomputing the mix costs tensor time that is free here; in exchange the logits never exist in memory.
 //
@@ -200,7 +200,6 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
     uint8_t* stage_base = smem + HM_A_BYTES;
     uint8_t* out_base = stage_base + HM_NSTAGE * HM_STAGE_BYTES;      // HM_NACC staging buffers of HM_OUT_BYTES
     uint8_t* fill_base = out_base + HM_NACC * HM_OUT_BYTES;           // one more, holding `fill` (0 for the softmax) everywhere
-    constexpr int PASSES = SOFTMAX ? 2 : 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int C = g.C, R = g.R;
 
@@ -259,7 +258,9 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
         if (u >= g.units) continue;                                                                    \
         const int n = (int)(u % g.N), p0 = g.row_begin + (g.groups - 1 - (int)(u / g.N)) * R;          \
         const int nt = hm_tiles(g, p0);                                                                \
-        (void)n;
+        const int hold = SOFTMAX ? min(nt, HM_NACC) : 0;      /* tiles whose accumulators wait for pass 2 */ \
+        const int count = SOFTMAX ? 2 * nt - hold : nt;       /* products of the unit */                 \
+        (void)n; (void)count;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -268,14 +269,14 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
             int it = 0;
             bool ok = true;
             HM_FOR_UNITS
-                for (int j = 0; j < PASSES * nt && ok; ++j, ++it) {
-                    const int kt = j < nt ? j : 2 * nt - 1 - j;
+                for (int j = 0; j < count && ok; ++j, ++it) {
+                    const int kt = j < nt ? j : 2 * nt - 1 - hold - j;
                     const int st = it % HM_NSTAGE;
                     const int use = it / HM_NSTAGE;
                     if (use > 0 && !(ok = mbar_wait(&empty_bar[st], (uint32_t)((use - 1) & 1), err_flag))) break;
                     uint8_t* dst = stage_base + st * HM_STAGE_BYTES;
                     mbar_expect_tx(&full_bar[st], HM_STAGE_BYTES);
-                    const uint64_t pol = (SOFTMAX && j < nt) ? pol_keep : pol_drop;
+                    const uint64_t pol = j < nt - hold && SOFTMAX ? pol_keep : pol_drop;
                     tma_load_3d_hint(dst, &mx, &full_bar[st], kt * HM_KEYS, p0 - g.x_row0, n * C, pol);
                     tma_load_3d_hint(dst + HM_BOX_BYTES, &mx, &full_bar[st], kt * HM_KEYS + 64, p0 - g.x_row0, n * C, pol);
                 }
@@ -291,9 +292,9 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
         int it = 0;
         bool ok = true;
         HM_FOR_UNITS
-            for (int j = 0; j < PASSES * nt && ok; ++j, ++it) {
+            for (int j = 0; j < count && ok; ++j, ++it) {
                 if (it % HM_ISSUERS != issuer) continue;
-                const int kt = j < nt ? j : 2 * nt - 1 - j;
+                const int kt = j < nt ? j : 2 * nt - 1 - hold - j;
                 const int st = it % HM_NSTAGE, ab = it % HM_NACC;
                 const int use = it / HM_NSTAGE, au = it / HM_NACC;
                 uint8_t* sb = stage_base + st * HM_STAGE_BYTES;
@@ -367,7 +368,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
 #pragma unroll 1
                 for (int c = 0; c < 4; ++c) {
                     tmem_ld_round32<T>(t_base + (uint32_t)(c * 32), cur);
-                    if (c == 3) {
+                    if (c == 3 && j < nt - hold) {
                         fence_before_sync();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&acc_empty[grp]);
@@ -400,13 +401,21 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
             // p = 2^(x log2 e - shift): the division by the sum is folded into the exponent
             shift = fmaf(mm, HM_LOG2E, log2f(ss));
             }
-            // ---- the output pass: for the softmax the tiles again, from the diagonal down ----
-            for (int j = 0; j < nt; ++j) {                         // no early exit after a wait gave up (see below)
-                const int t = it + j;
-                if (t % HM_NACC != grp) continue;
-                if (ok) ok = mbar_wait_spin(&acc_full[grp], (uint32_t)((t / HM_NACC) & 1), err_flag);
+            // ---- the output pass: for the softmax the tiles again, from the diagonal down; the last `hold` of them are still in the
+            // accumulators, this group's own tile of them comes first (j = -1) ----
+            for (int j = hold > 0 ? -1 : 0; j < nt - hold; ++j) {         // no early exit after a wait gave up (see below)
+                int key0;
+                if (j < 0) {
+                    const int first = nt - hold, own = first + ((grp - (it - nt + first)) & (HM_NACC - 1));
+                    if (own >= nt) continue;
+                    key0 = own * HM_KEYS;
+                } else {
+                    const int t = it + j;
+                    if (t % HM_NACC != grp) continue;
+                    if (ok) ok = mbar_wait_spin(&acc_full[grp], (uint32_t)((t / HM_NACC) & 1), err_flag);
+                    key0 = (SOFTMAX ? nt - 1 - hold - j : j) * HM_KEYS;
+                }
                 fence_after_sync();
-                const int key0 = (SOFTMAX ? nt - 1 - j : j) * HM_KEYS;
                 uint32_t cur[16];
 #pragma unroll 1
                 for (int c = 0; c < 4; ++c) {
@@ -440,7 +449,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
                     }
                 }
             }
-            it += nt;
+            it += nt - hold;
             if (g.write_upper && issuer) {
                 // Everything past the unit's last tile is `fill` (0 for the softmax): boxes of the constant buffer, the
                 // groups taking turns.  Nobody waits for these stores before the kernel ends.
