@@ -11,6 +11,8 @@
 // added in group order, so a row's sum depends only on which index lies in which block.
 // The accumulators are packed pairs of columns: the packed FMA needs half the issue slots, which the operand loads then use.
 // Measured at B1 H16 S2048 D64: P V 115 us (the general kernel: 532), Q K^T 131 us (183); the FMAs alone would take 64.
+// Few tiles leave SMs idle and an SM with four groups needs 10 000 cycles for 64 x 64 x 256: there the groups of QK are CTAs of their own
+// and the others take half as many columns.  B2 H8 S256 D64 inside the forward: Q K^T 18.7 -> 14.4 us, P V 16.4 -> 10.2.
 #include "kernels.cuh"
 
 namespace mta {
@@ -29,10 +31,12 @@ constexpr int OPER_N = BK * BT;      // floats of an operand staged [index][row]
 
 enum Kind { QK, PV, PT };
 constexpr int a_floats(Kind kind) { return kind == PT ? OPER_N : OPER_K; }
-constexpr int b_floats(Kind) { return OPER_N; }
-constexpr int stage_floats(Kind kind) { return a_floats(kind) + b_floats(kind); }
-constexpr int smem_bytes(Kind kind) { return GROUPS * NST * stage_floats(kind) * (int)sizeof(float); }
-static_assert(NST * stage_floats(PV) >= BT * BT && NST * stage_floats(PT) >= BT * BT, "the partial tiles reuse the rings");
+// bn: columns of an output tile, 64 or 32
+constexpr int stage_floats(Kind kind, int bn) { return a_floats(kind) + BK * bn; }
+constexpr int smem_bytes(Kind kind, int bn) { return GROUPS * NST * stage_floats(kind, bn) * (int)sizeof(float); }
+static_assert(NST * stage_floats(PV, 64) >= BT * 64 && NST * stage_floats(PT, 64) >= BT * 64 && NST * stage_floats(PV, 32) >= BT * 32 &&
+                  NST * stage_floats(PT, 32) >= BT * 32,
+              "the partial tiles reuse the rings");
 
 __device__ __forceinline__ void group_barrier(int group) { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(GTHREADS) : "memory"); }
 // 16 bytes to shared memory, of which only the first n floats come from src (none: src is not touched), the rest become 0.
@@ -48,27 +52,30 @@ template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.
 // 32 + tx * 4 + {0,1}, {2,3}.
 __device__ __forceinline__ int pair_col(int tx, int j) { return (j < 2 ? tx * 4 + 2 * j : 32 + tx * 4 + 2 * (j - 2)); }
 
-__global__ void __launch_bounds__(THREADS, 2)
+// G groups a CTA: four, a 2 x 2 block of tiles that share their operands in L1, or one, when there are fewer blocks than SMs.
+template <int G>
+__global__ void __launch_bounds__(G * GTHREADS, 8 / G)
 qk_f32_kernel(const float* __restrict__ q, const float* __restrict__ k, float* __restrict__ s, PlaneView sv, int S, int D, float scale,
               int causal, int row_begin, int row_end, int tiles_k) {
     extern __shared__ __align__(16) float smem[];
     pdl_wait();
     const long bh = blockIdx.x;
+    constexpr int EDGE = G == 1 ? BT : 2 * BT;           // of a CTA's block
     const int tq = blockIdx.y / tiles_k, tk = blockIdx.y % tiles_k;
-    if (causal && tk * 2 * BT > min(row_begin + (tq + 1) * 2 * BT, row_end) - 1) return;
+    if (causal && tk * EDGE > min(row_begin + (tq + 1) * EDGE, row_end) - 1) return;
     const int group = threadIdx.x / GTHREADS, gt = threadIdx.x % GTHREADS;
-    const int q0 = row_begin + tq * 2 * BT + (group >> 1) * BT, k0 = tk * 2 * BT + (group & 1) * BT;
+    const int q0 = row_begin + tq * EDGE + (group >> 1) * BT, k0 = tk * EDGE + (group & 1) * BT;
     const int q_end = min(q0 + BT, row_end);
     if (q0 >= row_end || k0 >= S || (causal && k0 > q_end - 1)) return;      // a whole group: its barrier has no other members
     const float* qp = q + (bh * S + q0) * D;
     const float* kp = k + (bh * S + k0) * D;
-    float* ring = smem + group * NST * stage_floats(QK);
+    float* ring = smem + group * NST * stage_floats(QK, BT);
     const int ty = gt >> 3, tx = gt & 7;
     const int blocks = (D + BK - 1) / BK;
     const int lm = gt >> 2, lq = gt & 3;          // loader: rows lm + 16 r, index quad lq of the block
     auto issue_q = [&](int b) {
         if (b < blocks) {
-            float* as = ring + (b % NST) * stage_floats(QK);
+            float* as = ring + (b % NST) * stage_floats(QK, BT);
             const int d = b * BK + lq * 4;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
@@ -98,8 +105,8 @@ qk_f32_kernel(const float* __restrict__ q, const float* __restrict__ k, float* _
     load_k(0);
 #pragma unroll 1
     for (int b = 0; b < blocks; ++b) {
-        const float* as = ring + (b % NST) * stage_floats(QK);
-        float* bs = ring + (b % NST) * stage_floats(QK) + OPER_K;
+        const float* as = ring + (b % NST) * stage_floats(QK, BT);
+        float* bs = ring + (b % NST) * stage_floats(QK, BT) + OPER_K;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int col = (lm + 16 * r + 8 * lq) & (BT - 1);
@@ -150,7 +157,8 @@ qk_f32_kernel(const float* __restrict__ q, const float* __restrict__ k, float* _
     }
 }
 
-template <Kind KIND>
+// BN: 64 columns of the output, or 32 (half of a thread's accumulators), when there are fewer tiles than SMs.
+template <Kind KIND, int BN>
 __global__ void __launch_bounds__(THREADS, 2)
 pv_f32_kernel(const float* __restrict__ p, PlaneView pv, const float* __restrict__ v, float* __restrict__ o, int planes, int S, int D,
               int causal, int row_begin, int row_end, int tiles_d, float scale) {
@@ -162,14 +170,14 @@ pv_f32_kernel(const float* __restrict__ p, PlaneView pv, const float* __restrict
     const int width = min(PLANE_GROUP, planes - p0);
     const long bh = p0 + in_group % width;
     const int t = in_group / width / tiles_d, td = in_group / width % tiles_d, tq = KIND == PT ? t : n_q - 1 - t;
-    const int q0 = row_begin + tq * BT, d0 = td * BT;
+    const int q0 = row_begin + tq * BT, d0 = td * BN;
     const int q_end = min(q0 + BT, row_end);
     // contraction indices [c_lo, c_hi), c_lo a multiple of BK
     const int c_lo = KIND == PT && causal ? q0 / BK * BK : 0, c_hi = KIND == PV && causal ? min(q_end, S) : S;
     const int group = threadIdx.x / GTHREADS, gt = threadIdx.x % GTHREADS;
     const float* vp = v + bh * (long)S * D + d0;
     const float* pp = p + bh * pv.plane_stride;
-    float* ring = smem + group * NST * stage_floats(KIND);
+    float* ring = smem + group * NST * stage_floats(KIND, BN);
     const int ty = gt >> 3, tx = gt & 7;
     // blocks of this group: the absolute block index modulo 4 says whose it is, so a row range changes no sum
     const int first = c_lo / BK + ((group - c_lo / BK) & (GROUPS - 1));
@@ -177,7 +185,7 @@ pv_f32_kernel(const float* __restrict__ p, PlaneView pv, const float* __restrict
     const int blocks = n_all > first ? (n_all - first + GROUPS - 1) / GROUPS : 0;
     auto issue = [&](int b) {
         if (b < blocks) {
-            float* as = ring + (b % NST) * stage_floats(KIND);
+            float* as = ring + (b % NST) * stage_floats(KIND, BN);
             float* bs = as + a_floats(KIND);
             const int c0 = (first + b * GROUPS) * BK;
 #pragma unroll
@@ -191,25 +199,27 @@ pv_f32_kernel(const float* __restrict__ p, PlaneView pv, const float* __restrict
                     const int n = qq < c_hi ? min(q_end, causal ? qq + 1 : q_end) - kk : 0;
                     copy16(as + c * BT + (gt & 15) * 4, n > 0 ? pp + (long)(qq - pv.row0) * pv.width + kk : p, n);
                 }
-                const int c = (gt >> 4) + 4 * r, d = (gt & 15) * 4;
-                const int n = c0 + c < c_hi ? D - d0 - d : 0;
-                copy16(bs + c * BT + d, n > 0 ? vp + (long)(c0 + c) * D + d : v, n);
+                if (r < BN / 16) {
+                    const int c = gt / (BN / 4) + 256 / BN * r, d = gt % (BN / 4) * 4;
+                    const int n = c0 + c < c_hi ? D - d0 - d : 0;
+                    copy16(bs + c * BN + d, n > 0 ? vp + (long)(c0 + c) * D + d : v, n);
+                }
             }
         }
         copy_commit();
     };
-    float2 acc[8][4];
+    float2 acc[8][BN / 16];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+        for (int j = 0; j < BN / 16; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int b = 0; b < NST - 1; ++b) issue(b);
     for (int b = 0; b < blocks; ++b) {
         copy_wait<NST - 2>();
         group_barrier(group);
         issue(b + NST - 1);
-        const float* as = ring + (b % NST) * stage_floats(KIND);
+        const float* as = ring + (b % NST) * stage_floats(KIND, BN);
         const float* bs = as + a_floats(KIND);
 #pragma unroll
         for (int k4 = 0; k4 < BK / 4; ++k4) {
@@ -221,9 +231,13 @@ pv_f32_kernel(const float* __restrict__ p, PlaneView pv, const float* __restrict
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int kk = k4 * 4 + e;
-                const float4 b0 = *reinterpret_cast<const float4*>(bs + kk * BT + tx * 4);
-                const float4 b1 = *reinterpret_cast<const float4*>(bs + kk * BT + 32 + tx * 4);
-                const float2 bv[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
+                float2 bv[BN / 16];
+#pragma unroll
+                for (int h = 0; h < BN / 32; ++h) {
+                    const float4 b0 = *reinterpret_cast<const float4*>(bs + kk * BN + 32 * h + tx * 4);
+                    bv[2 * h] = make_float2(b0.x, b0.y);
+                    bv[2 * h + 1] = make_float2(b0.z, b0.w);
+                }
                 float a[8];
                 if (KIND == PV) {
 #pragma unroll
@@ -238,36 +252,41 @@ pv_f32_kernel(const float* __restrict__ p, PlaneView pv, const float* __restrict
                 for (int i = 0; i < 8; ++i) {
                     const float2 a2 = make_float2(a[i], a[i]);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = __ffma2_rn(a2, bv[j], acc[i][j]);
+                    for (int j = 0; j < BN / 16; ++j) acc[i][j] = __ffma2_rn(a2, bv[j], acc[i][j]);
                 }
             }
         }
     }
     // the groups' partial tiles through shared memory, added in group order
     __syncthreads();
-    float* part = smem + group * BT * BT;
+    float* part = smem + group * BT * BN;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < BN / 16; ++j) {
             const int r = KIND == PV ? ty + 8 * i : (i < 4 ? ty * 4 + i : 32 + ty * 4 + i - 4);
-            *reinterpret_cast<float2*>(part + r * BT + pair_col(tx, j)) = acc[i][j];
+            *reinterpret_cast<float2*>(part + r * BN + pair_col(tx, j)) = acc[i][j];
         }
     __syncthreads();
     float* op = o + bh * (long)S * D;
-    for (int e = threadIdx.x; e < BT * BT; e += THREADS) {
-        const int r = e / BT, d = d0 + e % BT;
+    for (int e = threadIdx.x; e < BT * BN; e += THREADS) {
+        const int r = e / BN, d = d0 + e % BN;
         if (q0 + r >= q_end || d >= D) continue;
-        op[(long)(q0 + r) * D + d] = (smem[e] + smem[BT * BT + e] + smem[2 * BT * BT + e] + smem[3 * BT * BT + e]) * scale;
+        op[(long)(q0 + r) * D + d] = (smem[e] + smem[BT * BN + e] + smem[2 * BT * BN + e] + smem[3 * BT * BN + e]) * scale;
     }
 }
 
 template <Kind KIND>
 int launch_pv(const float* p, PlaneView pview, const float* v, float* o, int B, int H, int S, int D, int causal, int row_begin, int row_end,
               float scale, cudaStream_t st) {
-    const int tiles_q = (row_end - row_begin + BT - 1) / BT, tiles_d = (D + BT - 1) / BT;
-    return launch_kernel<pv_f32_kernel<KIND>>("pv_f32_kernel", (unsigned)(B * H * tiles_q * tiles_d), THREADS, smem_bytes(KIND), st, p, pview, v,
-                                              o, B * H, S, D, causal, row_begin, row_end, tiles_d, scale);
+    int sms = 0;
+    if (int bad = sm_count(&sms)) return bad;
+    const int tiles_q = (row_end - row_begin + BT - 1) / BT, tiles_d = (D + BT - 1) / BT, fine_d = (D + 31) / 32;
+    if ((long)B * H * tiles_q * tiles_d < sms)                // a sum does not depend on the choice
+        return launch_kernel<pv_f32_kernel<KIND, 32>>("pv_f32_kernel", (unsigned)(B * H * tiles_q * fine_d), THREADS, smem_bytes(KIND, 32), st, p, pview, v,
+                                                      o, B * H, S, D, causal, row_begin, row_end, fine_d, scale);
+    return launch_kernel<pv_f32_kernel<KIND, BT>>("pv_f32_kernel", (unsigned)(B * H * tiles_q * tiles_d), THREADS, smem_bytes(KIND, BT), st, p, pview, v, o,
+                                                  B * H, S, D, causal, row_begin, row_end, tiles_d, scale);
 }
 
 }  // namespace
@@ -281,10 +300,19 @@ bool gemm_f32_supported(const void* a, const void* b, const void* c, PlaneView p
 
 int qk_f32_launch(const void* q, const void* k, void* s, PlaneView sv, int B, int H, int S, int D, float scale, int causal, int row_begin,
                   int row_end, cudaStream_t st) {
-    const int tiles_q = (row_end - row_begin + 2 * BT - 1) / (2 * BT), tiles_k = (S + 2 * BT - 1) / (2 * BT);
-    return launch_kernel<qk_f32_kernel>("qk_f32_kernel", dim3((unsigned)(B * H), (unsigned)(tiles_q * tiles_k)), THREADS, smem_bytes(QK), st,
-                                        static_cast<const float*>(q), static_cast<const float*>(k), static_cast<float*>(s), sv, S, D, scale, causal,
-                                        row_begin, row_end, tiles_k);
+    int sms = 0;
+    if (int bad = sm_count(&sms)) return bad;
+    const float *qf = static_cast<const float*>(q), *kf = static_cast<const float*>(k);
+    float* sf = static_cast<float*>(s);
+    const int edge = 2 * BT, tiles_q = (row_end - row_begin + edge - 1) / edge, tiles_k = (S + edge - 1) / edge;
+    // About half of the blocks lie above the diagonal.  A sum does not depend on the choice.
+    if ((long)B * H * tiles_q * tiles_k < (causal ? 2l : 1l) * sms) {
+        const int fine_q = (row_end - row_begin + BT - 1) / BT, fine_k = (S + BT - 1) / BT;
+        return launch_kernel<qk_f32_kernel<1>>("qk_f32_kernel", dim3((unsigned)(B * H), (unsigned)(fine_q * fine_k)), GTHREADS, smem_bytes(QK, BT) / GROUPS, st,
+                                               qf, kf, sf, sv, S, D, scale, causal, row_begin, row_end, fine_k);
+    }
+    return launch_kernel<qk_f32_kernel<GROUPS>>("qk_f32_kernel", dim3((unsigned)(B * H), (unsigned)(tiles_q * tiles_k)), THREADS, smem_bytes(QK, BT), st, qf, kf,
+                                                sf, sv, S, D, scale, causal, row_begin, row_end, tiles_k);
 }
 
 int pv_f32_launch(const void* p, PlaneView pview, const void* v, void* o, int B, int H, int S, int D, int causal, int row_begin, int row_end,
