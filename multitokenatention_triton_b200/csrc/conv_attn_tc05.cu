@@ -13,7 +13,9 @@
 //   epilogue   O / row sum -> 16-bit -> global memory, once per unit (conv_attention_triton.py:352-356)
 // Rounding: the scores are rounded to the 16-bit dtype as the reference's matmul does (conv_attention_pytorch.py:48)
 // and so are the exponentials that enter P.V; the conv output and the scaled logits, which the reference rounds
-// too (:57-64), stay in fp32 here.
+// too (:57-64), stay in fp32 here.  The row sum is of the rounded exponentials: 0.3 % less error against a float64 evaluation than the
+// sum of the unrounded ones with the tiles of 128 keys before (H8-64 S512-1024), which with tiles of 80 would have 0.4 % more, the first reference
+// maximum being over fewer keys.  It costs up to 2 % of the time.
 //
 // Warps: 0 Q and K loads, 1 and 2 the score and conv MMAs of the even and of the odd tiles, 3 V loads and P.V MMAs (all from one thread, so
 // the result is bit-reproducible), 4-7 drain, 8-15 softmax + epilogue (a pair of warps per 32 rows, 40 columns each).
@@ -21,7 +23,7 @@
 // buffers, two accumulators and O then fit: every hand-over has a tile of slack.  With 112 keys one of the two would be single.
 // Bound: the softmax warps (1540 of a tile's 1830 cycles at 6 x 11) and the tensor pipe (400 cycles of scores, 88 a row tap of conv, 320 of
 // P.V); long launches run at the power limit (1.5 GHz).  Before, with the conv's operand in shared memory and tiles of 123 x 128: B8 H16
-// S4096 6x11 back to back 1.39 -> 1.12 ms, B1 S4096 154 -> 120 us, B2 S1024 36 -> 31, B1 S2048 D64 11x15 67 -> 52.
+// S4096 6x11 back to back 1.39 -> 1.14 ms, B1 S4096 154 -> 120 us, B2 S1024 36 -> 31, B1 S2048 D64 11x15 67 -> 52.
 // Work units: groups of planes, so that K and V stay in L2; within a group heaviest first, dealt in rounds of alternating direction,
 // which balances the CTAs' tile counts.
 // 16-bit dtypes, D in {64, 128}, odd key extent <= 17, up to 16 row taps, causal; any S (TMA zero-fills rows past the end).
@@ -379,7 +381,6 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
 #pragma unroll
                 for (int e = 0; e < HALF / 2; ++e) {
                     const float p0 = ex2_approx(fmaf(x[2 * e], c2, mb)), p1 = ex2_approx(fmaf(x[2 * e + 1], c2, mb));
-                    l_part += p0 + p1;
                     pk[e] = pack2q<T>(p0, p1);
                 }
                 tmem_st_32x16(tacc + (uint32_t)(half * (HALF / 2)), *reinterpret_cast<const uint32_t(*)[16]>(&pk[0]));
@@ -388,6 +389,16 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_ready[b]);
+                // The sum is of the rounded exponentials, the weights that P.V uses: what rounding adds to a weight it then also adds to the
+                // divisor.  Taken while P.V runs.
+                float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+                for (int e = 0; e < HALF / 2; ++e) {
+                    const float2 p = unpack2q<T>(pk[e]);
+                    s0 += p.x;
+                    s1 += p.y;
+                }
+                l_part += s0 + s1;
             }
             // ---- the unit's rows are complete once its last P.V has finished ----
             // (a barrier of its own, awaited once a unit: of pv_done, whose phases these warps skip, the last tile's phase could be taken for

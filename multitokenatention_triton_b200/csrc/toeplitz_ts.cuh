@@ -43,6 +43,11 @@ template <> __device__ __forceinline__ uint32_t pack2q<__half>(float lo, float h
     __half2 r = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&r);
 }
+template <typename T> __device__ __forceinline__ float2 unpack2q(uint32_t v);
+template <> __device__ __forceinline__ float2 unpack2q<__nv_bfloat16>(uint32_t v) {
+    return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+template <> __device__ __forceinline__ float2 unpack2q<__half>(uint32_t v) { return __half22float2(*reinterpret_cast<__half2*>(&v)); }
 // Two products in T, each rounded once (the exact product of two 16-bit values fits in fp32, so this is what fp32 and a
 // conversion would give).
 template <typename T> __device__ __forceinline__ uint32_t mul2q(uint32_t a, uint32_t b);
