@@ -89,19 +89,6 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, i
     return false;
 }
 
-// Whole-warp wait for several barriers at once: every lane with `active` polls its own barrier, the warp goes on when all are through.
-// One after the other the waits of an MMA-issuing warp cost some 50 cycles each, with nothing left to wait for.
-__device__ __forceinline__ bool mbar_wait_lanes(uint64_t* bar, uint32_t parity, bool active, int* err_flag) {
-    bool ok = !active;
-    for (uint32_t i = 0; i < WAIT_LIMIT * 8u; ++i) {
-        if (!ok) ok = mbar_try_wait(bar, parity);
-        if (__all_sync(0xffffffffu, ok)) return true;
-        if ((i & 8191u) == 8191u && __any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(err_flag) != 0)) return false;
-    }
-    if (!ok) raise_wait_flag(err_flag);
-    return false;
-}
-
 // The flag is looked at twice.  gave_up_before(): at a kernel's start, by the whole block; when it is up the block returns at once -
 // but not before its predecessors are complete, or its successors would overtake them.
 __device__ __forceinline__ bool gave_up_before(int* err_flag, int* slot) {
@@ -147,13 +134,6 @@ __device__ __forceinline__ uint64_t l2_policy_evict_last() {
     return pol;
 }
 
-// Plain (untiled) bulk copy global -> shared that completes on `bar`; both addresses 16-byte aligned, bytes % 16 == 0.
-__device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
 // 3-D tiled store of a shared-memory box; completion is tracked by the thread's bulk async-group.
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* src, int x, int y, int z) {
     asm volatile(
@@ -198,17 +178,6 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t lbo
     d |= (uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32;
     d |= (uint64_t)1 << 46;      // descriptor version for sm_100
     d |= (uint64_t)2 << 61;      // SWIZZLE_128B
-    return d;
-}
-
-// The same for the 32-byte swizzle: K-major rows of 32 bytes (16 elements), sbo = bytes between 8-row groups (256).
-__device__ __forceinline__ uint64_t smem_desc_sw32(uint32_t saddr, uint32_t sbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3ffffu) >> 4);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)6 << 61;      // SWIZZLE_32B
     return d;
 }
 

@@ -5,7 +5,7 @@
 
   conv2d       causal depthwise conv 6x11 on a (B=4, H=16, S=2048, S) bf16 score plane
   head_linear  16x16 head mix on post-softmax probabilities of the same shape
-  graph        the whole forward (five launches) at --batch/--heads/--seq/--dim, launched call by call and replayed
+  graph        the whole forward at --batch/--heads/--seq/--dim, launched call by call and replayed
                from a CUDA graph: what stream capture saves where the forward is launch-bound (not part of "all")
   train        the module's forward and backward, both convs with --taps (not part of "all")
   write        what memory takes when it is only written: torch's fill of a plane of the shape (not part of "all")
