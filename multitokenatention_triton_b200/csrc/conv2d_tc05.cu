@@ -43,10 +43,16 @@ struct ConvGeom : TileGeom {
     long zero_per_plane, zero_total;     // tiles wholly above the diagonal that must be written as zero (write_upper)
 };
 
-// Zero tiles to the right of row of tiles tm.
+// Zero tiles to the right of row of tiles tm.  The first begins where the compute tiles end, the others at multiples of ZERO_COLS, so that they
+// store whole lines; what the first two have in common is stored twice.
 __host__ __device__ __forceinline__ int zero_tiles(const ConvGeom& g, int tm) {
-    const int left = g.W - key_tiles(g, tm) * TN;
-    return left > 0 ? (left + ZERO_COLS - 1) / ZERO_COLS : 0;
+    const int c0 = key_tiles(g, tm) * TN;
+    return c0 < g.W ? (g.W + ZERO_COLS - 1) / ZERO_COLS - c0 / ZERO_COLS : 0;
+}
+
+__device__ __forceinline__ int zero_tile_col(const ConvGeom& g, int tm, int tn) {
+    const int c0 = key_tiles(g, tm) * TN;
+    return tn == 0 ? c0 : (c0 / ZERO_COLS + tn) * ZERO_COLS;
 }
 
 template <typename T>
@@ -146,7 +152,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
                 // the producer always reaches its last tile, and giving up early only changes the pacing)
                 const int due = (int)((long)zi * my_tiles / my_zero);
                 for (int spin = 0; *reinterpret_cast<volatile int*>(&tiles_loaded) < due && spin < (1 << 20); ++spin) __nanosleep(256);
-                tma_store_3d(&mz, zero_box, key_tiles(g, ztm) * TN + ztn * ZERO_COLS, g.row_begin + ztm * g.tmo - g.y_row0, zp);
+                tma_store_3d(&mz, zero_box, zero_tile_col(g, ztm, ztn), g.row_begin + ztm * g.tmo - g.y_row0, zp);
                 bulk_commit();
                 bulk_wait_read_1();
                 if (++ztn == nz && zi + 1 < my_zero) {
@@ -270,9 +276,10 @@ size_t conv2d_tc05_smem_bytes(int R, bool split_w, bool zeros, int nstage) {
 }
 
 // Of one group's tiles a CTA gets this many or more.  The fewer planes are in work at a time, the more of the rows that neighbouring tiles
-// share come from L2 (B4 H16 S2048 with zeros, forward and input gradient together: 353 us with 32 tiles, 345 with 8), but a CTA changes
-// its head with every group.
-constexpr int GROUP_TILES = 8;
+// share come from L2, but a CTA changes its head with every group.  With the zeros above the diagonal to be stored, HBM is the bound: forward and
+// gradients of B4 H16 S2048 take 513 us with 2, 521 with 8.  Without, the head changes show: 158 against 153 us (forward B1 H16 S2048 with two 7x7
+// convs), 674 against 650 (training step B4 H16 S1024).
+constexpr int GROUP_TILES = 8, GROUP_TILES_ZEROS = 2;
 
 template <typename T>
 int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, int w_dtype, void* y, PlaneView yv,
@@ -282,9 +289,9 @@ int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, 
     if ((rc = sm_count(&sms))) return rc;
     ConvGeom g{};
     set_tiles(g, planes, C, W, R, causal, row_begin, row_end);
-    set_groups(g, (long)g.tiles_per_plane * planes / ((long)GROUP_TILES * sms));
-    g.W = W; g.R = R; g.S = S; g.x_row0 = xv.row0; g.y_row0 = yv.row0;
     g.write_upper = causal && write_upper ? 1 : 0;
+    set_groups(g, (long)g.tiles_per_plane * planes / ((long)(g.write_upper ? GROUP_TILES_ZEROS : GROUP_TILES) * sms));
+    g.W = W; g.R = R; g.S = S; g.x_row0 = xv.row0; g.y_row0 = yv.row0;
     g.split_w = w_dtype == MTA_F32 ? 1 : 0;
     g.lead = grad_input ? 0 : R - 1;
     g.flip = grad_input ? 1 : 0;
