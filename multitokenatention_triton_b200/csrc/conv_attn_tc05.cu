@@ -13,9 +13,7 @@
 //   epilogue   O / row sum -> 16-bit -> global memory, once per unit (conv_attention_triton.py:352-356)
 // Rounding: the scores are rounded to the 16-bit dtype as the reference's matmul does (conv_attention_pytorch.py:48)
 // and so are the exponentials that enter P.V; the conv output and the scaled logits, which the reference rounds
-// too (:57-64), stay in fp32 here.  The row sum is of the rounded exponentials: 0.3 % less error against a float64 evaluation than the
-// sum of the unrounded ones with the tiles of 128 keys before (H8-64 S512-1024), which with tiles of 80 would have 0.4 % more, the first reference
-// maximum being over fewer keys.  It costs up to 2 % of the time.
+// too (:57-64), stay in fp32 here, and so do the exponentials that the row sum adds.
 //
 // Warps: 0 Q and K loads, 1 and 2 the score and conv MMAs of the even and of the odd tiles, 3 V loads and P.V MMAs (all from one thread, so
 // the result is bit-reproducible), 4-7 drain, 8-15 softmax + epilogue (a pair of warps per 32 rows, 40 columns each).
@@ -380,8 +378,9 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 uint32_t pk[HALF / 2];                       // this thread's 40 exponentials, two per column
 #pragma unroll
                 for (int e = 0; e < HALF / 2; ++e) {
-                    const float p0 = ex2_approx(fmaf(x[2 * e], c2, mb)), p1 = ex2_approx(fmaf(x[2 * e + 1], c2, mb));
-                    pk[e] = pack2q<T>(p0, p1);
+                    x[2 * e] = ex2_approx(fmaf(x[2 * e], c2, mb));
+                    x[2 * e + 1] = ex2_approx(fmaf(x[2 * e + 1], c2, mb));
+                    pk[e] = pack2q<T>(x[2 * e], x[2 * e + 1]);
                 }
                 tmem_st_32x16(tacc + (uint32_t)(half * (HALF / 2)), *reinterpret_cast<const uint32_t(*)[16]>(&pk[0]));
                 tmem_st_32x4(tacc + (uint32_t)(half * (HALF / 2) + 16), *reinterpret_cast<const uint32_t(*)[4]>(&pk[16]));
@@ -389,14 +388,11 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_ready[b]);
-                // The sum is of the rounded exponentials, the weights that P.V uses: what rounding adds to a weight it then also adds to the
-                // divisor.  Taken while P.V runs.
-                float s0 = 0.0f, s1 = 0.0f;
+                float s0 = 0.0f, s1 = 0.0f;                  // of the exponentials before rounding; taken while P.V runs
 #pragma unroll
                 for (int e = 0; e < HALF / 2; ++e) {
-                    const float2 p = unpack2q<T>(pk[e]);
-                    s0 += p.x;
-                    s1 += p.y;
+                    s0 += x[2 * e];
+                    s1 += x[2 * e + 1];
                 }
                 l_part += s0 + s1;
             }
