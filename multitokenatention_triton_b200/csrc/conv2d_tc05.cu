@@ -6,10 +6,11 @@
 // staged tile is the MMA's A operand in tensor memory, where the shift costs nothing (toeplitz_ts.cuh).
 //
 // Persistent, warp-specialised kernel; per output tile (4 (33 - R) rows x 112 keys; only tiles that touch keys <= query when causal):
-//   warp 0      TMA producer: two boxes of 64 columns (128-byte swizzle) of each of the four groups of 32 rows, a ring of tiles
+//   warp 0      TMA producer: two boxes of 64 columns (128-byte swizzle) of the tile's 4 (33 - R) + R - 1 rows, a ring of tiles
 //               (out-of-range rows / columns arrive as zero = the conv's zero padding)
-//   warps 4-11  shared memory -> registers -> tensor memory, one row and 64 columns a thread, keys above the causal diagonal replaced by
-//               zeros on the way; the Toeplitz slices when the head changes
+//   warps 4-11  shared memory -> registers -> tensor memory, one row and 64 columns a thread (the four groups of 32 rows share R - 1
+//               rows with the next, which are read twice here and not loaded twice), keys above the causal diagonal replaced by zeros
+//               on the way; the Toeplitz slices when the head changes
 //   warps 1, 2  the MMAs of the even and of the odd tiles, each with an accumulator and two A buffers
 //   warps 12-15 epilogue: accumulator -> 16-bit -> staging tiles -> TMA stores
 //   warp 3      stores zero tiles above the diagonal when the whole output is wanted
@@ -26,7 +27,9 @@ namespace {
 using namespace tc05;
 using namespace qc;
 
-constexpr int STAGE_BYTES = 2 * BOX_BYTES;        // a tile: two boxes of 64 columns x 128 rows
+constexpr int STAGE_BYTES = 2 * BOX_BYTES;        // a tile: two boxes of 64 columns x up to 128 rows
+// Rows of input that a tile's output rows reach.
+__host__ __device__ constexpr int staged_rows(int R) { return 4 * (33 - R) + R - 1; }
 constexpr int MAX_STAGES = 4;
 constexpr int ABUFS = 4;                          // A operands in tensor memory; buffer b in columns 128 (b / 2) + 32 (b % 2) .. + 31 and 64 more on
 constexpr uint32_t C_COL = 256;                   // accumulators
@@ -119,13 +122,10 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
             for (int n = 0; n < my_tiles; ++n, it.next(g)) {
                 mbar_wait_spin(&empty_bar[st], (use & 1) ^ 1, err_flag);
                 uint8_t* xa = stage_base + st * STAGE_BYTES;
-                mbar_expect_tx(&full_bar[st], (uint32_t)STAGE_BYTES);
-#pragma unroll 1
-                for (int gq = 0; gq < 4; ++gq)
+                mbar_expect_tx(&full_bar[st], (uint32_t)(2 * staged_rows(R) * 128));
 #pragma unroll
-                    for (int j = 0; j < 2; ++j)
-                        tma_load_3d(xa + j * BOX_BYTES + gq * QBOX_BYTES, &mx, &full_bar[st], it.n0() - 8 + 64 * j, it.m0(g) - g.lead - g.x_row0 + gq * gr,
-                                    it.plane);
+                for (int j = 0; j < 2; ++j)
+                    tma_load_3d(xa + j * BOX_BYTES, &mx, &full_bar[st], it.n0() - 8 + 64 * j, it.m0(g) - g.lead - g.x_row0, it.plane);
                 *reinterpret_cast<volatile int*>(&tiles_loaded) = n + 1;
                 if (++st == g.nstage) { st = 0; ++use; }
             }
@@ -183,7 +183,7 @@ conv2d_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant
     } else if (warp < 12) {
         // ---------------- staged tile -> tensor memory; Toeplitz slices ----------------
         const int quarter = warp & 3, half = warp >= 8 ? 1 : 0;
-        const int sr = quarter * 32 + lane;                  // staged row = TMEM lane of this thread
+        const int sr = quarter * gr + lane;                  // staged row that becomes TMEM lane 32 quarter + lane
         const int row = quarter * gr + lane - g.lead;        // its row relative to the tile's first output row
         const int ft = tid - 128;                            // 0..127 in the warps that build the slices
         if (half == 0) clear_taps(wsm, ft, 2);
@@ -301,7 +301,7 @@ int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, 
     g.zero_total = g.zero_per_plane * planes;
     CUtensorMap mx, my, mz;
     if ((rc = make_tensor_map_3d(&mx, x, (uint64_t)planes, (uint64_t)x_rows_stored, (uint64_t)W, (uint64_t)xv.width,
-                                 (uint64_t)xv.plane_stride, 64, 32, true)))
+                                 (uint64_t)xv.plane_stride, 64, (uint32_t)staged_rows(R), true)))
         return rc;
     // rows past row_end are outside these maps, so a tile's store never touches them
     if ((rc = make_tensor_map_3d(&my, y, (uint64_t)planes, (uint64_t)(row_end - yv.row0), (uint64_t)W, (uint64_t)yv.width,
