@@ -112,10 +112,8 @@ int run_forward(const void* q, const void* k, const void* v, const void* w1, con
     // B1 S512 18 / 25, B4 S1024 49 / 66, B1 S4096 139 / 215; H8 B1 S1024 18 / 26; H32 B1 S512 27 / 37, B1 S2048 100 / 113; H64 B1 S256
     // 26 / 35, B1 S1024 83 / 82, B4 S1024 249 / 240, B1 S4096 800 / 903 (two heads' rows of a group are two thirds of what it reads).
     // 2 x 3 gains more everywhere.  3 x 5 was level with two kernels (B4 H16 S2048 212 / 215) and 3 x 7 and more cost FMAs in proportion.
-    // Two forms keep the two kernels because of what is promised for them, not for speed: 8 heads up to 128 keys (the number of launches)
-    // and 16 heads of 64 (bit for bit the head mix kernel that head_linear_launch picks by the row).
     const void* weights = bufA;
-    const bool one = variant("fused") != 1 && variant("conv2d") == 0 && variant("head_linear") == 0 && (H > 8 || S > 128) && (H != 16 || D != 64) &&
+    const bool one = variant("fused") != 1 && variant("conv2d") == 0 && variant("head_linear") == 0 &&
                      conv_mix_supported(bufA, pv, bufB, pv, H, cq2, ck2, causal, dtype, w_dtype);
     if (one) {
         if ((rc = trace_mark("conv2+head_mix2", st))) return rc;

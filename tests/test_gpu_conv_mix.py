@@ -54,3 +54,14 @@ def test_against_the_two_kernels(B, H, S, dtype):
         _lib.set_variant("fused", 0)
     _lib.device_status()
     assert rel_fro(npf(one), npf(two)) <= (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12)
+
+
+@pytest.mark.parametrize("H,S,D", [(8, 64, 64), (8, 128, 128), (16, 128, 64), (16, 1024, 64), (16, 128, 128)])
+def test_the_choice_does_not_depend_on_the_head_dimension(H, S, D):
+    args = [t.to(DEV) for t in _inputs(1, H, S, D, 3, 3, torch.bfloat16, S + D)]
+    _lib.set_stage_trace(True)
+    try:
+        ops.mta_fused_fwd(*args)
+        assert [n for n, _ in _lib.stage_times_ms()][-2:] == ["conv2+head_mix2", "pv"]
+    finally:
+        _lib.set_stage_trace(False)

@@ -130,10 +130,11 @@ def test_stand_alone_ops_without_room_for_copies(monkeypatch):
 
 @pytest.mark.parametrize("S,variant", [(960, 2), (961, 3), (1021, 3), (1024, 3), (2048, 3), (2049, 2)])
 def test_lengths_of_one_padded_row_take_one_head_mix(S, variant):
-    """The second head mix of 16 heads is chosen by the padded row: bit for bit what the kernel of that row gives, not the other's."""
+    """The second head mix of 16 heads, where it is a kernel of its own (the second conv is not small), is chosen by the padded row: bit for bit
+    what the kernel of that row gives, not the other's."""
     g = torch.Generator(device=DEV).manual_seed(S)
     q, k, v = (torch.randn(1, 16, S, 64, device=DEV, generator=g).to(torch.bfloat16) for _ in range(3))
-    w = torch.randn(16, 3, 3, device=DEV, generator=g).to(torch.bfloat16)
+    w = torch.randn(16, 3, 5, device=DEV, generator=g).to(torch.bfloat16)
     mix = torch.randn(16, 16, device=DEV, generator=g).to(torch.bfloat16)
     out = {}
     for n in (0, 2, 3):
