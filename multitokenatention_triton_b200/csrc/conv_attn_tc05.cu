@@ -3,7 +3,7 @@
 // scratch.  Per work unit = (plane, block of 4 (33 - R) query rows) the CTA walks tiles of 80 keys, 0 .. diagonal:
 //   scores     S[128 x 96] = Q . K[keys n0-8 .. n0+87]^T on tcgen05 into score buffer n % 2 in tensor memory (TMEM); the 128 lanes are
 //              four groups of 32 rows, R - 1 of each shared with the next group (toeplitz_ts.cuh)
-//   drain      round(round(S) * score_scale), 0 above the diagonal, in place
+//   drain      round(S), 0 above the diagonal, in place
 //   conv       the MMAs of toeplitz_ts.cuh, A from the score buffer, into accumulator n % 2 (128 x 80 fp32)
 //   softmax    TMEM -> y = conv * scale * log2 e in fp32, -inf above the diagonal -> running (reference max, sum) per
 //              query row, P = 2^(y - m) in the 16-bit dtype -> back into the accumulator's own columns.  The output
@@ -51,8 +51,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 
 struct CaGeom {
-    int C, S, R, KS, row_begin, row_end, tiles_m, tmo, split_w, planes, group_planes, nq;
-    float score_scale, sm_scale;
+    int C, S, R, KS, row_begin, row_end, tiles_m, tmo, split_w, planes, group_planes;
+    float sm_scale;
     long units;
 };
 
@@ -97,7 +97,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     const int R = g.R, KS = g.KS;
     const int tb_bytes = toeplitz_bytes(R, g.split_w);
     uint8_t* q_base = smem;
-    uint8_t* k_base = q_base + g.nq * Q_BYTES;
+    uint8_t* k_base = q_base + 2 * Q_BYTES;
     uint8_t* v_base = k_base + 2 * K_BYTES;
     uint8_t* tb_base = v_base + 2 * V_BYTES;       // two sets of Toeplitz slices: units alternate between them
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
@@ -141,16 +141,16 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     if (warp == 0) {
         // ---------------- Q and K loads ----------------
         if (lane == 0) {
-            int n = 0, qs = 0, qu = 0;
-            for (bool more = un_it.first(g); more; more = un_it.next(g)) {
-                mbar_wait_spin(&q_free[qs], (qu & 1) ^ 1, err_flag);
+            int n = 0, un = 0;
+            for (bool more = un_it.first(g); more; more = un_it.next(g), ++un) {
+                const int qs = un & 1;
+                mbar_wait_spin(&q_free[qs], ((un >> 1) & 1) ^ 1, err_flag);
                 mbar_expect_tx(&q_full[qs], (uint32_t)Q_BYTES);
 #pragma unroll
                 for (int j = 0; j < DBOX; ++j)
 #pragma unroll 1
                     for (int gq = 0; gq < 4; ++gq)
                         tma_load_3d(q_base + qs * Q_BYTES + j * BOX_BYTES + gq * QBOX_BYTES, &mq, &q_full[qs], 64 * j, un_it.m0 - lead + gq * gr, un_it.plane);
-                if (++qs == g.nq) { qs = 0; ++qu; }
                 for (int tn = 0; tn < un_it.nk; ++tn, ++n) {
                     const int b = n & 1;
                     mbar_wait_spin(&k_free[b], ((n >> 1) & 1) ^ 1, err_flag);
@@ -167,12 +167,13 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
         const int b = warp - 1;
         const uint32_t t_s = tmem + (uint32_t)(b * CS), t_c = tmem + C_COL + (uint32_t)(b * CK), tb_addr = smem_u32(tb_base);
         const uint64_t k0 = smem_desc_sw128(smem_u32(k_base + b * K_BYTES), 16, 1024);
-        int n = 0, un = 0, qs = 0, qu = 0;
+        int n = 0, un = 0;
         uint32_t phase = 0;
         for (bool more = un_it.first(g); more; more = un_it.next(g), ++un) {
             const int nk = uniform(un_it.nk);
             const uint64_t db = desc_plain(tb_addr + (uint32_t)((un & 1) * tb_bytes), 512, 128);
-            mbar_wait_spin(&q_full[qs], qu & 1, err_flag);
+            const int qs = un & 1;
+            mbar_wait_spin(&q_full[qs], (un >> 1) & 1, err_flag);
             const uint64_t q0 = smem_desc_sw128(smem_u32(q_base + qs * Q_BYTES), 16, 1024);
             const int first = (n & 1) == b ? 0 : 1;               // this warp's first tile of the unit
             if (first >= nk && lane == 0) mbar_arrive(&q_free[qs]);
@@ -195,7 +196,6 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 mma_commit(&acc_full[b], el);
             }
             n += nk;
-            if (++qs == g.nq) { qs = 0; ++qu; }
         }
     } else if (warp == 3) {
         // ---------------- V loads (a tile ahead) and P.V MMAs: O[128 x D] (+)= P[128 x 80] V[80 x D] ----------------
@@ -241,12 +241,10 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
             }
         }
     } else if (warp < 8) {
-        // ---------------- drain: fp32 scores -> rounded, scaled, masked, in place; Toeplitz slices ----------------
+        // ---------------- drain: fp32 scores -> rounded, masked, in place; Toeplitz slices ----------------
         const int quarter = warp & 3;
         const int row = quarter * gr + lane - lead;          // staged row of this thread's lane, relative to the unit's first output row
         const int ft = tid - 128;                            // 0..127
-        const uint32_t sc = pack2q<T>(g.score_scale, g.score_scale);
-        const bool scaled = g.score_scale != 1.0f;           // raw scores (the conv attention) are rounded once
         int n = 0, un = 0;
         // The weights of a unit's head are fetched one unit ahead (successive units of a CTA belong to different planes,
         // so every unit rebuilds its slices): the global loads are in flight while the previous unit's tiles are drained.
@@ -279,10 +277,6 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                     tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < 24; ++i) pk[i] = pack2q<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-                    if (scaled) {
-#pragma unroll
-                        for (int i = 0; i < 24; ++i) pk[i] = mul2q<T>(pk[i], sc);
-                    }
                     if (diag) {
                         const int nl = live - h * 48;
 #pragma unroll
@@ -435,17 +429,17 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
 
 constexpr size_t CA_SMEM_LIMIT = 220 * 1024;     // what the static arrays leave
 
-size_t conv_attn_smem_bytes(int D, int R, bool split_w, int nq) {
-    return 1024 + (size_t)(D / 64) * (nq * BOX_BYTES + 2 * (CA_KBOX + CA_VBOX)) + 2 * (size_t)toeplitz_bytes(R, split_w ? 1 : 0);
+size_t conv_attn_smem_bytes(int D, int R, bool split_w) {
+    return 1024 + 2 * (size_t)(D / 64) * (BOX_BYTES + CA_KBOX + CA_VBOX) + 2 * (size_t)toeplitz_bytes(R, split_w ? 1 : 0);
 }
 
 template <typename T, int D>
 int launch_ca(const void* q, const void* k, const void* v, const void* w, int w_dtype, void* o, int B, int H, int S, int R, int KS,
-              float score_scale, float sm_scale, int row_begin, int row_end, cudaStream_t st) {
+              float sm_scale, int row_begin, int row_end, cudaStream_t st) {
     const long planes = (long)B * H;
     CaGeom g{};
     g.C = H; g.S = S; g.R = R; g.KS = KS; g.row_begin = row_begin; g.row_end = row_end;
-    g.score_scale = score_scale; g.sm_scale = sm_scale;
+    g.sm_scale = sm_scale;
     g.tmo = tile_rows(R);
     g.tiles_m = (row_end - row_begin + g.tmo - 1) / g.tmo;
     g.split_w = w_dtype == MTA_F32 ? 1 : 0;
@@ -463,8 +457,7 @@ int launch_ca(const void* q, const void* k, const void* v, const void* w, int w_
     int sms = 0;
     if (int bad = sm_count(&sms)) return bad;
     const unsigned grid = (unsigned)std::min<long>(g.units, sms);
-    g.nq = conv_attn_smem_bytes(D, R, g.split_w != 0, 2) <= CA_SMEM_LIMIT ? 2 : 1;
-    return launch_kernel<conv_attn_tc05_kernel<T, D>>("conv_attn_tc05_kernel", grid, CA_THREADS, conv_attn_smem_bytes(D, R, g.split_w != 0, g.nq), st, mq, mk,
+    return launch_kernel<conv_attn_tc05_kernel<T, D>>("conv_attn_tc05_kernel", grid, CA_THREADS, conv_attn_smem_bytes(D, R, g.split_w != 0), st, mq, mk,
                                                       mv, static_cast<T*>(o), w, w_dtype, g, flag);
 }
 
@@ -472,7 +465,7 @@ int launch_ca(const void* q, const void* k, const void* v, const void* w, int w_
 
 bool conv_attn_fused_shape_ok(int S, int D, int R, int KS, int causal, int dtype, int w_dtype) {
     return causal && dtype != MTA_F32 && (D == 64 || D == 128) && S >= 1 && KS % 2 == 1 && KS <= 17 && R >= 1 && R <= 16 &&
-           conv_attn_smem_bytes(D, R, w_dtype == MTA_F32, 1) <= CA_SMEM_LIMIT;
+           conv_attn_smem_bytes(D, R, w_dtype == MTA_F32) <= CA_SMEM_LIMIT;
 }
 
 bool conv_attn_fused_supported(const void* q, const void* k, const void* v, const void* o, int S, int D, int R, int KS, int causal,
@@ -481,9 +474,9 @@ bool conv_attn_fused_supported(const void* q, const void* k, const void* v, cons
 }
 
 int conv_attn_fused_launch(const void* q, const void* k, const void* v, const void* w, int w_dtype, void* o, int B, int H, int S, int D,
-                           int R, int KS, float score_scale, float sm_scale, int row_begin, int row_end, int dtype, cudaStream_t st) {
+                           int R, int KS, float sm_scale, int row_begin, int row_end, int dtype, cudaStream_t st) {
     if ((long)B * H == 0 || row_end <= row_begin) return MTA_OK;
-#define MTA_CA(TT, DD) return launch_ca<TT, DD>(q, k, v, w, w_dtype, o, B, H, S, R, KS, score_scale, sm_scale, row_begin, row_end, st)
+#define MTA_CA(TT, DD) return launch_ca<TT, DD>(q, k, v, w, w_dtype, o, B, H, S, R, KS, sm_scale, row_begin, row_end, st)
     if (dtype == MTA_BF16) { if (D == 64) MTA_CA(__nv_bfloat16, 64); MTA_CA(__nv_bfloat16, 128); }
     if (D == 64) MTA_CA(__half, 64);
     MTA_CA(__half, 128);

@@ -272,8 +272,8 @@ int mta_conv_attn_fwd(const void* q, const void* k, const void* v, const void* w
     if (conv_attn_one_kernel(S, D, cq, ck, causal, dtype, w_dtype)) {
         MTA_REQUIRE(conv_attn_fused_supported(q, k, v, o, S, D, cq, ck, causal, dtype, w_dtype),
                     "conv_attn_fwd: q, k, v and o must be 16-byte aligned");
-        // raw scores into the conv (score scale 1), the softmax scale after it, as the reference orders them
-        return conv_attn_fused_launch(q, k, v, w, w_dtype, o, B, H, S, D, cq, ck, 1.0f, scale, 0, S, dtype, st);
+        // raw scores into the conv, the softmax scale after it, as the reference orders them
+        return conv_attn_fused_launch(q, k, v, w, w_dtype, o, B, H, S, D, cq, ck, scale, 0, S, dtype, st);
     }
     const Plan pl = fit_plan(B, H, S, cq, 1, 0, S, dtype, workspace_bytes);
     MTA_REQUIRE(workspace && workspace_bytes >= pl.total(), "conv_attn_fwd: workspace of %zu bytes is smaller than the %zu needed",

@@ -177,7 +177,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
             mbar_wait_spin(&s_full[b], (n >> 1) & 1, err_flag);
             __syncwarp();
             fence_after_sync();
-            drain_half<T, true>(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * SN + 64 * half), sc, m0 + row - kbase + 1, kbase + 63 > m0 - lead);
+            drain_half<T>(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * SN + 64 * half), sc, m0 + row - kbase + 1, kbase + 63 > m0 - lead);
             fence_before_sync();
             fence_proxy_async();          // the slices, written through the generic proxy, must be visible to the MMAs (async proxy)
             __syncwarp();

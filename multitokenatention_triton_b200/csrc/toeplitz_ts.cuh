@@ -1,6 +1,6 @@
 // Pieces shared by the kernels that run the conv as Toeplitz MMAs with its input in tensor memory (TMEM): conv2d_tc05.cu, and with the
-// scores Q K^T computed on the spot qk_conv_tc05.cu and conv_attn_tc05.cu.  Tile geometry, the drain that turns the fp32 scores into the 16-bit operand in place, the
-// conv MMA schedule and the Toeplitz slices.
+// scores Q K^T computed on the spot qk_conv_tc05.cu and conv_attn_tc05.cu.  Tile geometry, the drain of the score
+// + conv kernel (the conv attention, whose tiles are narrower, has its own), the conv MMA schedule and the Toeplitz slices.
 //
 // The score tile never leaves TMEM.  S[128 x 128] comes out of the score MMAs as fp32, the drain warps round it to 16 bits in place
 // (64 columns of fp32 become 32 of the same columns), and the conv's MMAs read it there as their A operand.  A row tap is the A operand moved up by one
@@ -43,11 +43,6 @@ template <> __device__ __forceinline__ uint32_t pack2q<__half>(float lo, float h
     __half2 r = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&r);
 }
-template <typename T> __device__ __forceinline__ float2 unpack2q(uint32_t v);
-template <> __device__ __forceinline__ float2 unpack2q<__nv_bfloat16>(uint32_t v) {
-    return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
-}
-template <> __device__ __forceinline__ float2 unpack2q<__half>(uint32_t v) { return __half22float2(*reinterpret_cast<__half2*>(&v)); }
 // Two products in T, each rounded once (the exact product of two 16-bit values fits in fp32, so this is what fp32 and a
 // conversion would give).
 template <typename T> __device__ __forceinline__ uint32_t mul2q(uint32_t a, uint32_t b);
@@ -179,11 +174,11 @@ __device__ __forceinline__ void build_from_taps(uint8_t* tb, float* wsm, const f
     named_barrier(bar_id, 128);             // nobody refills wsm while another warp still reads it
 }
 
-// One thread's share of the drain: 64 of its lane's fp32 scores, at `tcol`, become 16-bit values, two per column, in the first 32 of the
-// same columns.  SCALED: round(round(S) * scale), the reference's 16-bit matmul followed by its 16-bit multiply (`sc2`: the scale
-// twice); otherwise round(S).  `live`: how many of the columns lie on or below the diagonal, the others become 0; `diag`
+// One thread's share of the score + conv kernel's drain: 64 of its lane's fp32 scores, at `tcol`, become 16-bit values, two per column, in the
+// first 32 of the same columns: round(round(S) * scale), the reference's 16-bit matmul followed by its 16-bit multiply (`sc2`: the scale
+// twice).  `live`: how many of the columns lie on or below the diagonal, the others become 0; `diag`
 // (warp-uniform): some lane has fewer than 64.  Whole-warp call; the stores are complete when it returns.
-template <typename T, bool SCALED>
+template <typename T>
 __device__ __forceinline__ void drain_half(uint32_t tcol, uint32_t sc2, int live, bool diag) {
     uint32_t r[64], pk[32];
     tmem_ld_32x32(tcol, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
@@ -191,8 +186,7 @@ __device__ __forceinline__ void drain_half(uint32_t tcol, uint32_t sc2, int live
     tmem_ld_wait();
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-        pk[i] = pack2q<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-        if (SCALED) pk[i] = mul2q<T>(pk[i], sc2);
+        pk[i] = mul2q<T>(pack2q<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), sc2);
     }
     if (diag) {
 #pragma unroll
