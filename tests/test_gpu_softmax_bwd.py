@@ -40,3 +40,40 @@ def test_rows(S, dtype):
         assert float((got - want).norm() / want.norm()) <= tol
     got, want = ins[0].grad[:, :, -8:].double(), ref_in[0].grad[:, :, -8:]
     assert float((got - want).norm() / want.norm()) <= 2 * tol
+
+
+@pytest.mark.parametrize("S,dtype", [(31, torch.bfloat16), (256, torch.bfloat16), (257, torch.float16), (519, torch.bfloat16), (1024, torch.bfloat16),
+                                     (1033, torch.float16), (2056, torch.bfloat16), (128, torch.float32), (135, torch.float32),
+                                     (513, torch.float32), (1024, torch.float32), (1029, torch.float32)])
+def test_every_chunk_counts_once(S, dtype):
+    """Entry by entry.  Queries of 0 make a row's probabilities 1 / n; the convs and mixes are identities; the values of a head are 0 but for eight
+    neighbouring keys, which alone make up the row's dot product; keys with a single 1 hand the gradient of 64 scores to one entry of dq each."""
+    H, D, G = 8, 64, 1024.0
+    g = torch.Generator(device=DEV).manual_seed(S)
+    first = [min(max(k, 0), S - 8) for k in (0, 124, 248, 256, S // 2 // 8 * 8, (S - 1) // 8 * 8, S - 16, S - 8)]
+    q, k, v = (torch.zeros(1, H, S, D, device=DEV, dtype=dtype) for _ in range(3))
+    seen = torch.zeros(H, D, dtype=torch.long, device=DEV)
+    for h, f in enumerate(first):
+        v[0, h, f:f + 8, 0] = (1 + torch.rand(8, device=DEV, generator=g)).to(dtype)
+        at = torch.cat([torch.arange(f, f + 8, device=DEV), torch.randperm(S, device=DEV, generator=g)[:D - 8]])
+        seen[h, :len(at)] = at
+        for j, key in enumerate(at.tolist()):
+            k[0, h, key, j] = 1.0
+    up = torch.zeros(1, S, H, D, device=DEV, dtype=dtype)
+    up[..., 0] = G
+    ins = [t.requires_grad_() for t in (q, k, v)]
+    w, mix = torch.ones(H, 1, 1, device=DEV, dtype=dtype), torch.eye(H, device=DEV, dtype=dtype)
+    MTAFunction.apply(*ins, w, mix, w, mix).transpose(1, 2).backward(up)
+    _lib.device_status()
+    n = torch.arange(1, S + 1, device=DEV, dtype=torch.float64)[None, :, None]
+    below = torch.ones(S, S, dtype=torch.bool, device=DEV).tril()
+    dp = (G * v[0, :, :, 0].detach().double())[:, None, :] * below                      # [head, query, key]
+    dot = dp.sum(-1, keepdim=True) / n
+    pick = seen[:, None, :].expand(H, S, D)
+    live = below.expand(H, S, S).gather(2, pick)
+    filled = torch.arange(D, device=DEV) < min(D, 8 + S)
+    want = ((dp.gather(2, pick) - dot) / n * live * filled) * D ** -0.5
+    # p (twice: in the dot and in front), the result and dq are rounded once each; the exponential, its sum and the dot in float32
+    u = {torch.float32: 2.0 ** -24, torch.float16: 2.0 ** -12, torch.bfloat16: 2.0 ** -9}[dtype]
+    bound = (5 * u + 2.0 ** -18) * (dp.gather(2, pick) + dot) / n * D ** -0.5
+    assert bool(((ins[0].grad[0].double() - want).abs() <= bound + 1e-30).all())
