@@ -39,16 +39,6 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t saddr) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr));
 }
 
-template <typename T> __device__ __forceinline__ uint32_t pack2w(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t pack2w<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-template <> __device__ __forceinline__ uint32_t pack2w<__half>(float lo, float hi) {
-    __half2 r = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-
 // Shared memory: [staged tile | output staging (aliases the tile)] [B fragments hi] [B fragments lo]
 //   B fragments: [row tap i][variant v (column offset delta = 8v - 8)][lane][2 words]
 template <typename T>
@@ -113,8 +103,8 @@ conv2d_mma_kernel(const __grid_constant__ CUtensorMap mx, const void* __restrict
             hi[e] = round_to<T>(wv);
             lo[e] = wv - hi[e];
         }
-        bfrag[idx] = pack2w<T>(hi[0], hi[1]);
-        if (split_w) bfrag_lo[idx] = pack2w<T>(lo[0], lo[1]);
+        bfrag[idx] = pack2<T>(hi[0], hi[1]);
+        if (split_w) bfrag_lo[idx] = pack2<T>(lo[0], lo[1]);
     }
 
     mbar_wait(&bar, 0, err_flag);
@@ -187,8 +177,8 @@ conv2d_mma_kernel(const __grid_constant__ CUtensorMap mx, const void* __restrict
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
             uint8_t* o0 = xs + (r0 + g) * OPITCH + (cw + nt * 8 + 2 * t4) * 2;
-            *reinterpret_cast<uint32_t*>(o0) = pack2w<T>(acc[nt][0], acc[nt][1]);
-            *reinterpret_cast<uint32_t*>(o0 + 8 * OPITCH) = pack2w<T>(acc[nt][2], acc[nt][3]);
+            *reinterpret_cast<uint32_t*>(o0) = pack2<T>(acc[nt][0], acc[nt][1]);
+            *reinterpret_cast<uint32_t*>(o0 + 8 * OPITCH) = pack2<T>(acc[nt][2], acc[nt][3]);
         }
     }
     __syncthreads();

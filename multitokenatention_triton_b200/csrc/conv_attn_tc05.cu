@@ -276,7 +276,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                     tmem_ld_32x16(tcol + (uint32_t)(h * 48 + 32), *reinterpret_cast<uint32_t(*)[16]>(&r[32]));
                     tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 24; ++i) pk[i] = pack2q<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                    for (int i = 0; i < 24; ++i) pk[i] = pack2<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
                     if (diag) {
                         const int nl = live - h * 48;
 #pragma unroll
@@ -374,7 +374,7 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 for (int e = 0; e < HALF / 2; ++e) {
                     x[2 * e] = ex2_approx(fmaf(x[2 * e], c2, mb));
                     x[2 * e + 1] = ex2_approx(fmaf(x[2 * e + 1], c2, mb));
-                    pk[e] = pack2q<T>(x[2 * e], x[2 * e + 1]);
+                    pk[e] = pack2<T>(x[2 * e], x[2 * e + 1]);
                 }
                 tmem_st_32x16(tacc + (uint32_t)(half * (HALF / 2)), *reinterpret_cast<const uint32_t(*)[16]>(&pk[0]));
                 tmem_st_32x4(tacc + (uint32_t)(half * (HALF / 2) + 16), *reinterpret_cast<const uint32_t(*)[4]>(&pk[16]));
@@ -410,10 +410,10 @@ conv_attn_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
 #pragma unroll
                     for (int v8 = 0; v8 < 4; ++v8) {
                         uint4 v;
-                        v.x = pack2q<T>(__uint_as_float(ro[v8 * 8 + 0]) * inv, __uint_as_float(ro[v8 * 8 + 1]) * inv);
-                        v.y = pack2q<T>(__uint_as_float(ro[v8 * 8 + 2]) * inv, __uint_as_float(ro[v8 * 8 + 3]) * inv);
-                        v.z = pack2q<T>(__uint_as_float(ro[v8 * 8 + 4]) * inv, __uint_as_float(ro[v8 * 8 + 5]) * inv);
-                        v.w = pack2q<T>(__uint_as_float(ro[v8 * 8 + 6]) * inv, __uint_as_float(ro[v8 * 8 + 7]) * inv);
+                        v.x = pack2<T>(__uint_as_float(ro[v8 * 8 + 0]) * inv, __uint_as_float(ro[v8 * 8 + 1]) * inv);
+                        v.y = pack2<T>(__uint_as_float(ro[v8 * 8 + 2]) * inv, __uint_as_float(ro[v8 * 8 + 3]) * inv);
+                        v.z = pack2<T>(__uint_as_float(ro[v8 * 8 + 4]) * inv, __uint_as_float(ro[v8 * 8 + 5]) * inv);
+                        v.w = pack2<T>(__uint_as_float(ro[v8 * 8 + 6]) * inv, __uint_as_float(ro[v8 * 8 + 7]) * inv);
                         *reinterpret_cast<uint4*>(orow + c * 32 + v8 * 8) = v;
                     }
                 }

@@ -47,15 +47,6 @@ template <typename T> struct AbFmtC;
 template <> struct AbFmtC<__nv_bfloat16> { static constexpr int value = 1; };
 template <> struct AbFmtC<__half> { static constexpr int value = 0; };
 
-template <typename T> __device__ __forceinline__ uint32_t cm_pack2(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t cm_pack2<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-template <> __device__ __forceinline__ uint32_t cm_pack2<__half>(float lo, float hi) {
-    __half2 r = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
 template <typename T> __device__ __forceinline__ float2 cm_unpack2(uint32_t w);
 template <> __device__ __forceinline__ float2 cm_unpack2<__nv_bfloat16>(uint32_t w) {
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
@@ -138,7 +129,7 @@ __device__ __forceinline__ void conv_item(const uint8_t* src, uint8_t* tile, int
             uint32_t o[4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                o[m] = cm_pack2<T>(a[m].x, a[m].y);
+                o[m] = pack2<T>(a[m].x, a[m].y);
                 if (DIAG) o[m] = cm_keep(o[m], m, live0 + rp - 2);
             }
             const int l = l0 + rp - (CQ - 1);
@@ -199,7 +190,7 @@ conv_mix_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_consta
                 const int k = 2 * (c0 + c);
                 const float lo = (k & (R - 1)) == r ? to_f32<T>(Wm[o * C + (k >> g.r_log)]) : 0.0f;
                 const float hi = ((k + 1) & (R - 1)) == r ? to_f32<T>(Wm[o * C + ((k + 1) >> g.r_log)]) : 0.0f;
-                pk[c] = cm_pack2<T>(lo, hi);
+                pk[c] = pack2<T>(lo, hi);
             }
             tmem_st_32x32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + CM_A_COL + (uint32_t)c0, pk);
         }
@@ -310,7 +301,7 @@ conv_mix_tc05_kernel(const __grid_constant__ CUtensorMap mx, const __grid_consta
                     uint32_t pk[16];
                     tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) pk[e] = cm_pack2<T>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+                    for (int e = 0; e < 16; ++e) pk[e] = pack2<T>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
                     if (c + 1 < chunks) {
                         tmem_ld_32x32(tacc + (uint32_t)(c * 32 + 32), r);        // on its way while this one is stored
                     } else {

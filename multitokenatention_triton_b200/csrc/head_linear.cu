@@ -144,16 +144,6 @@ template <> __device__ __forceinline__ uint32_t elem_bits<__half>(const uint4& v
     return __float_as_uint(__half2float(h));
 }
 
-template <typename T> __device__ __forceinline__ uint32_t pack2(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-template <> __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
-    __half2 r = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-
 // 32-byte global accesses (sm_100): a lane of the tensor-core kernels owns 16 consecutive keys of a head, and two
 // separate 16-byte stores would each write half of a 32-byte sector.
 __device__ __forceinline__ void st_global_v8(void* p, const uint4& a, const uint4& b) {

@@ -55,15 +55,6 @@ template <typename T> struct AbFmtH;
 template <> struct AbFmtH<__nv_bfloat16> { static constexpr int value = 1; };
 template <> struct AbFmtH<__half> { static constexpr int value = 0; };
 
-template <typename T> __device__ __forceinline__ uint32_t hm_pack2(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t hm_pack2<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-template <> __device__ __forceinline__ uint32_t hm_pack2<__half>(float lo, float hi) {
-    __half2 r = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
 template <typename T> __device__ __forceinline__ void hm_unpack2(uint32_t w, float& lo, float& hi);
 template <> __device__ __forceinline__ void hm_unpack2<__nv_bfloat16>(uint32_t w, float& lo, float& hi) {
     lo = __uint_as_float(w << 16);
@@ -143,7 +134,7 @@ __device__ __forceinline__ void hm_prob32(const uint32_t (&in)[16], uint32_t liv
             float2 f;
             hm_unpack2<T>(in[i], f.x, f.y);
             const float2 yv = __ffma2_rn(f, l2, ns);
-            pk[i] = hm_pack2<T>(hm_ex2(yv.x), hm_ex2(yv.y));
+            pk[i] = pack2<T>(hm_ex2(yv.x), hm_ex2(yv.y));
         }
     } else {
 #pragma unroll
@@ -151,7 +142,7 @@ __device__ __forceinline__ void hm_prob32(const uint32_t (&in)[16], uint32_t liv
             float2 f;
             hm_unpack2<T>(in[i], f.x, f.y);
             const float2 yv = __ffma2_rn(f, l2, ns);
-            pk[i] = hm_pack2<T>(live >> (2 * i) & 1u ? hm_ex2(yv.x) : 0.0f, live >> (2 * i + 1) & 1u ? hm_ex2(yv.y) : 0.0f);
+            pk[i] = pack2<T>(live >> (2 * i) & 1u ? hm_ex2(yv.x) : 0.0f, live >> (2 * i + 1) & 1u ? hm_ex2(yv.y) : 0.0f);
         }
     }
 }
@@ -163,7 +154,7 @@ __device__ __forceinline__ void hm_plain32(const uint32_t (&in)[16], uint32_t li
 #pragma unroll
         for (int i = 0; i < 16; ++i) pk[i] = in[i];
     } else {
-        const uint32_t f2 = hm_pack2<T>(fill, fill);
+        const uint32_t f2 = pack2<T>(fill, fill);
 #pragma unroll
         for (int i = 0; i < 16; ++i)
             pk[i] = (live >> (2 * i) & 1u ? in[i] & 0x0000ffffu : f2 & 0x0000ffffu) | (live >> (2 * i + 1) & 1u ? in[i] & 0xffff0000u : f2 & 0xffff0000u);
@@ -227,7 +218,7 @@ __device__ __forceinline__ void head_mix_tc05_body(const CUtensorMap& mx, const 
     // k = h * R + r (the order of the input box's lines).
     for (int i = tid; i < HM_A_BYTES / 16; i += HM_THREADS) reinterpret_cast<uint4*>(a_base)[i] = make_uint4(0u, 0u, 0u, 0u);
     {
-        const uint32_t f2 = SOFTMAX ? 0u : hm_pack2<T>(g.fill, g.fill);
+        const uint32_t f2 = SOFTMAX ? 0u : pack2<T>(g.fill, g.fill);
         for (int i = tid; i < HM_OUT_BYTES / 16; i += HM_THREADS) reinterpret_cast<uint4*>(fill_base)[i] = make_uint4(f2, f2, f2, f2);
     }
     __syncthreads();

@@ -156,7 +156,7 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
         const int row = quarter * gr + lane - lead;          // staged row of this thread's lane, relative to the tile's first output row
         const int half = warp >= 8 ? 1 : 0;                  // of the staged columns
         const int ft = tid - 128;                            // 0..127 in the warps that build the slices
-        const uint32_t sc = pack2q<T>(g.scale, g.scale);
+        const uint32_t sc = pack2<T>(g.scale, g.scale);
         if (half == 0) clear_taps(wsm, ft, 2);
         it.init(g);
         int cur_head = -1, hn = -1;

@@ -27,16 +27,6 @@ template <typename T> struct AbF;
 template <> struct AbF<__nv_bfloat16> { static constexpr int value = 1; };
 template <> struct AbF<__half> { static constexpr int value = 0; };
 
-template <typename T> __device__ __forceinline__ uint32_t pk2q(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t pk2q<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-template <> __device__ __forceinline__ uint32_t pk2q<__half>(float lo, float hi) {
-    __half2 r = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-
 struct QkGeom {
     int S, causal, row_begin, row_end, tiles_q, tiles_k;
     int mode;          // 0: every tile that touches keys <= query; 1: only the band (last tiles of a row); 2: only below the band
@@ -219,10 +209,10 @@ qk_persistent_kernel(const __grid_constant__ CUtensorMap ma, const __grid_consta
                         if (g.causal && k + x > q) f[x] = 0.0f;   // above the diagonal inside a visited tile: written as 0
                     }
                     uint4 o;
-                    o.x = pk2q<T>(f[0], f[1]);
-                    o.y = pk2q<T>(f[2], f[3]);
-                    o.z = pk2q<T>(f[4], f[5]);
-                    o.w = pk2q<T>(f[6], f[7]);
+                    o.x = pack2<T>(f[0], f[1]);
+                    o.y = pack2<T>(f[2], f[3]);
+                    o.z = pack2<T>(f[4], f[5]);
+                    o.w = pack2<T>(f[6], f[7]);
                     *reinterpret_cast<uint4*>(orow + (((col >> 3) ^ (row & 7)) << 4)) = o;
                 }
             }

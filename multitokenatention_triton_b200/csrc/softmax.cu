@@ -112,16 +112,6 @@ template <> __device__ __forceinline__ void unpack8<__half>(const uint4& v, floa
         f[2 * i] = t.x; f[2 * i + 1] = t.y;
     }
 }
-template <typename T> __device__ __forceinline__ uint32_t pack2s(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t pack2s<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-template <> __device__ __forceinline__ uint32_t pack2s<__half>(float lo, float hi) {
-    __half2 r = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-
 template <typename T, int NCH>
 __global__ void __launch_bounds__(VT)
 softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y, PlaneView yv, int Q, int causal,
@@ -184,10 +174,10 @@ softmax_rows_vec_kernel(const T* __restrict__ x, PlaneView xv, T* __restrict__ y
             if constexpr (sizeof(T) == 4) {
                 o = make_uint4(__float_as_uint(v[c][0] * inv), __float_as_uint(v[c][1] * inv), __float_as_uint(v[c][2] * inv), __float_as_uint(v[c][3] * inv));
             } else {
-                o.x = pack2s<T>(v[c][0] * inv, v[c][1] * inv);
-                o.y = pack2s<T>(v[c][2] * inv, v[c][3] * inv);
-                o.z = pack2s<T>(v[c][4] * inv, v[c][5] * inv);
-                o.w = pack2s<T>(v[c][6] * inv, v[c][7] * inv);
+                o.x = pack2<T>(v[c][0] * inv, v[c][1] * inv);
+                o.y = pack2<T>(v[c][2] * inv, v[c][3] * inv);
+                o.z = pack2<T>(v[c][4] * inv, v[c][5] * inv);
+                o.w = pack2<T>(v[c][6] * inv, v[c][7] * inv);
             }
             if (!write_upper && ch * VEC + VEC > n) {       // last chunk: keys past the diagonal stay untouched
                 T* dst = reinterpret_cast<T*>(yr + ch);

@@ -34,15 +34,6 @@ template <typename T> struct AbFmtQ;
 template <> struct AbFmtQ<__nv_bfloat16> { static constexpr int value = 1; };
 template <> struct AbFmtQ<__half> { static constexpr int value = 0; };
 
-template <typename T> __device__ __forceinline__ uint32_t pack2q(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t pack2q<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-template <> __device__ __forceinline__ uint32_t pack2q<__half>(float lo, float hi) {
-    __half2 r = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&r);
-}
 // Two products in T, each rounded once (the exact product of two 16-bit values fits in fp32, so this is what fp32 and a
 // conversion would give).
 template <typename T> __device__ __forceinline__ uint32_t mul2q(uint32_t a, uint32_t b);
@@ -164,8 +155,8 @@ __device__ __forceinline__ void build_from_taps(uint8_t* tb, float* wsm, const f
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float a = src[2 * e], b = src[2 * e + 1];
-            hi[e] = pack2q<T>(a, b);
-            lo[e] = pack2q<T>(a - round_to<T>(a), b - round_to<T>(b));
+            hi[e] = pack2<T>(a, b);
+            lo[e] = pack2<T>(a - round_to<T>(a), b - round_to<T>(b));
         }
         uint8_t* dst = tb + i * 1024 + half * 512 + (nn >> 3) * 128 + (nn & 7) * 16;
         *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -186,7 +177,7 @@ __device__ __forceinline__ void drain_half(uint32_t tcol, uint32_t sc2, int live
     tmem_ld_wait();
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-        pk[i] = mul2q<T>(pack2q<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), sc2);
+        pk[i] = mul2q<T>(pack2<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), sc2);
     }
     if (diag) {
 #pragma unroll
@@ -306,7 +297,7 @@ __device__ __forceinline__ void stage_row(uint32_t tacc, uint8_t* orow, int live
         tmem_ld_32x8(tacc + (uint32_t)(h * OUT_COLS + 48), *reinterpret_cast<uint32_t(*)[8]>(&r[48]));
         tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < OUT_COLS / 2; ++e) pk[e] = pack2q<T>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+        for (int e = 0; e < OUT_COLS / 2; ++e) pk[e] = pack2<T>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
         if (diag) {
             const int nl = live - h * OUT_COLS;
 #pragma unroll
