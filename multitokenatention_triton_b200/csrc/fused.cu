@@ -7,7 +7,8 @@
 // Both keep two score-plane scratch buffers in the caller's workspace, indexed by absolute query row
 // relative to the first row the request needs, so a query-row range [q_row_begin, q_row_end) costs
 // memory and work proportional to that range (plus the rows the convs reach back to).  Nothing above
-// the diagonal of a scratch plane is ever written or read.
+// the diagonal of a scratch plane is ever read as a score; kernels write zeros there, up to the end of the tiles
+// that the diagonal crosses.
 #include "kernels.cuh"
 
 namespace mta {

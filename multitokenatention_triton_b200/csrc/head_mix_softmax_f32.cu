@@ -5,7 +5,7 @@
 // A CTA owns one query row of all heads.  Its mixed logits live in shared memory: the keys are spread over the threads (a thread takes V
 // neighbouring keys of all heads, as head_linear_simt_kernel does, same sums in the same order), then a warp per head takes the maximum,
 // the exponentials and their sum, and writes the probabilities.  Bound: HBM, the planes are read once and written once; as two
-// kernels they were read and written twice.  It takes rows whose C logits fit into shared memory (16 heads: 3400 keys).
+// kernels they were read and written twice.  It takes rows whose C logits fit into shared memory (16 heads: 3504 keys).
 // Measured, both stages, B1 H16: S1024 45 -> 32 us, S2048 125 -> 108 (one CTA an SM); B2 H8 S256 18 -> 9.  With the row in the warp's
 // registers instead of three passes over shared memory: S1024 42, S256 11, S2048 the same.
 #include <algorithm>
@@ -32,11 +32,8 @@ __device__ __forceinline__ float row_sum(float v) {
     for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
     return v;
 }
-// (a row of nothing but -inf: zeros, as softmax.cu has it)
-__device__ __forceinline__ float4 exp4(float4 v, float mx) {
-    const bool none = mx == -INFINITY;
-    return make_float4(none ? 0.0f : __expf(v.x - mx), none ? 0.0f : __expf(v.y - mx), none ? 0.0f : __expf(v.z - mx), none ? 0.0f : __expf(v.w - mx));
-}
+// (a row of nothing but -inf becomes NaN, as in softmax.cu without a mask)
+__device__ __forceinline__ float4 exp4(float4 v, float mx) { return make_float4(__expf(v.x - mx), __expf(v.y - mx), __expf(v.z - mx), __expf(v.w - mx)); }
 
 template <int CP, int V, int THREADS>
 __global__ void __launch_bounds__(THREADS)

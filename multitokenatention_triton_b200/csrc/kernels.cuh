@@ -114,7 +114,7 @@ bool head_linear_tc05_supported(const void* x, PlaneView xv, const void* y, Plan
 int head_linear_tc05_launch(const void* x, PlaneView xv, const void* Wm, void* y, PlaneView yv, int N, int C, int Q, int causal,
                             float fill, int row_begin, int row_end, bool write_upper, bool wt, int dtype, cudaStream_t st, bool early_weights = false);
 
-// A small causal conv (2 or 3 row taps, 3 or 5 key taps) and the head mix that follows it in one kernel (conv_mix_tc05.cu): the conv's
+// A small causal conv (2 or 3 row taps, 3 key taps) and the head mix that follows it in one kernel (conv_mix_tc05.cu): the conv's
 // output never reaches memory.  16-bit dtypes, weights in the same one, C = 8, 16, 32 or 64, rows [row_begin,row_end).
 bool conv_mix_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int C, int CQ, int CK, int causal, int dtype, int w_dtype);
 int conv_mix_launch(const void* x, PlaneView xv, const void* w, const void* Wm, void* y, PlaneView yv, int N, int C, int Q, int CQ, int CK, int row_begin,
@@ -155,8 +155,8 @@ int qk_f32_launch(const void* q, const void* k, void* s, PlaneView sv, int B, in
 int pv_f32_launch(const void* p, PlaneView pview, const void* v, void* o, int B, int H, int S, int D, int causal, int row_begin, int row_end,
                   bool trans, float scale, cudaStream_t st);
 
-// tcgen05 version of the conv (conv2d_tc05.cu): 16-bit dtypes, S <= 17, any W on rows whose pitch is a multiple of 8 elements, R <= 16
-// and small enough for its shared-memory rings (float32 weights take two sets of slices: R <= 9).
+// tcgen05 version of the conv (conv2d_tc05.cu): 16-bit dtypes, S <= 17, any W on rows whose pitch is a multiple of 8 elements, R <= 16;
+// weights of the same type or float32 (then in two 16-bit parts).
 bool conv2d_tc05_supported(const void* x, PlaneView xv, const void* y, PlaneView yv, int W, int R, int S, int dtype,
                            int w_dtype);
 // `grad_input` (odd S): the same kernel evaluates the gradient with respect to the conv's input - taps reversed, rows
