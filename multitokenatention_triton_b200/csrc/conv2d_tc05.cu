@@ -276,10 +276,19 @@ size_t conv2d_tc05_smem_bytes(int R, bool split_w, bool zeros, int nstage) {
 }
 
 // Of one group's tiles a CTA gets this many or more.  The fewer planes are in work at a time, the more of the rows that neighbouring tiles
-// share come from L2, but a CTA changes its head with every group.  With the zeros above the diagonal to be stored, HBM is the bound: forward and
-// gradients of B4 H16 S2048 take 513 us with 2, 521 with 8.  Without, the head changes show: 158 against 153 us (forward B1 H16 S2048 with two 7x7
-// convs), 674 against 650 (training step B4 H16 S1024).
-constexpr int GROUP_TILES = 8, GROUP_TILES_ZEROS = 2;
+// share come from L2, but a CTA changes its head with every group and then builds R slices.  Where the zeros above the diagonal are stored and the
+// planes do not all fit into L2, HBM is the bound and small groups pay, up to 9 row taps.  Forward, us, with 2 / 8 / 16 tiles:
+//   B4 H16 S2048: 3x3 175 / 181 / 184, 6x11 175 / 178 / 180, 7x9 174 / 183 / 186, 11x15 176 (input gradient 195) / 190 (185) / 189, 16x17 339 / 257 / 248
+//   B4 H16 S1024: 3x3 49 / 50 / 50, 6x11 45 / 48 / 47, 11x15 59 / 51 / 47, 16x17 96 / 78 / 72;  B8 H16 S1024: 6x11 87 / 97 / 97
+//   B1 H8 S2048 (67 MB of output): 3x3 22 / 20 / 20, 6x11 22 / 20 / 21, 16x17 50 / 35 / 34
+// Without the zeros the head changes show at once: 158 against 153 us (forward B1 H16 S2048 with two 7x7 convs), 674 against 650 (training step
+// B4 H16 S1024).
+constexpr int GROUP_TILES = 8, GROUP_TILES_ZEROS = 2, GROUP_ZEROS_TAPS = 9;
+constexpr long GROUP_ZEROS_BYTES = 80 << 20;       // of output: with the lower triangles of the input what L2 holds
+
+int group_tiles(int R, bool zeros, long out_bytes) {
+    return zeros && R <= GROUP_ZEROS_TAPS && out_bytes > GROUP_ZEROS_BYTES ? GROUP_TILES_ZEROS : std::max(GROUP_TILES, R);
+}
 
 template <typename T>
 int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, int w_dtype, void* y, PlaneView yv,
@@ -290,7 +299,7 @@ int launch_tc05(const void* x, PlaneView xv, long x_rows_stored, const void* w, 
     ConvGeom g{};
     set_tiles(g, planes, C, W, R, causal, row_begin, row_end);
     g.write_upper = causal && write_upper ? 1 : 0;
-    set_groups(g, (long)g.tiles_per_plane * planes / ((long)(g.write_upper ? GROUP_TILES_ZEROS : GROUP_TILES) * sms));
+    set_groups(g, (long)g.tiles_per_plane * planes / ((long)group_tiles(R, g.write_upper != 0, planes * (row_end - row_begin) * W * (long)sizeof(T)) * sms));
     g.W = W; g.R = R; g.S = S; g.x_row0 = xv.row0; g.y_row0 = yv.row0;
     g.split_w = w_dtype == MTA_F32 ? 1 : 0;
     g.lead = grad_input ? 0 : R - 1;
