@@ -19,7 +19,8 @@
 //   epilogue  4 warps: rounded, staged, one TMA store per 32 keys x 128 rows
 // Warps: 0 TMA producer, 1 MMAs, 4-11 conv, 12-15 epilogue.  The conv is the longest of the roles (3 x 3: 288 packed
 // FMAs and as many other instructions for 64 results, at 2.5 cycles each), which is why larger convs stay on the tensor cores and apart.
-// Measured: B8 H16 S4096 3x3 0.93 ms, 1.67 as two kernels (HBM alone: 0.66); B4 S1024 44 us, 66.  On the way there: tap pairs with
+// Measured: B8 H16 S4096 3x3 1.09 to 1.18 ms as a stage of the forward (0.93 in a first run alone), 1.67 as two kernels (HBM alone: 0.66); B4 S1024
+// 49 us, 66.  On the way there: tap pairs with
 // zeros in them instead of the second unpacking 1.75 ms, rows in a loop 1.21; sixteen conv warps of four rows instead of eight of
 // eight are level; neighbours' pairs by shuffles instead of 4-byte reads 1.04.
 #include <algorithm>
