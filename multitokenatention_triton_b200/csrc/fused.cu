@@ -109,9 +109,18 @@ int run_forward(const void* q, const void* k, const void* v, const void* w1, con
         if ((rc = trace_mark("softmax", st))) return rc;
         if ((rc = softmax_launch(bufA, pv, bufA, pv, planes, S, S, causal, pl.rb, pl.r1, false, 1.0f, dtype, st, dead, H))) return rc;
     }
-    // The second conv and the second head mix: one kernel where the conv is small.  one / two kernels, us, 3 x 3: H16 B1 S64 14 / 20,
-    // B1 S512 18 / 25, B4 S1024 49 / 66, B1 S4096 139 / 215; H8 B1 S1024 18 / 26; H32 B1 S512 27 / 37, B1 S2048 100 / 113; H64 B1 S256
-    // 26 / 35, B1 S1024 83 / 82, B4 S1024 249 / 240, B1 S4096 800 / 903 (two heads' rows of a group are two thirds of what it reads).
+    // The second conv and the second head mix: one kernel where the conv is small.  one / two kernels, us, 3 x 3, the two stages: H16 B1 S64 14 / 20,
+    // B1 S512 18 / 25, B4 S1024 49 / 66, B1 S4096 139 / 215; H8 B1 S1024 18 / 26; H32 B1 S512 27 / 37, B1 S2048 100 / 113.  The whole forward (first
+    // conv 2 x 3), 3 x 3: H8 B1 S128 27 / 29, B1 S768 47 / 45, B8 S768 96 / 108, B1 S4096 215 / 247; H16 D64 B1 S128 27 / 29, B4 S1024 130 / 140,
+    // B1 S4096 404 / 485 (D128 402 / 495: the head dimension changes neither stage); H32 B1 S1024 84 / 84, B2 S2048 438 / 491.  64 heads, where two
+    // heads' rows of a group are two thirds of what it reads:
+    //         S128      S384        S512        S640        S768        S1024        S1536       S4096
+    //   B1    32 / 39   53 / 55     68 / 67     84 / 79     103 / 95    150 / 143    296 / 306   1818 / 2014
+    //   B2              78 / 77     108 / 103   138 / 133   178 / 175   273 / 281
+    //   B4    51 / 57   133 / 130   184 / 183   248 / 251   322 / 337   531 / 573
+    //   B8    76 / 84   222 / 231   328 / 342   472 / 491   615 / 673   1027 / 1112
+    // The choice depends on the heads, the conv and the types only, so that a row range or a part of a batch gets the same bits as the whole;
+    // over the batches the ratio's mean is 0.99, 1.01, 1.01, 0.99 and 0.97 from 384 to 1024 keys, so no line by length would gain.
     // 2 x 3 gains more everywhere.  3 x 5 was level with two kernels (B4 H16 S2048 212 / 215) and 3 x 7 and more cost FMAs in proportion.
     const void* weights = bufA;
     const bool one = variant("fused") != 1 && variant("conv2d") == 0 && variant("head_linear") == 0 &&
