@@ -14,6 +14,10 @@
 //   warps 1, 2  the MMAs of the even and of the odd tiles, each with an accumulator and two A buffers
 //   warps 12-15 epilogue: accumulator -> 16-bit -> staging tiles -> TMA stores
 //   warp 3      stores zero tiles above the diagonal when the whole output is wanted
+// Against the form with the staged tile as an operand in shared memory (tiles of 128 x 128), the zeros above the diagonal written, us, that form / this:
+//   S1024 B2: 3x3 23 / 22, 6x11 28 / 21, 11x15 38 / 25;  B4 S1024: 3x3 49 / 49, 6x11 47 / 45, 11x15 61 / 47;  B1 S3000: 3x3 110 / 104, 6x11 112 / 101;
+//   B4 S2048: 1x1 163 / 172, 3x3 173 / 178, 6x11 174 / 173, 7x9 168 / 171, 11x15 208 / 166;  B1 S4096: 3x3 172 / 174, 6x11 171 / 173, 7x9 168 / 177
+// (H16).  So it is up to 5 % behind where rows are 4 or 8 KB, a power of two, and taps are few, level or ahead everywhere else: not worth a second kernel.
 // Bound: 120 cycles of MMAs a row tap and tile for large kernels, HBM for small ones.  With the staged tile as an operand in shared
 // memory an MMA took 40 cycles instead of 16.  6 x 11, lower triangles only: B4 H16 S1024 41 -> 31 us; 7 x 7 B1 H16 S2048 fp16 42 -> 30;
 // with the zeros above the diagonal written (B4 H16 S2048, 805 MB) 171 us before and after: HBM, three quarters of it writes.
