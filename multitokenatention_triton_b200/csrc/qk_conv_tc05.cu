@@ -124,7 +124,9 @@ qk_conv_tc05_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
         // Each chain has its Q and K tile, its score buffer and its accumulator, and a warp that issues its MMAs, so while one chain waits
         // for its drain (or its warp for an instruction) the other has the tensor pipe.  One warp for all MMAs left the pipe idle
         // for half of the time, and a warp for the scores and one for the convs hold each other up MMA by MMA.
-        // The scores of tile n + 2 overwrite the A operand of the conv of tile n: MMAs of one thread execute in the order of issue.
+        // The scores of tile n + 2 overwrite the A operand of the conv of tile n: MMAs of one thread execute in the order of issue. (PTX
+        // promises that for MMAs of one shape on one accumulator.  Across shapes and accumulators, as here and between the row taps, whose shift each MMA
+        // leaves in A for the next, it is what the hardware was seen to do: results are the same bits in every run.)
         constexpr uint32_t idesc = instr_desc_f16(AbFmtQ<T>::value, 0, 0, TM, SN);
         const uint32_t el = elect_one();
         const int b = warp - 1;
